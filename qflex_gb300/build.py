@@ -36,7 +36,7 @@ def _sources():
 
 def _compile(src: Path, nvcc: str) -> Path:
     obj = BUILD / (src.name + ".o")
-    deps = [src] + list(CSRC.glob("*.h")) + [PKG.parent / "include" / "qflex_gb300.h"]
+    deps = [src] + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "qflex_gb300.h"]
     if obj.exists() and obj.stat().st_mtime >= max(d.stat().st_mtime for d in deps if d.exists()):
         return obj
     flags = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I", str(CSRC), "-I", str(PKG.parent / "include")]

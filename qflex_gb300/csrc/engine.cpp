@@ -191,11 +191,27 @@ void Engine::set_tc_variant(std::size_t m, std::size_t n, std::size_t k, int var
   ++options_version_;
 }
 
+// Whether the 3xFP16 product of n columns splits A inside the kernel. Every
+// 128 columns of the product read and split A again, beside the MMAs: with
+// shared memory's bandwidth the shared limit that costs 8 to 17 % of the
+// product, while splitting A beforehand costs a pass over it that does not
+// depend on n. Measured, split + product against direct:
+// (65536, 256, 256) x 4 211 + 309 against 340 us, (4096, 4096, 4096)
+// 50 + 947 against 1109 us; the lines cross between n = 1024 and 1700.
+bool Engine::direct_product(std::size_t n, const TcConfig& cfg) const {
+  return precision_ == FP16X3 && cfg.variant == 0 && cfg.chunk <= 2 && n <= 1024;
+}
+
 void Engine::launch_split_product(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
                                   std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch,
                                   float* ws) {
   const TcConfig cfg = tc_config(m, n, k);
-  if (precision_ == FP16X3)
+  if (direct_product(n, cfg)) {
+    const bool aligned = (reinterpret_cast<std::uintptr_t>(A) & 15) == 0 && k % 2 == 0 &&
+                         (batch == 1 || ac_stride % 2 == 0);
+    launch_cgemm_fp16x3_direct(A, make_a_rows(k, aligned), Bt, C, m, n, k, ac_stride, bt_stride, batch, ws,
+                               error_flag(), cfg, stream_);
+  } else if (precision_ == FP16X3)
     launch_cgemm_fp16x3(A, Bt, C, m, n, k, ac_stride, bt_stride, batch, ws, error_flag(), cfg, stream_);
   else if (precision_ == BF16X3)
     launch_cgemm_bf16x3(A, Bt, C, m, n, k, ac_stride, bt_stride, batch, ws, error_flag(), cfg, stream_);

@@ -130,6 +130,7 @@ class Engine {
   bool debias_ = true;    // tensor-core products compensate the truncation bias
   unsigned options_version_ = 0;  // part of the graph key: options change launches
   TcConfig tc_config(std::size_t m, std::size_t n, std::size_t k) const;
+  bool direct_product(std::size_t n, const TcConfig& cfg) const;
   // C = A * Bt^T on the tensor cores in the context's split precision.
   void launch_split_product(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
                             std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch, float* ws);

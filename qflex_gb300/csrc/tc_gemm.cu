@@ -48,6 +48,7 @@
 #include <string>
 
 #include "kernels.h"
+#include "tc_common.cuh"
 #include "tc_gemm.h"
 
 namespace qfx {
@@ -83,137 +84,7 @@ constexpr int DEEP_SMEM_BYTES = DEEP_STAGES * F16_STAGE_BYTES + DEEP_STAGING_BYT
 // warp in the same staging area. Needs the bulk-store output map.
 constexpr int WIDE_EPI_WARPS = 16;
 constexpr int WIDE_THREADS = 64 + 32 * WIDE_EPI_WARPS;
-constexpr unsigned long long WAIT_NS = 2000000000ull;  // 2 s per wait
 
-__device__ __forceinline__ std::uint32_t smem_u32(const void* p) {
-  return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(std::uint64_t* bar, std::uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(std::uint64_t* bar, std::uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_test(std::uint64_t* bar, std::uint32_t parity) {
-  std::uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Limit of a pipeline wait: the 64-bit value the host keeps after the error
-// code in the error-flag buffer (err[2..3], written when the buffer is
-// created and by the "tc_wait_ns" option), or WAIT_NS when it is 0. Read
-// only once a wait has to spin. The drains on the abort path keep WAIT_NS.
-__device__ __forceinline__ unsigned long long wait_limit_ns(const int* err) {
-  const unsigned long long v = *reinterpret_cast<const volatile unsigned long long*>(err + 2);
-  return v ? v : WAIT_NS;
-}
-// Bounded wait: false (and an error code) when the phase does not complete
-// within the wait limit or another warp of the CTA has already given up.
-__device__ __forceinline__ bool mbar_wait(std::uint64_t* bar, std::uint32_t parity, volatile int* abort_flag,
-                                          int* err, int code) {
-  if (mbar_test(bar, parity)) return true;  // the common case reads no timer
-  const unsigned long long t0 = now_ns(), limit = wait_limit_ns(err);
-  while (!mbar_test(bar, parity)) {
-    if (*abort_flag) return false;
-    if (now_ns() - t0 > limit) {
-      *abort_flag = 1;
-      atomicExch(err, code);
-      return false;
-    }
-  }
-  return true;
-}
-
-__device__ __forceinline__ void tma_load_4d(const CUtensorMap* map, std::uint64_t* bar, void* dst, int c0,
-                                            int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-      "%5}], [%6];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<std::uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// Bulk tensor store of a shared-memory box to global memory (C tiles), its
-// commit group, and the waits for the box's shared-memory reads / for the
-// global writes to finish.
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
-                   reinterpret_cast<std::uint64_t>(map)),
-               "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(src))
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// v * 2^e, exact unless the result leaves the normal range (then rounded
-// like ldexpf): a multiply by the power of two when 2^e is a normal float.
-__device__ __forceinline__ float scale2(float v, int e) {
-  return (e >= -126 && e <= 127) ? v * __uint_as_float(std::uint32_t(e + 127) << 23) : ldexpf(v, e);
-}
-
-// Shared-memory matrix descriptor: K-major operand inside rows of 128 bytes
-// in the 128-byte swizzle (the start address may sit 32, 64 or 96 bytes into
-// the row, as for a K offset), 8-row groups 1024 bytes apart.
-__device__ __forceinline__ std::uint64_t smem_desc_sw128(std::uint32_t addr) {
-  std::uint64_t d = 0;
-  d |= std::uint64_t((addr & 0x3FFFF) >> 4);       // start address
-  d |= std::uint64_t(1) << 16;                     // leading byte offset (unused here)
-  d |= std::uint64_t(1024 >> 4) << 32;             // stride byte offset
-  d |= std::uint64_t(1) << 46;                     // descriptor version
-  d |= std::uint64_t(2) << 61;                     // 128-byte swizzle
-  return d;
-}
-
-// The same for rows of 64 bytes in the 64-byte swizzle (8-row groups 512
-// bytes apart); the BF16x3 kernel keeps its third pieces there.
-__device__ __forceinline__ std::uint64_t smem_desc_sw64(std::uint32_t addr) {
-  std::uint64_t d = 0;
-  d |= std::uint64_t((addr & 0x3FFFF) >> 4);
-  d |= std::uint64_t(1) << 16;
-  d |= std::uint64_t(512 >> 4) << 32;
-  d |= std::uint64_t(1) << 46;
-  d |= std::uint64_t(4) << 61;                     // 64-byte swizzle
-  return d;
-}
-
-// Instruction descriptor, kind::tf32: D = F32, A = B = TF32, both K-major.
-__host__ __device__ constexpr std::uint32_t idesc_tf32(int m, int n, bool negate_a) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | (negate_a ? (1u << 13) : 0u) |
-         (std::uint32_t(n >> 3) << 17) | (std::uint32_t(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_tf32(std::uint32_t d_tmem, std::uint64_t a, std::uint64_t b,
-                                          std::uint32_t idesc, std::uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-// Instruction descriptor, kind::f16 with FP16 A and B (format 0), F32 D.
-__host__ __device__ constexpr std::uint32_t idesc_f16(int m, int n, bool negate_a) {
-  return (1u << 4) | (negate_a ? (1u << 13) : 0u) | (std::uint32_t(n >> 3) << 17) | (std::uint32_t(m >> 4) << 24);
-}
-__device__ __forceinline__ void umma_f16(std::uint32_t d_tmem, std::uint64_t a, std::uint64_t b, std::uint32_t idesc,
-                                         std::uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
 // One k-step of the 3xFP16 product (six M = 128, N = 256 MMAs, small terms
 // first) in one instruction block. The stage is A's 16 KB block of 128-byte
 // rows (re hi, lo, im hi, lo; 128-byte swizzle, high descriptor word `hia`)
@@ -243,29 +114,6 @@ __device__ __forceinline__ void umma_f16_kstep(std::uint32_t d, std::uint32_t lo
       "r"(lo), "r"(hia), "r"(hib), "r"(idesc), "r"(acc), "r"(bstep));
 }
 
-// Operand kinds of the single-CTA kernel: 3xTF32 planes (8 values of 4
-// bytes per plane and k-step) or 3xFP16 planes (16 values of 2 bytes, rows
-// scaled by powers of two).
-// BF16x3: three BF16 pieces per value (x = b0 + b1 + b2 to ~24 bits).
-enum SplitKind : int { KIND_TF32 = 0, KIND_FP16 = 1, KIND_BF16 = 2 };
-
-// Compensation of the truncation bias. The tensor core's FP32 accumulation
-// rounds toward zero, so every product comes out smaller by a fraction beta
-// of itself that depends on the split kind and on how many k-steps a TMEM
-// chunk accumulates (not on the shape). Measured on GB300 against complex128
-// products of Gaussian operands (python -m qflex_gb300.kernel_bench bias), for
-// chunks of one and two k-steps; other chunk lengths are not compensated.
-// With err[1] != 0 (option "tc_debias") every output x becomes x + beta x,
-// one fused multiply-add rounded to nearest (1 + beta itself is not a float:
-// beta is below the float spacing at 1).
-template <int KIND>
-__device__ __forceinline__ float debias_beta(const int* err, int chunk, int kblocks) {
-  if (*reinterpret_cast<const volatile int*>(err + 1) == 0) return 0.f;
-  const int c = chunk < kblocks ? chunk : kblocks;
-  if (c == 1) return KIND == KIND_FP16 ? 5.53e-8f : KIND == KIND_BF16 ? 4.47e-8f : 5.39e-8f;
-  if (c == 2) return KIND == KIND_FP16 ? 1.535e-7f : KIND == KIND_BF16 ? 2.226e-7f : 1.52e-7f;
-  return 0.f;
-}
 template <int KIND>
 __device__ __forceinline__ void umma(std::uint32_t d, std::uint64_t a, std::uint64_t b, std::uint32_t id,
                                      std::uint32_t acc) {
@@ -284,12 +132,6 @@ __host__ __device__ constexpr std::uint32_t idesc_kind(int m, int n, bool negate
                            : (KIND == KIND_FP16 ? idesc_f16(m, n, negate_a) : idesc_bf16(m, n, negate_a));
 }
 
-__device__ __forceinline__ void umma_commit(std::uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
 #define TMEM_LD32(taddr, r)                                                                            \
   asm volatile(                                                                                        \
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15," \
@@ -300,18 +142,6 @@ __device__ __forceinline__ void umma_commit(std::uint64_t* bar) {
         "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),    \
         "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])                                            \
       : "r"(taddr))
-
-#define TMEM_LD16(taddr, r)                                                                            \
-  asm volatile(                                                                                        \
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),          \
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),       \
-        "=r"(r[14]), "=r"(r[15])                                                                      \
-      : "r"(taddr))
-
-__device__ __forceinline__ void mbar_arrive(std::uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // ---- Cluster (CTA pair) helpers ------------------------------------------------
 
@@ -468,7 +298,8 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
   std::uint32_t* tmem_slot = reinterpret_cast<std::uint32_t*>(mma_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  // Uniform for the compiler: see the MMA issuer.
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32;
   // Work items (tiles) of this CTA (of this pair): first, first + stride, ...
   const std::uint32_t rank = PAIR ? cluster_rank() : 0;
   const int first = PAIR ? blockIdx.x / 2 : blockIdx.x;
@@ -585,8 +416,13 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
         }
       }
     }
-  } else if (warp == 1 && lane == 0 && rank == 0) {
-    // MMA issuer (of the pair: CTA 0). Planes in a stage: A re_hi, re_lo,
+  } else if (warp == 1 && rank == 0) {
+    // MMA issuer (of the pair: CTA 0). The whole warp runs the loop in step
+    // and one elected lane issues, so that descriptors and loop state live in
+    // uniform registers. Run by one lane alone, every descriptor word moved
+    // there before each MMA: beside the epilogue and shared-memory traffic a
+    // 3xFP16 k-step then took 860 cycles, 768 this way (the tensor pipe's
+    // rate; measured on the k-step, its commits and barrier tests alone). Planes in a stage: A re_hi, re_lo,
     // im_hi, im_lo, then B.
     // Chunk c (CHUNK k-steps of one tile; c counts across tiles) accumulates
     // from zero into TMEM buffer c % 2; the epilogue warps add it into their
@@ -600,6 +436,10 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
     std::uint32_t f16_lo = std::uint32_t(f16d0);
     // Stage s with phase bit ph, k-step kc of chunk c: counters, not
     // divisions, since this thread's instruction stream paces the MMAs.
+    const bool leader = elect_one();
+    auto wait_all = [&](std::uint64_t* bar, std::uint32_t parity, int code) {
+      return __all_sync(0xffffffffu, wait(bar, parity, code));
+    };
     int s = 0, c = 0, kc = 0;
     std::uint32_t ph = 0;
     bool go = true;
@@ -611,7 +451,7 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
         if (first && c >= NBUF) {
           // The epilogue's TMEM reads of this buffer precede the MMAs that
           // overwrite it.
-          if (!wait(&acc_empty[buf], ((c / NBUF) - 1) & 1, 4)) {
+          if (!wait_all(&acc_empty[buf], ((c / NBUF) - 1) & 1, 4)) {
             go = false;
             break;
           }
@@ -619,100 +459,104 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
         }
         // Operand stages need no fence: the TMA's complete_tx on the barrier
         // orders its shared-memory writes before the MMAs' reads.
-        if (!wait(&full[s], ph, 2)) {
+        if (!wait_all(&full[s], ph, 2)) {
           go = false;
           break;
         }
         const std::uint32_t d_re = tmem + buf * 2 * TBN, d_im = d_re + TBN;
         const std::uint32_t a0 = smem_u32(smem + s * SBYTES);
         const std::uint32_t acc = first ? 0u : 1u;
-        if constexpr (PAIR) {
-          // M = 256 over the pair; B rows (Br; Bi) at the stage's B offset
-          // and (-Bi; Br) 8 KB further, each half in its own CTA.
-          const std::uint32_t idw = idesc_f16(2 * BM, 2 * BN, false);
-          const std::uint32_t ar = a0, ai = a0 + F16_BLOCK, b1 = a0 + 2 * F16_BLOCK, b2 = a0 + 3 * F16_BLOCK;
-          const std::uint64_t arh = smem_desc_sw64(ar), arl = smem_desc_sw64(ar + 32);
-          const std::uint64_t aih = smem_desc_sw64(ai), ail = smem_desc_sw64(ai + 32);
-          const std::uint64_t b1h = smem_desc_sw64(b1), b1l = smem_desc_sw64(b1 + 32);
-          const std::uint64_t b2h = smem_desc_sw64(b2), b2l = smem_desc_sw64(b2 + 32);
-          umma_f16_pair(d_re, arh, b1l, idw, acc);
-          umma_f16_pair(d_re, arl, b1h, idw, 1);
-          umma_f16_pair(d_re, aih, b2l, idw, 1);
-          umma_f16_pair(d_re, ail, b2h, idw, 1);
-          umma_f16_pair(d_re, arh, b1h, idw, 1);
-          umma_f16_pair(d_re, aih, b2h, idw, 1);
-          (void)d_im;
-        } else if constexpr (KIND == KIND_FP16) {
-          // One M = 128, N = 256 product gives C_re (columns 0..127) and
-          // C_im (128..255) together: Ar against the B rows (Br; Bi) and Ai
-          // against (-Bi; Br), both read from the stage's B blocks
-          // (-Bi, Br, Bi). Six MMAs per k-step, small terms first.
-          // Stage s's descriptors: stage 0's with the start address moved
-          // by s * SBYTES (the 14-bit field cannot carry: shared memory is
-          // below 256 KB).
-          umma_f16_kstep(d_re, f16_lo, f16_hia, f16_hib, idesc_f16(BM, 2 * TBN, false), acc, F16_BBLOCK / 16);
-          (void)d_im;
-        } else {
-          const std::uint32_t b0 = a0 + TILE_A;
-          const std::uint64_t arh = smem_desc_sw128(a0), arl = smem_desc_sw128(a0 + 32),
-                              aih = smem_desc_sw128(a0 + 64), ail = smem_desc_sw128(a0 + 96);
-          const std::uint64_t brh = smem_desc_sw128(b0), brl = smem_desc_sw128(b0 + 32),
-                              bih = smem_desc_sw128(b0 + 64), bil = smem_desc_sw128(b0 + 96);
-          if constexpr (KIND == KIND_BF16) {
-            // Pieces 0 and 1 sit in the 128-byte rows (re0 re1 im0 im1, named
-            // *h and *l above), piece 2 in the 64-byte rows (re2 im2). Per real
-            // product x*y the terms x2y0, x1y1, x0y2 (~2^-16), x1y0, x0y1
-            // (~2^-8) and x0y0, smallest first.
-            const std::uint32_t at = a0 + 2 * TILE_A, bt = at + TAIL;
-            const std::uint64_t ar2 = smem_desc_sw64(at), ai2 = smem_desc_sw64(at + 32);
-            const std::uint64_t br2 = smem_desc_sw64(bt), bi2 = smem_desc_sw64(bt + 32);
-            // C_re = Ar Br - Ai Bi
-            umma<KIND>(d_re, ar2, brh, idp, acc);
-            umma<KIND>(d_re, arl, brl, idp, 1);
-            umma<KIND>(d_re, arh, br2, idp, 1);
-            umma<KIND>(d_re, ai2, bih, idn, 1);
-            umma<KIND>(d_re, ail, bil, idn, 1);
-            umma<KIND>(d_re, aih, bi2, idn, 1);
-            umma<KIND>(d_re, arl, brh, idp, 1);
-            umma<KIND>(d_re, arh, brl, idp, 1);
-            umma<KIND>(d_re, ail, bih, idn, 1);
-            umma<KIND>(d_re, aih, bil, idn, 1);
-            umma<KIND>(d_re, arh, brh, idp, 1);
-            umma<KIND>(d_re, aih, bih, idn, 1);
-            // C_im = Ar Bi + Ai Br
-            umma<KIND>(d_im, ar2, bih, idp, acc);
-            umma<KIND>(d_im, arl, bil, idp, 1);
-            umma<KIND>(d_im, arh, bi2, idp, 1);
-            umma<KIND>(d_im, ai2, brh, idp, 1);
-            umma<KIND>(d_im, ail, brl, idp, 1);
-            umma<KIND>(d_im, aih, br2, idp, 1);
-            umma<KIND>(d_im, arl, bih, idp, 1);
-            umma<KIND>(d_im, arh, bil, idp, 1);
-            umma<KIND>(d_im, ail, brh, idp, 1);
-            umma<KIND>(d_im, aih, brl, idp, 1);
-            umma<KIND>(d_im, arh, bih, idp, 1);
-            umma<KIND>(d_im, aih, brh, idp, 1);
+        const bool chunk_end = ++kc == CHUNK || kb == kblocks - 1;
+        if (leader) {
+          if constexpr (PAIR) {
+            // M = 256 over the pair; B rows (Br; Bi) at the stage's B offset
+            // and (-Bi; Br) 8 KB further, each half in its own CTA.
+            const std::uint32_t idw = idesc_f16(2 * BM, 2 * BN, false);
+            const std::uint32_t ar = a0, ai = a0 + F16_BLOCK, b1 = a0 + 2 * F16_BLOCK, b2 = a0 + 3 * F16_BLOCK;
+            const std::uint64_t arh = smem_desc_sw64(ar), arl = smem_desc_sw64(ar + 32);
+            const std::uint64_t aih = smem_desc_sw64(ai), ail = smem_desc_sw64(ai + 32);
+            const std::uint64_t b1h = smem_desc_sw64(b1), b1l = smem_desc_sw64(b1 + 32);
+            const std::uint64_t b2h = smem_desc_sw64(b2), b2l = smem_desc_sw64(b2 + 32);
+            umma_f16_pair(d_re, arh, b1l, idw, acc);
+            umma_f16_pair(d_re, arl, b1h, idw, 1);
+            umma_f16_pair(d_re, aih, b2l, idw, 1);
+            umma_f16_pair(d_re, ail, b2h, idw, 1);
+            umma_f16_pair(d_re, arh, b1h, idw, 1);
+            umma_f16_pair(d_re, aih, b2h, idw, 1);
+            (void)d_im;
+          } else if constexpr (KIND == KIND_FP16) {
+            // One M = 128, N = 256 product gives C_re (columns 0..127) and
+            // C_im (128..255) together: Ar against the B rows (Br; Bi) and Ai
+            // against (-Bi; Br), both read from the stage's B blocks
+            // (-Bi, Br, Bi). Six MMAs per k-step, small terms first.
+            // Stage s's descriptors: stage 0's with the start address moved
+            // by s * SBYTES (the 14-bit field cannot carry: shared memory is
+            // below 256 KB).
+            umma_f16_kstep(d_re, f16_lo, f16_hia, f16_hib, idesc_f16(BM, 2 * TBN, false), acc, F16_BBLOCK / 16);
+            (void)d_im;
           } else {
-            // The small hi*lo terms go first and the two large hi*hi terms
-            // last, so only those two additions round against a large
-            // accumulator.
-            umma<KIND>(d_re, arh, brl, idp, acc);
-            umma<KIND>(d_re, arl, brh, idp, 1);
-            umma<KIND>(d_re, aih, bil, idn, 1);
-            umma<KIND>(d_re, ail, bih, idn, 1);
-            umma<KIND>(d_re, arh, brh, idp, 1);
-            umma<KIND>(d_re, aih, bih, idn, 1);
-            umma<KIND>(d_im, arh, bil, idp, acc);
-            umma<KIND>(d_im, arl, bih, idp, 1);
-            umma<KIND>(d_im, aih, brl, idp, 1);
-            umma<KIND>(d_im, ail, brh, idp, 1);
-            umma<KIND>(d_im, arh, bih, idp, 1);
-            umma<KIND>(d_im, aih, brh, idp, 1);
+            const std::uint32_t b0 = a0 + TILE_A;
+            const std::uint64_t arh = smem_desc_sw128(a0), arl = smem_desc_sw128(a0 + 32),
+                                aih = smem_desc_sw128(a0 + 64), ail = smem_desc_sw128(a0 + 96);
+            const std::uint64_t brh = smem_desc_sw128(b0), brl = smem_desc_sw128(b0 + 32),
+                                bih = smem_desc_sw128(b0 + 64), bil = smem_desc_sw128(b0 + 96);
+            if constexpr (KIND == KIND_BF16) {
+              // Pieces 0 and 1 sit in the 128-byte rows (re0 re1 im0 im1, named
+              // *h and *l above), piece 2 in the 64-byte rows (re2 im2). Per real
+              // product x*y the terms x2y0, x1y1, x0y2 (~2^-16), x1y0, x0y1
+              // (~2^-8) and x0y0, smallest first.
+              const std::uint32_t at = a0 + 2 * TILE_A, bt = at + TAIL;
+              const std::uint64_t ar2 = smem_desc_sw64(at), ai2 = smem_desc_sw64(at + 32);
+              const std::uint64_t br2 = smem_desc_sw64(bt), bi2 = smem_desc_sw64(bt + 32);
+              // C_re = Ar Br - Ai Bi
+              umma<KIND>(d_re, ar2, brh, idp, acc);
+              umma<KIND>(d_re, arl, brl, idp, 1);
+              umma<KIND>(d_re, arh, br2, idp, 1);
+              umma<KIND>(d_re, ai2, bih, idn, 1);
+              umma<KIND>(d_re, ail, bil, idn, 1);
+              umma<KIND>(d_re, aih, bi2, idn, 1);
+              umma<KIND>(d_re, arl, brh, idp, 1);
+              umma<KIND>(d_re, arh, brl, idp, 1);
+              umma<KIND>(d_re, ail, bih, idn, 1);
+              umma<KIND>(d_re, aih, bil, idn, 1);
+              umma<KIND>(d_re, arh, brh, idp, 1);
+              umma<KIND>(d_re, aih, bih, idn, 1);
+              // C_im = Ar Bi + Ai Br
+              umma<KIND>(d_im, ar2, bih, idp, acc);
+              umma<KIND>(d_im, arl, bil, idp, 1);
+              umma<KIND>(d_im, arh, bi2, idp, 1);
+              umma<KIND>(d_im, ai2, brh, idp, 1);
+              umma<KIND>(d_im, ail, brl, idp, 1);
+              umma<KIND>(d_im, aih, br2, idp, 1);
+              umma<KIND>(d_im, arl, bih, idp, 1);
+              umma<KIND>(d_im, arh, bil, idp, 1);
+              umma<KIND>(d_im, ail, brh, idp, 1);
+              umma<KIND>(d_im, aih, brl, idp, 1);
+              umma<KIND>(d_im, arh, bih, idp, 1);
+              umma<KIND>(d_im, aih, brh, idp, 1);
+            } else {
+              // The small hi*lo terms go first and the two large hi*hi terms
+              // last, so only those two additions round against a large
+              // accumulator.
+              umma<KIND>(d_re, arh, brl, idp, acc);
+              umma<KIND>(d_re, arl, brh, idp, 1);
+              umma<KIND>(d_re, aih, bil, idn, 1);
+              umma<KIND>(d_re, ail, bih, idn, 1);
+              umma<KIND>(d_re, arh, brh, idp, 1);
+              umma<KIND>(d_re, aih, bih, idn, 1);
+              umma<KIND>(d_im, arh, bil, idp, acc);
+              umma<KIND>(d_im, arl, bih, idp, 1);
+              umma<KIND>(d_im, aih, brl, idp, 1);
+              umma<KIND>(d_im, ail, brh, idp, 1);
+              umma<KIND>(d_im, arh, bih, idp, 1);
+              umma<KIND>(d_im, aih, brh, idp, 1);
+            }
           }
+          commit(&empty[s]);
+          if (chunk_end) commit(&acc_full[buf]);
         }
-        commit(&empty[s]);
-        if (++kc == CHUNK || kb == kblocks - 1) {
-          commit(&acc_full[buf]);
+        __syncwarp();
+        if (chunk_end) {
           ++c;
           kc = 0;
         }
@@ -724,7 +568,8 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
         }
       }
     }
-    commit(mma_done);
+    if (leader) commit(mma_done);
+    __syncwarp();
   } else if (warp >= 2) {
     // Epilogue: warp w reads TMEM lanes [32 (w % 4), 32 (w % 4) + 32) and one
     // half of the tile's columns. The tensor core's FP32 accumulation rounds
@@ -1046,7 +891,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   std::uint32_t* tmem_slot = reinterpret_cast<std::uint32_t*>(mma_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32;
   const std::uint32_t rank = cluster_rank();
   const int pair = blockIdx.x / 2;
   const int tiles_m = (m + 2 * PBM - 1) / (2 * PBM);
@@ -1105,18 +950,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
       }
     }
-  } else if (warp == 1 && lane == 0 && rank == 0) {
-    // MMA issuer of the pair (even CTA).
+  } else if (warp == 1 && rank == 0) {
+    // MMA issuer of the pair (even CTA): the warp in step, one lane issues.
+    const bool leader = elect_one();
+    auto wait_all = [&](std::uint64_t* bar, std::uint32_t parity, int code) {
+      return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag, err, code));
+    };
     const std::uint32_t idp = idesc_tf32(2 * PBM, PBN, false), idn = idesc_tf32(2 * PBM, PBN, true);
     for (int kb = 0; kb < kblocks; ++kb) {
       const int s = kb % P_STAGES;
       const int c = kb / CHUNK, buf = c & 1;
       const bool first = kb % CHUNK == 0;
       if (first && c >= 2) {
-        if (!mbar_wait_cluster(&acc_empty[buf], ((c >> 1) - 1) & 1, abort_flag, err, 14)) break;
+        if (!wait_all(&acc_empty[buf], ((c >> 1) - 1) & 1, 14)) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
       }
-      if (!mbar_wait_cluster(&full[s], (kb / P_STAGES) & 1, abort_flag, err, 12)) break;
+      if (!wait_all(&full[s], (kb / P_STAGES) & 1, 12)) break;
       const std::uint32_t d_re = tmem + buf * 2 * PBN, d_im = d_re + PBN;
       const std::uint32_t a0 = smem_u32(smem + s * P_STAGE_BYTES);
       const std::uint32_t b0 = a0 + P_TILE_A;
@@ -1125,22 +974,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
       const std::uint64_t brh = smem_desc_sw128(b0), brl = smem_desc_sw128(b0 + 32),
                           bih = smem_desc_sw128(b0 + 64), bil = smem_desc_sw128(b0 + 96);
       const std::uint32_t acc = first ? 0u : 1u;
-      umma_tf32_pair(d_re, arh, brl, idp, acc);
-      umma_tf32_pair(d_re, arl, brh, idp, 1);
-      umma_tf32_pair(d_re, aih, bil, idn, 1);
-      umma_tf32_pair(d_re, ail, bih, idn, 1);
-      umma_tf32_pair(d_re, arh, brh, idp, 1);
-      umma_tf32_pair(d_re, aih, bih, idn, 1);
-      umma_tf32_pair(d_im, arh, bil, idp, acc);
-      umma_tf32_pair(d_im, arl, bih, idp, 1);
-      umma_tf32_pair(d_im, aih, brl, idp, 1);
-      umma_tf32_pair(d_im, ail, brh, idp, 1);
-      umma_tf32_pair(d_im, arh, bih, idp, 1);
-      umma_tf32_pair(d_im, aih, brh, idp, 1);
-      umma_commit_pair(&empty[s]);
-      if (kb % CHUNK == CHUNK - 1 || kb == kblocks - 1) umma_commit_pair(&acc_full[buf]);
+      if (leader) {
+        umma_tf32_pair(d_re, arh, brl, idp, acc);
+        umma_tf32_pair(d_re, arl, brh, idp, 1);
+        umma_tf32_pair(d_re, aih, bil, idn, 1);
+        umma_tf32_pair(d_re, ail, bih, idn, 1);
+        umma_tf32_pair(d_re, arh, brh, idp, 1);
+        umma_tf32_pair(d_re, aih, bih, idn, 1);
+        umma_tf32_pair(d_im, arh, bil, idp, acc);
+        umma_tf32_pair(d_im, arl, bih, idp, 1);
+        umma_tf32_pair(d_im, aih, brl, idp, 1);
+        umma_tf32_pair(d_im, ail, brh, idp, 1);
+        umma_tf32_pair(d_im, arh, bih, idp, 1);
+        umma_tf32_pair(d_im, aih, brh, idp, 1);
+        umma_commit_pair(&empty[s]);
+        if (kb % CHUNK == CHUNK - 1 || kb == kblocks - 1) umma_commit_pair(&acc_full[buf]);
+      }
+      __syncwarp();
     }
-    umma_commit_pair(mma_done);
+    if (leader) umma_commit_pair(mma_done);
+    __syncwarp();
   } else if (warp >= 2) {
     // Epilogue (both CTAs): this CTA's 128 rows from its own TMEM.
     const int q = warp % 4;
@@ -1394,30 +1247,6 @@ CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad,
   return map;
 }
 
-// 4-D map over FP16 planes laid out [batch][kpad / 16][rows][row_halves]
-// (64: re hi, lo, im hi, lo; 96: also -im hi, lo). Box {32, box_rows, 1, 1}:
-// the hi and lo planes of one part as 64-byte rows, 64-byte swizzle, the
-// part chosen by the box's x coordinate (0, 32, 64); or with box_inner = 64
-// whole 128-byte rows (all four planes of A) in the 128-byte swizzle.
-CUtensorMap plane_map_f16(const __half* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
-                          int row_halves, int box_inner = 32) {
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  const std::uint64_t kb = kpad / 16, rb = std::uint64_t(row_halves) * 2;
-  const cuuint64_t dims[4] = {(cuuint64_t)row_halves, rows, kb, (cuuint64_t)batch};
-  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
-  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half*>(base), dims, strides, box,
-                           estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
-        std::to_string((int)r);
-  return map;
-}
-
 // 4-D map over BF16 planes laid out [batch][kpad / 16][rows][inner] with
 // `inner` 64 (128-byte rows, 128-byte swizzle) or 32 (64-byte rows, 64-byte
 // swizzle); box {inner, box_rows, 1, 1}.
@@ -1440,13 +1269,43 @@ CUtensorMap plane_map_bf16(const __nv_bfloat16* base, std::uint64_t rows, std::u
   return map;
 }
 
+void check(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: CUDA ") + what + ") --> " + cudaGetErrorString(e);
+}
+
+}  // namespace
+
+// 4-D map over FP16 planes laid out [batch][kpad / 16][rows][row_halves]
+// (64: re hi, lo, im hi, lo; 96: also -im hi, lo). Box {32, box_rows, 1, 1}:
+// the hi and lo planes of one part as 64-byte rows, 64-byte swizzle, the
+// part chosen by the box's x coordinate (0, 32, 64); or with box_inner = 64
+// whole 128-byte rows (all four planes of A) in the 128-byte swizzle.
+CUtensorMap plane_map_f16(const __half* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
+                          int row_halves, int box_inner) {
+  CUtensorMap map;
+  std::memset(&map, 0, sizeof(map));
+  const std::uint64_t kb = kpad / 16, rb = std::uint64_t(row_halves) * 2;
+  const cuuint64_t dims[4] = {(cuuint64_t)row_halves, rows, kb, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
+  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half*>(base), dims, strides, box,
+                           estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
+        std::to_string((int)r);
+  return map;
+}
+
 // 3-D map over C as floats [batch][m][2n] for the epilogue's bulk stores,
 // box {32, 32, 1} (32 rows x 16 complex) in the 128-byte swizzle, or with
 // `narrow` {16, 32, 1} (8 complex) in the 64-byte swizzle. False (and the
 // epilogue stores with plain instructions) when C is not 16-byte aligned, n
 // or the batch stride is odd, or QFLEX_TC_TMA_STORE=0.
 bool output_map(float2* C, std::size_t m, std::size_t n, std::uint64_t batch_stride, int batch, CUtensorMap* map,
-                bool narrow = false) {
+                bool narrow) {
   static const bool enabled = [] {
     const char* e = std::getenv("QFLEX_TC_TMA_STORE");
     return !(e && std::atoi(e) == 0);
@@ -1463,11 +1322,12 @@ bool output_map(float2* C, std::size_t m, std::size_t n, std::uint64_t batch_str
                      CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-void check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: CUDA ") + what + ") --> " + cudaGetErrorString(e);
+void launch_split_fp16(const float2* src, __half* planes, int* exps, std::size_t rows, std::size_t k,
+                       std::uint64_t src_stride, int batch, int nplanes, cudaStream_t s) {
+  dim3 grid((unsigned)std::min<std::uint64_t>((rows + 7) / 8, 152 * 16), (unsigned)batch);
+  split_fp16_kernel<<<grid, 256, 0, s>>>(src, planes, exps, rows, k, (k + 15) / 16 * 16, src_stride, nplanes);
+  check(cudaGetLastError(), "split_fp16");
 }
-
-}  // namespace
 
 bool tc_eligible(std::size_t m, std::size_t n, std::size_t k) {
   return m >= 64 && n >= 64 && k >= 16 && k % 4 == 0 && m < (1u << 31) && n < (1u << 31) && k < (1u << 31);
@@ -1608,15 +1468,8 @@ void launch_cgemm_fp16x3(const float2* A, const float2* Bt, float2* C, std::size
   __half* pb = static_cast<__half*>(w.b_planes);
   int* ea = a_in_planes ? w.a_block_exps : w.a_exps;
   int* eb = w.b_exps;
-  {
-    if (!a_in_planes) {
-      dim3 ga((unsigned)std::min<std::uint64_t>((m + 7) / 8, 152 * 16), (unsigned)batch);
-      split_fp16_kernel<<<ga, 256, 0, s>>>(A, pa, ea, m, k, kpad, batch_stride, 4);
-    }
-    dim3 gb((unsigned)std::min<std::uint64_t>((n + 7) / 8, 152 * 16), (unsigned)batch);
-    split_fp16_kernel<<<gb, 256, 0, s>>>(Bt, pb, eb, n, k, kpad, bt_stride, 6);
-    check(cudaGetLastError(), "split_fp16");
-  }
+  if (!a_in_planes) launch_split_fp16(A, pa, ea, m, k, batch_stride, batch, 4, s);
+  launch_split_fp16(Bt, pb, eb, n, k, bt_stride, batch, 6, s);
   // A: whole 128-byte rows for the single-CTA kernels, re / im halves for
   // the pair; B: 64-byte halves.
   const CUtensorMap ma_rows = plane_map_f16(pa, m, kpad, batch, BM, 64, 64);

@@ -62,6 +62,37 @@ void launch_cgemm_fp16x3(const float2* A, const float2* Bt, float2* C, std::size
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s,
                          bool a_in_planes = false);
 
+// Where the direct 3xFP16 product finds A: copies of 16 bytes (two elements
+// adjacent in the source) fill a block of 128 rows x 32 values, copy
+// u = lt + 64 i by loader thread lt. Offsets of sources are in elements and
+// add up, offsets into the block are in bytes and combine by XOR.
+struct AGather {
+  static constexpr int kBits = 26;
+  std::uint64_t copy_src[32];   // copy i's part of the source offset
+  std::uint64_t lane_src[6];    // part of each bit of lt
+  std::uint64_t tile_src[kBits];   // of each bit of the row-tile number (not plain)
+  std::uint64_t block_src[kBits];  // of each bit of the 32-value block number (not plain)
+  std::uint32_t copy_dst[32];   // the same two in the block
+  std::uint32_t lane_dst[6];
+  std::uint32_t row_at[7];      // of each bit of a row, where its values are read
+  std::uint32_t value_at[32];   // of each value of a row
+  std::int32_t plain;           // rows of k values: tiles and blocks by arithmetic
+  std::int32_t aligned;         // plain: every row starts on 16 bytes
+  std::int32_t pairs;           // values 2 j and 2 j + 1 of a row are adjacent
+  std::int32_t copies_real;     // copies i below this exist (16 when k = 16)
+};
+// A as m rows of k values; `aligned`: base, row and batch strides are
+// multiples of 16 bytes.
+AGather make_a_rows(std::size_t k, bool aligned);
+
+// The same product with A split inside the kernel: A is read as complex64
+// through `gather`, every 32 values of a row scaled by their own power of
+// two, and no A planes exist in memory. Single CTA, cfg.chunk 1 or 2 (a TMEM
+// chunk never spans two of A's blocks); cfg.variant is ignored.
+void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* Bt, float2* C, std::size_t m,
+                                std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride,
+                                int batch, float* workspace, int* err, const TcConfig& cfg, cudaStream_t s);
+
 // The same product with BF16x3 planes: x = b0 + b1 + b2 in BF16 (no
 // scaling: BF16 has the FP32 exponent range), six products per real
 // product (x0y0, x0y1, x1y0, x0y2, x1y1, x2y0) on kind::f16 tensor cores.

@@ -1,0 +1,53 @@
+"""The 3xFP16 product that splits A inside the kernel (products of up to 1024
+columns at the default kernel choice), at the edges of its tiles and blocks
+and on rows whose magnitude changes from one block of 32 values to the next."""
+import numpy as np
+import pytest
+
+from qflex_gb300 import FP16X3, Context
+
+pytestmark = pytest.mark.gpu
+
+# Error of an element against FP64, relative to sum |a| |b|: operands carried
+# to 22 bits (2 * 2^-23 each), twelve truncating additions per chunk of two
+# k-steps (2^-23 each), the chunks' FP32 additions (k / 32 * 2^-24), real and
+# imaginary part together (sqrt 2): below 4e-6 for k <= 256.
+TOL = 4e-6
+
+
+def _rows(kind, g, m, k):
+    block = np.arange(k) // 32
+    scale = {"gauss": np.zeros(k), "grow": 13.0 * block, "shrink": -13.0 * block,
+             "zeros": np.where(block == 0, -np.inf, 0.0), "tiny": np.full(k, -118.0),
+             "jump": np.where(block % 2 == 0, 0.0, 3.0)}[kind]
+    return (g.standard_normal((m, k)) + 1j * g.standard_normal((m, k))) * np.exp2(scale)
+
+
+@pytest.mark.parametrize("kind", ["gauss", "grow", "shrink", "zeros", "tiny", "jump"])
+@pytest.mark.parametrize("m,n,k,batch,extra", [
+    (64, 64, 16, 1, 0), (128, 128, 32, 1, 0), (129, 64, 64, 2, 0), (300, 128, 64, 1, 1), (192, 256, 128, 3, 1),
+    (1024, 1024, 32, 1, 0), (20000, 64, 16, 1, 0)])
+def test_direct_product(built_lib, kind, m, n, k, batch, extra):
+    import torch
+    g = np.random.default_rng(m + n + k)
+    stride = m * k + k * n + m * n + extra  # an odd stride leaves rows on 8-byte boundaries
+    buf = np.zeros((batch, stride), np.complex64)
+    scale_b = 2.0 ** 40 if kind == "tiny" else 1.0
+    with np.errstate(under="ignore"):
+        for row in buf:
+            row[:m * k] = _rows(kind, g, m, k).reshape(-1)
+            row[m * k:m * k + k * n] = (g.standard_normal(k * n) + 1j * g.standard_normal(k * n)) * scale_b
+    d = torch.from_numpy(buf).cuda()
+    torch.cuda.synchronize()
+    ctx = Context(0, FP16X3)
+    at = d.data_ptr()
+    ctx.multiply(at, at + 8 * m * k, at + 8 * (m * k + k * n), m, n, k, batch, stride)
+    ctx.synchronize()
+    out = d.cpu().numpy()
+    for row, got in zip(buf, out):
+        A, B = row[:m * k].reshape(m, k).astype(complex), row[m * k:m * k + k * n].reshape(k, n).astype(complex)
+        C = got[m * k + k * n:m * k + k * n + m * n].reshape(m, n)
+        assert np.isfinite(C).all()
+        assert np.max(np.abs(C - A @ B) / (np.abs(A) @ np.abs(B) + 1e-300)) < TOL
+        assert np.array_equal(got[:m * k + k * n], row[:m * k + k * n])
+        assert np.array_equal(got[m * k + k * n + m * n:], row[m * k + k * n + m * n:])
