@@ -138,11 +138,13 @@ size_t qflex_gb300_last_ops(const qflex_gb300_context* ctx, double* out, size_t 
  *                replay it (default 1, or QFLEX_GB300_GRAPHS)
  *   "max_batch"  most output strings per device pass of evaluate_many
  *                (0: as many as fit in device memory; default 0)
- *   "fuse_splits" 1 (3xFP16): a permutation whose output is the next
- *                product's A operand and read by nothing else writes the FP16
- *                planes (scaled per 32 values of a row) directly instead of
- *                complex64, and the product skips splitting A (default 1,
- *                or QFLEX_GB300_FUSE)
+ *   "fuse_splits" 1 (3xFP16): a product of up to 1024 columns (kernel choice
+ *                0) reads A through the permutation that would lay it out,
+ *                and no permutation runs; for the others a permutation whose
+ *                output is the next product's A operand and read by nothing
+ *                else writes the FP16 planes (scaled per 32 values of a row)
+ *                directly instead of complex64, and the product skips
+ *                splitting A (default 1, or QFLEX_GB300_FUSE)
  *   "tc_debias"  1: the split tensor-core products multiply their outputs
  *                by 1 + beta, the mean fraction the tensor core's truncating
  *                accumulation loses (measured on GB300 per split kind for
@@ -201,6 +203,15 @@ int qflex_gb300_permute(qflex_gb300_context* ctx, const void* src, void* dst, si
  * and diagnostics; needs no GPU and no context. No reference counterpart. */
 int qflex_gb300_check_permute(size_t rank, const size_t* dims, const size_t* new_order,
                               const void* src_host, void* dst_host);
+
+/* Host-side check of how a 3xFP16 product reads its A operand through a
+ * permutation instead of after it: the product's own copies and block reads
+ * over HOST buffers of complex64; dst_host is the row-major m x (size / m)
+ * operand the product sees. QFLEX_GB300_ERR_INPUT when products do not read
+ * that permutation directly (it runs as qflex_gb300_permute does). For tests
+ * and diagnostics; needs no GPU and no context. No reference counterpart. */
+int qflex_gb300_check_gather(size_t rank, const size_t* dims, const size_t* new_order, size_t m,
+                             const void* src_host, void* dst_host);
 
 /* In-place reorder with caller-provided scratch of at least the tensor's
  * size: Tensor::reorder(new_ordering, scratch_copy) (src/tensor.h:215,

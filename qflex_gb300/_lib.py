@@ -26,7 +26,7 @@ EXPORTS = (
     "qflex_gb300_result_final_state", "qflex_gb300_last_stats", "qflex_gb300_last_shapes",
     "qflex_gb300_last_gemms", "qflex_gb300_set_profiling", "qflex_gb300_last_ops",
     "qflex_gb300_set_option", "qflex_gb300_get_option", "qflex_gb300_set_tc_variant",
-    "qflex_gb300_permute", "qflex_gb300_check_permute",
+    "qflex_gb300_permute", "qflex_gb300_check_permute", "qflex_gb300_check_gather",
     "qflex_gb300_reorder",
     "qflex_gb300_multiply", "qflex_gb300_synchronize", "qflex_gb300_mlp_param_count",
     "qflex_gb300_mlp_work_floats", "qflex_gb300_mlp_forward", "qflex_gb300_mlp_loss_grad",
@@ -101,6 +101,7 @@ def load_library(path: Optional[Path] = None) -> C.CDLL:
             "qflex_gb300_last_ops": (sz, [vp, C.POINTER(dbl), sz]),
             "qflex_gb300_permute": (i, [vp, vp, vp, sz, C.POINTER(sz), C.POINTER(sz), sz, sz]),
             "qflex_gb300_check_permute": (i, [sz, C.POINTER(sz), C.POINTER(sz), vp, vp]),
+            "qflex_gb300_check_gather": (i, [sz, C.POINTER(sz), C.POINTER(sz), sz, vp, vp]),
             "qflex_gb300_reorder": (i, [vp, vp, vp, sz, C.POINTER(sz), C.POINTER(sz)]),
             "qflex_gb300_multiply": (i, [vp, vp, vp, vp, sz, sz, sz, sz, sz]),
             "qflex_gb300_synchronize": (i, [vp]),
@@ -142,6 +143,23 @@ def check_permute(src, dims: Sequence[int], new_order: Sequence[int]):
     if rc != OK:
         raise QflexGb300Error(rc, "permutation schedule check failed")
     return out
+
+
+def check_gather(src, dims: Sequence[int], new_order: Sequence[int], m: int):
+    """The row-major operand of m rows that a 3xFP16 product sees when it
+    reads the host array `src` through a permutation, or None when products
+    do not read that permutation directly."""
+    import numpy as np
+    lib = load_library()
+    a = np.ascontiguousarray(src, dtype=np.complex64).reshape(-1)
+    out = np.full_like(a, np.nan)
+    rc = lib.qflex_gb300_check_gather(len(dims), _sizes(dims), _sizes(new_order), m,
+                                      a.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p))
+    if rc == ERR_INPUT:
+        return None
+    if rc != OK:
+        raise QflexGb300Error(rc, "gather schedule check failed")
+    return out.reshape(m, -1)
 
 
 def multiply_skinny_noalloc(A: int, B: int, Cp: int, m: int, n: int, k: int, stream: int = 0) -> None:

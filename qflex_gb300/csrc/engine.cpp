@@ -48,6 +48,7 @@ struct Engine::Plan {
   Network net;
   Program prog;
   std::vector<PermPlan> perm;  // indexed like prog.ops (unused for GEMM ops)
+  std::vector<AGather> gather; // of the products that read A through a permutation, in program order
   // 3xFP16 fusion, indexed like prog.ops: a permute that writes the next
   // product's A operand straight as FP16 planes has fused[i] = index of that
   // product; the product has fused[j] = j. -1 elsewhere. Recomputed when
@@ -329,6 +330,12 @@ Engine::Plan* Engine::get_plan(const std::string& circuit, const std::string& or
   key += std::to_string(precision_);
   key += open_terminals_ ? "o" : "p";
   key += std::to_string(exact_gates_);
+  if (precision_ == FP16X3 && fuse_splits_) {
+    // What decides which products read A through a permutation.
+    key += cat("f", tc_cfg_.chunk <= 2 ? 1 : 0, ",", tc_cfg_.variant);
+    for (const auto& [shape, variant] : tc_variant_)
+      key += cat(";", std::get<0>(shape), ",", std::get<1>(shape), ",", std::get<2>(shape), ",", variant);
+  }
   if (plan_ && plan_->key == key) return plan_.get();
   auto p = std::make_unique<Plan>();
   p->key = std::move(key);
@@ -457,7 +464,7 @@ void Engine::plan_fusion(Plan& p) {
       if (g.kind == DevOp::PERMUTE) continue;
       if (!g.b_nk || g.a != ops[i].c || g.m * g.k != (std::size_t(1) << ops[i].nbits)) break;
       const TcConfig cfg = tc_config(g.m, g.n, g.k);
-      if (g.k < 32 || (g.k & (g.k - 1)) != 0 || cfg.chunk > 2) break;
+      if (g.k < 32 || (g.k & (g.k - 1)) != 0 || cfg.chunk > 2 || direct_product(g.n, cfg)) break;
       if (only_read_by(ops, i, j)) {
         p.fused[i] = (int)j;
         p.fused[j] = (int)j;
@@ -481,6 +488,7 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
     }
   }
   if (p.fuse_version != options_version_ || p.fused.size() != prog.ops.size()) plan_fusion(p);
+  std::size_t gathered = 0;
   for (std::size_t i = 0; i < prog.ops.size(); ++i) {
     const DevOp& op = prog.ops[i];
     if (profile_) QFX_CUDA(cudaEventRecord(prof_events_[i], stream_));
@@ -499,13 +507,17 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
       launches += 1;
     } else if (op.b_nk) {
       const bool a_planes = p.fused[i] == (int)i;
-      if (a_planes)
+      const TcConfig cfg = tc_config(op.m, op.n, op.k);
+      if (op.a_gather)
+        launch_cgemm_fp16x3_direct(arena + op.a, p.gather[gathered++], arena + op.b, arena + op.c, op.m, op.n, op.k,
+                                   stride, stride, batch, tc_ws, error_flag(), cfg, stream_);
+      else if (a_planes)
         launch_cgemm_fp16x3(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, stride, batch,
-                            tc_ws, error_flag(), tc_config(op.m, op.n, op.k), stream_, true);
+                            tc_ws, error_flag(), cfg, stream_, true);
       else
         launch_split_product(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, stride, batch,
                              tc_ws);
-      launches += a_planes ? 2 : 3;  // plane splits and the product
+      launches += a_planes || direct_product(op.n, cfg) ? 2 : 3;  // plane splits and the product
     } else {
       launch_cgemm_fp32(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, batch,
                         stream_, scratch);
@@ -610,8 +622,17 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
     p.net = build_network(p.circuit, p.grid, initial, results[0].final_state, final_qubits, p.ops);
     std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor;
     if (precision_ != FP32 && !is_complex128(precision_)) b_kmajor = tc_eligible;
+    std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a;
+    if (precision_ == FP16X3 && fuse_splits_)
+      gather_a = [&](std::size_t m, std::size_t n, std::size_t k, int nbits, const std::uint8_t* perm) {
+        AGather g;
+        if (!direct_product(n, tc_config(m, n, k)) || !make_a_gather(nbits, perm, m, k, &g)) return false;
+        p.gather.push_back(g);
+        return true;
+      };
+    p.gather.clear();
     try {
-      p.prog = plan_contraction(p.net, p.ops, results[0].states.size(), INFINITY, b_kmajor, open_terminals_);
+      p.prog = plan_contraction(p.net, p.ops, results[0].states.size(), INFINITY, b_kmajor, open_terminals_, gather_a);
     } catch (const std::string& e) {
       throw QFX_WRAP("ContractGrid", e);
     }

@@ -135,8 +135,9 @@ double reference_plan_bytes(const Network& net, const std::vector<Op>& ops) {
 class Planner {
  public:
   Planner(const Network& net, const std::vector<Op>& ops, std::size_t n_amps,
-          std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor, bool open_terminals)
-      : net_(net), ops_(ops), b_kmajor_(std::move(b_kmajor)) {
+          std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor, bool open_terminals,
+          std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a)
+      : net_(net), ops_(ops), b_kmajor_(std::move(b_kmajor)), gather_a_(std::move(gather_a)) {
     prog_.n_amplitudes = n_amps;
     // Terminal cuts stay open indices when every one of them takes all its
     // values and no two-qubit cut follows the first of them: the ops after
@@ -226,25 +227,27 @@ class Planner {
     t.dim = nd;
   }
 
-  // Moves the data of `t` into index order `order` (an out-of-place
-  // permute into a fresh buffer) unless it is already laid out that way.
-  void physical(STensor& t, const std::vector<std::string>& order, std::size_t leaf_dst = 0) {
-    if (order.empty() && t.phys.empty()) return;
-    if (order == t.phys) return;
+  // The digit permutation that brings `t`'s data into index order `order`
+  // (nbits and perm of `op`); false when it already lies so.
+  bool digit_permutation(const STensor& t, const std::vector<std::string>& order, DevOp& op,
+                         std::vector<std::size_t>& new_dim) const {
     const std::size_t r = t.phys.size();
+    new_dim.assign(r, 0);
+    if (r == 0 || order == t.phys) {
+      new_dim = t.pdim;
+      return false;
+    }
     std::vector<int> lg(r);
     for (std::size_t i = 0; i < r; ++i) lg[i] = ilog2_exact(t.pdim[i]);
     std::vector<int> s_old(r, 0);
     for (std::size_t i = r; i-- > 1;) s_old[i - 1] = s_old[i] + lg[i];
     std::vector<std::size_t> new_pos(r);
-    std::vector<std::size_t> new_dim(r);
     for (std::size_t i = 0; i < r; ++i) {
       new_pos[i] = std::find(order.begin(), order.end(), t.phys[i]) - order.begin();
       new_dim[new_pos[i]] = t.pdim[i];
     }
     std::vector<int> s_new(r, 0);
     for (std::size_t p = r; p-- > 1;) s_new[p - 1] = s_new[p] + ilog2_exact(new_dim[p]);
-    DevOp op{DevOp::PERMUTE};
     int nbits = 0;
     for (std::size_t i = 0; i < r; ++i) nbits += lg[i];
     if (nbits > 40) throw QFX_ERR("Tensor of 2^", nbits, " elements is too large.");
@@ -253,7 +256,17 @@ class Planner {
       for (int b = 0; b < lg[i]; ++b) op.perm[s_old[i] + b] = (std::uint8_t)(s_new[new_pos[i]] + b);
     bool identity = true;
     for (int b = 0; b < nbits; ++b) identity &= (op.perm[b] == b);
-    if (!identity) {
+    return !identity;
+  }
+
+  // Moves the data of `t` into index order `order` (an out-of-place
+  // permute into a fresh buffer) unless it is already laid out that way.
+  void physical(STensor& t, const std::vector<std::string>& order, std::size_t leaf_dst = 0) {
+    if (order.empty() && t.phys.empty()) return;
+    if (order == t.phys) return;
+    DevOp op{DevOp::PERMUTE};
+    std::vector<std::size_t> new_dim;
+    if (digit_permutation(t, order, op, new_dim)) {
       const int nb = leaf_dst ? -1 : alloc(t.size());
       op.a = addr(t);
       op.c = leaf_dst ? leaf_dst : bufs_[nb].off;
@@ -288,7 +301,13 @@ class Planner {
     // Tensor-core products read B as (right, common) rows (K-major); the
     // CUDA-core kernels read the reference's (common, right) layout.
     const bool b_nk = b_kmajor_(m, n, k);
-    physical(A, concat(left, common));
+    // A product that can read A through the permutation leaves A's data where
+    // it is (and its buffer in use until C has one).
+    DevOp op{DevOp::GEMM};
+    std::vector<std::size_t> a_dim;
+    op.a_gather = b_nk && gather_a_ && digit_permutation(A, concat(left, common), op, a_dim) &&
+                  gather_a_(m, n, k, op.nbits, op.perm);
+    if (!op.a_gather) physical(A, concat(left, common));
     physical(B, b_nk ? concat(right, common) : concat(common, right));
     STensor C;
     C.idx = concat(left, right);
@@ -297,7 +316,6 @@ class Planner {
     C.phys = C.idx;
     C.pdim = C.dim;
     C.buf = alloc(m * n);
-    DevOp op{DevOp::GEMM};
     op.a = addr(A);
     op.b = addr(B);
     op.c = bufs_[C.buf].off;
@@ -497,6 +515,7 @@ class Planner {
   const Network& net_;
   const std::vector<Op>& ops_;
   std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor_;
+  std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a_;
   Program prog_;
   std::vector<Buf> bufs_;
   std::vector<int> free_[64];
@@ -515,14 +534,15 @@ class Planner {
 Program plan_contraction(const Network& net, const std::vector<Op>& ops, std::size_t n_amplitudes,
                          double memory_limit,
                          std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor,
-                         bool open_terminals) {
+                         bool open_terminals,
+                         std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a) {
   const double ref_bytes = reference_plan_bytes(net, ops);
   if (ref_bytes > memory_limit)
     throw QFX_ERR("Failed to call Initialize(). Error:\n\t[Required space (",
                   readable_memory_string(ref_bytes), ") exceeds memory limit (",
                   readable_memory_string(memory_limit), "). Cancelling simulation.]");
   if (!b_kmajor) b_kmajor = [](std::size_t, std::size_t, std::size_t) { return false; };
-  Planner p(net, ops, n_amplitudes, std::move(b_kmajor), open_terminals);
+  Planner p(net, ops, n_amplitudes, std::move(b_kmajor), open_terminals, std::move(gather_a));
   Program prog = p.run();
   prog.reference_bytes = ref_bytes;
   return prog;

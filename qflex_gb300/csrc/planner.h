@@ -23,10 +23,11 @@ struct DevOp {
   enum Kind : int { PERMUTE = 0, GEMM = 1 } kind;
   std::size_t a = 0, b = 0, c = 0;  // PERMUTE: a = source, c = destination
   std::size_t m = 1, n = 1, k = 1;  // GEMM: C[m,n] = A[m,k] * B[k,n]
-  int nbits = 0;                    // PERMUTE: log2(size)
-  std::uint8_t perm[40] = {};       // PERMUTE: output bit of each input bit
+  int nbits = 0;                    // PERMUTE (and gathered A): log2(size)
+  std::uint8_t perm[40] = {};       // output bit of each input bit
   int shape_id = -1;                // GEMM: index into Program::shapes
   bool b_nk = false;                // GEMM: B stored as [n][k] (K-major)
+  bool a_gather = false;            // GEMM: A is read through the digit permutation nbits, perm
 };
 
 struct GemmShape {
@@ -61,9 +62,13 @@ struct Program {
 // With `open_terminals`, terminal cuts that take all their values (and are
 // not followed by a two-qubit cut) stay open indices: the ops after them
 // run once and the final tensor holds the terminal region's amplitudes.
+// `gather_a(m, n, k, nbits, perm)` tells whether the product of that shape can
+// read an A operand through the digit permutation that would lay it out
+// row-major; then no permutation is recorded (by default none can).
 Program plan_contraction(const Network& net, const std::vector<Op>& ops,
                          std::size_t n_amplitudes, double memory_limit,
                          std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor = {},
-                         bool open_terminals = false);
+                         bool open_terminals = false,
+                         std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a = {});
 
 }  // namespace qfx

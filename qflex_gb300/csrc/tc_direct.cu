@@ -35,9 +35,11 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "tc_common.cuh"
 #include "tc_gemm.h"
@@ -693,6 +695,118 @@ AGather make_a_rows(std::size_t k, bool aligned) {
   }
   for (int b = 0; b < 7; ++b) g.row_at[b] = at(16u << b);
   return g;
+}
+
+bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size_t k, AGather* g) {
+  int kl = 0;
+  while ((std::size_t(1) << kl) < k) ++kl;
+  if ((std::size_t(1) << kl) != k || kl < 4 || nbits > 31 || m < std::size_t(BM) || (m << kl) >> nbits != 1)
+    return false;
+  int from[32] = {};  // source digit of every digit of the row-major operand
+  for (int p = 0; p < nbits; ++p) from[perm[p]] = p;
+  // A block's digits, 7 of the row and 5 of the value (4 when k = 16: then
+  // the block's top digit is one that no value has), in source order.
+  const int kb = kl < 5 ? kl : 5;
+  int at_e[12], n_e = 0, row_e[7], val_e[5];
+  for (int p = 0; p < nbits; ++p) {
+    const int d = perm[p];
+    if (d < kb)
+      val_e[d] = n_e;
+    else if (d >= kl && d < kl + 7)
+      row_e[d - kl] = n_e;
+    else
+      continue;
+    at_e[n_e++] = p;
+  }
+  if (kb < 5) val_e[4] = n_e;
+  // The source's three lowest digits lie in the block: every copy of 16
+  // bytes is a pair of neighbours and eight lanes read at least 64
+  // consecutive bytes. (Tensors of the grid contractions keep their last
+  // index, 3 or 4 digits, in one piece; anything else is permuted first.)
+  if (at_e[0] != 0 || at_e[1] != 1 || at_e[2] != 2) return false;
+  std::memset(g, 0, sizeof(*g));
+  // Where element e of the block (source order) lies: unit e / 2 with its low
+  // three bits XORed by one mask per higher bit, chosen so that the low row
+  // digits, which the lanes of a reading warp differ in, reach different
+  // units: lanes 0..7 read 16 bytes each (pairs) or lanes 0..15 8 bytes.
+  std::uint32_t mask[11] = {};
+  {
+    std::uint32_t used = 0;
+    int want[3], n_want = 0;
+    for (int d = 0; d < 4 && n_want < 3; ++d)
+      if (row_e[d] != 0) want[n_want++] = row_e[d] - 1;
+    for (int w : want)
+      if (w < 3) used |= 1u << w;
+    for (int w : want)
+      if (w >= 3) {
+        const std::uint32_t free_bit = (used & 1) == 0 ? 1u : (used & 2) == 0 ? 2u : 4u;
+        mask[w] = free_bit;
+        used |= free_bit;
+      }
+  }
+  auto at = [&](std::uint32_t e) {
+    std::uint32_t u = e >> 1, x = u;
+    for (int b = 3; b < 11; ++b)
+      if ((u >> b) & 1) x ^= mask[b];
+    return (x << 4) | ((e & 1u) << 3);
+  };
+  g->aligned = 1;
+  g->pairs = val_e[0] == 0 ? 1 : 0;
+  g->copies_real = kb < 5 ? 16 : 32;
+  for (int b = 0; b < 6; ++b) {
+    g->lane_src[b] = std::uint64_t(1) << at_e[b + 1];
+    g->lane_dst[b] = at(2u << b);
+  }
+  for (std::uint32_t i = 0; i < 32; ++i) {
+    for (int b = 0; b < 5; ++b)
+      if (((i >> b) & 1) && 7 + b < n_e) g->copy_src[i] += std::uint64_t(1) << at_e[7 + b];
+    g->copy_dst[i] = at(i << 7);
+    std::uint32_t e = 0;
+    for (int q = 0; q < 5; ++q)
+      if ((i >> q) & 1) e |= 1u << val_e[q];
+    g->value_at[i] = at(e);
+  }
+  for (int d = 0; d < 7; ++d) g->row_at[d] = at(1u << row_e[d]);
+  for (int b = 0; kl + 7 + b < nbits; ++b) g->tile_src[b] = std::uint64_t(1) << from[kl + 7 + b];
+  for (int b = 0; 5 + b < kl; ++b) g->block_src[b] = std::uint64_t(1) << from[5 + b];
+  return true;
+}
+
+void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const float2* src, float2* dst) {
+  std::vector<float2> block(A_BLOCK / sizeof(float2));
+  for (std::size_t mt = 0; mt < m / BM; ++mt)
+    for (std::size_t b = 0; b < (k + 31) / 32; ++b) {
+      std::uint64_t base = 0;
+      for (int x = 0; x < AGather::kBits; ++x) {
+        if ((mt >> x) & 1) base += g.tile_src[x];
+        if ((b >> x) & 1) base += g.block_src[x];
+      }
+      std::fill(block.begin(), block.end(), make_float2(NAN, NAN));
+      for (int u = 0; u < 2048; ++u) {
+        std::uint64_t from = base + g.copy_src[u / LOADERS];
+        std::uint32_t to = g.copy_dst[u / LOADERS];
+        for (int x = 0; x < 6; ++x)
+          if ((u >> x) & 1) {
+            from += g.lane_src[x];
+            to ^= g.lane_dst[x];
+          }
+        const bool real = u / LOADERS < g.copies_real;
+        if ((real && (from + 2 > m * k || from % 2)) || to + 16 > A_BLOCK || to % 16)
+          throw std::string("ERROR (qflex_gb300: product) --> copy out of range");
+        for (int h = 0; h < 2; ++h) block[to / 8 + h] = real ? src[from + h] : make_float2(0.f, 0.f);
+      }
+      for (int row = 0; row < BM; ++row) {
+        std::uint32_t at = 0;
+        for (int x = 0; x < 7; ++x)
+          if ((row >> x) & 1) at ^= g.row_at[x];
+        for (std::size_t v = 0; v < 32 && b * 32 + v < k; ++v) {
+          const std::uint32_t slot = at ^ g.value_at[v];
+          if (slot + 8 > A_BLOCK || (g.pairs && v % 2 && slot != ((at ^ g.value_at[v - 1]) | 8u)))
+            throw std::string("ERROR (qflex_gb300: product) --> block read out of range");
+          dst[(mt * BM + row) * k + b * 32 + v] = block[slot / 8];
+        }
+      }
+    }
 }
 
 void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* Bt, float2* C, std::size_t m,

@@ -84,6 +84,15 @@ struct AGather {
 // A as m rows of k values; `aligned`: base, row and batch strides are
 // multiples of 16 bytes.
 AGather make_a_rows(std::size_t k, bool aligned);
+// A as a tensor of 2^nbits elements whose digit p goes to digit perm[p] of
+// the row-major m x k operand (k = 2^j >= 16, m >= 128): the product reads it
+// where it lies. False when the permutation cannot be read that way (the
+// source's low digits outside a block); the base and the batch stride have to
+// be multiples of 16 bytes.
+bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size_t k, AGather* g);
+// The gather's copies and reads on host buffers, block by block, with bounds
+// checks: dst is the m x k operand the product sees. Tests use it.
+void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const float2* src, float2* dst);
 
 // The same product with A split inside the kernel: A is read as complex64
 // through `gather`, every 32 values of a row scaled by their own power of
