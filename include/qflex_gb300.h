@@ -138,9 +138,10 @@ size_t qflex_gb300_last_ops(const qflex_gb300_context* ctx, double* out, size_t 
  *                replay it (default 1, or QFLEX_GB300_GRAPHS)
  *   "max_batch"  most output strings per device pass of evaluate_many
  *                (0: as many as fit in device memory; default 0)
- *   "fuse_splits" 1 (3xFP16): a product of up to 1024 columns (kernel choice
- *                0) reads A through the permutation that would lay it out,
- *                and no permutation runs; for the others a permutation whose
+ *   "fuse_splits" 1: CUDA-core products, and 3xFP16 products of up to 1024
+ *                columns (kernel choice 0), read A through the permutation
+ *                that would lay it out, and no permutation runs; for the
+ *                other 3xFP16 products a permutation whose
  *                output is the next product's A operand and read by nothing
  *                else writes the FP16 planes (scaled per 32 values of a row)
  *                directly instead of complex64, and the product skips
@@ -204,14 +205,16 @@ int qflex_gb300_permute(qflex_gb300_context* ctx, const void* src, void* dst, si
 int qflex_gb300_check_permute(size_t rank, const size_t* dims, const size_t* new_order,
                               const void* src_host, void* dst_host);
 
-/* Host-side check of how a 3xFP16 product reads its A operand through a
- * permutation instead of after it: the product's own copies and block reads
- * over HOST buffers of complex64; dst_host is the row-major m x (size / m)
- * operand the product sees. QFLEX_GB300_ERR_INPUT when products do not read
- * that permutation directly (it runs as qflex_gb300_permute does). For tests
- * and diagnostics; needs no GPU and no context. No reference counterpart. */
-int qflex_gb300_check_gather(size_t rank, const size_t* dims, const size_t* new_order, size_t m,
-                             const void* src_host, void* dst_host);
+/* Host-side check of how the products of a contraction read their A operand
+ * through a permutation instead of after it (tensor_cores != 0: the 3xFP16
+ * products; 0: the tiled CUDA-core products of n columns): the product's own
+ * copies over HOST buffers of complex64. dst_host is the row-major
+ * m x (size / m) operand the product sees. QFLEX_GB300_ERR_INPUT when products
+ * do not read that permutation directly (it runs as qflex_gb300_permute
+ * does). For tests and diagnostics; needs no GPU and no context. No reference
+ * counterpart. */
+int qflex_gb300_check_gather(size_t rank, const size_t* dims, const size_t* new_order, size_t m, size_t n,
+                             int tensor_cores, const void* src_host, void* dst_host);
 
 /* In-place reorder with caller-provided scratch of at least the tensor's
  * size: Tensor::reorder(new_ordering, scratch_copy) (src/tensor.h:215,

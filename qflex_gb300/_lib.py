@@ -101,7 +101,7 @@ def load_library(path: Optional[Path] = None) -> C.CDLL:
             "qflex_gb300_last_ops": (sz, [vp, C.POINTER(dbl), sz]),
             "qflex_gb300_permute": (i, [vp, vp, vp, sz, C.POINTER(sz), C.POINTER(sz), sz, sz]),
             "qflex_gb300_check_permute": (i, [sz, C.POINTER(sz), C.POINTER(sz), vp, vp]),
-            "qflex_gb300_check_gather": (i, [sz, C.POINTER(sz), C.POINTER(sz), sz, vp, vp]),
+            "qflex_gb300_check_gather": (i, [sz, C.POINTER(sz), C.POINTER(sz), sz, sz, i, vp, vp]),
             "qflex_gb300_reorder": (i, [vp, vp, vp, sz, C.POINTER(sz), C.POINTER(sz)]),
             "qflex_gb300_multiply": (i, [vp, vp, vp, vp, sz, sz, sz, sz, sz]),
             "qflex_gb300_synchronize": (i, [vp]),
@@ -145,15 +145,16 @@ def check_permute(src, dims: Sequence[int], new_order: Sequence[int]):
     return out
 
 
-def check_gather(src, dims: Sequence[int], new_order: Sequence[int], m: int):
-    """The row-major operand of m rows that a 3xFP16 product sees when it
-    reads the host array `src` through a permutation, or None when products
-    do not read that permutation directly."""
+def check_gather(src, dims: Sequence[int], new_order: Sequence[int], m: int, n: int = 0):
+    """The row-major operand of m rows that a product sees when it reads the
+    host array `src` through a permutation, or None when products do not read
+    that permutation directly: a tiled CUDA-core product of n columns, or
+    (n = 0) a 3xFP16 product."""
     import numpy as np
     lib = load_library()
     a = np.ascontiguousarray(src, dtype=np.complex64).reshape(-1)
     out = np.full_like(a, np.nan)
-    rc = lib.qflex_gb300_check_gather(len(dims), _sizes(dims), _sizes(new_order), m,
+    rc = lib.qflex_gb300_check_gather(len(dims), _sizes(dims), _sizes(new_order), m, n, int(n == 0),
                                       a.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.c_void_p))
     if rc == ERR_INPUT:
         return None

@@ -348,8 +348,8 @@ int qflex_gb300_check_permute(size_t rank, const size_t* dims, const size_t* new
   }
 }
 
-int qflex_gb300_check_gather(size_t rank, const size_t* dims, const size_t* new_order, size_t m,
-                             const void* src_host, void* dst_host) {
+int qflex_gb300_check_gather(size_t rank, const size_t* dims, const size_t* new_order, size_t m, size_t n,
+                             int tensor_cores, const void* src_host, void* dst_host) {
   try {
     if (!src_host || !dst_host || !all_powers_of_two(rank, dims) || m == 0 || (m & (m - 1)) != 0)
       return QFLEX_GB300_ERR_ARG;
@@ -357,9 +357,17 @@ int qflex_gb300_check_gather(size_t rank, const size_t* dims, const size_t* new_
     std::uint8_t perm[40] = {};
     check_perm(rank, dims, new_order, &nbits, perm);
     const size_t size = size_t(1) << nbits;
-    qfx::AGather g;
-    if (m > size || !qfx::make_a_gather(nbits, perm, m, size / m, &g)) return QFLEX_GB300_ERR_INPUT;
-    qfx::a_gather_on_host(g, m, size / m, (const float2*)src_host, (float2*)dst_host);
+    if (m > size) return QFLEX_GB300_ERR_INPUT;
+    const size_t k = size / m;
+    if (tensor_cores) {
+      qfx::AGather g;
+      if (!qfx::make_a_gather(nbits, perm, m, k, &g)) return QFLEX_GB300_ERR_INPUT;
+      qfx::a_gather_on_host(g, m, k, (const float2*)src_host, (float2*)dst_host);
+    } else {
+      qfx::TileGather g;
+      if (!qfx::make_tile_gather(nbits, perm, m, n, k, &g)) return QFLEX_GB300_ERR_INPUT;
+      qfx::tile_gather_on_host(g, m, n, k, (const float2*)src_host, (float2*)dst_host);
+    }
     return QFLEX_GB300_OK;
   } catch (...) {
     return QFLEX_GB300_ERR_ARG;

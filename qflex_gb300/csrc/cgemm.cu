@@ -1,0 +1,396 @@
+// Complex64 products C = A * B (row-major) on the FP32 pipes of sm_103a.
+//
+// One kernel body for all tile shapes: BM x BN outputs per tile, TM x TN per
+// thread, k in steps of BK. Blocks are persistent over the tiles (and the
+// batch): the k-steps of a block's tiles form one sequence, whose operands
+// cp.async brings into a ring of STAGES buffers, so a tile's products run
+// while the next tile's operands are on their way. That matters most for the
+// long, narrow products of the contractions (2^20 x 16 x 16), where a tile is
+// two k-steps.
+//
+// Bound by the FP32 pipes where k is long (scalar FMAs reach about 61 TFLOP/s
+// from registers alone at these clocks), by HBM at small k. Measured against
+// one tile per block with operands staged through registers:
+//   (2048, 2048, 2048)       1541 -> 1460 us (47 TFLOP/s)
+//   (32768, 64, 64) x 16      462 ->  342 us (50 TFLOP/s)
+//   (32768, 64, 8) x 16       221 ->   71 us
+//   (32768, 8, 64) x 16       113 ->   72 us
+//   (2^20, 16, 16)             75 ->   65 us (4.1 TB/s)
+//   (2^20, 16, 256)           847 ->  747 us
+// Copies of 16 bytes are worth 10 to 25 % of that against copies of 8; k-steps
+// of 8 keep four blocks of the narrow tiles on an SM. Two-lane FMAs
+// (fma.rn.f32x2) have the same rate from registers and lose more to packing
+// their operands: 2049 us at 2048^3.
+//
+// Sums run over k in ascending order with four FMAs per complex term.
+//
+// A is read as it lies or, for the tensors of a contraction, through the digit
+// permutation that would have laid it out row-major (TileGather): then lanes
+// follow the source's order and each copy goes to its place in the tile.
+#include <algorithm>
+#include <cstring>
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "kernels.h"
+
+namespace qfx {
+
+namespace {
+
+__device__ __forceinline__ void cfma(float2& c, float2 a, float2 b) {
+  c.x = fmaf(a.x, b.x, c.x);
+  c.x = fmaf(-a.y, b.y, c.x);
+  c.y = fmaf(a.x, b.y, c.y);
+  c.y = fmaf(a.y, b.x, c.y);
+}
+__device__ __forceinline__ void copy8(float2* dst, const float2* src, bool real) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                   static_cast<std::uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(real ? 8u : 0u)
+               : "memory");
+}
+
+__device__ __forceinline__ void copy16(float2* dst, const float2* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   static_cast<std::uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+// Row stride of a staged A tile in elements: 16 bytes more than its values,
+// so that the rows a quarter-warp reads start in different banks.
+constexpr int a_row(int BK) { return BK + 2; }
+
+template <int BM, int BN, int BK, int TM, int TN, int STAGES, bool GATHER>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+    cgemm_kernel(const float2* __restrict__ A, const float2* __restrict__ B, float2* __restrict__ C, int m, int n,
+                 int k, std::uint64_t batch_stride, int tiles_m, long long tiles, int pairs,
+                 const __grid_constant__ TileGather g) {
+  constexpr int NT = (BM / TM) * (BN / TN);
+  constexpr int TX = BN / TN, TY = BM / TM;
+  constexpr int LA = BM * BK / NT, LB = (BK * BN + NT - 1) / NT;
+  constexpr int AR = a_row(BK);
+  constexpr int A_ELEMS = BM * AR, STAGE = A_ELEMS + BK * BN;
+  static_assert(LA * NT == BM * BK && BK % 2 == 0 && TN % 2 == 0, "tile / threads mismatch");
+  extern __shared__ __align__(16) float2 ring[];
+  const int t = threadIdx.x;
+  const int tx = t % TX, ty = t / TX;
+  const int ktiles = k > 0 ? (k + BK - 1) / BK : 1;  // no terms: one k-step of zeros
+  const int tiles_n = (n + BN - 1) / BN;
+  const long long mine = (long long)blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const long long steps = mine * ktiles;
+  // Consecutive tiles share their rows of A.
+  auto place = [&](long long tile, unsigned& mt, unsigned& nt, std::uint64_t& at) {
+    if (tiles <= 0xffffffffll) {  // 32-bit divisions are much the shorter
+      const unsigned r = unsigned(tile) / unsigned(tiles_n);
+      nt = unsigned(tile) % unsigned(tiles_n);
+      mt = r % unsigned(tiles_m);
+      at = std::uint64_t(r / unsigned(tiles_m)) * batch_stride;
+    } else {
+      const long long r = tile / tiles_n;
+      nt = unsigned(tile % tiles_n);
+      mt = unsigned(r % tiles_m);
+      at = std::uint64_t(r / tiles_m) * batch_stride;
+    }
+  };
+
+  const float2* lane_src = A;
+  int lane_dst = 0;
+  if constexpr (GATHER) {
+    for (int b = 0; (1 << b) < NT; ++b)
+      if ((t >> b) & 1) {
+        lane_src += g.lane_src[b];
+        lane_dst += g.lane_dst[b];
+      }
+  }
+
+  // Loader position: k-step lk of the block's tile lt.
+  long long lt = blockIdx.x;
+  int lk = 0;
+  auto load = [&](int slot) {
+    float2* As = ring + slot * STAGE;
+    float2* Bs = As + A_ELEMS;
+    unsigned mt, nt;
+    std::uint64_t at;
+    place(lt, mt, nt, at);
+    const int k0 = lk * BK;
+    if constexpr (GATHER) {
+      const float2* src = lane_src + at;
+      for (int b = 0; b < TileGather::kBits && (mt >> b); ++b)
+        if ((mt >> b) & 1) src += g.tile_src[b];
+      for (int b = 0; b < TileGather::kBits && (lk >> b); ++b)
+        if ((lk >> b) & 1) src += g.step_src[b];
+#pragma unroll
+      for (int i = 0; i < LA; ++i) copy8(As + lane_dst + g.copy_dst[i], src + g.copy_src[i], true);
+    } else if ((pairs & 2) && (mt + 1) * BM <= unsigned(m) && k0 + BK <= k) {
+      // Inside the matrix, rows on 16 bytes: pairs of values.
+      constexpr int P = BK / 2, LP = (BM * P + NT - 1) / NT, ROWS = NT / P;
+      static_assert(NT % P == 0, "pairs of a row of A / threads");
+      const int r = t / P, c = 2 * (t % P);
+      const float2* src = A + at + std::uint64_t(mt * BM + r) * k + k0 + c;
+#pragma unroll
+      for (int i = 0; i < LP; ++i) {
+        if (BM * P % NT == 0 || r + i * ROWS < BM) copy16(As + (r + i * ROWS) * AR + c, src);
+        src += std::uint64_t(ROWS) * k;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < LA; ++i) {
+        const int idx = t + i * NT;
+        const int r = idx / BK, c = idx % BK;
+        const unsigned row = mt * BM + r;
+        const bool real = row < unsigned(m) && k0 + c < k;
+        copy8(As + r * AR + c, real ? A + at + std::uint64_t(row) * k + k0 + c : A, real);
+      }
+    }
+    if ((pairs & 4) && (nt + 1) * BN <= unsigned(n) && k0 + BK <= k) {
+      constexpr int P = BN / 2, LP = (BK * P + NT - 1) / NT, ROWS = NT / P;
+      static_assert(NT % P == 0, "pairs of a row of B / threads");
+      const int r = t / P, c = 2 * (t % P);
+      const float2* src = B + at + std::uint64_t(k0 + r) * n + nt * BN + c;
+#pragma unroll
+      for (int i = 0; i < LP; ++i) {
+        if (BK * P % NT == 0 || r + i * ROWS < BK) copy16(Bs + (r + i * ROWS) * BN + c, src);
+        src += std::uint64_t(ROWS) * n;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < LB; ++i) {
+        const int idx = t + i * NT;
+        if (BK * BN % NT != 0 && idx >= BK * BN) break;
+        const int r = idx / BN, c = idx % BN;
+        const unsigned col = nt * BN + c;
+        const bool real = k0 + r < k && col < unsigned(n);
+        copy8(Bs + r * BN + c, real ? B + at + std::uint64_t(k0 + r) * n + col : B, real);
+      }
+    }
+    if (++lk == ktiles) {
+      lk = 0;
+      lt += gridDim.x;
+    }
+  };
+
+  float2 acc[TM][TN];
+  long long loaded = 0, tile = blockIdx.x;
+  int ks = 0, slot = 0, load_slot = 0;
+  for (; loaded < STAGES - 1; ++loaded) {
+    if (loaded < steps) load(load_slot);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (++load_slot == STAGES) load_slot = 0;
+  }
+  for (long long s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();  // step s has landed; everybody is done with the slot loaded next
+    if (loaded < steps) load(load_slot);
+    ++loaded;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (++load_slot == STAGES) load_slot = 0;
+
+    if (ks == 0) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    }
+    // Thread (tx, ty): rows ty + TY i, columns 2 tx, 2 tx + 1 of every 2 TX.
+    const float2* As = ring + slot * STAGE + ty * AR;
+    const float2* Bs = ring + slot * STAGE + A_ELEMS + 2 * tx;
+#pragma unroll 4
+    for (int kk = 0; kk < BK; kk += 2) {
+      float4 a[TM];  // values kk and kk + 1
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(As + i * TY * AR + kk);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float2 b[TN];
+#pragma unroll
+        for (int j = 0; j < TN; j += 2) {
+          const float4 v = *reinterpret_cast<const float4*>(Bs + (kk + h) * BN + j * TX);
+          b[j] = make_float2(v.x, v.y);
+          b[j + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+          const float2 x = h ? make_float2(a[i].z, a[i].w) : make_float2(a[i].x, a[i].y);
+#pragma unroll
+          for (int j = 0; j < TN; ++j) cfma(acc[i][j], x, b[j]);
+        }
+      }
+    }
+    if (++slot == STAGES) slot = 0;
+    if (++ks == ktiles) {
+      ks = 0;
+      unsigned mt, nt;
+      std::uint64_t at;
+      place(tile, mt, nt, at);
+      tile += gridDim.x;
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const unsigned r = mt * BM + ty + i * TY;
+        if (r >= unsigned(m)) continue;
+        float2* c = C + at + std::uint64_t(r) * n;
+#pragma unroll
+        for (int j = 0; j < TN; j += 2) {
+          const unsigned col = nt * BN + 2 * tx + j * TX;
+          const float2 v0 = acc[i][j], v1 = acc[i][j + 1];
+          if ((pairs & 1) && col + 1 < unsigned(n)) {
+            *reinterpret_cast<float4*>(c + col) = make_float4(v0.x, v0.y, v1.x, v1.y);
+          } else {
+            if (col < unsigned(n)) c[col] = v0;
+            if (col + 1 < unsigned(n)) c[col + 1] = v1;
+          }
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+struct Tile {
+  int bm, bn, bk, threads;
+};
+template <int BM, int BN, int BK, int TM, int TN, int STAGES>
+struct Shape {
+  static constexpr int nt = (BM / TM) * (BN / TN);
+  static constexpr Tile tile{BM, BN, BK, nt};
+  static constexpr int smem = STAGES * (BM * a_row(BK) + BK * BN) * (int)sizeof(float2);
+
+  template <bool GATHER>
+  static void run(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
+                  std::uint64_t stride, int batch, const TileGather& g, cudaStream_t s) {
+    auto* kernel = cgemm_kernel<BM, BN, BK, TM, TN, STAGES, GATHER>;
+    // Blocks that are resident at once on the current device.
+    static std::once_flag once;
+    static int resident = 152;
+    std::call_once(once, [&] {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      int dev = 0, sms = 152, per = 1;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
+      resident = sms * std::max(per, 1);
+    });
+    const long long tiles_m = (long long)((m + BM - 1) / BM);
+    const long long tiles = tiles_m * (long long)((n + BN - 1) / BN) * batch;
+    // Which of C's, A's and B's rows start on 16 bytes (bits 0, 1, 2).
+    const bool even = batch == 1 || stride % 2 == 0;
+    auto rows16 = [&](const float2* p, std::size_t row) {
+      return even && row % 2 == 0 && (reinterpret_cast<std::uintptr_t>(p) & 15) == 0;
+    };
+    const int pairs = (rows16(C, n) ? 1 : 0) | (rows16(A, k) ? 2 : 0) | (rows16(B, n) ? 4 : 0);
+    kernel<<<(unsigned)std::min<long long>(tiles, resident), nt, smem, s>>>(A, B, C, (int)m, (int)n, (int)k, stride,
+                                                                            (int)tiles_m, tiles, pairs, g);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch cgemm) --> ") + cudaGetErrorString(e);
+  }
+  static void launch(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
+                     std::uint64_t stride, int batch, const TileGather* g, cudaStream_t s) {
+    if (g)
+      run<true>(A, B, C, m, n, k, stride, batch, *g, s);
+    else
+      run<false>(A, B, C, m, n, k, stride, batch, TileGather{}, s);
+  }
+};
+
+// Calls f with the shape that a product takes: the narrowest that holds its
+// columns (or rows), so that no more than half of a tile's outputs are padding
+// from 5 columns on; k-steps of 16 where there are 16 terms and the tile is
+// wide enough to keep two blocks on an SM.
+template <typename F>
+auto with_shape(std::size_t m, std::size_t n, std::size_t k, F&& f) {
+  if (n <= 8) return f(Shape<256, 8, 8, 4, 4, 3>{});
+  if (n <= 16) return f(Shape<256, 16, 8, 8, 4, 2>{});
+  if (n <= 32) return f(Shape<128, 32, 8, 8, 4, 3>{});
+  if (m <= 32) return f(Shape<16, 256, 8, 4, 8, 3>{});
+  if (k <= 8) return f(Shape<128, 64, 8, 8, 4, 3>{});
+  return f(Shape<128, 64, 16, 8, 4, 3>{});
+}
+
+}  // namespace
+
+bool make_tile_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size_t n, std::size_t k, TileGather* g) {
+  const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
+  int kl = 0, ml = 0, bk = 0, bm = 0, lanes = 0;
+  while ((std::size_t(1) << kl) < k) ++kl;
+  while ((std::size_t(1) << ml) < m) ++ml;
+  while ((1 << bk) < tile.bk) ++bk;
+  while ((1 << bm) < tile.bm) ++bm;
+  while ((1 << lanes) < tile.threads) ++lanes;
+  if ((std::size_t(1) << kl) != k || (std::size_t(1) << ml) != m || kl + ml != nbits || nbits > 31 || kl < bk ||
+      ml < bm)
+    return false;
+  std::memset(g, 0, sizeof(*g));
+  int n_e = 0;
+  for (int p = 0; p < nbits; ++p) {
+    const int d = perm[p];
+    const bool value = d < bk, row = d >= kl && d < kl + bm;
+    if (!value && !row) {
+      // The source's three lowest digits lie in the tile: eight lanes read 64
+      // consecutive bytes.
+      if (p < 3) return false;
+      if (d < kl)
+        g->step_src[d - bk] = std::uint64_t(1) << p;
+      else
+        g->tile_src[d - kl - bm] = std::uint64_t(1) << p;
+      continue;
+    }
+    const std::uint32_t dst = value ? 1u << d : (std::uint32_t)a_row(tile.bk) << (d - kl);
+    if (n_e < lanes) {
+      g->lane_src[n_e] = std::uint64_t(1) << p;
+      g->lane_dst[n_e] = dst;
+    } else {
+      const int b = n_e - lanes;
+      for (int i = 0; i < TileGather::kCopies; ++i)
+        if ((i >> b) & 1) {
+          g->copy_src[i] += std::uint64_t(1) << p;
+          g->copy_dst[i] += dst;
+        }
+    }
+    ++n_e;
+  }
+  return true;
+}
+
+void tile_gather_on_host(const TileGather& g, std::size_t m, std::size_t n, std::size_t k, const float2* src,
+                         float2* dst) {
+  const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
+  const int ar = a_row(tile.bk), copies = tile.bm * tile.bk / tile.threads;
+  std::vector<float2> staged(std::size_t(tile.bm) * ar);
+  for (std::size_t mt = 0; mt < m / tile.bm; ++mt)
+    for (std::size_t ks = 0; ks < k / tile.bk; ++ks) {
+      std::uint64_t base = 0;
+      for (int b = 0; b < TileGather::kBits; ++b) {
+        if ((mt >> b) & 1) base += g.tile_src[b];
+        if ((ks >> b) & 1) base += g.step_src[b];
+      }
+      for (int t = 0; t < tile.threads; ++t)
+        for (int i = 0; i < copies; ++i) {
+          std::uint64_t from = base + g.copy_src[i], to = g.copy_dst[i];
+          for (int b = 0; (1 << b) < tile.threads; ++b)
+            if ((t >> b) & 1) {
+              from += g.lane_src[b];
+              to += g.lane_dst[b];
+            }
+          if (copies > TileGather::kCopies || from >= m * k || to >= staged.size())
+            throw std::string("ERROR (qflex_gb300: cgemm) --> copy out of range");
+          staged[to] = src[from];
+        }
+      for (int r = 0; r < tile.bm; ++r)
+        for (int v = 0; v < tile.bk; ++v)
+          dst[(mt * tile.bm + r) * k + ks * tile.bk + v] = staged[std::size_t(r) * ar + v];
+    }
+}
+
+void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
+                        std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, cudaStream_t s) {
+  if (m > 0x7fffffffull || n > 0x7fffffffull || k > 0x7fffffffull)
+    throw std::string("ERROR (qflex_gb300: cgemm) --> dimension exceeds 2^31");
+  with_shape(m, n, k, [&](auto shape) {
+    decltype(shape)::launch(A, B, C, m, n, k, batch_stride, batch, gather, s);
+    return 0;
+  });
+}
+
+}  // namespace qfx

@@ -48,7 +48,10 @@ struct Engine::Plan {
   Network net;
   Program prog;
   std::vector<PermPlan> perm;  // indexed like prog.ops (unused for GEMM ops)
-  std::vector<AGather> gather; // of the products that read A through a permutation, in program order
+  // Of the products that read A through a permutation, in program order:
+  // the tensor-core ones and the CUDA-core ones.
+  std::vector<AGather> gather;
+  std::vector<TileGather> tile_gather;
   // 3xFP16 fusion, indexed like prog.ops: a permute that writes the next
   // product's A operand straight as FP16 planes has fused[i] = index of that
   // product; the product has fused[j] = j. -1 elsewhere. Recomputed when
@@ -330,6 +333,7 @@ Engine::Plan* Engine::get_plan(const std::string& circuit, const std::string& or
   key += std::to_string(precision_);
   key += open_terminals_ ? "o" : "p";
   key += std::to_string(exact_gates_);
+  if (!fuse_splits_) key += "n";
   if (precision_ == FP16X3 && fuse_splits_) {
     // What decides which products read A through a permutation.
     key += cat("f", tc_cfg_.chunk <= 2 ? 1 : 0, ",", tc_cfg_.variant);
@@ -488,7 +492,7 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
     }
   }
   if (p.fuse_version != options_version_ || p.fused.size() != prog.ops.size()) plan_fusion(p);
-  std::size_t gathered = 0;
+  std::size_t gathered = 0, tile_gathered = 0;
   for (std::size_t i = 0; i < prog.ops.size(); ++i) {
     const DevOp& op = prog.ops[i];
     if (profile_) QFX_CUDA(cudaEventRecord(prof_events_[i], stream_));
@@ -518,6 +522,10 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
         launch_split_product(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, stride, batch,
                              tc_ws);
       launches += a_planes || direct_product(op.n, cfg) ? 2 : 3;  // plane splits and the product
+    } else if (op.a_gather) {
+      launch_cgemm_tiled(arena + op.a, &p.tile_gather[tile_gathered++], arena + op.b, arena + op.c, op.m, op.n, op.k,
+                         stride, batch, stream_);
+      launches += 1;
     } else {
       launch_cgemm_fp32(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, batch,
                         stream_, scratch);
@@ -623,14 +631,21 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
     std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor;
     if (precision_ != FP32 && !is_complex128(precision_)) b_kmajor = tc_eligible;
     std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a;
-    if (precision_ == FP16X3 && fuse_splits_)
+    p.gather.clear();
+    p.tile_gather.clear();
+    if (fuse_splits_ && !is_complex128(precision_))
       gather_a = [&](std::size_t m, std::size_t n, std::size_t k, int nbits, const std::uint8_t* perm) {
-        AGather g;
-        if (!direct_product(n, tc_config(m, n, k)) || !make_a_gather(nbits, perm, m, k, &g)) return false;
-        p.gather.push_back(g);
+        if (b_kmajor && b_kmajor(m, n, k)) {
+          AGather g;
+          if (!direct_product(n, tc_config(m, n, k)) || !make_a_gather(nbits, perm, m, k, &g)) return false;
+          p.gather.push_back(g);
+        } else {
+          TileGather g;
+          if (m < 2 || n < 2 || m * n <= 64 || !make_tile_gather(nbits, perm, m, n, k, &g)) return false;
+          p.tile_gather.push_back(g);
+        }
         return true;
       };
-    p.gather.clear();
     try {
       p.prog = plan_contraction(p.net, p.ops, results[0].states.size(), INFINITY, b_kmajor, open_terminals_, gather_a);
     } catch (const std::string& e) {

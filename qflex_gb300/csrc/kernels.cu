@@ -250,106 +250,9 @@ __global__ void __launch_bounds__(256) permute_general_kernel(const __grid_const
 }
 
 // ---------------------------------------------------------------------------
-// Complex64 GEMM on CUDA cores (C = A * B, row-major).
-// Block tile BM x BN, k-step BK; each thread owns a TM x TN sub-tile.
-// Operands pass through shared memory with a register-staged prefetch of
-// the next k-step.
+// Complex64 products with a single row or column, or few outputs and a long
+// contraction (the tiled products are in cgemm.cu).
 // ---------------------------------------------------------------------------
-template <int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-    cgemm_kernel(const float2* __restrict__ A, const float2* __restrict__ B, float2* __restrict__ C,
-                 int m, int n, int k, std::uint64_t batch_stride) {
-  constexpr int NT = (BM / TM) * (BN / TN);
-  constexpr int TX = BN / TN;
-  constexpr int LA = BM * BK / NT;
-  constexpr int LB = BK * BN / NT;
-  static_assert(LA * NT == BM * BK && LB * NT == BK * BN, "tile/threads mismatch");
-  __shared__ __align__(16) float2 As[BK][BM + 2];
-  __shared__ __align__(16) float2 Bs[BK][BN + 2];
-
-  const std::uint64_t boff = std::uint64_t(blockIdx.z) * batch_stride;
-  A += boff;
-  B += boff;
-  C += boff;
-  const int tiles_m = (m + BM - 1) / BM;
-  const int m0 = int(blockIdx.x % tiles_m) * BM;
-  const int n0 = int(blockIdx.x / tiles_m) * BN;
-  const int t = threadIdx.x;
-  const int tx = t % TX, ty = t / TX;
-
-  float2 acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
-
-  float2 ra[LA], rb[LB];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < LA; ++i) {
-      const int idx = t + i * NT;
-      const int r = idx / BK, c = idx % BK;
-      const int gr = m0 + r, gc = k0 + c;
-      ra[i] = (gr < m && gc < k) ? A[std::size_t(gr) * k + gc] : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int i = 0; i < LB; ++i) {
-      const int idx = t + i * NT;
-      const int r = idx / BN, c = idx % BN;
-      const int gr = k0 + r, gc = n0 + c;
-      rb[i] = (gr < k && gc < n) ? B[std::size_t(gr) * n + gc] : make_float2(0.f, 0.f);
-    }
-  };
-  auto store = [&]() {
-#pragma unroll
-    for (int i = 0; i < LA; ++i) {
-      const int idx = t + i * NT;
-      As[idx % BK][idx / BK] = ra[i];
-    }
-#pragma unroll
-    for (int i = 0; i < LB; ++i) {
-      const int idx = t + i * NT;
-      Bs[idx / BN][idx % BN] = rb[i];
-    }
-  };
-
-  const int ktiles = (k + BK - 1) / BK;
-  load(0);
-  store();
-  __syncthreads();
-  for (int kt = 0; kt < ktiles; ++kt) {
-    const bool more = kt + 1 < ktiles;
-    if (more) load((kt + 1) * BK);
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float2 a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx * TN + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = cfma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-    if (more) {
-      store();
-      __syncthreads();
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int gr = m0 + ty * TM + i;
-    if (gr >= m) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gc = n0 + tx * TN + j;
-      if (gc < n) C[std::size_t(gr) * n + gc] = acc[i][j];
-    }
-  }
-}
-
 __device__ __forceinline__ float2 warp_sum(float2 v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -534,16 +437,6 @@ __global__ void reduce_amplitudes_kernel(const float2* __restrict__ results, std
   double2& out = amps[std::size_t(b) * n_amps + a];
   out.x += re;
   out.y += im;
-}
-
-template <int BM, int BN, int BK, int TM, int TN>
-void run_cgemm(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n,
-               std::size_t k, std::uint64_t stride, int batch, cudaStream_t s) {
-  const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-  dim3 grid((unsigned)tiles, 1, (unsigned)batch);
-  cgemm_kernel<BM, BN, BK, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, s>>>(A, B, C, (int)m, (int)n,
-                                                                         (int)k, stride);
-  check_launch("cgemm");
 }
 
 }  // namespace
@@ -802,14 +695,7 @@ void launch_cgemm_fp32(const float2* A, const float2* B, float2* C, std::size_t 
     check_launch("gemv_cols");
     return;
   }
-  if (m > 0x7fffffffull || n > 0x7fffffffull || k > 0x7fffffffull)
-    throw std::string("ERROR (qflex_gb300: cgemm) --> dimension exceeds 2^31");
-  if (n <= 32)
-    run_cgemm<256, 16, 16, 8, 2>(A, B, C, m, n, k, stride, batch, s);
-  else if (m <= 32)
-    run_cgemm<16, 256, 16, 2, 8>(A, B, C, m, n, k, stride, batch, s);
-  else
-    run_cgemm<128, 64, 16, 8, 4>(A, B, C, m, n, k, stride, batch, s);
+  launch_cgemm_tiled(A, nullptr, B, C, m, n, k, stride, batch, s);
 }
 
 void launch_reduce_amplitudes(const float2* results, std::uint64_t stride, const std::uint32_t* ptr,

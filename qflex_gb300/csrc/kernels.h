@@ -125,6 +125,32 @@ void launch_cgemm_fp32(const float2* A, const float2* B, float2* C, std::size_t 
                        std::size_t k, std::uint64_t batch_stride, int batch, cudaStream_t s,
                        float2* scratch);
 
+// Where a tiled product finds A when it reads it through a digit permutation:
+// copy i of thread t goes from source offset lane(t) + copy i's part (plus the
+// tile's and k-step's) to place lane(t) + copy i's part of the staged tile;
+// all offsets in elements.
+struct TileGather {
+  static constexpr int kBits = 26, kCopies = 32;
+  std::uint64_t copy_src[kCopies];
+  std::uint64_t lane_src[8];        // of each bit of the thread
+  std::uint64_t tile_src[kBits];    // of each bit of the row-tile number
+  std::uint64_t step_src[kBits];    // of each bit of the k-step number
+  std::uint32_t copy_dst[kCopies];
+  std::uint32_t lane_dst[8];
+};
+// A as a tensor of 2^nbits elements whose digit p goes to digit perm[p] of the
+// row-major m x k operand of an m x n x k product. False when the product's
+// tile does not divide the operand or the source's three lowest digits lie
+// outside a tile.
+bool make_tile_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size_t n, std::size_t k, TileGather* g);
+// The gather's copies on host buffers with bounds checks: dst is the m x k
+// operand that the product sees. Tests use it.
+void tile_gather_on_host(const TileGather& g, std::size_t m, std::size_t n, std::size_t k, const float2* src,
+                         float2* dst);
+// The tiled product, A row-major or (gather not null) through a permutation.
+void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
+                        std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, cudaStream_t s);
+
 // One skinny product (m * n outputs) with k split over `splits` blocks per
 // output; `partial` holds m * n * splits float2, every one of which is
 // written before it is read.

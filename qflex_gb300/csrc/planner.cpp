@@ -305,7 +305,7 @@ class Planner {
     // it is (and its buffer in use until C has one).
     DevOp op{DevOp::GEMM};
     std::vector<std::size_t> a_dim;
-    op.a_gather = b_nk && gather_a_ && digit_permutation(A, concat(left, common), op, a_dim) &&
+    op.a_gather = gather_a_ && digit_permutation(A, concat(left, common), op, a_dim) &&
                   gather_a_(m, n, k, op.nbits, op.perm);
     if (!op.a_gather) physical(A, concat(left, common));
     physical(B, b_nk ? concat(right, common) : concat(common, right));

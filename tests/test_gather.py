@@ -47,3 +47,28 @@ def test_gather_refuses_what_no_block_holds(built_lib):
     assert check_gather(src, [64, 64], [1, 0], 64) is None           # fewer than 128 rows
     assert check_gather(src, [512, 8], [1, 0], 512) is None          # rows of 8 values
     assert check_gather(src, [16, 16, 16], [0, 1, 2], 256) is not None
+
+
+@pytest.mark.parametrize("n", [8, 16, 32, 64, 256])
+@pytest.mark.parametrize("seed", range(8))
+def test_tile_gather_matches_transpose(built_lib, seed, n):
+    """The same for the tiled CUDA-core products, whose tile depends on the
+    product's columns, rows and terms."""
+    rng = random.Random(1000 * n + seed)
+    accepted = 0
+    for _ in range(60):
+        lg = [rng.randint(1, 5) for _ in range(rng.randint(2, 7))]
+        if not 8 <= sum(lg) <= 17:
+            continue
+        order = list(range(len(lg)))
+        rng.shuffle(order)
+        if rng.random() < 0.3:
+            order.sort()
+        src = _source(1 << sum(lg))
+        kl = rng.randint(2, sum(lg) - 3)
+        got = check_gather(src, [1 << x for x in lg], order, 1 << (sum(lg) - kl), n)
+        if got is not None:
+            accepted += 1
+            want = src.reshape([1 << x for x in lg]).transpose(order).reshape(got.shape)
+            assert np.array_equal(got, want)
+    assert accepted
