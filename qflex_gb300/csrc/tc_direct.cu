@@ -23,10 +23,13 @@
 // A block is two k-steps of 16, one TMEM chunk at the default chunk length,
 // so the epilogue applies the block's exponent as it adds the chunk.
 //
-// What bounds it: the tensor pipe. Six N = 256 MMAs' worth of work per k-step
-// take 768 cycles; shared-memory traffic of the conversion (32 KB written,
-// read and written again per two k-steps) measured no slowdown of the MMAs
-// beside it.
+// What bounds it: shared memory's 128 bytes a cycle. A k-step's MMAs take 768
+// cycles of the tensor pipe and read 84 KB of operands (672 cycles); loading
+// B takes another 128, and A's way through shared memory (written by the
+// copies, read by the converter, written as planes) 384. 1125 cycles measured
+// at k = 4096. (The kernel that loads A's planes reads 72 KB and loads 40:
+// 896, where the card's power limit is near.) A tile's store overlaps two
+// chunks of the next tile's MMAs.
 //
 // B holds no negated copy: Ar multiplies (Br; Bi) in one N = 256 MMA, and Ai
 // takes two N = 128 MMAs, -Ai Bi (the descriptor's negate-A bit) and Ai Br.
