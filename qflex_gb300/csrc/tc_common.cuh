@@ -131,6 +131,17 @@ __device__ __forceinline__ std::uint64_t smem_desc_sw64(std::uint32_t addr) {
   return d;
 }
 
+// Rows of 32 bytes in the 32-byte swizzle (8-row groups 256 bytes apart).
+__device__ __forceinline__ std::uint64_t smem_desc_sw32(std::uint32_t addr) {
+  std::uint64_t d = 0;
+  d |= std::uint64_t((addr & 0x3FFFF) >> 4);
+  d |= std::uint64_t(1) << 16;
+  d |= std::uint64_t(256 >> 4) << 32;
+  d |= std::uint64_t(1) << 46;
+  d |= std::uint64_t(6) << 61;                     // 32-byte swizzle
+  return d;
+}
+
 // Instruction descriptor, kind::tf32: D = F32, A = B = TF32, both K-major.
 __host__ __device__ constexpr std::uint32_t idesc_tf32(int m, int n, bool negate_a) {
   return (1u << 4) | (2u << 7) | (2u << 10) | (negate_a ? (1u << 13) : 0u) |

@@ -9,9 +9,10 @@
 // (hi*hi + hi*lo + lo*hi) and the complex product uses four real products:
 //   C_re = Ar Br - Ai Bi,   C_im = Ar Bi + Ai Br,
 // i.e. 12 TF32 MMAs per k-step. The minus sign is the instruction
-// descriptor's negate-A bit. The 3xFP16 kind (below) instead keeps a
-// negated copy of Bt's imaginary planes so that one N = 256 MMA yields C_re
-// and C_im side by side: 6 MMAs per k-step, each twice as large.
+// descriptor's negate-A bit (BF16x3, the 3xTF32 CTA pair). The 3xTF32 and
+// 3xFP16 kinds keep a negated copy of Bt's imaginary planes so that one
+// N = 256 MMA yields C_re and C_im side by side: 6 MMAs per k-step, each twice
+// as large.
 //
 // Accumulation. The tensor core accumulates in FP32 but rounds toward zero,
 // so a long sum in one TMEM accumulator drifts in proportion to the number
@@ -24,9 +25,9 @@
 // Kernel structure (persistent, one CTA per SM taking 128 x 128 complex
 // output tiles in turn, 320 threads):
 //   warp 0      TMA producer: 4-D boxes bring one k-step of the operands'
-//               planes per stage (3xTF32 / BF16x3: all planes of a row in
-//               one 128-byte row; 3xFP16: A's 128-byte rows and three
-//               blocks of 64-byte B rows, see umma_f16_kstep)
+//               planes per stage (BF16x3: all planes of a row in one
+//               128-byte row; else A's 128-byte rows and three blocks of
+//               64-byte B rows, see umma_kstep)
 //   warp 1      TMEM allocation and the single MMA-issuing thread, whose
 //               instruction stream paces the tensor core: its loops count
 //               stages and chunks instead of dividing, and a barrier test
@@ -62,7 +63,7 @@ constexpr int STAGES = 5;
 constexpr int TILE_A = BM * 128;
 constexpr int TILE_B = BN * 128;
 constexpr int STAGE_BYTES = TILE_A + TILE_B;
-// 3xFP16 stage: 40 KB of five 8 KB blocks, one k-step: A's 128 rows of 128
+// 3xFP16 and 3xTF32 stage: 40 KB of five 8 KB blocks, one k-step: A's 128 rows of 128
 // bytes (re hi, lo, im hi, lo; 128-byte swizzle) fill the first two, then B
 // rows of 64 bytes (hi, lo; 64-byte swizzle) of -im, re and im. (The CTA
 // pair loads A's re and im halves as separate 64-byte blocks instead.)
@@ -85,33 +86,39 @@ constexpr int DEEP_SMEM_BYTES = DEEP_STAGES * F16_STAGE_BYTES + DEEP_STAGING_BYT
 constexpr int WIDE_EPI_WARPS = 16;
 constexpr int WIDE_THREADS = 64 + 32 * WIDE_EPI_WARPS;
 
-// One k-step of the 3xFP16 product (six M = 128, N = 256 MMAs, small terms
-// first) in one instruction block. The stage is A's 16 KB block of 128-byte
-// rows (re hi, lo, im hi, lo; 128-byte swizzle, high descriptor word `hia`)
-// and B's 8 KB blocks of 64-byte rows (-im, re, im; 64-byte swizzle, `hib`).
-// The low descriptor words differ from `lo` (A re hi) by fixed offsets in
-// 16-byte units: A re lo +2, A im hi +4, lo +6; B -im +1024, +1026, B re
-// +1536, +1538. `acc` = 0 starts the accumulator.
-__device__ __forceinline__ void umma_f16_kstep(std::uint32_t d, std::uint32_t lo, std::uint32_t hia,
-                                               std::uint32_t hib, std::uint32_t idesc, std::uint32_t acc,
-                                               std::uint32_t bstep = 512) {
-  // bstep: distance from the -Bi block to the Br block in 16-byte units
-  // (rows of the tile x 64 bytes / 16).
-  asm volatile(
-      "{\n .reg .pred p0, p1;\n .reg .b32 l1, l2, l3, l4, l5, l6, l7;\n"
-      " .reg .b64 arh, arl, aih, ail, b2h, b2l, b1h, b1l;\n"
-      " setp.ne.b32 p0, %5, 0;\n setp.eq.b32 p1, %5, %5;\n"
-      " add.u32 l1, %1, 2;\n add.u32 l2, %1, 4;\n add.u32 l3, %1, 6;\n add.u32 l4, %1, 1024;\n"
-      " add.u32 l5, %1, 1026;\n add.u32 l6, l4, %6;\n add.u32 l7, l6, 2;\n"
-      " mov.b64 arh, {%1, %2};\n mov.b64 arl, {l1, %2};\n mov.b64 aih, {l2, %2};\n mov.b64 ail, {l3, %2};\n"
-      " mov.b64 b2h, {l4, %3};\n mov.b64 b2l, {l5, %3};\n mov.b64 b1h, {l6, %3};\n mov.b64 b1l, {l7, %3};\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], arh, b1l, %4, p0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], arl, b1h, %4, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], aih, b2l, %4, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], ail, b2h, %4, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], arh, b1h, %4, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], aih, b2h, %4, p1;\n}\n" ::"r"(d),
-      "r"(lo), "r"(hia), "r"(hib), "r"(idesc), "r"(acc), "r"(bstep));
+// One k-step of the 3xFP16 or 3xTF32 product (six M = 128, N = 256 MMAs, small
+// terms first) in one instruction block. The stage is A's 16 KB block of
+// 128-byte rows (re hi, lo, im hi, lo; 128-byte swizzle, high descriptor word
+// `hia`) and B's 8 KB blocks of 64-byte rows (-im, re, im; 64-byte swizzle,
+// `hib`). The low descriptor words differ from `lo` (A re hi) by fixed offsets
+// in 16-byte units: A re lo +2, A im hi +4, lo +6; B -im +1024, +1026, B re
+// `bstep` (rows of the tile x 64 bytes / 16) further. `acc` = 0 starts the
+// accumulator. N = 256 matters twice: an MMA of N = 128 reads 8 KB of shared
+// memory in the time that it takes, all there is, one of N = 256 12 KB in
+// twice the time.
+#define QFX_KSTEP(KIND_)                                                                                              \
+  asm volatile(                                                                                                       \
+      "{\n .reg .pred p0, p1;\n .reg .b32 l1, l2, l3, l4, l5, l6, l7;\n"                                              \
+      " .reg .b64 arh, arl, aih, ail, b2h, b2l, b1h, b1l;\n"                                                          \
+      " setp.ne.b32 p0, %5, 0;\n setp.eq.b32 p1, %5, %5;\n"                                                           \
+      " add.u32 l1, %1, 2;\n add.u32 l2, %1, 4;\n add.u32 l3, %1, 6;\n add.u32 l4, %1, 1024;\n"                       \
+      " add.u32 l5, %1, 1026;\n add.u32 l6, l4, %6;\n add.u32 l7, l6, 2;\n"                                           \
+      " mov.b64 arh, {%1, %2};\n mov.b64 arl, {l1, %2};\n mov.b64 aih, {l2, %2};\n mov.b64 ail, {l3, %2};\n"          \
+      " mov.b64 b2h, {l4, %3};\n mov.b64 b2l, {l5, %3};\n mov.b64 b1h, {l6, %3};\n mov.b64 b1l, {l7, %3};\n"          \
+      " tcgen05.mma.cta_group::1.kind::" KIND_ " [%0], arh, b1l, %4, p0;\n"                                           \
+      " tcgen05.mma.cta_group::1.kind::" KIND_ " [%0], arl, b1h, %4, p1;\n"                                           \
+      " tcgen05.mma.cta_group::1.kind::" KIND_ " [%0], aih, b2l, %4, p1;\n"                                           \
+      " tcgen05.mma.cta_group::1.kind::" KIND_ " [%0], ail, b2h, %4, p1;\n"                                           \
+      " tcgen05.mma.cta_group::1.kind::" KIND_ " [%0], arh, b1h, %4, p1;\n"                                           \
+      " tcgen05.mma.cta_group::1.kind::" KIND_ " [%0], aih, b2h, %4, p1;\n}\n" ::"r"(d),                              \
+      "r"(lo), "r"(hia), "r"(hib), "r"(idesc), "r"(acc), "r"(bstep))
+template <int KIND>
+__device__ __forceinline__ void umma_kstep(std::uint32_t d, std::uint32_t lo, std::uint32_t hia, std::uint32_t hib,
+                                           std::uint32_t idesc, std::uint32_t acc, std::uint32_t bstep) {
+  if constexpr (KIND == KIND_TF32)
+    QFX_KSTEP("tf32");
+  else
+    QFX_KSTEP("f16");
 }
 
 template <int KIND>
@@ -228,9 +235,9 @@ __device__ __forceinline__ void umma_f16_pair(std::uint32_t d_tmem, std::uint64_
 // (value = plane value * 2^-e) per row, or for A with a_blocks > 0 per 32
 // values of a row (a_blocks = k / 32 per row; then every TMEM chunk, which
 // lies inside one block, is scaled as it is added); the epilogue removes
-// them. KIND_BF16 operands have
-// six planes per k-step: b0, b1 of re and im in a 128-byte row (map_a /
-// map_b) and b2 of re and im in a 64-byte row (map_a2 / map_b2).
+// them. KIND_BF16 operands have six planes per k-step: b0, b1 of re and im
+// (map_a whole 128-byte rows, map_b 64-byte halves) and b2 of re and im
+// (map_a2 whole 64-byte rows, map_b2 32-byte halves).
 //
 // PAIR (3xFP16 only; a cluster of two CTAs, cta_group::2): a tile is 256
 // rows x 128 complex columns. CTA r holds rows m0 + 128 r .. + 127 of A and
@@ -266,11 +273,12 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
   constexpr int KSTEP = KIND == KIND_TF32 ? 8 : 16;  // k values per plane row of 32 bytes
   constexpr int TAIL = BM * 64;                       // BF16 third-piece tile of one operand
   constexpr bool NARROW = TBN != BN;
-  constexpr int NST = KIND == KIND_BF16 ? 3 : (KIND == KIND_FP16 ? (PAIR || DEEP || NARROW ? 5 : 4) : STAGES);
+  constexpr int NST = KIND == KIND_BF16 ? 3 : (PAIR || DEEP || NARROW ? 5 : 4);
   constexpr int F16_BBLOCK = TBN * 64;  // one B block: TBN rows of 64 bytes
-  constexpr int SBYTES = KIND == KIND_BF16   ? 2 * (TILE_A + TAIL)
-                         : KIND == KIND_FP16 ? (PAIR ? 4 * F16_BLOCK : 2 * F16_BLOCK + 3 * F16_BBLOCK)
-                                             : STAGE_BYTES;
+  constexpr int SBYTES = KIND == KIND_BF16 ? 2 * (TILE_A + TAIL)
+                                           : (PAIR ? 4 * F16_BLOCK : 2 * F16_BLOCK + 3 * F16_BBLOCK);
+  // x coordinate of B's re, im and -im blocks (hi and lo: 64 bytes each).
+  constexpr int BX = KIND == KIND_TF32 ? 16 : 32;
   constexpr int NBUF = TMEM_COLS / (2 * TBN);  // TMEM chunk buffers of (re, im)
   static_assert(!NARROW || (TBN == 64 && KIND == KIND_FP16 && !PAIR && !DEEP && EPI == EPI_WARPS),
                 "the narrow tile is a single-CTA 3xFP16 kernel");
@@ -384,20 +392,21 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
           tma_load_4d_pair(map_b, bar, st + 3 * F16_BLOCK, rank ? 0 : 64, n0, kb, batch);
         } else {
           mbar_expect_tx(&full[s], SBYTES);
-          if constexpr (KIND == KIND_FP16) {
-            // A: one box of whole 128-byte rows (16 KB); B: planes x = 64
-            // (-im), 0 (re) and 32 (im), hi and lo each.
+          if constexpr (KIND != KIND_BF16) {
+            // A: one box of whole 128-byte rows (16 KB); B: -im, re and im,
+            // hi and lo each.
             tma_load_4d(map_a, &full[s], st, 0, m0, kb, batch);
-            tma_load_4d(map_b, &full[s], st + 2 * F16_BLOCK, 64, n0, kb, batch);
+            tma_load_4d(map_b, &full[s], st + 2 * F16_BLOCK, 2 * BX, n0, kb, batch);
             tma_load_4d(map_b, &full[s], st + 2 * F16_BLOCK + F16_BBLOCK, 0, n0, kb, batch);
-            tma_load_4d(map_b, &full[s], st + 2 * F16_BLOCK + 2 * F16_BBLOCK, 32, n0, kb, batch);
+            tma_load_4d(map_b, &full[s], st + 2 * F16_BLOCK + 2 * F16_BBLOCK, BX, n0, kb, batch);
           } else {
+            std::uint8_t* bt = st + TILE_A + TAIL;  // re rows, im rows, re2 rows, im2 rows
             tma_load_4d(map_a, &full[s], st, 0, m0, kb, batch);
-            tma_load_4d(map_b, &full[s], st + TILE_A, 0, n0, kb, batch);
-          }
-          if constexpr (KIND == KIND_BF16) {
-            tma_load_4d(map_a2, &full[s], st + 2 * TILE_A, 0, m0, kb, batch);
-            tma_load_4d(map_b2, &full[s], st + 2 * TILE_A + TAIL, 0, n0, kb, batch);
+            tma_load_4d(map_a2, &full[s], st + TILE_A, 0, m0, kb, batch);
+            tma_load_4d(map_b, &full[s], bt, 0, n0, kb, batch);
+            tma_load_4d(map_b, &full[s], bt + BN * 64, 32, n0, kb, batch);
+            tma_load_4d(map_b2, &full[s], bt + BN * 128, 0, n0, kb, batch);
+            tma_load_4d(map_b2, &full[s], bt + BN * 160, 16, n0, kb, batch);
           }
         }
         ++g;
@@ -429,7 +438,7 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
     // FP32 registers and free it.
     const std::uint32_t idp = idesc_kind<KIND>(BM, TBN, false), idn = idesc_kind<KIND>(BM, TBN, true);
     // 3xFP16: descriptor of stage 0's A re hi plane; the stage's others
-    // follow at fixed offsets (umma_f16_kstep), stage s at + s SBYTES / 16.
+    // follow at fixed offsets (umma_kstep), stage s at + s SBYTES / 16.
     const std::uint64_t f16d0 = smem_desc_sw128(smem_u32(smem));
     const std::uint32_t f16_hia = std::uint32_t(f16d0 >> 32);
     const std::uint32_t f16_hib = std::uint32_t(smem_desc_sw64(smem_u32(smem)) >> 32);
@@ -484,7 +493,7 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
             umma_f16_pair(d_re, arh, b1h, idw, 1);
             umma_f16_pair(d_re, aih, b2h, idw, 1);
             (void)d_im;
-          } else if constexpr (KIND == KIND_FP16) {
+          } else if constexpr (KIND != KIND_BF16) {
             // One M = 128, N = 256 product gives C_re (columns 0..127) and
             // C_im (128..255) together: Ar against the B rows (Br; Bi) and Ai
             // against (-Bi; Br), both read from the stage's B blocks
@@ -492,65 +501,43 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
             // Stage s's descriptors: stage 0's with the start address moved
             // by s * SBYTES (the 14-bit field cannot carry: shared memory is
             // below 256 KB).
-            umma_f16_kstep(d_re, f16_lo, f16_hia, f16_hib, idesc_f16(BM, 2 * TBN, false), acc, F16_BBLOCK / 16);
+            umma_kstep<KIND>(d_re, f16_lo, f16_hia, f16_hib, idesc_kind<KIND>(BM, 2 * TBN, false), acc,
+                             F16_BBLOCK / 16);
             (void)d_im;
           } else {
-            const std::uint32_t b0 = a0 + TILE_A;
-            const std::uint64_t arh = smem_desc_sw128(a0), arl = smem_desc_sw128(a0 + 32),
-                                aih = smem_desc_sw128(a0 + 64), ail = smem_desc_sw128(a0 + 96);
-            const std::uint64_t brh = smem_desc_sw128(b0), brl = smem_desc_sw128(b0 + 32),
-                                bih = smem_desc_sw128(b0 + 64), bil = smem_desc_sw128(b0 + 96);
-            if constexpr (KIND == KIND_BF16) {
-              // Pieces 0 and 1 sit in the 128-byte rows (re0 re1 im0 im1, named
-              // *h and *l above), piece 2 in the 64-byte rows (re2 im2). Per real
-              // product x*y the terms x2y0, x1y1, x0y2 (~2^-16), x1y0, x0y1
-              // (~2^-8) and x0y0, smallest first.
-              const std::uint32_t at = a0 + 2 * TILE_A, bt = at + TAIL;
-              const std::uint64_t ar2 = smem_desc_sw64(at), ai2 = smem_desc_sw64(at + 32);
-              const std::uint64_t br2 = smem_desc_sw64(bt), bi2 = smem_desc_sw64(bt + 32);
-              // C_re = Ar Br - Ai Bi
-              umma<KIND>(d_re, ar2, brh, idp, acc);
-              umma<KIND>(d_re, arl, brl, idp, 1);
-              umma<KIND>(d_re, arh, br2, idp, 1);
-              umma<KIND>(d_re, ai2, bih, idn, 1);
-              umma<KIND>(d_re, ail, bil, idn, 1);
-              umma<KIND>(d_re, aih, bi2, idn, 1);
-              umma<KIND>(d_re, arl, brh, idp, 1);
-              umma<KIND>(d_re, arh, brl, idp, 1);
-              umma<KIND>(d_re, ail, bih, idn, 1);
-              umma<KIND>(d_re, aih, bil, idn, 1);
-              umma<KIND>(d_re, arh, brh, idp, 1);
-              umma<KIND>(d_re, aih, bih, idn, 1);
-              // C_im = Ar Bi + Ai Br
-              umma<KIND>(d_im, ar2, bih, idp, acc);
-              umma<KIND>(d_im, arl, bil, idp, 1);
-              umma<KIND>(d_im, arh, bi2, idp, 1);
-              umma<KIND>(d_im, ai2, brh, idp, 1);
-              umma<KIND>(d_im, ail, brl, idp, 1);
-              umma<KIND>(d_im, aih, br2, idp, 1);
-              umma<KIND>(d_im, arl, bih, idp, 1);
-              umma<KIND>(d_im, arh, bil, idp, 1);
-              umma<KIND>(d_im, ail, brh, idp, 1);
-              umma<KIND>(d_im, aih, brl, idp, 1);
-              umma<KIND>(d_im, arh, bih, idp, 1);
-              umma<KIND>(d_im, aih, brh, idp, 1);
-            } else {
-              // The small hi*lo terms go first and the two large hi*hi terms
-              // last, so only those two additions round against a large
-              // accumulator.
-              umma<KIND>(d_re, arh, brl, idp, acc);
-              umma<KIND>(d_re, arl, brh, idp, 1);
-              umma<KIND>(d_re, aih, bil, idn, 1);
-              umma<KIND>(d_re, ail, bih, idn, 1);
-              umma<KIND>(d_re, arh, brh, idp, 1);
-              umma<KIND>(d_re, aih, bih, idn, 1);
-              umma<KIND>(d_im, arh, bil, idp, acc);
-              umma<KIND>(d_im, arl, bih, idp, 1);
-              umma<KIND>(d_im, aih, brl, idp, 1);
-              umma<KIND>(d_im, ail, brh, idp, 1);
-              umma<KIND>(d_im, arh, bih, idp, 1);
-              umma<KIND>(d_im, aih, brh, idp, 1);
-            }
+            // BF16x3. Pieces 0 and 1 of A sit in 128-byte rows (re0 re1 im0 im1),
+            // piece 2 in 64-byte rows (re2 im2); B's re rows and im rows lie one
+            // block after the other, 64-byte rows of pieces 0 and 1 and 32-byte
+            // rows of piece 2, so that Ar multiplies (Br; Bi) in MMAs of N = 256.
+            // Ai takes two of N = 128, -Ai Bi (the descriptor's negate-A bit) and
+            // Ai Br. Per real product x y the terms x2 y0, x1 y1, x0 y2 (~2^-16),
+            // x1 y0, x0 y1 (~2^-8) and x0 y0, smallest first. (24 MMAs of N = 128
+            // read 192 KB of shared memory per k-step, these 168.)
+            const std::uint32_t idw = idesc_kind<KIND>(BM, 2 * TBN, false);
+            const std::uint32_t at = a0 + TILE_A, br = at + TAIL, bi = br + BN * 64, br2_ = bi + BN * 64;
+            const std::uint64_t ar0 = smem_desc_sw128(a0), ar1 = smem_desc_sw128(a0 + 32),
+                                ai0 = smem_desc_sw128(a0 + 64), ai1 = smem_desc_sw128(a0 + 96);
+            const std::uint64_t ar2 = smem_desc_sw64(at), ai2 = smem_desc_sw64(at + 32);
+            const std::uint64_t br0 = smem_desc_sw64(br), br1 = smem_desc_sw64(br + 32);
+            const std::uint64_t bi0 = smem_desc_sw64(bi), bi1 = smem_desc_sw64(bi + 32);
+            const std::uint64_t br2 = smem_desc_sw32(br2_), bi2 = smem_desc_sw32(br2_ + BN * 32);
+            auto wide = [&](std::uint64_t x, std::uint64_t y, std::uint32_t on) { umma<KIND>(d_re, x, y, idw, on); };
+            auto both = [&](std::uint64_t x, std::uint64_t yr, std::uint64_t yi) {
+              umma<KIND>(d_re, x, yi, idn, 1);
+              umma<KIND>(d_im, x, yr, idp, 1);
+            };
+            wide(ar2, br0, acc);
+            wide(ar1, br1, 1);
+            wide(ar0, br2, 1);
+            both(ai2, br0, bi0);
+            both(ai1, br1, bi1);
+            both(ai0, br2, bi2);
+            wide(ar1, br0, 1);
+            wide(ar0, br1, 1);
+            both(ai1, br0, bi0);
+            both(ai0, br1, bi1);
+            wide(ar0, br0, 1);
+            both(ai0, br0, bi0);
           }
           commit(&empty[s]);
           if (chunk_end) commit(&acc_full[buf]);
@@ -1085,16 +1072,17 @@ struct RowReader {
 };
 
 // Output layout per batch entry: [k / 8][row][plane][8] fp32 with planes
-// re_hi, re_lo, im_hi, im_lo; k is padded to a multiple of 8 with zeros.
+// re_hi, re_lo, im_hi, im_lo and with nplanes = 6 also -im_hi, -im_lo; k is
+// padded to a multiple of 8 with zeros.
 // k-step-major, so the 128 rows of one k-step that a tile loads are one
 // contiguous 16 KB block. One warp per row; lane j covers k = 2j, 2j + 1 of
 // every 64.
 __global__ void __launch_bounds__(256) split_tf32_kernel(const float2* __restrict__ src, float* __restrict__ planes,
                                                          std::uint64_t rows, std::uint64_t k, std::uint64_t kpad,
-                                                         std::uint64_t src_batch_stride) {
+                                                         std::uint64_t src_batch_stride, int nplanes) {
   const std::uint64_t b = blockIdx.y;
   const float2* sb = src + b * src_batch_stride;
-  float* pb = planes + b * 4 * rows * kpad;
+  float* pb = planes + b * nplanes * rows * kpad;
   const int lane = threadIdx.x % 32;
   const std::uint64_t warps = std::uint64_t(gridDim.x) * (blockDim.x / 32);
   for (std::uint64_t row = (std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; row < rows; row += warps) {
@@ -1104,11 +1092,16 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float2* __restric
       float2 v0, v1;
       rd.pair(kk, v0, v1);
       const float rh0 = tf32_rn(v0.x), ih0 = tf32_rn(v0.y), rh1 = tf32_rn(v1.x), ih1 = tf32_rn(v1.y);
-      float* o = pb + ((kk / 8) * rows + row) * 32 + (kk % 8);
+      const float il0 = tf32_rn(v0.y - ih0), il1 = tf32_rn(v1.y - ih1);
+      float* o = pb + ((kk / 8) * rows + row) * (8 * nplanes) + (kk % 8);
       *reinterpret_cast<float2*>(o) = make_float2(rh0, rh1);
       *reinterpret_cast<float2*>(o + 8) = make_float2(tf32_rn(v0.x - rh0), tf32_rn(v1.x - rh1));
       *reinterpret_cast<float2*>(o + 16) = make_float2(ih0, ih1);
-      *reinterpret_cast<float2*>(o + 24) = make_float2(tf32_rn(v0.y - ih0), tf32_rn(v1.y - ih1));
+      *reinterpret_cast<float2*>(o + 24) = make_float2(il0, il1);
+      if (nplanes == 6) {
+        *reinterpret_cast<float2*>(o + 32) = make_float2(-ih0, -ih1);
+        *reinterpret_cast<float2*>(o + 40) = make_float2(-il0, -il1);
+      }
     }
   }
 }
@@ -1228,18 +1221,22 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// 4-D map over split planes laid out [batch][kpad / 8][rows][32] (fp32),
-// box {32, box_rows, 1, 1} (one 128-byte row per tile row), 128-byte swizzle.
-CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows) {
+// 4-D map over split planes laid out [batch][kpad / 8][rows][row_floats] (32:
+// re hi, lo, im hi, lo; 48: also -im hi, lo). Box {32, box_rows, 1, 1}: whole
+// 128-byte rows, 128-byte swizzle; or with box_inner = 16 the hi and lo planes
+// of one part as 64-byte rows, 64-byte swizzle.
+CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
+                      int row_floats = 32, int box_inner = 32) {
   CUtensorMap map;
   std::memset(&map, 0, sizeof(map));
-  const std::uint64_t kb = kpad / 8;
-  const cuuint64_t dims[4] = {32, rows, kb, (cuuint64_t)batch};
-  const cuuint64_t strides[3] = {128, rows * 128, kb * rows * 128};
-  const cuuint32_t box[4] = {32, (cuuint32_t)box_rows, 1, 1};
+  const std::uint64_t kb = kpad / 8, rb = std::uint64_t(row_floats) * 4;
+  const cuuint64_t dims[4] = {(cuuint64_t)row_floats, rows, kb, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
+  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides,
-                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
@@ -1247,21 +1244,23 @@ CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad,
   return map;
 }
 
-// 4-D map over BF16 planes laid out [batch][kpad / 16][rows][inner] with
-// `inner` 64 (128-byte rows, 128-byte swizzle) or 32 (64-byte rows, 64-byte
-// swizzle); box {inner, box_rows, 1, 1}.
+// 4-D map over BF16 planes laid out [batch][kpad / 16][rows][inner]; box
+// {box_inner, box_rows, 1, 1}: rows of 128, 64 or 32 bytes in the swizzle of
+// that width.
 CUtensorMap plane_map_bf16(const __nv_bfloat16* base, std::uint64_t rows, std::uint64_t kpad, int batch,
-                           int box_rows, int inner) {
+                           int box_rows, int inner, int box_inner) {
   CUtensorMap map;
   std::memset(&map, 0, sizeof(map));
   const std::uint64_t kb = kpad / 16, rb = std::uint64_t(inner) * 2;
   const cuuint64_t dims[4] = {(cuuint64_t)inner, rows, kb, (cuuint64_t)batch};
   const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
-  const cuuint32_t box[4] = {(cuuint32_t)inner, (cuuint32_t)box_rows, 1, 1};
+  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(base), dims,
                            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           box_inner == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                           : box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                             : CU_TENSOR_MAP_SWIZZLE_32B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
@@ -1334,10 +1333,10 @@ bool tc_eligible(std::size_t m, std::size_t n, std::size_t k) {
 }
 
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k) {
-  // The largest of the 3xTF32 planes (4 fp32 per element), the 3xFP16
-  // planes (4 fp16 per element of A, 6 of Bt) plus their exponents and the BF16x3
+  // The largest of the 3xTF32 planes (4 fp32 per element of A, 6 of Bt), the
+  // 3xFP16 planes (4 fp16 per element of A, 6 of Bt) plus their exponents and the BF16x3
   // planes (6 bf16 per element, fewer than the 3xTF32 ones).
-  const std::size_t tf32 = 4 * (m + n) * ((k + 7) / 8 * 8);
+  const std::size_t tf32 = (4 * m + 6 * n) * ((k + 7) / 8 * 8);
   const std::size_t fp16 = (2 * m + 3 * n) * ((k + 15) / 16 * 16) + (m + n) + m * ((k + 31) / 32) + 64;
   return tf32 > fp16 ? tf32 : fp16;
 }
@@ -1400,9 +1399,9 @@ void launch_cgemm_tf32x3(const float2* A, const float2* Bt, float2* C, std::size
   float* pb = workspace + 4 * m * kpad * (std::size_t)batch;
   {
     dim3 ga((unsigned)std::min<std::uint64_t>((m + 7) / 8, 152 * 16), (unsigned)batch);
-    split_tf32_kernel<<<ga, 256, 0, s>>>(A, pa, m, k, kpad, batch_stride);
+    split_tf32_kernel<<<ga, 256, 0, s>>>(A, pa, m, k, kpad, batch_stride, 4);
     dim3 gb((unsigned)std::min<std::uint64_t>((n + 7) / 8, 152 * 16), (unsigned)batch);
-    split_tf32_kernel<<<gb, 256, 0, s>>>(Bt, pb, n, k, kpad, bt_stride);
+    split_tf32_kernel<<<gb, 256, 0, s>>>(Bt, pb, n, k, kpad, bt_stride, use_pair ? 4 : 6);
     check(cudaGetLastError(), "split_tf32");
   }
   if (use_pair) {
@@ -1416,7 +1415,7 @@ void launch_cgemm_tf32x3(const float2* A, const float2* Bt, float2* C, std::size
     return;
   }
   const CUtensorMap ma = plane_map(pa, m, kpad, batch, BM);
-  const CUtensorMap mb = plane_map(pb, n, kpad, batch, BN);
+  const CUtensorMap mb = plane_map(pb, n, kpad, batch, BN, 48, 16);
   const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
   dim3 grid(persistent_grid(tiles * (std::size_t)batch), 1, 1);
   CUtensorMap mc;
@@ -1562,10 +1561,10 @@ void launch_cgemm_bf16x3(const float2* A, const float2* Bt, float2* C, std::size
     split_bf16_kernel<<<gb, 256, 0, s>>>(Bt, bm, bt, n, k, kpad, bt_stride);
     check(cudaGetLastError(), "split_bf16");
   }
-  const CUtensorMap ma = plane_map_bf16(am, m, kpad, batch, BM, 64);
-  const CUtensorMap mb = plane_map_bf16(bm, n, kpad, batch, BN, 64);
-  const CUtensorMap ma2 = plane_map_bf16(at, m, kpad, batch, BM, 32);
-  const CUtensorMap mb2 = plane_map_bf16(bt, n, kpad, batch, BN, 32);
+  const CUtensorMap ma = plane_map_bf16(am, m, kpad, batch, BM, 64, 64);
+  const CUtensorMap mb = plane_map_bf16(bm, n, kpad, batch, BN, 64, 32);
+  const CUtensorMap ma2 = plane_map_bf16(at, m, kpad, batch, BM, 32, 32);
+  const CUtensorMap mb2 = plane_map_bf16(bt, n, kpad, batch, BN, 32, 16);
   const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
   dim3 grid(persistent_grid(tiles * (std::size_t)batch), 1, 1);
   CUtensorMap mc;

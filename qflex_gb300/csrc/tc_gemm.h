@@ -11,7 +11,7 @@ namespace qfx {
 // Shapes the tensor-core kernel takes (k a multiple of 4 for the TMA row
 // stride; smaller products stay on the CUDA-core kernels).
 bool tc_eligible(std::size_t m, std::size_t n, std::size_t k);
-// fp32 elements of split planes one batch entry needs (A and B, 4 planes).
+// fp32 elements of split planes one batch entry needs (A and B of any split kind).
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k);
 
 // Kernel choice of one product.
