@@ -60,6 +60,7 @@ struct Engine::Plan {
   unsigned fuse_version = ~0u;
   int precision = -1;          // precision the program was planned for
   std::size_t tc_ws_elems = 0; // split-plane workspace of one batch entry
+  unsigned ws_version = ~0u;   // options it was computed for
   std::uint32_t max_size_log2 = 0;
   ColumnDesc* d_cols = nullptr;
   StepDesc* d_steps = nullptr;
@@ -206,21 +207,26 @@ bool Engine::direct_product(std::size_t n, const TcConfig& cfg) const {
   return precision_ == FP16X3 && cfg.variant == 0 && cfg.chunk <= 2 && n <= 1024;
 }
 
-void Engine::launch_split_product(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                                  std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch,
-                                  float* ws) {
+std::size_t Engine::workspace_elems(std::size_t m, std::size_t n, std::size_t k) const {
+  return direct_product(n, tc_config(m, n, k)) ? tc_direct_workspace_elems(n, k) : tc_workspace_elems(m, n, k);
+}
+
+void Engine::launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                                  std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride,
+                                  int batch, float* ws) {
   const TcConfig cfg = tc_config(m, n, k);
   if (direct_product(n, cfg)) {
     const bool aligned = (reinterpret_cast<std::uintptr_t>(A) & 15) == 0 && k % 2 == 0 &&
                          (batch == 1 || ac_stride % 2 == 0);
-    launch_cgemm_fp16x3_direct(A, make_a_rows(k, aligned), Bt, C, m, n, k, ac_stride, bt_stride, batch, ws,
+    launch_cgemm_fp16x3_direct(A, make_a_rows(k, aligned), B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws,
                                error_flag(), cfg, stream_);
-  } else if (precision_ == FP16X3)
-    launch_cgemm_fp16x3(A, Bt, C, m, n, k, ac_stride, bt_stride, batch, ws, error_flag(), cfg, stream_);
-  else if (precision_ == BF16X3)
-    launch_cgemm_bf16x3(A, Bt, C, m, n, k, ac_stride, bt_stride, batch, ws, error_flag(), cfg, stream_);
-  else
-    launch_cgemm_tf32x3(A, Bt, C, m, n, k, ac_stride, bt_stride, batch, ws, error_flag(), cfg, stream_);
+  } else if (precision_ == FP16X3) {
+    launch_cgemm_fp16x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
+  } else if (precision_ == BF16X3) {
+    launch_cgemm_bf16x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
+  } else {
+    launch_cgemm_tf32x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
+  }
 }
 
 TcConfig Engine::tc_config(std::size_t m, std::size_t n, std::size_t k) const {
@@ -260,30 +266,29 @@ void Engine::check_error_flag() {
   }
 }
 
+// Whether multiply runs a product on the tensor cores in a split precision:
+// the sizes that contractions have (n and k powers of two), and any others
+// with at least 96 terms, where every split precision is as accurate as FP32
+// sums or more so. Relative RMS errors against complex128 products of
+// Gaussian operands, (1000, 256, k), FP32 / 3xFP16 / 3xTF32 / BF16x3:
+// k = 64 2.0 / 1.6 / 1.5 / 2.3e-7, 128 2.9 / 1.7 / 1.6 / 2.3e-7,
+// 1024 8.1 / 1.9 / 2.1 / 2.5e-7. (3001, 690, 1100) in 3xFP16: 424 -> 65 us.
+bool Engine::split_multiply(std::size_t m, std::size_t n, std::size_t k) const {
+  if (m >= 64 && n >= 64 && k >= 96 && tc_runs(m, n, k)) return true;
+  return tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
+}
+
 void Engine::multiply(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n,
                       std::size_t k, std::uint64_t stride, int batch) {
   if (is_complex128(precision_))
     throw QFX_ERR("The complex64 tensor operations need a complex64 precision mode (this context is complex128).");
-  if (precision_ != FP32 && tc_eligible(m, n, k)) {
-    // The tensor-core kernel reads B as [n][k]: transpose into the front of
-    // the workspace, split planes after it.
-    const std::size_t bt = ((n * k * (std::size_t)batch + 63) / 64) * 64;
-    float* ws = tc_workspace(2 * bt + tc_workspace_elems(m, n, k) * (std::size_t)batch);
-    float2* Bt = reinterpret_cast<float2*>(ws);
-    int nbits = 0;
-    std::uint8_t perm[40] = {};
-    int ln = 0, lk = 0;
-    while ((std::size_t(1) << ln) < n) ++ln;
-    while ((std::size_t(1) << lk) < k) ++lk;
-    if ((std::size_t(1) << ln) == n && (std::size_t(1) << lk) == k) {
-      nbits = ln + lk;
-      for (int b = 0; b < ln; ++b) perm[b] = (std::uint8_t)(lk + b);   // n digits move up
-      for (int b = 0; b < lk; ++b) perm[ln + b] = (std::uint8_t)b;     // k digits move down
-      PermPlan plan;
-      make_perm_plan(nbits, perm, &plan);
-      for (int b = 0; b < batch; ++b)
-        launch_permute(plan, B + (std::size_t)b * stride, Bt + (std::size_t)b * n * k, 0, 1, stream_);
-      launch_split_product(A, Bt, C, m, n, k, stride, n * k, batch, ws + 2 * bt);
+  if (precision_ != FP32 && split_multiply(m, n, k)) {
+    const std::size_t bytes = workspace_elems(m, n, k) * (std::size_t)batch * sizeof(float);
+    // A product that FP32 can run as well needs no more memory than that.
+    const bool contraction = tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
+    if (contraction || fits(bytes, 4)) {
+      float* ws = tc_workspace(bytes / sizeof(float));
+      launch_split_product(A, B, BLayout::kn, C, m, n, k, stride, stride, batch, ws);
       return;
     }
   }
@@ -311,6 +316,14 @@ void* Engine::reserve(std::size_t bytes, int slot) {
     b.bytes = bytes;
   }
   return b.ptr;
+}
+
+bool Engine::fits(std::size_t bytes, int slot) const {
+  const std::size_t have = (int)bufs_.size() > slot ? bufs_[slot].bytes : 0;
+  if (have >= bytes) return true;
+  std::size_t free_b = 0, total_b = 0;
+  QFX_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  return bytes < free_b + have;
 }
 
 const std::vector<GemmShape>& Engine::last_shapes() const {
@@ -513,14 +526,14 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
       const bool a_planes = p.fused[i] == (int)i;
       const TcConfig cfg = tc_config(op.m, op.n, op.k);
       if (op.a_gather)
-        launch_cgemm_fp16x3_direct(arena + op.a, p.gather[gathered++], arena + op.b, arena + op.c, op.m, op.n, op.k,
-                                   stride, stride, batch, tc_ws, error_flag(), cfg, stream_);
+        launch_cgemm_fp16x3_direct(arena + op.a, p.gather[gathered++], arena + op.b, BLayout::nk, arena + op.c, op.m, op.n,
+                                   op.k, stride, stride, batch, tc_ws, error_flag(), cfg, stream_);
       else if (a_planes)
-        launch_cgemm_fp16x3(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, stride, batch,
-                            tc_ws, error_flag(), cfg, stream_, true);
+        launch_cgemm_fp16x3(arena + op.a, arena + op.b, BLayout::nk, arena + op.c, op.m, op.n, op.k, stride, stride,
+                            batch, tc_ws, error_flag(), cfg, stream_, true);
       else
-        launch_split_product(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, stride, batch,
-                             tc_ws);
+        launch_split_product(arena + op.a, arena + op.b, BLayout::nk, arena + op.c, op.m, op.n, op.k, stride, stride,
+                             batch, tc_ws);
       launches += a_planes || direct_product(op.n, cfg) ? 2 : 3;  // plane splits and the product
     } else if (op.a_gather) {
       launch_cgemm_tiled(arena + op.a, &p.tile_gather[tile_gathered++], arena + op.b, arena + op.c, op.m, op.n, op.k,
@@ -652,10 +665,6 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
       throw QFX_WRAP("ContractGrid", e);
     }
     p.precision = precision_;
-    p.tc_ws_elems = 0;
-    for (const auto& op : p.prog.ops)
-      if (op.kind == DevOp::GEMM && op.b_nk)
-        p.tc_ws_elems = std::max(p.tc_ws_elems, tc_workspace_elems(op.m, op.n, op.k));
     p.perm.resize(p.prog.ops.size());
     for (std::size_t i = 0; i < p.prog.ops.size(); ++i)
       if (p.prog.ops[i].kind == DevOp::PERMUTE)
@@ -709,6 +718,13 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
                                                 "). Cancelling simulation.")));
   }
 
+  if (p.ws_version != options_version_) {
+    p.tc_ws_elems = 0;
+    for (const auto& op : p.prog.ops)
+      if (op.kind == DevOp::GEMM && op.b_nk)
+        p.tc_ws_elems = std::max(p.tc_ws_elems, workspace_elems(op.m, op.n, op.k));
+    p.ws_version = options_version_;
+  }
   const Program& prog = p.prog;
   const std::size_t n_cols = p.net.columns.size();
   const std::size_t n_amps = prog.n_amplitudes;

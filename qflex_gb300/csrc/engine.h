@@ -131,9 +131,15 @@ class Engine {
   unsigned options_version_ = 0;  // part of the graph key: options change launches
   TcConfig tc_config(std::size_t m, std::size_t n, std::size_t k) const;
   bool direct_product(std::size_t n, const TcConfig& cfg) const;
-  // C = A * Bt^T on the tensor cores in the context's split precision.
-  void launch_split_product(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                            std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch, float* ws);
+  bool split_multiply(std::size_t m, std::size_t n, std::size_t k) const;
+  // fp32 elements of split planes that one product of this shape needs.
+  std::size_t workspace_elems(std::size_t m, std::size_t n, std::size_t k) const;
+  // Whether device buffer `slot` holds `bytes` or can be made to.
+  bool fits(std::size_t bytes, int slot) const;
+  // C = A * B on the tensor cores in the context's split precision.
+  void launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                            std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride, int batch,
+                            float* ws);
   std::vector<cudaEvent_t> prof_events_;
   std::vector<double> op_ms_;
   std::unique_ptr<Plan> plan_;

@@ -18,9 +18,24 @@ CUtensorMap plane_map_f16(const __half* base, std::uint64_t rows, std::uint64_t 
 bool output_map(float2* C, std::size_t m, std::size_t n, std::uint64_t batch_stride, int batch, CUtensorMap* map,
                 bool narrow = false);
 unsigned persistent_grid(std::size_t tiles);
-// FP16 planes and row exponents of `rows` x k complex64 (split_fp16_kernel).
-void launch_split_fp16(const float2* src, __half* planes, int* exps, std::size_t rows, std::size_t k,
-                       std::uint64_t src_stride, int batch, int nplanes, cudaStream_t s);
+// Operand kinds of the single-CTA kernel: 3xTF32 planes (8 values of 4
+// bytes per plane and k-step) or 3xFP16 planes (16 values of 2 bytes, rows
+// scaled by powers of two).
+// BF16x3: three BF16 pieces per value (x = b0 + b1 + b2 to ~24 bits).
+enum SplitKind : int { KIND_TF32 = 0, KIND_FP16 = 1, KIND_BF16 = 2 };
+
+// Splits `batch` operands into planes (split.cu): `rows` rows of k values, or
+// with `columns` the columns of a row-major k x rows matrix. `nplanes` 4, or 6
+// with the negated imaginary planes (not BF16). `top` holds rows * batch words
+// for 3xFP16 columns.
+struct SplitOut {
+  void* main;
+  void* tail;          // BF16x3: the third pieces
+  int* exps;           // 3xFP16: one exponent per row
+  std::uint32_t* top;
+};
+void launch_split(SplitKind kind, int nplanes, const SplitOut& out, const float2* src, std::size_t rows,
+                  std::size_t k, std::uint64_t src_stride, int batch, bool columns, cudaStream_t s);
 
 namespace {
 
@@ -189,12 +204,6 @@ __device__ __forceinline__ void umma_commit(std::uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive(std::uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-
-// Operand kinds of the single-CTA kernel: 3xTF32 planes (8 values of 4
-// bytes per plane and k-step) or 3xFP16 planes (16 values of 2 bytes, rows
-// scaled by powers of two).
-// BF16x3: three BF16 pieces per value (x = b0 + b1 + b2 to ~24 bits).
-enum SplitKind : int { KIND_TF32 = 0, KIND_FP16 = 1, KIND_BF16 = 2 };
 
 // Compensation of the truncation bias. The tensor core's FP32 accumulation
 // rounds toward zero, so every product comes out smaller by a fraction beta

@@ -812,10 +812,15 @@ void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const floa
     }
 }
 
-void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* Bt, float2* C, std::size_t m,
-                                std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride,
-                                int batch, float* workspace, int* err, const TcConfig& cfg, cudaStream_t s) {
-  if (!tc_eligible(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
+std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k) {
+  return 2 * n * ((k + 15) / 16 * 16) + 2 * n;  // B's planes, exponents and largest components
+}
+
+void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* B, BLayout b_layout, float2* C,
+                                std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
+                                std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
+                                cudaStream_t s) {
+  if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk < 1 || cfg.chunk > 2)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct product takes chunks of 1 or 2 k-steps");
   static std::once_flag attr;
@@ -826,7 +831,8 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   const std::size_t kpad = (k + 15) / 16 * 16;
   __half* pb = reinterpret_cast<__half*>(workspace);
   int* eb = reinterpret_cast<int*>(pb + 4 * n * kpad * (std::size_t)batch);
-  launch_split_fp16(Bt, pb, eb, n, k, bt_stride, batch, 4, s);
+  std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
+  launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, BN, 64);
   CUtensorMap mc;
   const int tma_c = output_map(C, m, n, ac_stride, batch, &mc, true) ? 1 : 0;

@@ -1041,171 +1041,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
   }
 }
 
-// Splits complex64 rows into the four TF32 planes (round-to-nearest).
-__device__ __forceinline__ float tf32_rn(float x) {
-  std::uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
-// Row access shared by the split kernels: one warp per row, lanes over k.
-// A row whose start is 16-byte aligned (and k even) is read as float4 pairs.
-struct RowReader {
-  const float2* r;
-  std::uint64_t k;
-  bool vec;
-  __device__ RowReader(const float2* row, std::uint64_t k_)
-      : r(row), k(k_), vec(((reinterpret_cast<std::uintptr_t>(row) & 15) == 0) && (k_ % 2 == 0)) {}
-  // Values kk and kk + 1 (kk even), zero beyond k.
-  __device__ __forceinline__ void pair(std::uint64_t kk, float2& v0, float2& v1) const {
-    if (kk >= k) {
-      v0 = v1 = make_float2(0.f, 0.f);
-    } else if (vec) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(r + kk));
-      v0 = make_float2(v.x, v.y);
-      v1 = make_float2(v.z, v.w);
-    } else {
-      v0 = r[kk];
-      v1 = kk + 1 < k ? r[kk + 1] : make_float2(0.f, 0.f);
-    }
-  }
-};
-
-// Output layout per batch entry: [k / 8][row][plane][8] fp32 with planes
-// re_hi, re_lo, im_hi, im_lo and with nplanes = 6 also -im_hi, -im_lo; k is
-// padded to a multiple of 8 with zeros.
-// k-step-major, so the 128 rows of one k-step that a tile loads are one
-// contiguous 16 KB block. One warp per row; lane j covers k = 2j, 2j + 1 of
-// every 64.
-__global__ void __launch_bounds__(256) split_tf32_kernel(const float2* __restrict__ src, float* __restrict__ planes,
-                                                         std::uint64_t rows, std::uint64_t k, std::uint64_t kpad,
-                                                         std::uint64_t src_batch_stride, int nplanes) {
-  const std::uint64_t b = blockIdx.y;
-  const float2* sb = src + b * src_batch_stride;
-  float* pb = planes + b * nplanes * rows * kpad;
-  const int lane = threadIdx.x % 32;
-  const std::uint64_t warps = std::uint64_t(gridDim.x) * (blockDim.x / 32);
-  for (std::uint64_t row = (std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; row < rows; row += warps) {
-    const RowReader rd(sb + row * k, k);
-#pragma unroll 4
-    for (std::uint64_t kk = 2 * lane; kk < kpad; kk += 64) {
-      float2 v0, v1;
-      rd.pair(kk, v0, v1);
-      const float rh0 = tf32_rn(v0.x), ih0 = tf32_rn(v0.y), rh1 = tf32_rn(v1.x), ih1 = tf32_rn(v1.y);
-      const float il0 = tf32_rn(v0.y - ih0), il1 = tf32_rn(v1.y - ih1);
-      float* o = pb + ((kk / 8) * rows + row) * (8 * nplanes) + (kk % 8);
-      *reinterpret_cast<float2*>(o) = make_float2(rh0, rh1);
-      *reinterpret_cast<float2*>(o + 8) = make_float2(tf32_rn(v0.x - rh0), tf32_rn(v1.x - rh1));
-      *reinterpret_cast<float2*>(o + 16) = make_float2(ih0, ih1);
-      *reinterpret_cast<float2*>(o + 24) = make_float2(il0, il1);
-      if (nplanes == 6) {
-        *reinterpret_cast<float2*>(o + 32) = make_float2(-ih0, -ih1);
-        *reinterpret_cast<float2*>(o + 40) = make_float2(-il0, -il1);
-      }
-    }
-  }
-}
-
-// 3xFP16 planes. One warp per row: the row's largest |re| or |im| sets a
-// power-of-two scale e with max * 2^e in [2^14, 2^15) (FP16 holds up to
-// 65504), then hi = fp16(x 2^e) and lo = fp16(x 2^e - hi) for re and im,
-// both round-to-nearest, so x 2^e = hi + lo to ~22 significant bits.
-// Output per batch entry: planes [k / 16][row][plane][16] fp16 (re_hi,
-// re_lo, im_hi, im_lo, and with nplanes = 6 also -im_hi, -im_lo; one 128- or
-// 192-byte row per k-step, k zero-padded to a multiple of 16) and the
-// exponents [row] (int).
-__global__ void __launch_bounds__(256) split_fp16_kernel(const float2* __restrict__ src, __half* __restrict__ planes,
-                                                         int* __restrict__ exps, std::uint64_t rows, std::uint64_t k,
-                                                         std::uint64_t kpad, std::uint64_t src_batch_stride,
-                                                         int nplanes) {
-  const std::uint64_t b = blockIdx.y;
-  const float2* sb = src + b * src_batch_stride;
-  __half* pb = planes + b * nplanes * rows * kpad;
-  int* eb = exps + b * rows;
-  const int lane = threadIdx.x % 32;
-  const std::uint64_t warps = std::uint64_t(gridDim.x) * (blockDim.x / 32);
-  for (std::uint64_t row = (std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; row < rows; row += warps) {
-    const RowReader rd(sb + row * k, k);
-    float mx = 0.f;
-#pragma unroll 4
-    for (std::uint64_t kk = 2 * lane; kk < k; kk += 64) {
-      float2 v0, v1;
-      rd.pair(kk, v0, v1);
-      mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v0.x), fabsf(v0.y)), fmaxf(fabsf(v1.x), fabsf(v1.y))));
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int e = 0;
-    if (mx > 0.f && isfinite(mx)) {
-      int ex;
-      frexpf(mx, &ex);  // mx in [2^(ex-1), 2^ex)
-      e = 15 - ex;
-    }
-    if (lane == 0) eb[row] = e;
-#pragma unroll 4
-    for (std::uint64_t kk = 2 * lane; kk < kpad; kk += 64) {
-      float2 v0, v1;
-      rd.pair(kk, v0, v1);
-      const float r0 = ldexpf(v0.x, e), i0 = ldexpf(v0.y, e), r1 = ldexpf(v1.x, e), i1 = ldexpf(v1.y, e);
-      const __half2 rh = __floats2half2_rn(r0, r1), ih = __floats2half2_rn(i0, i1);
-      const float2 rhf = __half22float2(rh), ihf = __half22float2(ih);
-      __half* o = pb + ((kk / 16) * rows + row) * (16 * nplanes) + (kk % 16);
-      const __half2 il = __floats2half2_rn(i0 - ihf.x, i1 - ihf.y);
-      *reinterpret_cast<__half2*>(o) = rh;
-      *reinterpret_cast<__half2*>(o + 16) = __floats2half2_rn(r0 - rhf.x, r1 - rhf.y);
-      *reinterpret_cast<__half2*>(o + 32) = ih;
-      *reinterpret_cast<__half2*>(o + 48) = il;
-      if (nplanes == 6) {
-        *reinterpret_cast<__half2*>(o + 64) = __hneg2(ih);
-        *reinterpret_cast<__half2*>(o + 80) = __hneg2(il);
-      }
-    }
-  }
-}
-
-// BF16x3 planes: x = b0 + b1 + b2 with b0 = bf16(x), b1 = bf16(x - b0),
-// b2 = bf16(x - b0 - b1), all round-to-nearest. Output per batch entry:
-// main planes [k / 16][row][64] bf16 (re0, re1, im0, im1; 128 bytes per
-// k-step) and tail planes [k / 16][row][32] bf16 (re2, im2; 64 bytes), k
-// zero-padded to a multiple of 16.
-__global__ void __launch_bounds__(256) split_bf16_kernel(const float2* __restrict__ src,
-                                                         __nv_bfloat16* __restrict__ main_planes,
-                                                         __nv_bfloat16* __restrict__ tail_planes, std::uint64_t rows,
-                                                         std::uint64_t k, std::uint64_t kpad,
-                                                         std::uint64_t src_batch_stride) {
-  const std::uint64_t b = blockIdx.y;
-  const float2* sb = src + b * src_batch_stride;
-  __nv_bfloat16* mb = main_planes + b * 4 * rows * kpad;
-  __nv_bfloat16* tb = tail_planes + b * 2 * rows * kpad;
-  const int lane = threadIdx.x % 32;
-  const std::uint64_t warps = std::uint64_t(gridDim.x) * (blockDim.x / 32);
-  for (std::uint64_t row = (std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; row < rows; row += warps) {
-    const RowReader rd(sb + row * k, k);
-#pragma unroll 4
-    for (std::uint64_t kk = 2 * lane; kk < kpad; kk += 64) {
-      float2 v0, v1;
-      rd.pair(kk, v0, v1);
-      // Pieces of (re, im) of values kk and kk + 1, two at a time.
-      const __nv_bfloat162 r0 = __floats2bfloat162_rn(v0.x, v1.x), i0 = __floats2bfloat162_rn(v0.y, v1.y);
-      const float2 r0f = __bfloat1622float2(r0), i0f = __bfloat1622float2(i0);
-      const float2 rr = make_float2(v0.x - r0f.x, v1.x - r0f.y), ir = make_float2(v0.y - i0f.x, v1.y - i0f.y);
-      const __nv_bfloat162 r1 = __floats2bfloat162_rn(rr.x, rr.y), i1 = __floats2bfloat162_rn(ir.x, ir.y);
-      const float2 r1f = __bfloat1622float2(r1), i1f = __bfloat1622float2(i1);
-      const __nv_bfloat162 r2 = __floats2bfloat162_rn(rr.x - r1f.x, rr.y - r1f.y);
-      const __nv_bfloat162 i2 = __floats2bfloat162_rn(ir.x - i1f.x, ir.y - i1f.y);
-      const std::uint64_t slot = (kk / 16) * rows + row;
-      __nv_bfloat16* m = mb + slot * 64 + (kk % 16);
-      *reinterpret_cast<__nv_bfloat162*>(m) = r0;
-      *reinterpret_cast<__nv_bfloat162*>(m + 16) = r1;
-      *reinterpret_cast<__nv_bfloat162*>(m + 32) = i0;
-      *reinterpret_cast<__nv_bfloat162*>(m + 48) = i1;
-      __nv_bfloat16* t = tb + slot * 32 + (kk % 16);
-      *reinterpret_cast<__nv_bfloat162*>(t) = r2;
-      *reinterpret_cast<__nv_bfloat162*>(t + 16) = i2;
-    }
-  }
-}
-
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
@@ -1321,11 +1156,8 @@ bool output_map(float2* C, std::size_t m, std::size_t n, std::uint64_t batch_str
                      CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-void launch_split_fp16(const float2* src, __half* planes, int* exps, std::size_t rows, std::size_t k,
-                       std::uint64_t src_stride, int batch, int nplanes, cudaStream_t s) {
-  dim3 grid((unsigned)std::min<std::uint64_t>((rows + 7) / 8, 152 * 16), (unsigned)batch);
-  split_fp16_kernel<<<grid, 256, 0, s>>>(src, planes, exps, rows, k, (k + 15) / 16 * 16, src_stride, nplanes);
-  check(cudaGetLastError(), "split_fp16");
+bool tc_runs(std::size_t m, std::size_t n, std::size_t k) {
+  return m >= 1 && n >= 1 && k >= 1 && m < (1u << 31) && n < (1u << 31) && k < (1u << 31);
 }
 
 bool tc_eligible(std::size_t m, std::size_t n, std::size_t k) {
@@ -1337,7 +1169,7 @@ std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k) {
   // 3xFP16 planes (4 fp16 per element of A, 6 of Bt) plus their exponents and the BF16x3
   // planes (6 bf16 per element, fewer than the 3xTF32 ones).
   const std::size_t tf32 = (4 * m + 6 * n) * ((k + 7) / 8 * 8);
-  const std::size_t fp16 = (2 * m + 3 * n) * ((k + 15) / 16 * 16) + (m + n) + m * ((k + 31) / 32) + 64;
+  const std::size_t fp16 = (2 * m + 3 * n) * ((k + 15) / 16 * 16) + (m + 2 * n) + m * ((k + 31) / 32) + 64;
   return tf32 > fp16 ? tf32 : fp16;
 }
 
@@ -1378,10 +1210,10 @@ TcConfig tc_default_config() {
   return c;
 }
 
-void launch_cgemm_tf32x3(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                         std::size_t k, std::uint64_t batch_stride, std::uint64_t bt_stride, int batch,
+void launch_cgemm_tf32x3(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                         std::size_t n, std::size_t k, std::uint64_t batch_stride, std::uint64_t b_stride, int batch,
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s) {
-  if (!tc_eligible(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
+  if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk < 1 || cfg.chunk > 64)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> chunk length must be 1..64");
   const int chunk = cfg.chunk;
@@ -1397,13 +1229,8 @@ void launch_cgemm_tf32x3(const float2* A, const float2* Bt, float2* C, std::size
   float* pa = workspace;
   const std::size_t kpad = (k + BK - 1) / BK * BK;
   float* pb = workspace + 4 * m * kpad * (std::size_t)batch;
-  {
-    dim3 ga((unsigned)std::min<std::uint64_t>((m + 7) / 8, 152 * 16), (unsigned)batch);
-    split_tf32_kernel<<<ga, 256, 0, s>>>(A, pa, m, k, kpad, batch_stride, 4);
-    dim3 gb((unsigned)std::min<std::uint64_t>((n + 7) / 8, 152 * 16), (unsigned)batch);
-    split_tf32_kernel<<<gb, 256, 0, s>>>(Bt, pb, n, k, kpad, bt_stride, use_pair ? 4 : 6);
-    check(cudaGetLastError(), "split_tf32");
-  }
+  launch_split(KIND_TF32, 4, {pa}, A, m, k, batch_stride, batch, false, s);
+  launch_split(KIND_TF32, use_pair ? 4 : 6, {pb}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   if (use_pair) {
     const CUtensorMap ma = plane_map(pa, m, kpad, batch, PBM);
     const CUtensorMap mb = plane_map(pb, n, kpad, batch, PBN_CTA);
@@ -1435,13 +1262,14 @@ Fp16Workspace fp16_workspace(float* workspace, std::size_t m, std::size_t n, std
   w.a_exps = reinterpret_cast<int*>(pb + 6 * n * kpad * nb);
   w.b_exps = w.a_exps + m * nb;
   w.a_block_exps = w.b_exps + n * nb;
+  w.b_top = reinterpret_cast<std::uint32_t*>(w.a_block_exps + m * ((k + 31) / 32) * nb);
   return w;
 }
 
-void launch_cgemm_fp16x3(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                         std::size_t k, std::uint64_t batch_stride, std::uint64_t bt_stride, int batch,
+void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                         std::size_t n, std::size_t k, std::uint64_t batch_stride, std::uint64_t b_stride, int batch,
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s, bool a_in_planes) {
-  if (!tc_eligible(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
+  if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk < 1 || cfg.chunk > 64)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> chunk length must be 1..64");
   if (a_in_planes && (k < 32 || (k & (k - 1)) != 0 || cfg.chunk > 2))
@@ -1467,8 +1295,8 @@ void launch_cgemm_fp16x3(const float2* A, const float2* Bt, float2* C, std::size
   __half* pb = static_cast<__half*>(w.b_planes);
   int* ea = a_in_planes ? w.a_block_exps : w.a_exps;
   int* eb = w.b_exps;
-  if (!a_in_planes) launch_split_fp16(A, pa, ea, m, k, batch_stride, batch, 4, s);
-  launch_split_fp16(Bt, pb, eb, n, k, bt_stride, batch, 6, s);
+  if (!a_in_planes) launch_split(KIND_FP16, 4, {pa, nullptr, ea}, A, m, k, batch_stride, batch, false, s);
+  launch_split(KIND_FP16, 6, {pb, nullptr, eb, w.b_top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   // A: whole 128-byte rows for the single-CTA kernels, re / im halves for
   // the pair; B: 64-byte halves.
   const CUtensorMap ma_rows = plane_map_f16(pa, m, kpad, batch, BM, 64, 64);
@@ -1537,10 +1365,10 @@ void launch_cgemm_fp16x3(const float2* A, const float2* Bt, float2* C, std::size
   check(cudaGetLastError(), "cgemm_fp16x3");
 }
 
-void launch_cgemm_bf16x3(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                         std::size_t k, std::uint64_t batch_stride, std::uint64_t bt_stride, int batch,
+void launch_cgemm_bf16x3(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                         std::size_t n, std::size_t k, std::uint64_t batch_stride, std::uint64_t b_stride, int batch,
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s) {
-  if (!tc_eligible(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
+  if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk < 1 || cfg.chunk > 64)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> chunk length must be 1..64");
   static std::once_flag attr;
@@ -1554,13 +1382,8 @@ void launch_cgemm_bf16x3(const float2* A, const float2* Bt, float2* C, std::size
   __nv_bfloat16* at = am + 4 * m * kpad * nb;
   __nv_bfloat16* bm = at + 2 * m * kpad * nb;
   __nv_bfloat16* bt = bm + 4 * n * kpad * nb;
-  {
-    dim3 ga((unsigned)std::min<std::uint64_t>((m + 7) / 8, 152 * 16), (unsigned)batch);
-    split_bf16_kernel<<<ga, 256, 0, s>>>(A, am, at, m, k, kpad, batch_stride);
-    dim3 gb((unsigned)std::min<std::uint64_t>((n + 7) / 8, 152 * 16), (unsigned)batch);
-    split_bf16_kernel<<<gb, 256, 0, s>>>(Bt, bm, bt, n, k, kpad, bt_stride);
-    check(cudaGetLastError(), "split_bf16");
-  }
+  launch_split(KIND_BF16, 4, {am, at}, A, m, k, batch_stride, batch, false, s);
+  launch_split(KIND_BF16, 4, {bm, bt}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   const CUtensorMap ma = plane_map_bf16(am, m, kpad, batch, BM, 64, 64);
   const CUtensorMap mb = plane_map_bf16(bm, n, kpad, batch, BN, 64, 32);
   const CUtensorMap ma2 = plane_map_bf16(at, m, kpad, batch, BM, 32, 32);

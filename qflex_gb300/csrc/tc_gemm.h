@@ -8,9 +8,13 @@
 
 namespace qfx {
 
-// Shapes the tensor-core kernel takes (k a multiple of 4 for the TMA row
-// stride; smaller products stay on the CUDA-core kernels).
+// Shapes that a contraction gives to the tensor-core kernels (smaller products
+// stay on the CUDA-core kernels).
 bool tc_eligible(std::size_t m, std::size_t n, std::size_t k);
+// Shapes the kernels can run.
+bool tc_runs(std::size_t m, std::size_t n, std::size_t k);
+// How B lies in memory: n rows of k values, or k rows of n.
+enum class BLayout { nk, kn };
 // fp32 elements of split planes one batch entry needs (A and B of any split kind).
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k);
 
@@ -26,13 +30,13 @@ struct TcConfig {
 // QFLEX_TC_DEEP=1.
 TcConfig tc_default_config();
 
-// C[m,n] = A[m,k] * Bt[n,k]^T (complex64, both K-major), 3xTF32 split,
-// FP32 accumulation. Batch entry b reads A + b * ac_stride,
-// Bt + b * bt_stride and writes C + b * ac_stride. `workspace` holds
+// C[m,n] = A[m,k] * B (complex64, B in either layout), 3xTF32 split, FP32
+// accumulation. Batch entry b reads A + b * ac_stride, B + b * b_stride and
+// writes C + b * ac_stride. `workspace` holds
 // batch * tc_workspace_elems fp32; `err` (device int) receives a nonzero
 // code if a pipeline wait expired.
-void launch_cgemm_tf32x3(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                         std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch,
+void launch_cgemm_tf32x3(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                         std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride, int batch,
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s);
 
 // Where the 3xFP16 product keeps its operands in `workspace` (batch entries
@@ -45,6 +49,7 @@ struct Fp16Workspace {
   int* a_exps;
   int* b_exps;
   int* a_block_exps;
+  std::uint32_t* b_top;  // largest components of B's columns while it is split
 };
 Fp16Workspace fp16_workspace(float* workspace, std::size_t m, std::size_t n, std::size_t k, int batch);
 
@@ -57,8 +62,8 @@ Fp16Workspace fp16_workspace(float* workspace, std::size_t m, std::size_t n, std
 // workspace (written by launch_permute_fp16_planes; k a power of two >= 32,
 // cfg.chunk <= 2 so that a TMEM chunk never spans two exponent blocks) and
 // A is not read.
-void launch_cgemm_fp16x3(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                         std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch,
+void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                         std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride, int batch,
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s,
                          bool a_in_planes = false);
 
@@ -94,20 +99,23 @@ bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size
 // checks: dst is the m x k operand the product sees. Tests use it.
 void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const float2* src, float2* dst);
 
+// fp32 elements that launch_cgemm_fp16x3_direct's workspace takes per batch entry.
+std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k);
 // The same product with A split inside the kernel: A is read as complex64
 // through `gather`, every 32 values of a row scaled by their own power of
 // two, and no A planes exist in memory. Single CTA, cfg.chunk 1 or 2 (a TMEM
 // chunk never spans two of A's blocks); cfg.variant is ignored.
-void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* Bt, float2* C, std::size_t m,
-                                std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride,
-                                int batch, float* workspace, int* err, const TcConfig& cfg, cudaStream_t s);
+void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* B, BLayout b_layout, float2* C,
+                                std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
+                                std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
+                                cudaStream_t s);
 
 // The same product with BF16x3 planes: x = b0 + b1 + b2 in BF16 (no
 // scaling: BF16 has the FP32 exponent range), six products per real
 // product (x0y0, x0y1, x1y0, x0y2, x1y1, x2y0) on kind::f16 tensor cores.
 // Single-CTA kernel; cfg.variant is ignored.
-void launch_cgemm_bf16x3(const float2* A, const float2* Bt, float2* C, std::size_t m, std::size_t n,
-                         std::size_t k, std::uint64_t ac_stride, std::uint64_t bt_stride, int batch,
+void launch_cgemm_bf16x3(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
+                         std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride, int batch,
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s);
 
 }  // namespace qfx
