@@ -89,18 +89,30 @@ void launch_permute_fp16_planes(const PermPlan& plan, const float2* src, std::ui
                                 void* planes, int* exps, std::uint64_t rows, int k_log2, int batch,
                                 cudaStream_t s);
 
-// ---- permutation of indices of any dimension -------------------------------------
-// Output element o (row-major over the permuted dimensions) reads input
-// element sum_i digit_i(o) * in_stride[i], where in_stride[i] is the input
-// stride of the index that goes to position i. One thread per output
-// element: writes coalesced, reads gathered. For tensors whose dimensions
-// are not all powers of two.
+// ---- permutation of indices of any dimension (permute_general.cu) -----------------
+// For tensors whose dimensions are not all powers of two. Output element o
+// (row-major over the permuted dimensions) is input element
+// sum_i digit_i(o) * in_stride[i], where in_stride[i] is the input stride of
+// the index that goes to position i.
 constexpr int kGeneralPermMaxRank = 32;
+// Division by a constant: n / d = (hi32(n * mul) + n) >> shift for n < 2^31.
+struct FastDiv {
+  std::uint32_t d, mul, shift;
+};
 struct GeneralPerm {
   std::uint32_t rank;
   std::uint64_t size;
   std::uint64_t out_dims[kGeneralPermMaxRank];
   std::uint64_t in_stride[kGeneralPermMaxRank];
+  // The schedule for sizes below 2^31 (`runs` != 0): a thread moves a run of
+  // `run` elements that are neighbours in the input, to run_out[u] past its
+  // output offset; the other indices, fastest output index first, make the
+  // thread's number (`runs` threads). A last index cuts a long input index
+  // into runs, the last of which has `last_run` elements.
+  std::uint32_t runs, run, last_run, n_div;
+  FastDiv div[kGeneralPermMaxRank + 1];
+  std::uint32_t div_in[kGeneralPermMaxRank + 1], div_out[kGeneralPermMaxRank + 1];
+  std::uint32_t run_out[16];
 };
 // Throws (std::string) for a rank above kGeneralPermMaxRank, a zero
 // dimension, an element count above 2^40 or a new_order that is not a
