@@ -69,6 +69,9 @@ struct Engine::Plan {
   double2* d_mats64 = nullptr;  // complex128 programs: the double gate data
   std::uint32_t* d_ptr = nullptr;
   std::uint32_t* d_leaves = nullptr;
+  // The program as one kernel, when it is small (small.n_ops != 0).
+  SmallProgram small = {};
+  SmallOp* d_small_ops = nullptr;
   // Captured device pass and the buffers it was captured with.
   cudaGraphExec_t graph = nullptr;
   GraphKey graph_key, seen_key;
@@ -82,6 +85,7 @@ struct Engine::Plan {
     cudaFree(d_mats64);
     cudaFree(d_ptr);
     cudaFree(d_leaves);
+    cudaFree(d_small_ops);
   }
 };
 
@@ -440,6 +444,40 @@ T* upload(const std::vector<T>& v) {
 
 namespace {
 
+// The ops of a program as the one-kernel form takes them; empty when it does
+// not. A block runs its string's operations one after the other, at about 9
+// complex multiply-adds a cycle (256 x 16 x 16: 7000 cycles, 3.7 us) plus
+// 0.4 us per operation, against 3.3 us for the launch of an operation of its
+// own: the line lies where the average operation takes as long either way.
+std::vector<SmallOp> small_ops(const Program& prog) {
+  constexpr double kFlopPerOp = 400e3;
+  std::vector<SmallOp> out;
+  if (prog.arena_elems * sizeof(float2) > SmallProgram::kMaxSmem || prog.gemm_flop > kFlopPerOp * prog.ops.size())
+    return out;
+  for (const DevOp& op : prog.ops) {
+    SmallOp s{};
+    s.a = (std::uint32_t)op.a;
+    s.b = (std::uint32_t)op.b;
+    s.c = (std::uint32_t)op.c;
+    if (op.kind == DevOp::PERMUTE) {
+      s.m = 1u << op.nbits;
+      s.bits = (std::uint32_t)op.nbits;  // at most 14: the arena is below 226 KB
+      for (int b = 0; b < op.nbits; ++b) s.to[b] = op.perm[b];
+    } else {
+      if (op.b_nk || op.k == 0 || op.k > (std::size_t)SmallProgram::kMaxK) return {};
+      s.m = (std::uint32_t)op.m;
+      s.n = (std::uint32_t)op.n;
+      s.k = (std::uint32_t)op.k;
+      if (op.a_gather) {
+        s.bits = (std::uint32_t)op.nbits;
+        for (int b = 0; b < op.nbits; ++b) s.to[op.perm[b]] = (std::uint8_t)b;
+      }
+    }
+    out.push_back(s);
+  }
+  return out;
+}
+
 bool overlaps(std::size_t a0, std::size_t a1, std::size_t b0, std::size_t b1) { return a0 < b1 && b0 < a1; }
 
 // Whether the output of permute i, the A operand of product j, is read by no
@@ -696,6 +734,20 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
       }
       p.d_ptr = upload(ptr);
       p.d_leaves = upload(leaves);
+      std::vector<SmallOp> small;
+      if (!wide) small = small_ops(p.prog);
+      if (!small.empty()) {
+        p.d_small_ops = upload(small);
+        p.small = {p.d_cols, p.d_steps, p.d_mats, p.d_mats_lo, p.d_small_ops, p.d_ptr, p.d_leaves};
+        p.small.n_cols = (std::uint32_t)cols.size();
+        p.small.n_steps = (std::uint32_t)steps.size();
+        p.small.n_mats = (std::uint32_t)mats.size();
+        p.small.n_ops = (std::uint32_t)small.size();
+        p.small.n_amps = (std::uint32_t)p.prog.n_amplitudes;
+        p.small.arena_elems = (std::uint32_t)p.prog.arena_elems;
+        p.small.results = (std::uint32_t)p.prog.results_offset;
+        if (small_program_smem(p.small) > SmallProgram::kMaxSmem) p.small.n_ops = 0;
+      }
     }
     p.built = true;
   } else {
@@ -744,22 +796,29 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
     return results;
   }
 
-  // How many final states fit on the device at once.
-  std::size_t free_b = 0, total_b = 0;
-  QFX_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  std::size_t have = 0;
-  for (int slot : {0, 4})
-    if ((int)bufs_.size() > slot) have += bufs_[slot].bytes;
-  const std::size_t usable = free_b + have > (std::size_t(2) << 30) ? free_b + have - (std::size_t(2) << 30) : 0;
-  const std::size_t per_entry = arena_bytes + p.tc_ws_elems * sizeof(float);
-  int chunk = (int)std::max<std::size_t>(1, std::min<std::size_t>((std::size_t)total, usable / std::max<std::size_t>(per_entry, 1)));
-  chunk = std::min(chunk, 65535);
+  // How many final states fit on the device at once. A program that runs as
+  // one kernel keeps its tensors in shared memory.
+  const bool small = p.small.n_ops != 0 && !profile_;
+  int chunk = std::min(total, 65535);
+  float2* arena = nullptr;
+  float* tc_ws = nullptr;
+  if (!small) {
+    std::size_t free_b = 0, total_b = 0;
+    QFX_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    std::size_t have = 0;
+    for (int slot : {0, 4})
+      if ((int)bufs_.size() > slot) have += bufs_[slot].bytes;
+    const std::size_t usable = free_b + have > (std::size_t(2) << 30) ? free_b + have - (std::size_t(2) << 30) : 0;
+    const std::size_t per_entry = arena_bytes + p.tc_ws_elems * sizeof(float);
+    chunk = (int)std::max<std::size_t>(1, std::min<std::size_t>((std::size_t)chunk, usable / std::max<std::size_t>(per_entry, 1)));
+  }
   if (max_batch_ > 0) chunk = std::min(chunk, max_batch_);
-
-  float2* arena = (float2*)reserve(arena_bytes * (std::size_t)chunk, 0);
-  float* tc_ws = p.tc_ws_elems ? tc_workspace(p.tc_ws_elems * (std::size_t)chunk) : nullptr;
-  skinny_scratch();
-  QFX_CUDA(cudaMemsetAsync(error_flag(), 0, sizeof(int), stream_));
+  if (!small) {
+    arena = (float2*)reserve(arena_bytes * (std::size_t)chunk, 0);
+    tc_ws = p.tc_ws_elems ? tc_workspace(p.tc_ws_elems * (std::size_t)chunk) : nullptr;
+    skinny_scratch();
+    QFX_CUDA(cudaMemsetAsync(error_flag(), 0, sizeof(int), stream_));
+  }
   double2* d_amps = (double2*)reserve(std::max<std::size_t>(n_amps, 1) * sizeof(double2) * (std::size_t)chunk, 1);
   std::uint8_t* d_bits = (std::uint8_t*)reserve(std::max<std::size_t>(n_cols, 1) * 2 * (std::size_t)chunk, 2);
 
@@ -782,7 +841,7 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
       }
     }
     QFX_CUDA(cudaMemcpyAsync(d_bits, bits.data(), bits.size(), cudaMemcpyHostToDevice, stream_));
-    QFX_CUDA(cudaMemsetAsync(d_amps, 0, std::max<std::size_t>(n_amps, 1) * sizeof(double2) * nb, stream_));
+    if (!small) QFX_CUDA(cudaMemsetAsync(d_amps, 0, std::max<std::size_t>(n_amps, 1) * sizeof(double2) * nb, stream_));
     QFX_CUDA(cudaEventRecord(ev0_, stream_));
     auto enqueue = [&]() -> std::size_t {
       if (wide) {
@@ -805,7 +864,10 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
     // same batch size and buffers repeat: the first pass runs eagerly, the
     // second is captured, later ones replay the graph.
     const GraphKey gk{nb, arena, tc_ws, d_bits, d_amps, options_version_, precision_};
-    if (!profile_ && p.graph && p.graph_key == gk) {
+    if (small) {
+      launch_small_program(p.small, d_bits, d_bits + n_cols * (std::size_t)nb, d_amps, nb, stream_);
+      launches += 1;
+    } else if (!profile_ && p.graph && p.graph_key == gk) {
       QFX_CUDA(cudaGraphLaunch(p.graph, stream_));
       launches += p.graph_launches;
     } else if (!profile_ && graphs_ && p.seen_key == gk) {

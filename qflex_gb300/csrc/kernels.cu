@@ -8,72 +8,18 @@
 
 #include <cuda_fp16.h>
 
+#include "flatten.cuh"
 #include "kernels.h"
 
 namespace qfx {
 
 namespace {
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {
-  c.x = fmaf(a.x, b.x, c.x);
-  c.x = fmaf(-a.y, b.y, c.x);
-  c.y = fmaf(a.x, b.y, c.y);
-  c.y = fmaf(a.y, b.x, c.y);
-  return c;
-}
-
 void check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch ") + what + ") --> " + cudaGetErrorString(e);
 }
 
-// ---------------------------------------------------------------------------
-// Column flatten.
-// ---------------------------------------------------------------------------
-// Float-float numbers (an unevaluated sum h + l of two floats, ~44
-// significant bits) built from the classic error-free transformations:
-// Knuth's two-sum and the FMA-based exact product.
-struct ff {
-  float h, l;
-};
-__device__ __forceinline__ ff ff_add(ff a, ff b) {
-  const float s = a.h + b.h;
-  const float bb = s - a.h;
-  float e = (a.h - (s - bb)) + (b.h - bb);
-  e += a.l + b.l;
-  const float h = s + e;
-  return {h, e - (h - s)};
-}
-__device__ __forceinline__ ff ff_mul(ff a, ff b) {
-  const float p = a.h * b.h;
-  float e = fmaf(a.h, b.h, -p);
-  e = fmaf(a.h, b.l, e);
-  e = fmaf(a.l, b.h, e);
-  const float h = p + e;
-  return {h, e - (h - p)};
-}
-__device__ __forceinline__ ff ff_neg(ff a) { return {-a.h, -a.l}; }
-struct cff {
-  ff re, im;
-};
-__device__ __forceinline__ cff cff_mul(cff a, cff b) {
-  return {ff_add(ff_mul(a.re, b.re), ff_neg(ff_mul(a.im, b.im))),
-          ff_add(ff_mul(a.re, b.im), ff_mul(a.im, b.re))};
-}
-__device__ __forceinline__ cff cff_add(cff a, cff b) { return {ff_add(a.re, b.re), ff_add(a.im, b.im)}; }
-__device__ __forceinline__ cff cff_load(const float2* hi, const float2* lo, std::uint32_t i) {
-  const float2 h = __ldg(hi + i), l = __ldg(lo + i);
-  return {{h.x, l.x}, {h.y, l.y}};
-}
-
-// Element e of a column's 2D tensor: <final| G_K ... G_1 |init> with every
-// two-qubit half reading its virtual digit of e. Plain FP32 repeats the
-// reference's complex<float> arithmetic on its float gate constants; the
-// compensated form carries float-float values and gate constants (hi + lo
-// of the double-precision gate) and rounds once at the end.
 template <bool kCompensated>
 __global__ void __launch_bounds__(256) flatten_kernel(const ColumnDesc* __restrict__ cols,
                                                       const StepDesc* __restrict__ steps,
@@ -89,41 +35,11 @@ __global__ void __launch_bounds__(256) flatten_kernel(const ColumnDesc* __restri
   const std::uint64_t e = std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= (std::uint64_t(1) << cd.size_log2)) return;
   const bool one = init_bits[std::size_t(b) * n_cols + c] != 0;
-  float2 p0 = make_float2(one ? 0.f : 1.f, 0.f), p1 = make_float2(one ? 1.f : 0.f, 0.f);
-  cff f0 = {{p0.x, 0.f}, {0.f, 0.f}}, f1 = {{p1.x, 0.f}, {0.f, 0.f}};
-  for (std::uint32_t s = cd.step_begin; s < cd.step_end; ++s) {
-    const StepDesc sd = steps[s];
-    std::uint32_t g = sd.mat;
-    std::uint32_t row = 2;  // distance between input rows of the gate data
-    if (sd.kind == 2) {
-      const std::uint32_t v = std::uint32_t(e >> sd.shift) & (sd.V - 1);
-      g += 2 * v;
-      row = 2 * sd.V;
-    }
-    if constexpr (kCompensated) {
-      const cff q0 = cff_add(cff_mul(f0, cff_load(mats, mats_lo, g)),
-                             cff_mul(f1, cff_load(mats, mats_lo, g + row)));
-      const cff q1 = cff_add(cff_mul(f0, cff_load(mats, mats_lo, g + 1)),
-                             cff_mul(f1, cff_load(mats, mats_lo, g + row + 1)));
-      f0 = q0;
-      f1 = q1;
-    } else {
-      const float2 q0 = cfma(p1, __ldg(mats + g + row), cmul(p0, __ldg(mats + g)));
-      const float2 q1 = cfma(p1, __ldg(mats + g + row + 1), cmul(p0, __ldg(mats + g + 1)));
-      p0 = q0;
-      p1 = q1;
-    }
-  }
-  if constexpr (kCompensated) {
-    p0 = make_float2(f0.re.h + f0.re.l, f0.im.h + f0.im.l);
-    p1 = make_float2(f1.re.h + f1.re.l, f1.im.h + f1.im.l);
-  }
-  int bit;
-  if (cd.o_shift >= 0)
-    bit = int((e >> cd.o_shift) & 1);
-  else
-    bit = final_bits[std::size_t(b) * n_cols + c];
-  arena[std::uint64_t(b) * arena_stride + cd.out_offset + e] = bit ? p1 : p0;
+  const bool bit = cd.o_shift >= 0 ? ((e >> cd.o_shift) & 1) != 0 : final_bits[std::size_t(b) * n_cols + c] != 0;
+  const std::uint64_t at[1] = {e};
+  float2 out[1];
+  column_elements<kCompensated, 1>(cd, steps, mats, mats_lo, one, at, out, [&](int) { return bit; });
+  arena[std::uint64_t(b) * arena_stride + cd.out_offset + e] = out[0];
 }
 
 // ---------------------------------------------------------------------------

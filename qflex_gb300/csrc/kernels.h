@@ -190,6 +190,33 @@ void launch_reduce_amplitudes64(const double2* results, std::uint64_t stride, co
                                 const std::uint32_t* leaves, int n_amps, double2* amps, int batch,
                                 cudaStream_t s);
 
+// ---- a whole contraction in one kernel (small_program.cu) ------------------------
+struct SmallOp {
+  std::uint32_t a, b, c;  // arena offsets
+  std::uint32_t m, n, k;  // k = 0: permutation of m elements
+  alignas(8) std::uint8_t to[16];  // permutation: input digit -> output digit; A: operand digit -> source digit
+  std::uint32_t bits;     // digits of `to`: of a permutation, or of A read through one
+  std::uint32_t unused;
+};
+struct SmallProgram {
+  static constexpr std::size_t kMaxSmem = 226 * 1024;
+  static constexpr int kMaxK = 1024;
+  const ColumnDesc* cols;
+  const StepDesc* steps;
+  const float2* mats;
+  const float2* mats_lo;  // null: plain FP32 columns
+  const SmallOp* ops;
+  const std::uint32_t* ptr;
+  const std::uint32_t* leaves;
+  std::uint32_t n_cols, n_steps, n_mats, n_ops, n_amps;
+  std::uint32_t arena_elems, results;
+};
+// Shared memory of one block.
+std::size_t small_program_smem(const SmallProgram& p);
+// Amplitudes of `batch` strings, one block each; amps[b * n_amps + a] is written.
+void launch_small_program(const SmallProgram& p, const std::uint8_t* init_bits, const std::uint8_t* final_bits,
+                          double2* amps, int batch, cudaStream_t s);
+
 // ---- FP64 amplitude sums -------------------------------------------------------
 // amps[b * n_amps + a] += sum of results[b * stride + leaf] over the leaves
 // of amplitude a (CSR: leaves[ptr[a] .. ptr[a+1])), in leaf order.
