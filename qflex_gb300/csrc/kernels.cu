@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include "flatten.cuh"
+#include "half_split.cuh"
 #include "kernels.h"
 
 namespace qfx {
@@ -124,15 +125,14 @@ __global__ void __launch_bounds__(256, 8) permute_kernel(const __grid_constant__
       const bool direct = e >= -126 && e <= 127;
       const float sc = __uint_as_float(std::uint32_t(direct ? e + 127 : 127) << 23);
       const float xr = direct ? v.x * sc : ldexpf(v.x, e), xi = direct ? v.y * sc : ldexpf(v.y, e);
-      const __half2 hi = __floats2half2_rn(xr, xi);  // (re_hi, im_hi)
-      const float2 hf = __half22float2(hi);
-      const __half2 lo = __floats2half2_rn(xr - hf.x, xi - hf.y);
+      std::uint32_t hi, lo;  // (re, im)
+      split_pair(xr, xi, hi, lo);
       __half* pl = po.planes + std::uint64_t(blockIdx.y) * 4 * po.rows * k + ((kk / 16) * po.rows + row) * 64 +
                    (kk % 16);
-      pl[0] = __low2half(hi);
-      pl[16] = __low2half(lo);
-      pl[32] = __high2half(hi);
-      pl[48] = __high2half(lo);
+      pl[0] = __ushort_as_half(std::uint16_t(hi));
+      pl[16] = __ushort_as_half(std::uint16_t(lo));
+      pl[32] = __ushort_as_half(std::uint16_t(hi >> 16));
+      pl[48] = __ushort_as_half(std::uint16_t(lo >> 16));
       if ((threadIdx.x & 31) == 0)
         po.exps[std::uint64_t(blockIdx.y) * po.rows * (k / 32) + row * (k / 32) + kk / 32] = e;
       }

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <string>
 
+#include "half_split.cuh"
 #include "tc_common.cuh"
 
 namespace qfx {
@@ -93,7 +94,7 @@ __device__ __forceinline__ void emit(const float2 (&v)[unit_values<KIND>()], int
     // Scaling by 2^e is exact; two steps when 2^e is no normal float.
     const float s1 = __uint_as_float(std::uint32_t(min(e, 127) + 127) << 23);
     const float s2 = __uint_as_float(std::uint32_t(max(e - 127, 0) + 127) << 23);
-    __half2 rh[4], rl[4], ih[4], il[4];
+    std::uint32_t rh[4], rl[4], ih[4], il[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float r0 = v[2 * j].x * s1, i0 = v[2 * j].y * s1, r1 = v[2 * j + 1].x * s1, i1 = v[2 * j + 1].y * s1;
@@ -103,11 +104,8 @@ __device__ __forceinline__ void emit(const float2 (&v)[unit_values<KIND>()], int
         r1 *= s2;
         i1 *= s2;
       }
-      rh[j] = __floats2half2_rn(r0, r1);
-      ih[j] = __floats2half2_rn(i0, i1);
-      const float2 rf = __half22float2(rh[j]), jf = __half22float2(ih[j]);
-      rl[j] = __floats2half2_rn(r0 - rf.x, r1 - rf.y);
-      il[j] = __floats2half2_rn(i0 - jf.x, i1 - jf.y);
+      split_pair(r0, r1, rh[j], rl[j]);
+      split_pair(i0, i1, ih[j], il[j]);
     }
     uint4* o = reinterpret_cast<uint4*>(static_cast<__half*>(main_planes) + ((kk / 16) * rows + row) * (16 * NP) +
                                         kk % 16);
@@ -118,8 +116,8 @@ __device__ __forceinline__ void emit(const float2 (&v)[unit_values<KIND>()], int
     if constexpr (NP == 6) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        ih[j] = __hneg2(ih[j]);
-        il[j] = __hneg2(il[j]);
+        ih[j] ^= 0x80008000u;
+        il[j] ^= 0x80008000u;
       }
       o[8] = as_unit(ih);
       o[10] = as_unit(il);

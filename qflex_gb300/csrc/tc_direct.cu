@@ -12,9 +12,9 @@
 // 176, 104 per thread: 128 on average, the launch's own share).
 //   warp 0       B producer: two 8 KB TMA boxes per k-step (re and im rows of
 //                64 bytes, hi and lo)
-//   warp 1       TMEM allocation; one thread issues every MMA
+//   warp 1       TMEM allocation; issues every MMA
 //   warps 2, 3   A loader: 16-byte cp.async copies of one 128 x 32 block of A
-//                (32 KB) into a ring of four blocks
+//                (32 KB) into a ring of three blocks
 //   warps 4..11  epilogue: drains TMEM chunks, scales and stores the tile
 //   warps 12..15 A converter: thread r reads row r of the block, finds the
 //                largest component, scales by the power of two that brings it
@@ -23,13 +23,14 @@
 // A block is two k-steps of 16, one TMEM chunk at the default chunk length,
 // so the epilogue applies the block's exponent as it adds the chunk.
 //
-// What bounds it: shared memory's 128 bytes a cycle. A k-step's MMAs take 768
-// cycles of the tensor pipe and read 84 KB of operands (672 cycles); loading
-// B takes another 128, and A's way through shared memory (written by the
-// copies, read by the converter, written as planes) 384. 1125 cycles measured
-// at k = 4096. (The kernel that loads A's planes reads 72 KB and loads 40:
-// 896, where the card's power limit is near.) A tile's store overlaps two
-// chunks of the next tile's MMAs.
+// What bounds it: a k-step's MMAs take 768 cycles of the tensor pipe and read
+// 84 KB of operands; those reads (672 cycles at 128 bytes a cycle) share the
+// way with the fills, 128 cycles of B's TMA boxes and 128 of A's copies: 928,
+// and 938 measured at k = 4096. (The kernel that loads A's planes: 576 + 320 =
+// 896, where the card's power limit is near.) At short k the converter comes
+// next, about 1800 cycles a block of two k-steps, and a tile's store, 6100
+// cycles of which two chunks of the next tile's MMAs overlap: (65536, 256,
+// 256) x 4 takes 2930 cycles a block, 341 us; (65536, 256, 16) x 4 93 us.
 //
 // B holds no negated copy: Ar multiplies (Br; Bi) in one N = 256 MMA, and Ai
 // takes two N = 128 MMAs, -Ai Bi (the descriptor's negate-A bit) and Ai Br.
@@ -44,6 +45,7 @@
 #include <string>
 #include <vector>
 
+#include "half_split.cuh"
 #include "tc_common.cuh"
 #include "tc_gemm.h"
 
@@ -51,14 +53,14 @@ namespace qfx {
 namespace {
 
 constexpr int BM = 128, BN = 128;
-constexpr int A_RING = 4;                   // blocks of 128 rows x 32 values
+constexpr int A_RING = 3;                   // blocks of 128 rows x 32 values
 constexpr int A_BLOCK = 128 * 32 * 8;       // bytes, complex64 or two k-steps of planes
 constexpr int B_STAGES = 4;                 // one k-step each
 constexpr int B_PART = BN * 64;             // re or im rows of a k-step (hi, lo)
 constexpr int B_STAGE = 2 * B_PART;
 constexpr int EXP_RING = 6;                 // block exponents, see the converter
 constexpr int OFF_B = A_RING * A_BLOCK;
-constexpr int SLOT = 2048;                  // output box: 32 rows x 8 complex
+constexpr int SLOT = 4096;                  // output box: 32 rows x 16 complex
 constexpr int OFF_STAGING = OFF_B + B_STAGES * B_STAGE;
 constexpr int OFF_SCALE = OFF_STAGING + 8 * 2 * SLOT;
 constexpr int OFF_EXP = OFF_SCALE + 8 * (BN / 2) * 4;  // after each epilogue warp's column exponents
@@ -451,13 +453,8 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int j = 0; j < 4; ++j) {
             const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
             const float2 r = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
-            const __half2 hr = __floats2half2_rn(r.x, r.y), hi = __floats2half2_rn(im.x, im.y);
-            const float2 fr = __half22float2(hr), fi = __half22float2(hi);
-            const __half2 lr = __floats2half2_rn(r.x - fr.x, r.y - fr.y), li = __floats2half2_rn(im.x - fi.x, im.y - fi.y);
-            rh[j] = *reinterpret_cast<const std::uint32_t*>(&hr);
-            rl[j] = *reinterpret_cast<const std::uint32_t*>(&lr);
-            ih[j] = *reinterpret_cast<const std::uint32_t*>(&hi);
-            il[j] = *reinterpret_cast<const std::uint32_t*>(&li);
+            split_pair(r.x, r.y, rh[j], rl[j]);
+            split_pair(im.x, im.y, ih[j], il[j]);
           }
           // k-step i / 16; unit u of the 128-byte row (two per plane) lies at
           // u ^ (row % 8).
@@ -473,9 +470,9 @@ __global__ void __launch_bounds__(THREADS, 1)
           put(4, ih);
           put(6, il);
         }
-        // Exponents live in a ring of their own: this block is at most five
+        // Exponents live in a ring of their own: this block is at most four
         // ahead of the one the slowest epilogue warp drains (its MMAs are
-        // done with the block four back, which needed all chunks up to six
+        // done with the block three back, which needed all chunks up to five
         // back drained).
         exps[x * BM + row] = std::int8_t(e);
         fence_proxy_async();
@@ -602,34 +599,35 @@ __global__ void __launch_bounds__(THREADS, 1)
         sc_row[32 + lane] = 0;
         __syncwarp();
       }
-      auto scaled = [&](float2 v, float2 w, int ex, int ey, float4& out) {
-        // Two columns: v = re pair, w = im pair, exponents ex, ey (<< 23).
-        v = fma2(v, beta2, v);
-        w = fma2(w, beta2, w);
-        const float s0 = __uint_as_float(c0 - std::uint32_t(ex)), s1 = __uint_as_float(c0 - std::uint32_t(ey));
-        out = make_float4(v.x * s0, w.x * s0, v.y * s1, w.y * s1);
-      };
-      float2* cb = C + std::uint64_t(batch) * ac_stride;
 #pragma unroll
-      for (int j0 = 0; j0 < COLS; j0 += 8) {
-        // A box of 32 rows x 8 complex, two slots in turn. (A thread storing
-        // its own row piece in 32-byte sectors, without this pass through
-        // shared memory, took 9400 cycles a tile against 7300.)
-        std::uint8_t* slot = staging + ((j0 / 8) & 1) * SLOT;
+      for (int j = 0; j < COLS / 2; ++j) {
+        re[j] = fma2(re[j], beta2, re[j]);
+        im[j] = fma2(im[j], beta2, im[j]);
+      }
+      float2* cb = C + std::uint64_t(batch) * ac_stride;
+      // Four boxes of 32 rows x 16 complex, two slots in turn. (Boxes of 8
+      // columns: twice the fences and barriers, a tile's store took 7200
+      // cycles. A thread storing its own row piece in 32-byte sectors,
+      // without shared memory, 9400.)
+#pragma unroll
+      for (int j0 = 0; j0 < COLS; j0 += 16) {
+        std::uint8_t* slot = staging + ((j0 / 16) & 1) * SLOT;
         if (tma_c) {
           if (lane == 0) bulk_wait_read1();
           __syncwarp();
         }
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) {
+        for (int j = 0; j < 16; j += 4) {
           const int4 es = *reinterpret_cast<const int4*>(sc_row + j0 + j);
-          float4 o0, o1;
-          scaled(re[(j0 + j) / 2], im[(j0 + j) / 2], es.x, es.y, o0);
-          scaled(re[(j0 + j) / 2 + 1], im[(j0 + j) / 2 + 1], es.z, es.w, o1);
-          // 64-byte swizzle: unit u of row r lies at u ^ ((r / 2) % 4).
-          const std::uint32_t u = j / 2, w = (lane >> 1) & 3;
-          *reinterpret_cast<float4*>(slot + lane * 64 + ((u ^ w) << 4)) = o0;
-          *reinterpret_cast<float4*>(slot + lane * 64 + (((u + 1) ^ w) << 4)) = o1;
+          const float s0 = __uint_as_float(c0 - std::uint32_t(es.x)), s1 = __uint_as_float(c0 - std::uint32_t(es.y));
+          const float s2 = __uint_as_float(c0 - std::uint32_t(es.z)), s3 = __uint_as_float(c0 - std::uint32_t(es.w));
+          const int p = (j0 + j) / 2;
+          // 128-byte swizzle: unit u of row r lies at u ^ (r % 8).
+          const std::uint32_t u = j / 2, w = lane & 7;
+          *reinterpret_cast<float4*>(slot + lane * 128 + ((u ^ w) << 4)) =
+              make_float4(re[p].x * s0, im[p].x * s0, re[p].y * s1, im[p].y * s1);
+          *reinterpret_cast<float4*>(slot + lane * 128 + (((u + 1) ^ w) << 4)) =
+              make_float4(re[p + 1].x * s2, im[p + 1].x * s2, re[p + 1].y * s3, im[p + 1].y * s3);
         }
         if (tma_c) {
           fence_proxy_async();
@@ -640,11 +638,11 @@ __global__ void __launch_bounds__(THREADS, 1)
             bulk_commit();
           }
         } else {
-          // Odd n and unaligned outputs: four rows of 8 columns at a time.
+          // Odd n and unaligned outputs: two rows of 16 columns at a time.
           __syncwarp();
-          for (int r0 = 0; r0 < 32; r0 += 4) {
-            const int r = r0 + lane / 8, col = lane % 8;
-            const float2 v = *reinterpret_cast<const float2*>(slot + r * 64 + (((col / 2) ^ ((r >> 1) & 3)) << 4) +
+          for (int r0 = 0; r0 < 32; r0 += 2) {
+            const int r = r0 + lane / 16, col = lane % 16;
+            const float2 v = *reinterpret_cast<const float2*>(slot + r * 128 + (((col / 2) ^ (r & 7)) << 4) +
                                                               (col & 1) * 8);
             const int gr = m0 + q * 32 + r;
             if (gr < m && j0 + col < ncols) cb[std::uint64_t(gr) * n + n0 + j0 + col] = v;
@@ -835,7 +833,7 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, BN, 64);
   CUtensorMap mc;
-  const int tma_c = output_map(C, m, n, ac_stride, batch, &mc, true) ? 1 : 0;
+  const int tma_c = output_map(C, m, n, ac_stride, batch, &mc) ? 1 : 0;
   const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * (std::size_t)batch;
   cgemm_fp16x3_direct_kernel<<<persistent_grid(tiles), THREADS, SMEM, s>>>(
       mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err, cfg.chunk, eb);
