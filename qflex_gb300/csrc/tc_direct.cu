@@ -365,17 +365,22 @@ __global__ void __launch_bounds__(THREADS, 1)
           } else {
             // Edge blocks and rows that are not 16-byte aligned (plain rows:
             // copy u covers row u / 16, values 2 (u % 16) and the next).
-            const int kk = b * 32 + 2 * (lt & 15);
-            for (int i = 0; i < 32; ++i) {
-              const int row = mt * BM + (lt >> 4) + 4 * i;
-              const int have = row < m ? min(2, k - kk) : 0;  // values of the pair that exist
-              const float2* from = have > 0 ? src + g.copy_src[i] : A;
-              const std::uint32_t to = dst + (lane_dst ^ g.copy_dst[i]);
-              if (g.aligned) {
-                cp_async16(to, from, have > 0 ? 8u * have : 0u);
-              } else {
-                cp_async8(to, from, have > 0 ? 8u : 0u);
-                cp_async8(to + 8, have > 1 ? from + 1 : A, have > 1 ? 8u : 0u);
+            const int have = min(2, k - (b * 32 + 2 * (lt & 15)));  // values of a pair that exist
+            const int rows = have > 0 ? m - (mt * BM + (lt >> 4)) : 0;
+            if (g.aligned) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const bool in = 4 * i < rows;
+                cp_async16(dst + (lane_dst ^ g.copy_dst[i]), in ? src + g.copy_src[i] : A, in ? 8u * have : 0u);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const bool in = 4 * i < rows, in2 = in && have > 1;
+                const float2* from = src + g.copy_src[i];
+                const std::uint32_t to = dst + (lane_dst ^ g.copy_dst[i]);
+                cp_async8(to, in ? from : A, in ? 8u : 0u);
+                cp_async8(to + 8, in2 ? from + 1 : A, in2 ? 8u : 0u);
               }
             }
           }
