@@ -208,7 +208,7 @@ void Engine::set_tc_variant(std::size_t m, std::size_t n, std::size_t k, int var
 // (65536, 256, 256) x 4 211 + 309 against 340 us, (4096, 4096, 4096)
 // 50 + 947 against 1109 us; the lines cross between n = 1024 and 1700.
 bool Engine::direct_product(std::size_t n, const TcConfig& cfg) const {
-  return precision_ == FP16X3 && cfg.variant == 0 && cfg.chunk <= 2 && n <= 1024;
+  return precision_ == FP16X3 && cfg.variant == 0 && cfg.chunk == 2 && n <= 1024;
 }
 
 std::size_t Engine::workspace_elems(std::size_t m, std::size_t n, std::size_t k) const {
@@ -353,7 +353,7 @@ Engine::Plan* Engine::get_plan(const std::string& circuit, const std::string& or
   if (!fuse_splits_) key += "n";
   if (precision_ == FP16X3 && fuse_splits_) {
     // What decides which products read A through a permutation.
-    key += cat("f", tc_cfg_.chunk <= 2 ? 1 : 0, ",", tc_cfg_.variant);
+    key += cat("f", tc_cfg_.chunk == 2 ? 1 : 0, ",", tc_cfg_.variant);
     for (const auto& [shape, variant] : tc_variant_)
       key += cat(";", std::get<0>(shape), ",", std::get<1>(shape), ",", std::get<2>(shape), ",", variant);
   }

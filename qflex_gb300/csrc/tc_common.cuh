@@ -13,6 +13,10 @@
 namespace qfx {
 
 // Host helpers, defined in tc_gemm.cu next to the plane layouts.
+// Map over complex64 elements (`dims`, byte `strides` of the dimensions from
+// the second on) for boxes with rows of 16 elements, 128-byte swizzle.
+CUtensorMap element_map(const float2* base, int rank, const std::uint64_t* dims, const std::uint64_t* strides,
+                        const std::uint32_t* box);
 CUtensorMap plane_map_f16(const __half* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
                           int row_halves, int box_inner = 32);
 bool output_map(float2* C, std::size_t m, std::size_t n, std::uint64_t batch_stride, int batch, CUtensorMap* map,
@@ -97,6 +101,23 @@ __device__ __forceinline__ void tma_load_4d(const CUtensorMap* map, std::uint64_
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
       "%5}], [%6];" ::"r"(smem_u32(dst)),
       "l"(reinterpret_cast<std::uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+      : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, std::uint64_t* bar, std::uint32_t dst, int c0,
+                                            int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          dst),
+      "l"(reinterpret_cast<std::uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+      : "memory");
+}
+// Box at the origin of the first four dimensions.
+__device__ __forceinline__ void tma_load_5d(const CUtensorMap* map, std::uint64_t* bar, std::uint32_t dst, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %2, %2, %3}], "
+      "[%4];" ::"r"(dst),
+      "l"(reinterpret_cast<std::uint64_t>(map)), "r"(0), "r"(c4), "r"(smem_u32(bar))
       : "memory");
 }
 

@@ -9,32 +9,36 @@
 //
 // Structure: persistent, one CTA per SM over 128 x 128 complex tiles, 512
 // threads in four warpgroups whose registers setmaxnreg divides (56, 176,
-// 176, 104 per thread: 128 on average, the launch's own share).
-//   warp 0       B producer: two 8 KB TMA boxes per k-step (re and im rows of
-//                64 bytes, hi and lo)
+// 176, 104 per thread: 128 on average, the launch's own share). Work goes by
+// blocks of A, 128 rows x 32 values (two k-steps of 16):
+//   warp 0       B producer: four 8 KB TMA boxes a block (re and im rows of
+//                64 bytes, hi and lo, of each k-step)
 //   warp 1       TMEM allocation; issues every MMA
-//   warps 2, 3   A loader: 16-byte cp.async copies of one 128 x 32 block of A
-//                (32 KB) into a ring of three blocks
-//   warps 4..11  epilogue: drains TMEM chunks, scales and stores the tile
+//   warp 2       A loader: TMA boxes into a ring of three blocks (with warp 3,
+//                16- or 8-byte cp.async copies where no box fits)
+//   warps 4..11  epilogue: drains TMEM sums, scales and stores the tile
 //   warps 12..15 A converter: thread r reads row r of the block, finds the
 //                largest component, scales by the power of two that brings it
-//                into [2^14, 2^15), splits into hi + lo and writes the two
-//                k-steps' 128-byte plane rows over the block it came from
-// A block is two k-steps of 16, one TMEM chunk at the default chunk length,
-// so the epilogue applies the block's exponent as it adds the chunk.
+//                into [2^14, 2^15), splits into hi + lo and writes the planes
+//                to its TMEM lane, where the MMAs read A
+// TMEM holds two blocks of planes (128 columns) and three sums of 128
+// columns: a block's real part is summed from zero into one, its imaginary
+// part into the next, and the epilogue, which applies the block's exponent as
+// it adds a sum to the tile, drains one while the others fill.
 //
-// What bounds it: a k-step's MMAs take 768 cycles of the tensor pipe and read
-// 84 KB of operands; those reads (672 cycles at 128 bytes a cycle) share the
-// way with the fills, 128 cycles of B's TMA boxes and 128 of A's copies: 928,
-// and 938 measured at k = 4096. (The kernel that loads A's planes: 576 + 320 =
-// 896, where the card's power limit is near.) At short k the converter comes
-// next, about 1800 cycles a block of two k-steps, and a tile's store, 6100
-// cycles of which two chunks of the next tile's MMAs overlap: (65536, 256,
-// 256) x 4 takes 2930 cycles a block, 341 us; (65536, 256, 16) x 4 93 us.
+// What bounds it: a block's 24 MMAs take 1536 cycles of the tensor pipe, and
+// one warp issues them, one converts per SM partition, so what these do
+// between MMAs counts as much. Measured at k = 4096 (1024 x 1024, 64 CTAs: no
+// power limit), cycles a block: A's planes in shared memory, A by cp.async
+// and five waits and commits a block 2360; planes in TMEM the same; two waits
+// and commits 2030; A by TMA boxes 1950. Without the loads and the conversion
+// (wrong sums) 1700. (65536, 256, 256) x 4 went from 341 to 308 us, (4096,
+// 1024, 4096) from 319 to 275, (65536, 256, 16) x 4 takes 96, of which
+// writing C alone is 80.
 //
-// B holds no negated copy: Ar multiplies (Br; Bi) in one N = 256 MMA, and Ai
-// takes two N = 128 MMAs, -Ai Bi (the descriptor's negate-A bit) and Ai Br.
-// N = 128 MMAs run at the same rate, and a k-step loads 16 KB of B, not 24.
+// B holds no negated copy: the real part takes -Ai Bi by the descriptor's
+// negate-A bit, and a k-step loads 16 KB of B, not 24. MMAs of N = 128 run at
+// the rate of N = 256 when A lies in TMEM.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -54,50 +58,74 @@ namespace {
 
 constexpr int BM = 128, BN = 128;
 constexpr int A_RING = 3;                   // blocks of 128 rows x 32 values
-constexpr int A_BLOCK = 128 * 32 * 8;       // bytes, complex64 or two k-steps of planes
-constexpr int B_STAGES = 4;                 // one k-step each
+constexpr int A_BLOCK = 128 * 32 * 8;       // bytes
+constexpr int A_BUFS = 2;                   // blocks of planes in TMEM
+constexpr int HALVES = 3;                   // sums, the real or imaginary part of a block
+constexpr int B_STAGES = 2;                 // two k-steps each
+constexpr int DONE = 3;                     // barriers of finished blocks in turn
 constexpr int B_PART = BN * 64;             // re or im rows of a k-step (hi, lo)
-constexpr int B_STAGE = 2 * B_PART;
-constexpr int EXP_RING = 6;                 // block exponents, see the converter
+constexpr int B_STAGE = 4 * B_PART;
+constexpr int EXP_RING = 4;                 // block exponents, see the converter
 constexpr int OFF_B = A_RING * A_BLOCK;
 constexpr int SLOT = 4096;                  // output box: 32 rows x 16 complex
 constexpr int OFF_STAGING = OFF_B + B_STAGES * B_STAGE;
 constexpr int OFF_SCALE = OFF_STAGING + 8 * 2 * SLOT;
 constexpr int OFF_EXP = OFF_SCALE + 8 * (BN / 2) * 4;  // after each epilogue warp's column exponents
 constexpr int OFF_BAR = OFF_EXP + EXP_RING * BM;
-constexpr int N_BARS = 3 * A_RING + 2 * B_STAGES + 4 + 1;
+constexpr int N_BARS = 2 * A_RING + A_BUFS + B_STAGES + 2 * DONE + HALVES + 1;
 constexpr int SMEM = OFF_BAR + N_BARS * 8 + 8;
 static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
-constexpr int TMEM_COLS = 512;  // two chunk buffers of (re, im) x 128 columns
+constexpr int TMEM_COLS = 512;
+constexpr int TMEM_A = HALVES * BN;  // two blocks of planes after the accumulators
+constexpr int TMEM_A_BLOCK = 64;     // 2 k-steps x 4 planes x 8 words
+static_assert(TMEM_A + A_BUFS * TMEM_A_BLOCK == TMEM_COLS, "TMEM is full");
 constexpr int THREADS = 512;
 constexpr int LOADERS = 64, CONVERTERS = 128;
 
-// One k-step: A's planes (re hi, lo, im hi, lo 32 bytes apart in 128-byte
-// rows) against B's re rows (`blo`, hi and lo 32 bytes apart) and im rows
-// (B_PART further), small terms first.
-__device__ __forceinline__ void mma_kstep(std::uint32_t d, std::uint32_t alo, std::uint32_t ahi, std::uint32_t blo,
-                                          std::uint32_t bhi, std::uint32_t acc) {
-  constexpr std::uint32_t wide = idesc_f16(BM, 2 * BN, false), pos = idesc_f16(BM, BN, false),
-                          neg = idesc_f16(BM, BN, true);
-  static_assert(B_PART / 16 == 512, "offset of the im rows below");
+// The real (IM = 0) or imaginary part of a block: two k-steps of A's planes in
+// TMEM (re hi, lo, im hi, lo, 8 columns each from `a`) against B's re rows
+// (`blo`, hi and lo 32 bytes apart) and im rows (B_PART further), small terms
+// first.
+template <int IM>
+__device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std::uint32_t blo, std::uint32_t bhi) {
+  constexpr std::uint32_t pos = idesc_f16(BM, BN, false), neg = idesc_f16(BM, BN, true);
+  static_assert(B_PART / 16 == 512, "offset of the im rows and of the second k-step");
+  // Ar multiplies B's part of the same name, Ai the other one (negated for
+  // the real part).
+  const std::uint32_t x = IM ? blo + 512 : blo, y = IM ? blo : blo + 512;
+#define QFX_MMA(a_, b_, id, p) " tcgen05.mma.cta_group::1.kind::f16 [%0], [" a_ "], " b_ ", " id ", " p ";\n"
+#define QFX_KSTEP(rh, rl, ih, il, p)                                                                  \
+  QFX_MMA(rh, "xl", "%5", p)                                                                          \
+  QFX_MMA(rl, "xh", "%5", "p1")                                                                       \
+  QFX_MMA(ih, "yl", "%6", "p1")                                                                       \
+  QFX_MMA(il, "yh", "%6", "p1") QFX_MMA(rh, "xh", "%5", "p1") QFX_MMA(ih, "yh", "%6", "p1")
+#define QFX_BDESC " mov.b64 xh, {x0, %4};\n mov.b64 xl, {x1, %4};\n mov.b64 yh, {y0, %4};\n mov.b64 yl, {y1, %4};\n"
   asm volatile(
-      "{\n .reg .pred p0, p1;\n .reg .b32 l1, l2, l3, m1, m2, m3, dm;\n"
-      " .reg .b64 arh, arl, aih, ail, brh, brl, bih, bil;\n"
-      " setp.ne.b32 p0, %5, 0;\n setp.eq.b32 p1, %5, %5;\n"
-      " add.u32 l1, %1, 2;\n add.u32 l2, %1, 4;\n add.u32 l3, %1, 6;\n"
-      " add.u32 m1, %3, 2;\n add.u32 m2, %3, 512;\n add.u32 m3, %3, 514;\n add.u32 dm, %0, 128;\n"
-      " mov.b64 arh, {%1, %2};\n mov.b64 arl, {l1, %2};\n mov.b64 aih, {l2, %2};\n mov.b64 ail, {l3, %2};\n"
-      " mov.b64 brh, {%3, %4};\n mov.b64 brl, {m1, %4};\n mov.b64 bih, {m2, %4};\n mov.b64 bil, {m3, %4};\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], arh, brl, %6, p0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], arl, brh, %6, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], aih, bil, %8, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [dm], aih, brl, %7, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], ail, bih, %8, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [dm], ail, brh, %7, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], arh, brh, %6, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], aih, bih, %8, p1;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [dm], aih, brh, %7, p1;\n}\n" ::"r"(d),
-      "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(acc), "r"(wide), "r"(pos), "r"(neg));
+      "{\n .reg .pred p0, p1;\n .reg .b32 a1, a2, a3, a4, a5, a6, a7, x0, x1, y0, y1;\n"
+      " .reg .b64 xh, xl, yh, yl;\n"
+      " setp.ne.b32 p0, %1, %1;\n setp.eq.b32 p1, %1, %1;\n"
+      " add.u32 a1, %1, 8;\n add.u32 a2, %1, 16;\n add.u32 a3, %1, 24;\n add.u32 a4, %1, 32;\n"
+      " add.u32 a5, %1, 40;\n add.u32 a6, %1, 48;\n add.u32 a7, %1, 56;\n"
+      " mov.b32 x0, %2;\n mov.b32 y0, %3;\n add.u32 x1, %2, 2;\n add.u32 y1, %3, 2;\n"  //
+      QFX_BDESC QFX_KSTEP("%1", "a1", "a2", "a3", "p0")
+      " add.u32 x0, %2, 1024;\n add.u32 y0, %3, 1024;\n add.u32 x1, %2, 1026;\n add.u32 y1, %3, 1026;\n"  //
+      QFX_BDESC QFX_KSTEP("a4", "a5", "a6", "a7", "p1") "}\n" ::"r"(d),
+      "r"(a), "r"(x), "r"(y), "r"(bhi), "r"(pos), "r"(IM ? pos : neg));
+#undef QFX_BDESC
+#undef QFX_KSTEP
+#undef QFX_MMA
+}
+
+// 32 words of the thread's TMEM lane.
+__device__ __forceinline__ void tmem_st32(std::uint32_t at, const std::uint32_t* w) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(at),
+      "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+      "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15]), "r"(w[16]), "r"(w[17]), "r"(w[18]),
+      "r"(w[19]), "r"(w[20]), "r"(w[21]), "r"(w[22]), "r"(w[23]), "r"(w[24]), "r"(w[25]), "r"(w[26]), "r"(w[27]),
+      "r"(w[28]), "r"(w[29]), "r"(w[30]), "r"(w[31])
+      : "memory");
 }
 
 // Two-lane FP32 arithmetic (round to nearest, each lane as the scalar form).
@@ -131,36 +159,25 @@ __device__ __forceinline__ void cp_async8(std::uint32_t dst, const void* src, st
 __device__ __forceinline__ void cp_async_arrive(std::uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Whether every converter thread says yes; also their barrier.
-__device__ __forceinline__ bool converters_all(bool ok) {
-  int r;
-  asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.and.pred q, 1, %2, p;\n"
-      " selp.b32 %0, 1, 0, q;\n}\n"
-      : "=r"(r)
-      : "r"(int(ok)), "n"(CONVERTERS)
-      : "memory");
-  return r != 0;
-}
 
 #define QFX_SETMAXNREG_DEC(n) asm volatile("setmaxnreg.dec.sync.aligned.u32 " #n ";")
 #define QFX_SETMAXNREG_INC(n) asm volatile("setmaxnreg.inc.sync.aligned.u32 " #n ";")
 
 __global__ void __launch_bounds__(THREADS, 1)
-    cgemm_fp16x3_direct_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
-                               const __grid_constant__ AGather g, const float2* __restrict__ A,
-                               float2* __restrict__ C, int tma_c, int m, int n, int k, int batches,
-                               std::uint64_t ac_stride, int* __restrict__ err, int CHUNK,
+    cgemm_fp16x3_direct_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                               const __grid_constant__ CUtensorMap map_c, const __grid_constant__ AGather g,
+                               const float2* __restrict__ A, float2* __restrict__ C, int tma_c, int m, int n, int k,
+                               int batches, std::uint64_t ac_stride, int* __restrict__ err,
                                const int* __restrict__ exp_b) {
   extern __shared__ __align__(1024) std::uint8_t smem[];
   std::uint64_t* raw_full = reinterpret_cast<std::uint64_t*>(smem + OFF_BAR);  // a block of A has landed
-  std::uint64_t* a_full = raw_full + A_RING;                                   // its planes are written
-  std::uint64_t* a_empty = a_full + A_RING;                                    // its MMAs are done
-  std::uint64_t* b_full = a_empty + A_RING;
-  std::uint64_t* b_empty = b_full + B_STAGES;
-  std::uint64_t* acc_full = b_empty + B_STAGES;
-  std::uint64_t* acc_empty = acc_full + 2;
-  std::uint64_t* mma_done = acc_empty + 2;
+  std::uint64_t* raw_empty = raw_full + A_RING;                                // and is in registers
+  std::uint64_t* a_full = raw_empty + A_RING;                                  // its planes are in TMEM
+  std::uint64_t* b_full = a_full + A_BUFS;
+  std::uint64_t* re_full = b_full + B_STAGES;   // a block's real part is summed
+  std::uint64_t* done = re_full + DONE;         // all MMAs of a block are done
+  std::uint64_t* acc_empty = done + DONE;       // an accumulator was drained
+  std::uint64_t* mma_done = acc_empty + HALVES;
   std::uint32_t* tmem_slot = reinterpret_cast<std::uint32_t*>(mma_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   if (smem_u32(smem) & 1023) {  // the swizzles need it; the layout leaves no room to round up
@@ -189,27 +206,31 @@ __global__ void __launch_bounds__(THREADS, 1)
   auto wait = [&](std::uint64_t* bar, std::uint32_t parity, int code) {
     return mbar_wait(bar, parity, abort_flag, err, code);
   };
-  const int kblocks = (k + 15) / 16;       // k-steps
-  const int blocks = (kblocks + 1) / 2;    // blocks of A
+  const int blocks = (k + 31) / 32;
+  // Blocks of all the CTA's tiles.
+  const int work = first < total ? ((total - 1 - first) / stride + 1) * blocks : 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < A_RING; ++s) {
-      mbar_init(&raw_full[s], LOADERS);
-      mbar_init(&a_full[s], CONVERTERS / 32);
-      mbar_init(&a_empty[s], 1);
+      mbar_init(&raw_full[s], g.boxes ? 1 : LOADERS);
+      mbar_init(&raw_empty[s], CONVERTERS / 32);
     }
-    for (int s = 0; s < B_STAGES; ++s) {
-      mbar_init(&b_full[s], 1);
-      mbar_init(&b_empty[s], 1);
+    for (int s = 0; s < A_BUFS; ++s) mbar_init(&a_full[s], CONVERTERS / 32);
+    for (int s = 0; s < B_STAGES; ++s) mbar_init(&b_full[s], 1);
+    for (int s = 0; s < DONE; ++s) {
+      mbar_init(&re_full[s], 1);
+      mbar_init(&done[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 8);
-    }
+    for (int s = 0; s < HALVES; ++s) mbar_init(&acc_empty[s], 8);
     mbar_init(mma_done, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // The second half of a block that a k of 16 does not have.
+  if (g.boxes && !g.plain && g.copies_real < 32)
+    for (int i = threadIdx.x; i < A_RING * A_BLOCK / 32; i += THREADS)
+      *reinterpret_cast<float4*>(smem + i / (A_BLOCK / 32) * A_BLOCK + A_BLOCK / 2 + i % (A_BLOCK / 32) * 16) =
+          make_float4(0.f, 0.f, 0.f, 0.f);
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TMEM_COLS));
@@ -225,21 +246,24 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (warp == 0 && lane == 0) {
       // B producer.
       int q = 0, s = 0;
-      std::uint32_t ph = 0;
       for (int t = first; t < total && !*abort_flag; t += stride) {
         int mt, nt, batch;
         tile_of(t, mt, nt, batch);
-        for (int kb = 0; kb < kblocks; ++kb) {
-          if (q >= B_STAGES && !wait(&b_empty[s], ph ^ 1u, 1)) break;
+        for (int b = 0; b < blocks; ++b) {
+          if (q >= B_STAGES) {
+            const int free = q - B_STAGES;
+            if (!wait(&done[free % DONE], (free / DONE) & 1, 1)) break;
+          }
+          // A k of an odd number of k-steps: the last one's rows lie outside
+          // the map and arrive as zeros.
           std::uint8_t* st = smem + OFF_B + s * B_STAGE;
           mbar_expect_tx(&b_full[s], B_STAGE);
-          tma_load_4d(&map_b, &b_full[s], st, 0, nt * BN, kb, batch);
-          tma_load_4d(&map_b, &b_full[s], st + B_PART, 32, nt * BN, kb, batch);
+          tma_load_4d(&map_b, &b_full[s], st, 0, nt * BN, 2 * b, batch);
+          tma_load_4d(&map_b, &b_full[s], st + B_PART, 32, nt * BN, 2 * b, batch);
+          tma_load_4d(&map_b, &b_full[s], st + 2 * B_PART, 0, nt * BN, 2 * b + 1, batch);
+          tma_load_4d(&map_b, &b_full[s], st + 3 * B_PART, 32, nt * BN, 2 * b + 1, batch);
           ++q;
-          if (++s == B_STAGES) {
-            s = 0;
-            ph ^= 1u;
-          }
+          if (++s == B_STAGES) s = 0;
         }
       }
       if (*abort_flag) {
@@ -258,66 +282,97 @@ __global__ void __launch_bounds__(THREADS, 1)
       // beside the other warps' work a k-step took 980 cycles instead of 775
       // (768 at the tensor pipe's rate; measured with this k-step, its
       // commits and barrier tests, a TMEM drain and shared-memory traffic).
-      // Chunk c (CHUNK k-steps of one tile, c counts across tiles)
-      // accumulates from zero into TMEM buffer c % 2.
+      // What the warp does between two MMAs counts as well: a block's MMAs
+      // take 1536 cycles, and a loop with five waits, each by the whole warp,
+      // and five commits a block took 2370. So a block waits twice, its lanes
+      // testing different barriers, and commits twice.
+      //
+      // A block is summed from zero, first its real, then its imaginary part,
+      // each into the next of the three TMEM buffers. Lane kinds: 0 and 3
+      // wait for the buffers of the real and the imaginary part, 1 for A's
+      // planes, 2 for B's.
       const bool leader = elect_one();
-      const std::uint64_t da = smem_desc_sw128(smem_u32(smem)), db = smem_desc_sw64(smem_u32(smem + OFF_B));
-      const std::uint32_t a_hi = std::uint32_t(da >> 32), b_hi = std::uint32_t(db >> 32);
-      const std::uint32_t a_lo0 = std::uint32_t(da), b_lo0 = std::uint32_t(db);
-      auto wait_all = [&](std::uint64_t* bar, std::uint32_t parity, int code) {
-        return __all_sync(0xffffffffu, wait(bar, parity, code));
-      };
-      int sa = 0, sb = 0, c = 0, kc = 0;
-      std::uint32_t pa = 0, pb = 0;
-      bool go = true;
-      for (int t = first; t < total && go; t += stride) {
-        kc = 0;
-        for (int kb = 0; kb < kblocks; ++kb) {
-          const int buf = c & 1;
-          const bool start = kc == 0;
-          if (start && c >= 2) {
-            // The epilogue's TMEM reads of this buffer precede the MMAs that
-            // overwrite it.
-            if (!wait_all(&acc_empty[buf], ((c >> 1) - 1) & 1, 4)) {
-              go = false;
-              break;
+      const std::uint64_t db = smem_desc_sw64(smem_u32(smem + OFF_B));
+      const std::uint32_t b_hi = std::uint32_t(db >> 32), b_lo0 = std::uint32_t(db);
+      const int kind = lane & 3;
+      std::uint64_t* const bars = kind == 1 ? a_full : kind == 2 ? b_full : acc_empty;
+      const int ring = kind == 1 ? A_BUFS : kind == 2 ? B_STAGES : HALVES;
+      const int step = kind == 1 || kind == 2 ? 1 : 2;
+      int at = kind == 3 ? 1 : 0;
+      std::uint32_t parity = kind == 1 || kind == 2 ? 0u : 1u;  // a fresh buffer is empty
+      int xa = 0, sb = 0, h = 0, r = 0;
+      for (int w = 0; w < work; ++w) {
+        if (!__all_sync(0xffffffffu, kind == 3 || wait(bars + at, parity, 2))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const std::uint32_t a = tmem + TMEM_A + xa * TMEM_A_BLOCK, b = b_lo0 + sb * (B_STAGE >> 4);
+        if (leader) {
+          mma_block<0>(tmem + h * BN, a, b, b_hi);
+          umma_commit(&re_full[r]);
+        }
+        h = h == HALVES - 1 ? 0 : h + 1;
+        // The epilogue's TMEM reads of a buffer precede the MMAs that
+        // overwrite it.
+        if (!__all_sync(0xffffffffu, kind != 3 || wait(bars + at, parity, 4))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (leader) {
+          mma_block<1>(tmem + h * BN, a, b, b_hi);
+          umma_commit(&done[r]);
+        }
+        h = h == HALVES - 1 ? 0 : h + 1;
+        xa ^= 1;
+        sb = sb == B_STAGES - 1 ? 0 : sb + 1;
+        r = r == DONE - 1 ? 0 : r + 1;
+        at += step;
+        if (at >= ring) {
+          at -= ring;
+          parity ^= 1u;
+        }
+      }
+      __syncwarp();
+      if (leader) umma_commit(mma_done);
+      __syncwarp();
+    } else if (warp >= 2 && g.boxes) {
+      // A loader, by TMA boxes.
+      if (warp == 2 && lane == 0) {
+        const std::uint32_t ring = smem_u32(smem);
+        const std::uint32_t bytes = g.copies_real == 32 ? A_BLOCK : A_BLOCK / 2;
+        int q = 0, s = 0;
+        std::uint32_t ph = 0;
+        for (int t = first; t < total && !*abort_flag; t += stride) {
+          int mt, nt, batch;
+          tile_of(t, mt, nt, batch);
+          std::uint64_t tile_src = std::uint64_t(batch) * ac_stride;
+          if (!g.plain)
+            for (int x = 0; x < AGather::kBits && (mt >> x); ++x)
+              if ((mt >> x) & 1) tile_src += g.tile_src[x];
+          for (int b = 0; b < blocks; ++b) {
+            if (q >= A_RING && !wait(&raw_empty[s], ph ^ 1u, 5)) break;
+            const std::uint32_t dst = ring + s * A_BLOCK;
+            mbar_expect_tx(&raw_full[s], bytes);
+            if (g.plain) {
+              tma_load_3d(&map_a, &raw_full[s], dst, b * 32, mt * BM, batch);
+              tma_load_3d(&map_a, &raw_full[s], dst + A_BLOCK / 2, b * 32 + 16, mt * BM, batch);
+            } else {
+              std::uint64_t src = tile_src;
+              for (int x = 0; x < AGather::kBits && (b >> x); ++x)
+                if ((b >> x) & 1) src += g.block_src[x];
+              tma_load_5d(&map_a, &raw_full[s], dst, int(src / 16));
             }
-            asm volatile("tcgen05.fence::after_thread_sync;");
+            ++q;
+            if (++s == A_RING) {
+              s = 0;
+              ph ^= 1u;
+            }
           }
-          if (!(kb & 1) && !wait_all(&a_full[sa], pa, 7)) {
-            go = false;
-            break;
-          }
-          if (!wait_all(&b_full[sb], pb, 2)) {
-            go = false;
-            break;
-          }
-          const bool block_end = (kb & 1) || kb == kblocks - 1;
-          const bool chunk_end = ++kc == CHUNK || kb == kblocks - 1;
-          if (leader) {
-            mma_kstep(tmem + buf * 2 * BN, a_lo0 + ((sa * A_BLOCK + (kb & 1) * (A_BLOCK / 2)) >> 4), a_hi,
-                      b_lo0 + ((sb * B_STAGE) >> 4), b_hi, start ? 0u : 1u);
-            umma_commit(&b_empty[sb]);
-            if (block_end) umma_commit(&a_empty[sa]);
-            if (chunk_end) umma_commit(&acc_full[buf]);
-          }
-          __syncwarp();
-          if (++sb == B_STAGES) {
-            sb = 0;
-            pb ^= 1u;
-          }
-          if (block_end && ++sa == A_RING) {
-            sa = 0;
-            pa ^= 1u;
-          }
-          if (chunk_end) {
-            ++c;
-            kc = 0;
+        }
+        if (*abort_flag) {
+          for (int w = q > A_RING ? q - A_RING : 0; w < q; ++w) {
+            const unsigned long long t0 = now_ns();
+            while (!mbar_test(&raw_full[w % A_RING], (w / A_RING) & 1) && now_ns() - t0 < WAIT_NS) {
+            }
           }
         }
       }
-      if (leader) umma_commit(mma_done);
-      __syncwarp();
     } else if (warp >= 2) {
       // A loader. A block is 2048 copies of 16 bytes (a pair of elements
       // adjacent in the source); thread lt takes copies lt + 64 i, whose
@@ -344,7 +399,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int b = 0; b < AGather::kBits && (mt >> b); ++b)
             if ((mt >> b) & 1) tile_src += g.tile_src[b];
         for (int b = 0; b < blocks; ++b) {
-          if (q >= A_RING && !wait(&a_empty[s], ph ^ 1u, 5)) {
+          if (q >= A_RING && !wait(&raw_empty[s], ph ^ 1u, 5)) {
             ok = false;
             break;
           }
@@ -355,7 +410,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int x = 0; x < AGather::kBits && (b >> x); ++x)
               if ((b >> x) & 1) src += g.block_src[x];
           const std::uint32_t dst = ring + s * A_BLOCK;
-          if (!g.plain || (g.aligned && (mt + 1) * BM <= m && (b + 1) * 32 <= k)) {
+          if (!g.plain) {
             // Copies from copies_real on belong to the half of a block that a
             // k of 16 does not have: zeros.
 #pragma unroll
@@ -363,25 +418,17 @@ __global__ void __launch_bounds__(THREADS, 1)
               cp_async16(dst + (lane_dst ^ g.copy_dst[i]), i < g.copies_real ? src + g.copy_src[i] : A,
                          i < g.copies_real ? 16u : 0u);
           } else {
-            // Edge blocks and rows that are not 16-byte aligned (plain rows:
-            // copy u covers row u / 16, values 2 (u % 16) and the next).
-            const int have = min(2, k - (b * 32 + 2 * (lt & 15)));  // values of a pair that exist
+            // Rows that are not 16-byte aligned (copy u covers row u / 16,
+            // values 2 (u % 16) and the next).
+            const int have = k - (b * 32 + 2 * (lt & 15));  // values from the pair on
             const int rows = have > 0 ? m - (mt * BM + (lt >> 4)) : 0;
-            if (g.aligned) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const bool in = 4 * i < rows;
-                cp_async16(dst + (lane_dst ^ g.copy_dst[i]), in ? src + g.copy_src[i] : A, in ? 8u * have : 0u);
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const bool in = 4 * i < rows, in2 = in && have > 1;
-                const float2* from = src + g.copy_src[i];
-                const std::uint32_t to = dst + (lane_dst ^ g.copy_dst[i]);
-                cp_async8(to, in ? from : A, in ? 8u : 0u);
-                cp_async8(to + 8, in2 ? from + 1 : A, in2 ? 8u : 0u);
-              }
+            for (int i = 0; i < 32; ++i) {
+              const bool in = 4 * i < rows, in2 = in && have > 1;
+              const float2* from = src + g.copy_src[i];
+              const std::uint32_t to = dst + (lane_dst ^ g.copy_dst[i]);
+              cp_async8(to, in ? from : A, in ? 8u : 0u);
+              cp_async8(to + 8, in2 ? from + 1 : A, in2 ? 8u : 0u);
             }
           }
           cp_async_arrive(&raw_full[s]);
@@ -403,91 +450,76 @@ __global__ void __launch_bounds__(THREADS, 1)
       if ((row >> b) & 1) row_at ^= g.row_at[b];
     std::int8_t* exps = reinterpret_cast<std::int8_t*>(smem + OFF_EXP);
     const std::uint32_t ring = smem_u32(smem);
-    int s = 0, x = 0;
-    std::uint32_t ph = 0;
-    bool ok = true;
-    for (int t = first; t < total && ok; t += stride) {
-      for (int b = 0; b < blocks; ++b) {
-        const bool here = wait(&raw_full[s], ph, 6);
-        const std::uint32_t block = ring + s * A_BLOCK;
-        float2 v[32];
-        if (here) {
-          if (g.pairs) {
+    const std::uint32_t lanes = tmem + TMEM_A + (std::uint32_t((warp - 12) * 32) << 16);
+    int s = 0, x = 0, xa = 0, r = DONE - A_BUFS;
+    std::uint32_t ph = 0, pd = 1;  // block w - A_BUFS: barrier r
+    for (int w = 0; w < work; ++w) {
+      if (!__all_sync(0xffffffffu, wait(&raw_full[s], ph, 6))) break;
+      const std::uint32_t block = ring + s * A_BLOCK;
+      float2 v[32];
+      if (g.pairs) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 2)
-              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                           : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i + 1].x), "=f"(v[i + 1].y)
-                           : "r"(block + (row_at ^ g.value_at[i]))
-                           : "memory");
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-                           : "=f"(v[i].x), "=f"(v[i].y)
-                           : "r"(block + (row_at ^ g.value_at[i]))
-                           : "memory");
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = make_float2(0.f, 0.f);
-        }
-        // Every row is in registers before any thread writes planes over the
-        // block.
-        if (!converters_all(here)) {
-          ok = false;
-          break;
-        }
-        // Bit patterns of non-negative floats order like their values.
-        std::uint32_t mx[4] = {0u, 0u, 0u, 0u};
+        for (int i = 0; i < 32; i += 2)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i + 1].x), "=f"(v[i + 1].y)
+                       : "r"(block + (row_at ^ g.value_at[i]))
+                       : "memory");
+      } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i)
-          mx[i & 3] = max(mx[i & 3], max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
-        // e with max * 2^e in [2^14, 2^15), at most 126 (2^e and 2^-e stay
-        // normal floats; smaller blocks keep all their bits: below 2^-112 the
-        // lo planes reach further down than FP32 itself). A block of zeros
-        // takes 126 so that it never sets the scale of the sum; infinities
-        // and NaN keep 0.
-        const int be = int(max(max(mx[0], mx[1]), max(mx[2], mx[3])) >> 23);
-        const int e = be == 255 ? 0 : min(141 - be, 126);
-        const float sc = __uint_as_float(std::uint32_t(e + 127) << 23);
-        const float2 sc2 = make_float2(sc, sc);
+          asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                       : "=f"(v[i].x), "=f"(v[i].y)
+                       : "r"(block + (row_at ^ g.value_at[i]))
+                       : "memory");
+      }
+      // Bit patterns of non-negative floats order like their values.
+      std::uint32_t mx[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-        for (int i = 0; i < 32; i += 8) {  // 8 values: one 16-byte unit of every plane
-          std::uint32_t rh[4], rl[4], ih[4], il[4];
+      for (int i = 0; i < 32; ++i)
+        mx[i & 3] = max(mx[i & 3], max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
+      // e with max * 2^e in [2^14, 2^15), at most 126 (2^e and 2^-e stay
+      // normal floats; smaller blocks keep all their bits: below 2^-112 the
+      // lo planes reach further down than FP32 itself). A block of zeros
+      // takes 126 so that it never sets the scale of the sum; infinities
+      // and NaN keep 0.
+      const int be = int(max(max(mx[0], mx[1]), max(mx[2], mx[3])) >> 23);
+      const int e = be == 255 ? 0 : min(141 - be, 126);
+      const float sc = __uint_as_float(std::uint32_t(e + 127) << 23);
+      const float2 sc2 = make_float2(sc, sc);
+      // The block is in registers: its place in the ring is free.
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&raw_empty[s]);
+      if (!__all_sync(0xffffffffu, wait(&done[r], pd, 10))) break;
+      if (++r == DONE) {
+        r = 0;
+        pd ^= 1u;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
-            const float2 r = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
-            split_pair(r.x, r.y, rh[j], rl[j]);
-            split_pair(im.x, im.y, ih[j], il[j]);
-          }
-          // k-step i / 16; unit u of the 128-byte row (two per plane) lies at
-          // u ^ (row % 8).
-          const std::uint32_t at = block + (i / 16) * (A_BLOCK / 2) + row * 128;
-          const std::uint32_t h = (i / 8) & 1;
-          auto put = [&](std::uint32_t u, const std::uint32_t* w) {
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + (((u + h) ^ (row & 7)) << 4)), "r"(w[0]),
-                         "r"(w[1]), "r"(w[2]), "r"(w[3])
-                         : "memory");
-          };
-          put(0, rh);
-          put(2, rl);
-          put(4, ih);
-          put(6, il);
+      for (int i = 0; i < 32; i += 16) {  // a k-step: 8 words of every plane
+        std::uint32_t p[32];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
+          const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
+          split_pair(re.x, re.y, p[j], p[8 + j]);
+          split_pair(im.x, im.y, p[16 + j], p[24 + j]);
         }
-        // Exponents live in a ring of their own: this block is at most four
-        // ahead of the one the slowest epilogue warp drains (its MMAs are
-        // done with the block three back, which needed all chunks up to five
-        // back drained).
-        exps[x * BM + row] = std::int8_t(e);
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&a_full[s]);
-        if (++x == EXP_RING) x = 0;
-        if (++s == A_RING) {
-          s = 0;
-          ph ^= 1u;
-        }
+        tmem_st32(lanes + xa * TMEM_A_BLOCK + i * 2, p);
+      }
+      // Exponents live in a ring of their own: the MMAs of the block two
+      // back are done, so every epilogue warp has read the exponents of the
+      // block three back.
+      exps[x * BM + row] = std::int8_t(e);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&a_full[xa]);
+      xa ^= 1;
+      if (++x == EXP_RING) x = 0;
+      if (++s == A_RING) {
+        s = 0;
+        ph ^= 1u;
       }
     }
   } else {
@@ -503,12 +535,34 @@ __global__ void __launch_bounds__(THREADS, 1)
     const std::int8_t* exps = reinterpret_cast<const std::int8_t*>(smem + OFF_EXP);
     std::uint8_t* staging = smem + OFF_STAGING + (warp - 4) * 2 * SLOT;
     int* sc_row = reinterpret_cast<int*>(smem + OFF_SCALE) + (warp - 4) * COLS;
-    const float beta = debias_beta<KIND_FP16>(err, CHUNK, kblocks);
+    const float beta = debias_beta<KIND_FP16>(err, 2, (k + 15) / 16);
     const float2 beta2 = make_float2(beta, beta);
-    const int per_block = CHUNK == 1 ? 2 : 1;  // chunks of a whole block
-    const int chunks = (kblocks + CHUNK - 1) / CHUNK;
-    int c = 0, x = 0;
+    int h = 0, x = 0, r = 0;
+    std::uint32_t pr = 0;
     bool ok = true;
+    const std::uint32_t base0 = tmem + (std::uint32_t(q * 32) << 16) + part * COLS;
+    // Adds the next TMEM buffer, times `f`, to `sum`.
+    auto drain = [&](float2(&sum)[COLS / 2], float2 f) {
+      const std::uint32_t base = base0 + h * BN;
+#pragma unroll
+      for (int j0 = 0; j0 < COLS; j0 += 32) {
+        std::uint32_t v0[16], v1[16];
+        TMEM_LD16(base + j0, v0);
+        TMEM_LD16(base + j0 + 16, v1);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float2& a = sum[j0 / 2 + j];
+          float2& b = sum[j0 / 2 + 8 + j];
+          a = fma2(make_float2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1])), f, a);
+          b = fma2(make_float2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1])), f, b);
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[h]);
+      h = h == HALVES - 1 ? 0 : h + 1;
+    };
     for (int t = first; t < total && ok; t += stride) {
       int mt, nt, batch;
       tile_of(t, mt, nt, batch);
@@ -526,18 +580,15 @@ __global__ void __launch_bounds__(THREADS, 1)
       // two below the first block's exponent and drops, rescaling the sums,
       // only when a later block is more than four times larger.
       int eref = 0;
-      for (int cc = 0; cc < chunks; ++cc, ++c) {
-        const int buf = c & 1;
-        if (!__all_sync(0xffffffffu, wait(&acc_full[buf], (c >> 1) & 1, 3))) {
+      for (int b = 0; b < blocks; ++b) {
+        if (!__all_sync(0xffffffffu, wait(&re_full[r], pr, 3))) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const int e = exps[x * BM + row];
-        if (cc % per_block == per_block - 1 || cc == chunks - 1) {
-          if (++x == EXP_RING) x = 0;
-        }
-        if (cc == 0) {
+        if (++x == EXP_RING) x = 0;
+        if (b == 0) {
           eref = e - 2;
         } else if (__any_sync(0xffffffffu, e < eref)) {
           const int next = e < eref ? e - 2 : eref;
@@ -552,23 +603,17 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         const float sa = pow2(eref - e);
         const float2 sa2 = make_float2(sa, sa);
-        const std::uint32_t base = tmem + (std::uint32_t(q * 32) << 16) + buf * 2 * BN + part * COLS;
-#pragma unroll
-        for (int j0 = 0; j0 < COLS; j0 += 16) {
-          std::uint32_t vr[16], vi[16];
-          TMEM_LD16(base + j0, vr);
-          TMEM_LD16(base + BN + j0, vi);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int p = j0 / 2 + j;
-            re[p] = fma2(make_float2(__uint_as_float(vr[2 * j]), __uint_as_float(vr[2 * j + 1])), sa2, re[p]);
-            im[p] = fma2(make_float2(__uint_as_float(vi[2 * j]), __uint_as_float(vi[2 * j + 1])), sa2, im[p]);
-          }
+        drain(re, sa2);
+        if (!__all_sync(0xffffffffu, wait(&done[r], pr, 3))) {
+          ok = false;
+          break;
         }
-        asm volatile("tcgen05.fence::before_thread_sync;");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        drain(im, sa2);
+        if (++r == DONE) {
+          r = 0;
+          pr ^= 1u;
+        }
       }
       if (!ok) break;
       // The MMA issuer already works on the next tiles. The columns'
@@ -683,12 +728,13 @@ AGather make_a_rows(std::size_t k, bool aligned) {
   AGather g;
   std::memset(&g, 0, sizeof(g));
   g.plain = 1;
-  g.aligned = aligned ? 1 : 0;
   g.pairs = 1;
   g.copies_real = 32;
-  // Copy u = 16 row + pair; its unit of the block is u with the low three
-  // bits XORed with the row's, so that a quarter-warp of rows reading the
-  // same values hits eight different units.
+  g.boxes = aligned ? 1 : 0;
+  // Boxes: rows of 16 values, 128 bytes, unit u of row r at u ^ (r % 8).
+  // Copies: copy u = 16 row + pair; its unit of the block is u with the low
+  // three bits XORed with the row's. Either way a quarter-warp of rows reading
+  // the same values hits eight different units.
   auto at = [](std::uint32_t u) { return (u ^ ((u >> 4) & 7u)) << 4; };
   for (int b = 0; b < 6; ++b) {
     g.lane_src[b] = b < 4 ? std::uint64_t(2) << b : std::uint64_t(k) << (b - 4);
@@ -697,9 +743,9 @@ AGather make_a_rows(std::size_t k, bool aligned) {
   for (std::uint32_t i = 0; i < 32; ++i) {
     g.copy_src[i] = std::uint64_t(4) * i * k;
     g.copy_dst[i] = at(64u * i);
-    g.value_at[i] = at(i >> 1) | ((i & 1u) << 3);
+    g.value_at[i] = (aligned ? (i >> 4) * (A_BLOCK / 2) | ((i & 15) >> 1) << 4 : at(i >> 1)) | (i & 1u) << 3;
   }
-  for (int b = 0; b < 7; ++b) g.row_at[b] = at(16u << b);
+  for (int b = 0; b < 7; ++b) g.row_at[b] = aligned ? 128u << b ^ (b < 3 ? 16u << b : 0u) : at(16u << b);
   return g;
 }
 
@@ -731,6 +777,7 @@ bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size
   // index, 3 or 4 digits, in one piece; anything else is permuted first.)
   if (at_e[0] != 0 || at_e[1] != 1 || at_e[2] != 2) return false;
   std::memset(g, 0, sizeof(*g));
+  g->nbits = nbits;
   // Where element e of the block (source order) lies: unit e / 2 with its low
   // three bits XORed by one mask per higher bit, chosen so that the low row
   // digits, which the lanes of a reading warp differ in, reach different
@@ -756,7 +803,6 @@ bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size
       if ((u >> b) & 1) x ^= mask[b];
     return (x << 4) | ((e & 1u) << 3);
   };
-  g->aligned = 1;
   g->pairs = val_e[0] == 0 ? 1 : 0;
   g->copies_real = kb < 5 ? 16 : 32;
   for (int b = 0; b < 6; ++b) {
@@ -773,6 +819,50 @@ bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size
     g->value_at[i] = at(e);
   }
   for (int d = 0; d < 7; ++d) g->row_at[d] = at(1u << row_e[d]);
+  // As one TMA box when the block is 16 neighbours by at most three runs of
+  // neighbouring digits: the run with the lowest row digit that is not among
+  // the 16 comes next to them, where the 128-byte swizzle spreads the rows
+  // that a reading warp's lanes differ in.
+  if (at_e[3] == 3) {
+    int start[4], len[4], runs = 0;
+    for (int e = 4; e < n_e; ++e) {
+      if (e == 4 || at_e[e] != at_e[e - 1] + 1) {
+        if (runs == 3) {
+          runs = 4;
+          break;
+        }
+        start[runs] = e;
+        len[runs++] = 0;
+      }
+      ++len[runs - 1];
+    }
+    if (runs <= 3) {
+      int low = 0;
+      while (low < 6 && row_e[low] < 4) ++low;
+      for (int x = 1; x < runs; ++x)
+        if (row_e[low] >= start[x] && row_e[low] < start[x] + len[x]) {
+          std::swap(start[0], start[x]);
+          std::swap(len[0], len[x]);
+        }
+      std::uint32_t box_at[12];  // where the block's digits lie in the box
+      for (int e = 0; e < 4; ++e) box_at[e] = 8u << e;
+      std::uint32_t next = 128;
+      for (int x = 0; x < 3; ++x) {
+        g->run_bits[x] = x < runs ? len[x] : 0;
+        g->run_src[x] = x < runs ? std::uint64_t(1) << at_e[start[x]] : 16;
+        for (int e = 0; e < g->run_bits[x]; ++e, next <<= 1)
+          box_at[start[x] + e] = next < 1024 ? next | next >> 3 : next;
+      }
+      box_at[11] = n_e == 11 ? 1u << 14 : box_at[11];
+      g->boxes = 1;
+      for (std::uint32_t i = 0; i < 32; ++i) {
+        g->value_at[i] = 0;
+        for (int q = 0; q < 5; ++q)
+          if ((i >> q) & 1) g->value_at[i] ^= box_at[val_e[q]];
+      }
+      for (int d = 0; d < 7; ++d) g->row_at[d] = box_at[row_e[d]];
+    }
+  }
   for (int b = 0; kl + 7 + b < nbits; ++b) g->tile_src[b] = std::uint64_t(1) << from[kl + 7 + b];
   for (int b = 0; 5 + b < kl; ++b) g->block_src[b] = std::uint64_t(1) << from[5 + b];
   return true;
@@ -788,7 +878,22 @@ void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const floa
         if ((b >> x) & 1) base += g.block_src[x];
       }
       std::fill(block.begin(), block.end(), make_float2(NAN, NAN));
-      for (int u = 0; u < 2048; ++u) {
+      if (g.boxes && g.copies_real < 32)
+        std::fill(block.begin() + A_BLOCK / 16, block.end(), make_float2(0.f, 0.f));
+      const std::uint32_t rows = 8u << (g.run_bits[0] + g.run_bits[1] + g.run_bits[2] + 4);
+      if (g.boxes && rows != (g.copies_real == 32 ? A_BLOCK : A_BLOCK / 2))
+        throw std::string("ERROR (qflex_gb300: product) --> box of a wrong size");
+      for (std::uint32_t at = 0; g.boxes && at < rows; at += 8) {
+        std::uint64_t from = base + ((at >> 3) & 15);
+        std::uint32_t rest = at >> 7;
+        for (int x = 0; x < 3; ++x) {
+          from += (rest & ((1u << g.run_bits[x]) - 1)) * g.run_src[x];
+          rest >>= g.run_bits[x];
+        }
+        if (base % 16 || from >= m * k) throw std::string("ERROR (qflex_gb300: product) --> box out of range");
+        block[(at ^ ((at >> 3) & 0x70)) / 8] = src[from];
+      }
+      for (int u = 0; !g.boxes && u < 2048; ++u) {
         std::uint64_t from = base + g.copy_src[u / LOADERS];
         std::uint32_t to = g.copy_dst[u / LOADERS];
         for (int x = 0; x < 6; ++x)
@@ -824,24 +929,53 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
                                 std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
                                 cudaStream_t s) {
   if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
-  if (cfg.chunk < 1 || cfg.chunk > 2)
-    throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct product takes chunks of 1 or 2 k-steps");
+  if (cfg.chunk != 2)
+    throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct product takes chunks of 2 k-steps");
   static std::once_flag attr;
   std::call_once(attr, [] {
     check(cudaFuncSetAttribute(cgemm_fp16x3_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM),
           "cudaFuncSetAttribute");
   });
+  if (gather.boxes && !gather.plain && batch > 1) {
+    if (ac_stride % 16) throw std::string("ERROR (qflex_gb300: tensor cores) --> batch stride of a gathered operand");
+    // The box's last coordinate counts 128 bytes in 31 bits.
+    const std::uint64_t most = ((std::uint64_t(1) << 35) - (std::uint64_t(1) << gather.nbits)) / ac_stride + 1;
+    if (most < (std::uint64_t)batch) {
+      for (int at = 0; at < batch; at += (int)most)
+        launch_cgemm_fp16x3_direct(A + at * ac_stride, gather, B + at * b_stride, b_layout, C + at * ac_stride, m, n, k,
+                                   ac_stride, b_stride, (int)std::min<std::uint64_t>(most, batch - at), workspace, err,
+                                   cfg, s);
+      return;
+    }
+  }
   const std::size_t kpad = (k + 15) / 16 * 16;
   __half* pb = reinterpret_cast<__half*>(workspace);
   int* eb = reinterpret_cast<int*>(pb + 4 * n * kpad * (std::size_t)batch);
   std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
   launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, BN, 64);
+  CUtensorMap ma;
+  std::memset(&ma, 0, sizeof(ma));
+  if (gather.boxes && gather.plain) {
+    const std::uint64_t dims[3] = {k, m, (std::uint64_t)batch};
+    const std::uint64_t strides[2] = {k * 8, (batch > 1 ? ac_stride : m * k + (m * k & 1)) * 8};
+    const std::uint32_t box[3] = {16, BM, 1};
+    ma = element_map(A, 3, dims, strides, box);
+  } else if (gather.boxes) {
+    const std::uint64_t units = ((batch - 1) * ac_stride + (std::uint64_t(1) << gather.nbits)) / 16;
+    std::uint64_t dims[5] = {16, 1, 1, 1, units}, strides[4] = {0, 0, 0, 128};
+    std::uint32_t box[5] = {16, 1, 1, 1, 1};
+    for (int x = 0; x < 3; ++x) {
+      dims[1 + x] = box[1 + x] = 1u << gather.run_bits[x];
+      strides[x] = gather.run_src[x] * 8;
+    }
+    ma = element_map(A, 5, dims, strides, box);
+  }
   CUtensorMap mc;
   const int tma_c = output_map(C, m, n, ac_stride, batch, &mc) ? 1 : 0;
   const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * (std::size_t)batch;
   cgemm_fp16x3_direct_kernel<<<persistent_grid(tiles), THREADS, SMEM, s>>>(
-      mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err, cfg.chunk, eb);
+      ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err, eb);
   check(cudaGetLastError(), "cgemm_fp16x3_direct");
 }
 

@@ -1133,6 +1133,27 @@ CUtensorMap plane_map_f16(const __half* base, std::uint64_t rows, std::uint64_t 
   return map;
 }
 
+CUtensorMap element_map(const float2* base, int rank, const std::uint64_t* dims, const std::uint64_t* strides,
+                        const std::uint32_t* box) {
+  CUtensorMap map;
+  std::memset(&map, 0, sizeof(map));
+  cuuint64_t d[5], st[4];
+  cuuint32_t b[5], e[5];
+  for (int i = 0; i < rank; ++i) {
+    d[i] = dims[i];
+    if (i) st[i - 1] = strides[i - 1];
+    b[i] = box[i];
+    e[i] = 1;
+  }
+  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (cuuint32_t)rank, const_cast<float2*>(base), d, st,
+                           b, e, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
+        std::to_string((int)r);
+  return map;
+}
+
 // 3-D map over C as floats [batch][m][2n] for the epilogue's bulk stores,
 // box {32, 32, 1} (32 rows x 16 complex) in the 128-byte swizzle, or with
 // `narrow` {16, 32, 1} (8 complex) in the 64-byte swizzle. False (and the

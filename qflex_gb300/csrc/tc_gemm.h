@@ -67,10 +67,14 @@ void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, flo
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s,
                          bool a_in_planes = false);
 
-// Where the direct 3xFP16 product finds A: copies of 16 bytes (two elements
-// adjacent in the source) fill a block of 128 rows x 32 values, copy
+// Where the direct 3xFP16 product finds A: TMA boxes or, where no box fits,
+// cp.async copies (16 bytes: two elements adjacent in the source; 8 bytes for
+// plain rows on odd addresses) fill a block of 128 rows x 32 values, copy
 // u = lt + 64 i by loader thread lt. Offsets of sources are in elements and
-// add up, offsets into the block are in bytes and combine by XOR.
+// add up, offsets into the block are in bytes and combine by XOR. With boxes
+// one thread issues two copies or one a block, where 64 threads spent 2000
+// cycles issuing 32 each: (65536, 256, 256) x 4 323 -> 308 us, (3001, 690,
+// 1100) 63 -> 42 us.
 struct AGather {
   static constexpr int kBits = 26;
   std::uint64_t copy_src[32];   // copy i's part of the source offset
@@ -82,9 +86,15 @@ struct AGather {
   std::uint32_t row_at[7];      // of each bit of a row, where its values are read
   std::uint32_t value_at[32];   // of each value of a row
   std::int32_t plain;           // rows of k values: tiles and blocks by arithmetic
-  std::int32_t aligned;         // plain: every row starts on 16 bytes
   std::int32_t pairs;           // values 2 j and 2 j + 1 of a row are adjacent
   std::int32_t copies_real;     // copies i below this exist (16 when k = 16)
+  // TMA boxes instead of copies. Plain: two boxes of 128 rows x 16 values.
+  // Otherwise one box whose dimensions are the 16 lowest digits' values (rows
+  // of 128 bytes), then `runs` of neighbouring digits.
+  std::int32_t boxes;
+  std::int32_t run_bits[3];
+  std::uint64_t run_src[3];     // source offset of a run's lowest digit
+  std::int32_t nbits;           // digits of the source (not plain)
 };
 // A as m rows of k values; `aligned`: base, row and batch strides are
 // multiples of 16 bytes.
@@ -103,8 +113,8 @@ void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const floa
 std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k);
 // The same product with A split inside the kernel: A is read as complex64
 // through `gather`, every 32 values of a row scaled by their own power of
-// two, and no A planes exist in memory. Single CTA, cfg.chunk 1 or 2 (a TMEM
-// chunk never spans two of A's blocks); cfg.variant is ignored.
+// two, and no A planes exist in memory. Single CTA, cfg.chunk 2 (a TMEM
+// chunk is one of A's blocks); cfg.variant is ignored.
 void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* B, BLayout b_layout, float2* C,
                                 std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
                                 std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
