@@ -211,6 +211,16 @@ bool Engine::direct_product(std::size_t n, const TcConfig& cfg) const {
   return precision_ == FP16X3 && cfg.variant == 0 && cfg.chunk == 2 && n <= 1024;
 }
 
+// Products of 16 to 63 columns in the direct kernel's tiles of 32 or 64, from
+// the number of terms on where its error is below that of FP32 sums (see
+// split_multiply): A is then nearly all there is to read. FP32 products
+// against these, with B's split: (1048576, 16, 256) 746 and 361 us, (131072,
+// 32, 256) 194 and 63, (256, 16, 256) 39 and 15, (1000, 50, 100) 26 and 14.
+// Contractions with fewer rows may run as one small program instead.
+bool Engine::narrow_product(std::size_t m, std::size_t n, std::size_t k) const {
+  return m >= 256 && n >= 16 && n < 64 && k >= 96 && tc_runs(m, n, k) && direct_product(n, tc_config(m, n, k));
+}
+
 std::size_t Engine::workspace_elems(std::size_t m, std::size_t n, std::size_t k) const {
   return direct_product(n, tc_config(m, n, k)) ? tc_direct_workspace_elems(n, k) : tc_workspace_elems(m, n, k);
 }
@@ -279,6 +289,7 @@ void Engine::check_error_flag() {
 // 1024 8.1 / 1.9 / 2.1 / 2.5e-7. (3001, 690, 1100) in 3xFP16: 424 -> 65 us.
 bool Engine::split_multiply(std::size_t m, std::size_t n, std::size_t k) const {
   if (m >= 64 && n >= 64 && k >= 96 && tc_runs(m, n, k)) return true;
+  if (narrow_product(m, n, k)) return true;
   return tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
 }
 
@@ -351,8 +362,8 @@ Engine::Plan* Engine::get_plan(const std::string& circuit, const std::string& or
   key += open_terminals_ ? "o" : "p";
   key += std::to_string(exact_gates_);
   if (!fuse_splits_) key += "n";
-  if (precision_ == FP16X3 && fuse_splits_) {
-    // What decides which products read A through a permutation.
+  if (precision_ == FP16X3) {
+    // What decides which products run in the direct kernel.
     key += cat("f", tc_cfg_.chunk == 2 ? 1 : 0, ",", tc_cfg_.variant);
     for (const auto& [shape, variant] : tc_variant_)
       key += cat(";", std::get<0>(shape), ",", std::get<1>(shape), ",", std::get<2>(shape), ",", variant);
@@ -680,7 +691,9 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
   if (!p.built) {
     p.net = build_network(p.circuit, p.grid, initial, results[0].final_state, final_qubits, p.ops);
     std::function<bool(std::size_t, std::size_t, std::size_t)> b_kmajor;
-    if (precision_ != FP32 && !is_complex128(precision_)) b_kmajor = tc_eligible;
+    if (precision_ != FP32 && !is_complex128(precision_)) b_kmajor = [this](std::size_t m, std::size_t n, std::size_t k) {
+        return tc_eligible(m, n, k) || narrow_product(m, n, k);
+      };
     std::function<bool(std::size_t, std::size_t, std::size_t, int, const std::uint8_t*)> gather_a;
     p.gather.clear();
     p.tile_gather.clear();

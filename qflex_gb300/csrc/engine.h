@@ -133,6 +133,7 @@ class Engine {
   bool direct_product(std::size_t n, const TcConfig& cfg) const;
   bool split_multiply(std::size_t m, std::size_t n, std::size_t k) const;
   // fp32 elements of split planes that one product of this shape needs.
+  bool narrow_product(std::size_t m, std::size_t n, std::size_t k) const;
   std::size_t workspace_elems(std::size_t m, std::size_t n, std::size_t k) const;
   // Whether device buffer `slot` holds `bytes` or can be made to.
   bool fits(std::size_t bytes, int slot) const;

@@ -7,22 +7,22 @@
 // kernel (or a plane-writing permutation) before the product that saves one
 // pass over A: 8 B read and 8 B written per element.
 //
-// Structure: persistent, one CTA per SM over 128 x 128 complex tiles, 512
-// threads in four warpgroups whose registers setmaxnreg divides (56, 176,
+// Structure: persistent, one CTA per SM over tiles of 128 rows x BN (128, 64
+// or 32) columns, 512 threads in four warpgroups whose registers setmaxnreg divides (56, 176,
 // 176, 104 per thread: 128 on average, the launch's own share). Work goes by
 // blocks of A, 128 rows x 32 values (two k-steps of 16):
 //   warp 0       B producer: four 8 KB TMA boxes a block (re and im rows of
 //                64 bytes, hi and lo, of each k-step)
 //   warp 1       TMEM allocation; issues every MMA
-//   warp 2       A loader: TMA boxes into a ring of three blocks (with warp 3,
+//   warp 2       A loader: TMA boxes into a ring of blocks (with warp 3,
 //                16- or 8-byte cp.async copies where no box fits)
 //   warps 4..11  epilogue: drains TMEM sums, scales and stores the tile
 //   warps 12..15 A converter: thread r reads row r of the block, finds the
 //                largest component, scales by the power of two that brings it
 //                into [2^14, 2^15), splits into hi + lo and writes the planes
 //                to its TMEM lane, where the MMAs read A
-// TMEM holds two blocks of planes (128 columns) and three sums of 128
-// columns: a block's real part is summed from zero into one, its imaginary
+// TMEM holds two blocks of planes (128 columns) and three sums of BN columns:
+// a block's real part is summed from zero into one, its imaginary
 // part into the next, and the epilogue, which applies the block's exponent as
 // it adds a sum to the tile, drains one while the others fill.
 //
@@ -47,6 +47,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "half_split.cuh"
@@ -56,43 +57,50 @@
 namespace qfx {
 namespace {
 
-constexpr int BM = 128, BN = 128;
-constexpr int A_RING = 3;                   // blocks of 128 rows x 32 values
-constexpr int A_BLOCK = 128 * 32 * 8;       // bytes
-constexpr int A_BUFS = 2;                   // blocks of planes in TMEM
-constexpr int HALVES = 3;                   // sums, the real or imaginary part of a block
-constexpr int B_STAGES = 2;                 // two k-steps each
-constexpr int DONE = 3;                     // barriers of finished blocks in turn
-constexpr int B_PART = BN * 64;             // re or im rows of a k-step (hi, lo)
-constexpr int B_STAGE = 4 * B_PART;
-constexpr int EXP_RING = 4;                 // block exponents, see the converter
-constexpr int OFF_B = A_RING * A_BLOCK;
-constexpr int SLOT = 4096;                  // output box: 32 rows x 16 complex
-constexpr int OFF_STAGING = OFF_B + B_STAGES * B_STAGE;
-constexpr int OFF_SCALE = OFF_STAGING + 8 * 2 * SLOT;
-constexpr int OFF_EXP = OFF_SCALE + 8 * (BN / 2) * 4;  // after each epilogue warp's column exponents
-constexpr int OFF_BAR = OFF_EXP + EXP_RING * BM;
-constexpr int N_BARS = 2 * A_RING + A_BUFS + B_STAGES + 2 * DONE + HALVES + 1;
-constexpr int SMEM = OFF_BAR + N_BARS * 8 + 8;
-static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
-constexpr int TMEM_COLS = 512;
-constexpr int TMEM_A = HALVES * BN;  // two blocks of planes after the accumulators
-constexpr int TMEM_A_BLOCK = 64;     // 2 k-steps x 4 planes x 8 words
-static_assert(TMEM_A + A_BUFS * TMEM_A_BLOCK == TMEM_COLS, "TMEM is full");
+constexpr int BM = 128;
+constexpr int A_BLOCK = 128 * 32 * 8;  // bytes
+constexpr int A_BUFS = 2;              // blocks of planes in TMEM
+constexpr int HALVES = 3;              // sums, the real or imaginary part of a block
+constexpr int B_STAGES = 2;            // two k-steps each
+constexpr int DONE = 3;                // barriers of finished blocks in turn
+constexpr int EXP_RING = 4;            // block exponents, see the converter
+constexpr int SLOT = 4096;             // output box: 32 rows x 16 complex
+constexpr int TMEM_A_BLOCK = 64;       // 2 k-steps x 4 planes x 8 words
 constexpr int THREADS = 512;
 constexpr int LOADERS = 64, CONVERTERS = 128;
+
+// Shared memory and TMEM for tiles of 128 rows and BN columns.
+template <int BN>
+struct Layout {
+  static constexpr int A_RING = BN == 128 ? 3 : BN == 64 ? 4 : 5;  // blocks of 128 rows x 32 values
+  static constexpr int B_PART = BN * 64;                           // re or im rows of a k-step (hi, lo)
+  static constexpr int B_STAGE = 4 * B_PART;
+  static constexpr int SLOTS = BN == 32 ? 1 : 2;  // of each epilogue warp
+  static constexpr int COLS = BN / 2;             // columns of an epilogue warp
+  static constexpr int OFF_B = A_RING * A_BLOCK;
+  static constexpr int OFF_STAGING = OFF_B + B_STAGES * B_STAGE;
+  static constexpr int OFF_SCALE = OFF_STAGING + 8 * SLOTS * SLOT;
+  static constexpr int OFF_EXP = OFF_SCALE + 8 * COLS * 4;  // after each epilogue warp's column exponents
+  static constexpr int OFF_BAR = OFF_EXP + EXP_RING * BM;
+  static constexpr int N_BARS = 2 * A_RING + A_BUFS + B_STAGES + 2 * DONE + HALVES + 1;
+  static constexpr int SMEM = OFF_BAR + N_BARS * 8 + 8;
+  static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
+  static constexpr int TMEM_A = HALVES * BN;  // the planes, after the sums
+  static constexpr int TMEM_COLS = BN == 32 ? 256 : 512;
+  static_assert(TMEM_A + A_BUFS * TMEM_A_BLOCK <= TMEM_COLS, "TMEM");
+};
 
 // The real (IM = 0) or imaginary part of a block: two k-steps of A's planes in
 // TMEM (re hi, lo, im hi, lo, 8 columns each from `a`) against B's re rows
 // (`blo`, hi and lo 32 bytes apart) and im rows (B_PART further), small terms
 // first.
-template <int IM>
+template <int BN, int IM>
 __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std::uint32_t blo, std::uint32_t bhi) {
   constexpr std::uint32_t pos = idesc_f16(BM, BN, false), neg = idesc_f16(BM, BN, true);
-  static_assert(B_PART / 16 == 512, "offset of the im rows and of the second k-step");
+  constexpr std::uint32_t part = Layout<BN>::B_PART / 16;
   // Ar multiplies B's part of the same name, Ai the other one (negated for
   // the real part).
-  const std::uint32_t x = IM ? blo + 512 : blo, y = IM ? blo : blo + 512;
+  const std::uint32_t x = IM ? blo + part : blo, y = IM ? blo : blo + part;
 #define QFX_MMA(a_, b_, id, p) " tcgen05.mma.cta_group::1.kind::f16 [%0], [" a_ "], " b_ ", " id ", " p ";\n"
 #define QFX_KSTEP(rh, rl, ih, il, p)                                                                  \
   QFX_MMA(rh, "xl", "%5", p)                                                                          \
@@ -108,9 +116,9 @@ __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std:
       " add.u32 a5, %1, 40;\n add.u32 a6, %1, 48;\n add.u32 a7, %1, 56;\n"
       " mov.b32 x0, %2;\n mov.b32 y0, %3;\n add.u32 x1, %2, 2;\n add.u32 y1, %3, 2;\n"  //
       QFX_BDESC QFX_KSTEP("%1", "a1", "a2", "a3", "p0")
-      " add.u32 x0, %2, 1024;\n add.u32 y0, %3, 1024;\n add.u32 x1, %2, 1026;\n add.u32 y1, %3, 1026;\n"  //
+      " add.u32 x0, %2, %7;\n add.u32 y0, %3, %7;\n add.u32 x1, x0, 2;\n add.u32 y1, y0, 2;\n"  //
       QFX_BDESC QFX_KSTEP("a4", "a5", "a6", "a7", "p1") "}\n" ::"r"(d),
-      "r"(a), "r"(x), "r"(y), "r"(bhi), "r"(pos), "r"(IM ? pos : neg));
+      "r"(a), "r"(x), "r"(y), "r"(bhi), "r"(pos), "r"(IM ? pos : neg), "n"(2 * part));
 #undef QFX_BDESC
 #undef QFX_KSTEP
 #undef QFX_MMA
@@ -163,14 +171,17 @@ __device__ __forceinline__ void cp_async_arrive(std::uint64_t* bar) {
 #define QFX_SETMAXNREG_DEC(n) asm volatile("setmaxnreg.dec.sync.aligned.u32 " #n ";")
 #define QFX_SETMAXNREG_INC(n) asm volatile("setmaxnreg.inc.sync.aligned.u32 " #n ";")
 
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     cgemm_fp16x3_direct_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ AGather g,
                                const float2* __restrict__ A, float2* __restrict__ C, int tma_c, int m, int n, int k,
                                int batches, std::uint64_t ac_stride, int* __restrict__ err,
                                const int* __restrict__ exp_b) {
+  using L = Layout<BN>;
+  constexpr int A_RING = L::A_RING, B_PART = L::B_PART, B_STAGE = L::B_STAGE, TMEM_A = L::TMEM_A, COLS = L::COLS;
   extern __shared__ __align__(1024) std::uint8_t smem[];
-  std::uint64_t* raw_full = reinterpret_cast<std::uint64_t*>(smem + OFF_BAR);  // a block of A has landed
+  std::uint64_t* raw_full = reinterpret_cast<std::uint64_t*>(smem + L::OFF_BAR);  // a block of A has landed
   std::uint64_t* raw_empty = raw_full + A_RING;                                // and is in registers
   std::uint64_t* a_full = raw_empty + A_RING;                                  // its planes are in TMEM
   std::uint64_t* b_full = a_full + A_BUFS;
@@ -233,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           make_float4(0.f, 0.f, 0.f, 0.f);
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS));
+                 "r"(L::TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -256,7 +267,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           // A k of an odd number of k-steps: the last one's rows lie outside
           // the map and arrive as zeros.
-          std::uint8_t* st = smem + OFF_B + s * B_STAGE;
+          std::uint8_t* st = smem + L::OFF_B + s * B_STAGE;
           mbar_expect_tx(&b_full[s], B_STAGE);
           tma_load_4d(&map_b, &b_full[s], st, 0, nt * BN, 2 * b, batch);
           tma_load_4d(&map_b, &b_full[s], st + B_PART, 32, nt * BN, 2 * b, batch);
@@ -292,7 +303,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       // wait for the buffers of the real and the imaginary part, 1 for A's
       // planes, 2 for B's.
       const bool leader = elect_one();
-      const std::uint64_t db = smem_desc_sw64(smem_u32(smem + OFF_B));
+      const std::uint64_t db = smem_desc_sw64(smem_u32(smem + L::OFF_B));
       const std::uint32_t b_hi = std::uint32_t(db >> 32), b_lo0 = std::uint32_t(db);
       const int kind = lane & 3;
       std::uint64_t* const bars = kind == 1 ? a_full : kind == 2 ? b_full : acc_empty;
@@ -306,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;");
         const std::uint32_t a = tmem + TMEM_A + xa * TMEM_A_BLOCK, b = b_lo0 + sb * (B_STAGE >> 4);
         if (leader) {
-          mma_block<0>(tmem + h * BN, a, b, b_hi);
+          mma_block<BN, 0>(tmem + h * BN, a, b, b_hi);
           umma_commit(&re_full[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
@@ -315,7 +326,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!__all_sync(0xffffffffu, kind != 3 || wait(bars + at, parity, 4))) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (leader) {
-          mma_block<1>(tmem + h * BN, a, b, b_hi);
+          mma_block<BN, 1>(tmem + h * BN, a, b, b_hi);
           umma_commit(&done[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
@@ -448,7 +459,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     std::uint32_t row_at = 0;
     for (int b = 0; b < 7; ++b)
       if ((row >> b) & 1) row_at ^= g.row_at[b];
-    std::int8_t* exps = reinterpret_cast<std::int8_t*>(smem + OFF_EXP);
+    std::int8_t* exps = reinterpret_cast<std::int8_t*>(smem + L::OFF_EXP);
     const std::uint32_t ring = smem_u32(smem);
     const std::uint32_t lanes = tmem + TMEM_A + (std::uint32_t((warp - 12) * 32) << 16);
     int s = 0, x = 0, xa = 0, r = DONE - A_BUFS;
@@ -528,13 +539,12 @@ __global__ void __launch_bounds__(THREADS, 1)
     // zero; keeping each chunk short and adding the chunks here with
     // round-to-nearest keeps the product as accurate as FP32 arithmetic.
     QFX_SETMAXNREG_INC(176);
-    constexpr int COLS = BN / 2;
     const int q = warp % 4;
     const int part = (warp - 4) / 4;
     const int row = q * 32 + lane;
-    const std::int8_t* exps = reinterpret_cast<const std::int8_t*>(smem + OFF_EXP);
-    std::uint8_t* staging = smem + OFF_STAGING + (warp - 4) * 2 * SLOT;
-    int* sc_row = reinterpret_cast<int*>(smem + OFF_SCALE) + (warp - 4) * COLS;
+    const std::int8_t* exps = reinterpret_cast<const std::int8_t*>(smem + L::OFF_EXP);
+    std::uint8_t* staging = smem + L::OFF_STAGING + (warp - 4) * L::SLOTS * SLOT;
+    int* sc_row = reinterpret_cast<int*>(smem + L::OFF_SCALE) + (warp - 4) * COLS;
     const float beta = debias_beta<KIND_FP16>(err, 2, (k + 15) / 16);
     const float2 beta2 = make_float2(beta, beta);
     int h = 0, x = 0, r = 0;
@@ -544,18 +554,18 @@ __global__ void __launch_bounds__(THREADS, 1)
     // Adds the next TMEM buffer, times `f`, to `sum`.
     auto drain = [&](float2(&sum)[COLS / 2], float2 f) {
       const std::uint32_t base = base0 + h * BN;
+      constexpr int STEP = COLS < 32 ? COLS : 32;  // columns of one wait
 #pragma unroll
-      for (int j0 = 0; j0 < COLS; j0 += 32) {
-        std::uint32_t v0[16], v1[16];
-        TMEM_LD16(base + j0, v0);
-        TMEM_LD16(base + j0 + 16, v1);
+      for (int j0 = 0; j0 < COLS; j0 += STEP) {
+        std::uint32_t v[2][16];
+#pragma unroll
+        for (int i = 0; i < STEP / 16; ++i) TMEM_LD16(base + j0 + 16 * i, v[i]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < STEP / 2; ++j) {
+          const std::uint32_t* w = v[j / 8] + 2 * (j % 8);
           float2& a = sum[j0 / 2 + j];
-          float2& b = sum[j0 / 2 + 8 + j];
-          a = fma2(make_float2(__uint_as_float(v0[2 * j]), __uint_as_float(v0[2 * j + 1])), f, a);
-          b = fma2(make_float2(__uint_as_float(v1[2 * j]), __uint_as_float(v1[2 * j + 1])), f, b);
+          a = fma2(make_float2(__uint_as_float(w[0]), __uint_as_float(w[1])), f, a);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -570,8 +580,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int ncols = n - n0;
       // Exponents of the lane's columns, fetched before the drain.
       const int* eb = exp_b + std::uint64_t(batch) * n + n0;
-      const int eb0 = lane < ncols ? eb[lane] : 0;
-      const int eb1 = 32 + lane < ncols ? eb[32 + lane] : eb0;
+      const int eb0 = lane < min(ncols, COLS) ? eb[lane] : 0;
+      const int eb1 = COLS > 32 && 32 + lane < ncols ? eb[32 + lane] : eb0;
       float2 re[COLS / 2], im[COLS / 2];  // columns 2 j, 2 j + 1
 #pragma unroll
       for (int j = 0; j < COLS / 2; ++j) re[j] = im[j] = make_float2(0.f, 0.f);
@@ -620,8 +630,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       // exponents go through 64 words of the warp's own shared memory, from
       // where four at a time are read as one broadcast.
       __syncwarp();
-      sc_row[lane] = eb0 << 23;
-      sc_row[32 + lane] = eb1 << 23;
+      if (lane < COLS) sc_row[lane] = eb0 << 23;
+      if (COLS > 32) sc_row[32 + lane] = eb1 << 23;
       // When every scale 2^-(eref + eb) of the warp's block is a normal float
       // each element takes one multiply by it (exact unless the result leaves
       // the normal range). Otherwise the sums are scaled here, by two powers
@@ -645,8 +655,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         c0 = 127u << 23;
         __syncwarp();
-        sc_row[lane] = 0;
-        sc_row[32 + lane] = 0;
+        if (lane < COLS) sc_row[lane] = 0;
+        if (COLS > 32) sc_row[32 + lane] = 0;
         __syncwarp();
       }
 #pragma unroll
@@ -655,15 +665,20 @@ __global__ void __launch_bounds__(THREADS, 1)
         im[j] = fma2(im[j], beta2, im[j]);
       }
       float2* cb = C + std::uint64_t(batch) * ac_stride;
-      // Four boxes of 32 rows x 16 complex, two slots in turn. (Boxes of 8
+      // Boxes of 32 rows x 16 complex, the warp's slots in turn. (Boxes of 8
       // columns: twice the fences and barriers, a tile's store took 7200
       // cycles. A thread storing its own row piece in 32-byte sectors,
       // without shared memory, 9400.)
 #pragma unroll
       for (int j0 = 0; j0 < COLS; j0 += 16) {
-        std::uint8_t* slot = staging + ((j0 / 16) & 1) * SLOT;
+        std::uint8_t* slot = staging + (j0 / 16) % L::SLOTS * SLOT;
         if (tma_c) {
-          if (lane == 0) bulk_wait_read1();
+          if (lane == 0) {
+            if (L::SLOTS == 2)
+              bulk_wait_read1();
+            else
+              bulk_wait_read();
+          }
           __syncwarp();
         }
 #pragma unroll
@@ -714,7 +729,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     while (!mbar_test(mma_done, 0) && now_ns() - t0 < WAIT_NS) {
     }
     asm volatile("tcgen05.fence::after_thread_sync;");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS));
   }
 }
 
@@ -920,6 +935,12 @@ void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const floa
     }
 }
 
+// Columns of a tile: the narrowest that holds n, for fewer MMAs and smaller
+// B stages and so more blocks of A in flight. In tiles of 128, 64 and 32:
+// (32768, 64, 64) x 16 112 and 86 us (reading A and writing C alone 80),
+// (1048576, 16, 256) 498 and, in tiles of 32, 353 us (342).
+static int direct_columns(std::size_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : 128; }
+
 std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k) {
   return 2 * n * ((k + 15) / 16 * 16) + 2 * n;  // B's planes, exponents and largest components
 }
@@ -931,11 +952,6 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk != 2)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct product takes chunks of 2 k-steps");
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    check(cudaFuncSetAttribute(cgemm_fp16x3_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM),
-          "cudaFuncSetAttribute");
-  });
   if (gather.boxes && !gather.plain && batch > 1) {
     if (ac_stride % 16) throw std::string("ERROR (qflex_gb300: tensor cores) --> batch stride of a gathered operand");
     // The box's last coordinate counts 128 bytes in 31 bits.
@@ -953,7 +969,8 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   int* eb = reinterpret_cast<int*>(pb + 4 * n * kpad * (std::size_t)batch);
   std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
   launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
-  const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, BN, 64);
+  const int bn = direct_columns(n);
+  const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, bn, 64);
   CUtensorMap ma;
   std::memset(&ma, 0, sizeof(ma));
   if (gather.boxes && gather.plain) {
@@ -973,9 +990,24 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   }
   CUtensorMap mc;
   const int tma_c = output_map(C, m, n, ac_stride, batch, &mc) ? 1 : 0;
-  const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * (std::size_t)batch;
-  cgemm_fp16x3_direct_kernel<<<persistent_grid(tiles), THREADS, SMEM, s>>>(
-      ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err, eb);
+  const std::size_t tiles = ((m + BM - 1) / BM) * ((n + bn - 1) / bn) * (std::size_t)batch;
+  auto run = [&](auto columns) {
+    constexpr int BN = decltype(columns)::value;
+    auto* kernel = cgemm_fp16x3_direct_kernel<BN>;
+    static std::once_flag attr;
+    std::call_once(attr, [&] {
+      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BN>::SMEM),
+            "cudaFuncSetAttribute");
+    });
+    kernel<<<persistent_grid(tiles), THREADS, Layout<BN>::SMEM, s>>>(ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n,
+                                                                     (int)k, batch, ac_stride, err, eb);
+  };
+  if (bn == 32)
+    run(std::integral_constant<int, 32>{});
+  else if (bn == 64)
+    run(std::integral_constant<int, 64>{});
+  else
+    run(std::integral_constant<int, 128>{});
   check(cudaGetLastError(), "cgemm_fp16x3_direct");
 }
 

@@ -51,3 +51,12 @@ def test_direct_product(built_lib, kind, m, n, k, batch, extra):
         assert np.max(np.abs(C - A @ B) / (np.abs(A) @ np.abs(B) + 1e-300)) < TOL
         assert np.array_equal(got[:m * k + k * n], row[:m * k + k * n])
         assert np.array_equal(got[m * k + k * n + m * n:], row[m * k + k * n + m * n:])
+
+
+@pytest.mark.parametrize("kind", ["gauss", "grow", "tiny"])
+@pytest.mark.parametrize("m,n,k,batch,extra", [
+    (256, 16, 96, 1, 0), (300, 17, 100, 2, 0), (257, 31, 129, 1, 1), (1000, 32, 256, 1, 0), (384, 33, 128, 3, 1),
+    (257, 50, 97, 1, 0), (20000, 63, 112, 1, 0), (300, 64, 96, 2, 0)])
+def test_narrow_tiles(built_lib, kind, m, n, k, batch, extra):
+    """Tiles of 32 and 64 columns, also of products that FP32 kernels ran."""
+    test_direct_product(built_lib, kind, m, n, k, batch, extra)
