@@ -226,6 +226,68 @@ __device__ __forceinline__ void mbar_arrive(std::uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// ---- Pairs of CTAs (clusters of two, cta_group::2) ---------------------------
+
+__device__ __forceinline__ std::uint32_t cluster_rank() {
+  std::uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Shared::cluster address of the same shared-memory offset in CTA `rank`.
+__device__ __forceinline__ std::uint32_t peer_addr(const void* p, std::uint32_t rank) {
+  std::uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool mbar_test_cluster(std::uint64_t* bar, std::uint32_t parity) {
+  std::uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_cluster(std::uint64_t* bar, std::uint32_t parity, volatile int* abort_flag,
+                                                  int* err, int code) {
+  if (mbar_test_cluster(bar, parity)) return true;
+  const unsigned long long t0 = now_ns(), limit = wait_limit_ns(err);
+  while (!mbar_test_cluster(bar, parity)) {
+    if (*abort_flag) return false;
+    if (now_ns() - t0 > limit) {
+      *abort_flag = 1;
+      atomicExch(err, code);
+      return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ void mbar_arrive_remote(std::uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// TMA load into this CTA's shared memory that completes on a barrier of
+// either CTA of the pair (`bar` is a shared::cluster address).
+__device__ __forceinline__ void tma_load_4d_pair(const CUtensorMap* map, std::uint32_t bar, void* dst, int c0, int c1,
+                                                 int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+      "%4, %5}], [%6];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<std::uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
+// Commit of the issuing thread's MMAs, arriving on `bar` in both CTAs.
+__device__ __forceinline__ void umma_commit_pair(std::uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(std::uint16_t(3))
+      : "memory");
+}
+
 // Compensation of the truncation bias. The tensor core's FP32 accumulation
 // rounds toward zero, so every product comes out smaller by a fraction beta
 // of itself that depends on the split kind and on how many k-steps a TMEM

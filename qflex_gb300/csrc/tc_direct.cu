@@ -26,15 +26,23 @@
 // part into the next, and the epilogue, which applies the block's exponent as
 // it adds a sum to the tile, drains one while the others fill.
 //
+// PAIR (clusters of two CTAs, cta_group::2): CTA r has rows 128 r .. + 127 of a
+// tile of 256, their planes in its own tensor memory, and half of B's columns
+// in its shared memory; CTA 0 issues MMAs of M = 256 for both. B's stages and
+// the MMAs' reads of them halve. CTA 0's barriers take both CTAs' arrivals
+// (planes written, sums drained) and B's bytes; commits go to both CTAs.
+//
 // What bounds it: a block's 24 MMAs take 1536 cycles of the tensor pipe, and
 // one warp issues them, one converts per SM partition, so what these do
-// between MMAs counts as much. Measured at k = 4096 (1024 x 1024, 64 CTAs: no
+// between MMAs counts as much; next shared memory, of which the MMAs read 64
+// bytes a cycle (a pair's 32). Measured at k = 4096 (1024 x 1024, 64 CTAs: no
 // power limit), cycles a block: A's planes in shared memory, A by cp.async
 // and five waits and commits a block 2360; planes in TMEM the same; two waits
-// and commits 2030; A by TMA boxes 1950. Without the loads and the conversion
-// (wrong sums) 1700. (65536, 256, 256) x 4 went from 341 to 308 us, (4096,
-// 1024, 4096) from 319 to 275, (65536, 256, 16) x 4 takes 96, of which
-// writing C alone is 80.
+// and commits 2030; A by TMA boxes 1950; pairs 1640. At (4096, 4096, 4096),
+// 901 us, the card's power limit is reached. (65536, 256, 256) x 4 went from
+// 341 to 286 us, of which each tile's store, 5600 cycles, leaves the tensor
+// pipe idle for 3300; (4096, 1024, 4096) from 319 to 240; (65536, 256, 16) x
+// 4 takes 96, of which writing C alone is 80.
 //
 // B holds no negated copy: the real part takes -Ai Bi by the descriptor's
 // negate-A bit, and a k-step loads 16 KB of B, not 24. MMAs of N = 128 run at
@@ -61,19 +69,22 @@ constexpr int BM = 128;
 constexpr int A_BLOCK = 128 * 32 * 8;  // bytes
 constexpr int A_BUFS = 2;              // blocks of planes in TMEM
 constexpr int HALVES = 3;              // sums, the real or imaginary part of a block
-constexpr int B_STAGES = 2;            // two k-steps each
-constexpr int DONE = 3;                // barriers of finished blocks in turn
 constexpr int EXP_RING = 4;            // block exponents, see the converter
 constexpr int SLOT = 4096;             // output box: 32 rows x 16 complex
 constexpr int TMEM_A_BLOCK = 64;       // 2 k-steps x 4 planes x 8 words
 constexpr int THREADS = 512;
 constexpr int LOADERS = 64, CONVERTERS = 128;
 
-// Shared memory and TMEM for tiles of 128 rows and BN columns.
-template <int BN>
+// Shared memory and TMEM for tiles of 128 rows and BN columns; of a PAIR, with
+// half of B's columns.
+template <int BN, bool PAIR>
 struct Layout {
   static constexpr int A_RING = BN == 128 ? 3 : BN == 64 ? 4 : 5;  // blocks of 128 rows x 32 values
-  static constexpr int B_PART = BN * 64;                           // re or im rows of a k-step (hi, lo)
+  static constexpr int B_COLS = PAIR ? BN / 2 : BN;
+  static constexpr int B_PART = B_COLS * 64;      // re or im rows of a k-step (hi, lo)
+  static constexpr int B_STAGES = PAIR ? 4 : 2;  // two k-steps each
+  static constexpr int DONE = PAIR ? 4 : 3;      // barriers of finished blocks in turn
+  static_assert(DONE >= B_STAGES && DONE > A_BUFS, "a barrier's phase is read before the next but one");
   static constexpr int B_STAGE = 4 * B_PART;
   static constexpr int SLOTS = BN == 32 ? 1 : 2;  // of each epilogue warp
   static constexpr int COLS = BN / 2;             // columns of an epilogue warp
@@ -94,31 +105,38 @@ struct Layout {
 // TMEM (re hi, lo, im hi, lo, 8 columns each from `a`) against B's re rows
 // (`blo`, hi and lo 32 bytes apart) and im rows (B_PART further), small terms
 // first.
-template <int BN, int IM>
+template <int BN, bool PAIR, int IM>
 __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std::uint32_t blo, std::uint32_t bhi) {
-  constexpr std::uint32_t pos = idesc_f16(BM, BN, false), neg = idesc_f16(BM, BN, true);
-  constexpr std::uint32_t part = Layout<BN>::B_PART / 16;
+  constexpr int rows = PAIR ? 2 * BM : BM;
+  constexpr std::uint32_t pos = idesc_f16(rows, BN, false), neg = idesc_f16(rows, BN, true);
+  constexpr std::uint32_t part = Layout<BN, PAIR>::B_PART / 16;
   // Ar multiplies B's part of the same name, Ai the other one (negated for
   // the real part).
   const std::uint32_t x = IM ? blo + part : blo, y = IM ? blo : blo + part;
-#define QFX_MMA(a_, b_, id, p) " tcgen05.mma.cta_group::1.kind::f16 [%0], [" a_ "], " b_ ", " id ", " p ";\n"
-#define QFX_KSTEP(rh, rl, ih, il, p)                                                                  \
-  QFX_MMA(rh, "xl", "%5", p)                                                                          \
-  QFX_MMA(rl, "xh", "%5", "p1")                                                                       \
-  QFX_MMA(ih, "yl", "%6", "p1")                                                                       \
-  QFX_MMA(il, "yh", "%6", "p1") QFX_MMA(rh, "xh", "%5", "p1") QFX_MMA(ih, "yh", "%6", "p1")
+#define QFX_MMA(g, a_, b_, id, p) " tcgen05.mma.cta_group::" g ".kind::f16 [%0], [" a_ "], " b_ ", " id ", " p ";\n"
+#define QFX_KSTEP(g, rh, rl, ih, il, p)                                                                  \
+  QFX_MMA(g, rh, "xl", "%5", p)                                                                          \
+  QFX_MMA(g, rl, "xh", "%5", "p1")                                                                       \
+  QFX_MMA(g, ih, "yl", "%6", "p1")                                                                       \
+  QFX_MMA(g, il, "yh", "%6", "p1") QFX_MMA(g, rh, "xh", "%5", "p1") QFX_MMA(g, ih, "yh", "%6", "p1")
 #define QFX_BDESC " mov.b64 xh, {x0, %4};\n mov.b64 xl, {x1, %4};\n mov.b64 yh, {y0, %4};\n mov.b64 yl, {y1, %4};\n"
-  asm volatile(
-      "{\n .reg .pred p0, p1;\n .reg .b32 a1, a2, a3, a4, a5, a6, a7, x0, x1, y0, y1;\n"
-      " .reg .b64 xh, xl, yh, yl;\n"
-      " setp.ne.b32 p0, %1, %1;\n setp.eq.b32 p1, %1, %1;\n"
-      " add.u32 a1, %1, 8;\n add.u32 a2, %1, 16;\n add.u32 a3, %1, 24;\n add.u32 a4, %1, 32;\n"
-      " add.u32 a5, %1, 40;\n add.u32 a6, %1, 48;\n add.u32 a7, %1, 56;\n"
-      " mov.b32 x0, %2;\n mov.b32 y0, %3;\n add.u32 x1, %2, 2;\n add.u32 y1, %3, 2;\n"  //
-      QFX_BDESC QFX_KSTEP("%1", "a1", "a2", "a3", "p0")
-      " add.u32 x0, %2, %7;\n add.u32 y0, %3, %7;\n add.u32 x1, x0, 2;\n add.u32 y1, y0, 2;\n"  //
-      QFX_BDESC QFX_KSTEP("a4", "a5", "a6", "a7", "p1") "}\n" ::"r"(d),
-      "r"(a), "r"(x), "r"(y), "r"(bhi), "r"(pos), "r"(IM ? pos : neg), "n"(2 * part));
+#define QFX_BLOCK(g) \
+    asm volatile( \
+        "{\n .reg .pred p0, p1;\n .reg .b32 a1, a2, a3, a4, a5, a6, a7, x0, x1, y0, y1;\n" \
+        " .reg .b64 xh, xl, yh, yl;\n" \
+        " setp.ne.b32 p0, %1, %1;\n setp.eq.b32 p1, %1, %1;\n" \
+        " add.u32 a1, %1, 8;\n add.u32 a2, %1, 16;\n add.u32 a3, %1, 24;\n add.u32 a4, %1, 32;\n" \
+        " add.u32 a5, %1, 40;\n add.u32 a6, %1, 48;\n add.u32 a7, %1, 56;\n" \
+        " mov.b32 x0, %2;\n mov.b32 y0, %3;\n add.u32 x1, %2, 2;\n add.u32 y1, %3, 2;\n" \
+        QFX_BDESC QFX_KSTEP(g, "%1", "a1", "a2", "a3", "p0") \
+        " add.u32 x0, %2, %7;\n add.u32 y0, %3, %7;\n add.u32 x1, x0, 2;\n add.u32 y1, y0, 2;\n" \
+        QFX_BDESC QFX_KSTEP(g, "a4", "a5", "a6", "a7", "p1") "}\n" ::"r"(d), \
+        "r"(a), "r"(x), "r"(y), "r"(bhi), "r"(pos), "r"(IM ? pos : neg), "n"(2 * part))
+  if constexpr (PAIR)
+    QFX_BLOCK("2");
+  else
+    QFX_BLOCK("1");
+#undef QFX_BLOCK
 #undef QFX_BDESC
 #undef QFX_KSTEP
 #undef QFX_MMA
@@ -171,14 +189,15 @@ __device__ __forceinline__ void cp_async_arrive(std::uint64_t* bar) {
 #define QFX_SETMAXNREG_DEC(n) asm volatile("setmaxnreg.dec.sync.aligned.u32 " #n ";")
 #define QFX_SETMAXNREG_INC(n) asm volatile("setmaxnreg.inc.sync.aligned.u32 " #n ";")
 
-template <int BN>
+template <int BN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
     cgemm_fp16x3_direct_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ AGather g,
                                const float2* __restrict__ A, float2* __restrict__ C, int tma_c, int m, int n, int k,
                                int batches, std::uint64_t ac_stride, int* __restrict__ err,
                                const int* __restrict__ exp_b) {
-  using L = Layout<BN>;
+  using L = Layout<BN, PAIR>;
+  constexpr int B_STAGES = L::B_STAGES, DONE = L::DONE;
   constexpr int A_RING = L::A_RING, B_PART = L::B_PART, B_STAGE = L::B_STAGE, TMEM_A = L::TMEM_A, COLS = L::COLS;
   extern __shared__ __align__(1024) std::uint8_t smem[];
   std::uint64_t* raw_full = reinterpret_cast<std::uint64_t*>(smem + L::OFF_BAR);  // a block of A has landed
@@ -198,24 +217,44 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   // Uniform for the compiler: see the MMA issuer.
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32;
-  const int first = blockIdx.x, stride = gridDim.x;
-  const int tiles_m = (m + BM - 1) / BM;
+  const std::uint32_t rank = PAIR ? cluster_rank() : 0;
+  const int first = PAIR ? blockIdx.x / 2 : blockIdx.x, stride = PAIR ? gridDim.x / 2 : gridDim.x;
+  constexpr int TILE_M = PAIR ? 2 * BM : BM, GROUP = PAIR ? 4 : 8;
+  const int tiles_m = (m + TILE_M - 1) / TILE_M;
   const int tiles_n = (n + BN - 1) / BN;
   const int per_batch = tiles_m * tiles_n;
   const int total = per_batch * batches;
-  // Tiles run in groups of 8 row-tiles so that the CTAs working at one time
+  // Tiles run in groups of 1024 rows so that the CTAs working at one time
   // share A rows and B columns in L2.
   auto tile_of = [&](int t, int& mt, int& nt, int& batch) {
     batch = t / per_batch;
     const int r = t % per_batch;
-    const int per_group = 8 * tiles_n;
+    const int per_group = GROUP * tiles_n;
     const int group = r / per_group, in_group = r % per_group;
-    const int group_m = min(8, tiles_m - group * 8);
-    mt = group * 8 + in_group % group_m;
+    const int group_m = min(GROUP, tiles_m - group * GROUP);
+    mt = group * GROUP + in_group % group_m;
+    if (PAIR) mt = 2 * mt + int(rank);
     nt = in_group / group_m;
   };
+  // Waits and arrivals keep CTA scope in a pair as well: what the barriers
+  // between its CTAs order are tensor-memory accesses (with the tcgen05
+  // fences) and TMA writes. At cluster scope a block took 3200 cycles.
   auto wait = [&](std::uint64_t* bar, std::uint32_t parity, int code) {
     return mbar_wait(bar, parity, abort_flag, err, code);
+  };
+  // Arrival at, and MMA completion on, barriers that a pair's CTA 0 waits on
+  // or that both wait on.
+  auto arrive = [&](std::uint64_t* bar) {
+    if constexpr (PAIR)
+      asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(peer_addr(bar, 0)) : "memory");
+    else
+      mbar_arrive(bar);
+  };
+  auto commit = [&](std::uint64_t* bar) {
+    if constexpr (PAIR)
+      umma_commit_pair(bar);
+    else
+      umma_commit(bar);
   };
   const int blocks = (k + 31) / 32;
   // Blocks of all the CTA's tiles.
@@ -226,13 +265,13 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_init(&raw_full[s], g.boxes ? 1 : LOADERS);
       mbar_init(&raw_empty[s], CONVERTERS / 32);
     }
-    for (int s = 0; s < A_BUFS; ++s) mbar_init(&a_full[s], CONVERTERS / 32);
+    for (int s = 0; s < A_BUFS; ++s) mbar_init(&a_full[s], (PAIR ? 2 : 1) * CONVERTERS / 32);
     for (int s = 0; s < B_STAGES; ++s) mbar_init(&b_full[s], 1);
     for (int s = 0; s < DONE; ++s) {
       mbar_init(&re_full[s], 1);
       mbar_init(&done[s], 1);
     }
-    for (int s = 0; s < HALVES; ++s) mbar_init(&acc_empty[s], 8);
+    for (int s = 0; s < HALVES; ++s) mbar_init(&acc_empty[s], PAIR ? 16 : 8);
     mbar_init(mma_done, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -243,12 +282,19 @@ __global__ void __launch_bounds__(THREADS, 1)
       *reinterpret_cast<float4*>(smem + i / (A_BLOCK / 32) * A_BLOCK + A_BLOCK / 2 + i % (A_BLOCK / 32) * 16) =
           make_float4(0.f, 0.f, 0.f, 0.f);
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(L::TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(L::TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(L::TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  if constexpr (PAIR) cluster_sync();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const std::uint32_t tmem = *tmem_slot;
 
@@ -268,26 +314,41 @@ __global__ void __launch_bounds__(THREADS, 1)
           // A k of an odd number of k-steps: the last one's rows lie outside
           // the map and arrive as zeros.
           std::uint8_t* st = smem + L::OFF_B + s * B_STAGE;
-          mbar_expect_tx(&b_full[s], B_STAGE);
-          tma_load_4d(&map_b, &b_full[s], st, 0, nt * BN, 2 * b, batch);
-          tma_load_4d(&map_b, &b_full[s], st + B_PART, 32, nt * BN, 2 * b, batch);
-          tma_load_4d(&map_b, &b_full[s], st + 2 * B_PART, 0, nt * BN, 2 * b + 1, batch);
-          tma_load_4d(&map_b, &b_full[s], st + 3 * B_PART, 32, nt * BN, 2 * b + 1, batch);
+          const int col = nt * BN + int(rank) * L::B_COLS;
+          if constexpr (PAIR) {
+            // Both CTAs' halves complete on CTA 0's barrier.
+            if (rank == 0) mbar_expect_tx(&b_full[s], 2 * B_STAGE);
+            const std::uint32_t bar = peer_addr(&b_full[s], 0);
+            tma_load_4d_pair(&map_b, bar, st, 0, col, 2 * b, batch);
+            tma_load_4d_pair(&map_b, bar, st + B_PART, 32, col, 2 * b, batch);
+            tma_load_4d_pair(&map_b, bar, st + 2 * B_PART, 0, col, 2 * b + 1, batch);
+            tma_load_4d_pair(&map_b, bar, st + 3 * B_PART, 32, col, 2 * b + 1, batch);
+          } else {
+            mbar_expect_tx(&b_full[s], B_STAGE);
+            tma_load_4d(&map_b, &b_full[s], st, 0, col, 2 * b, batch);
+            tma_load_4d(&map_b, &b_full[s], st + B_PART, 32, col, 2 * b, batch);
+            tma_load_4d(&map_b, &b_full[s], st + 2 * B_PART, 0, col, 2 * b + 1, batch);
+            tma_load_4d(&map_b, &b_full[s], st + 3 * B_PART, 32, col, 2 * b + 1, batch);
+          }
           ++q;
           if (++s == B_STAGES) s = 0;
         }
       }
       if (*abort_flag) {
         // The copies already issued land before the CTA's shared memory is
-        // released (bounded as well).
-        for (int w = q > B_STAGES ? q - B_STAGES : 0; w < q; ++w) {
+        // released (bounded as well). Those of a pair's CTA 1 complete on CTA
+        // 0, which may have expected fewer: time for them to land.
+        const unsigned long long t1 = now_ns();
+        while (rank == 1 && now_ns() - t1 < 1000000) {
+        }
+        for (int w = q > B_STAGES ? q - B_STAGES : 0; w < q && rank == 0; ++w) {
           const unsigned long long t0 = now_ns();
           while (!mbar_test(&b_full[w % B_STAGES], (w / B_STAGES) & 1) && now_ns() - t0 < WAIT_NS) {
           }
         }
       }
-    } else if (warp == 1) {
-      // MMA issuer. The whole warp runs the loop in step and one elected lane
+    } else if (warp == 1 && rank == 0) {
+      // MMA issuer (of a pair: CTA 0). The whole warp runs the loop in step and one elected lane
       // issues: the descriptors then live in uniform registers. Run by one
       // lane alone, every descriptor word moved there before each MMA, and
       // beside the other warps' work a k-step took 980 cycles instead of 775
@@ -317,8 +378,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;");
         const std::uint32_t a = tmem + TMEM_A + xa * TMEM_A_BLOCK, b = b_lo0 + sb * (B_STAGE >> 4);
         if (leader) {
-          mma_block<BN, 0>(tmem + h * BN, a, b, b_hi);
-          umma_commit(&re_full[r]);
+          mma_block<BN, PAIR, 0>(tmem + h * BN, a, b, b_hi);
+          commit(&re_full[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
         // The epilogue's TMEM reads of a buffer precede the MMAs that
@@ -326,8 +387,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!__all_sync(0xffffffffu, kind != 3 || wait(bars + at, parity, 4))) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (leader) {
-          mma_block<BN, 1>(tmem + h * BN, a, b, b_hi);
-          umma_commit(&done[r]);
+          mma_block<BN, PAIR, 1>(tmem + h * BN, a, b, b_hi);
+          commit(&done[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
         xa ^= 1;
@@ -340,7 +401,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
       }
       __syncwarp();
-      if (leader) umma_commit(mma_done);
+      if (leader) commit(mma_done);
       __syncwarp();
     } else if (warp >= 2 && g.boxes) {
       // A loader, by TMA boxes.
@@ -500,24 +561,24 @@ __global__ void __launch_bounds__(THREADS, 1)
       // The block is in registers: its place in the ring is free.
       __syncwarp();
       if (lane == 0) mbar_arrive(&raw_empty[s]);
+      std::uint32_t p[2][32];  // of each k-step: 8 words of every plane
+#pragma unroll
+      for (int i = 0; i < 32; i += 16)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
+          const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
+          split_pair(re.x, re.y, p[i / 16][j], p[i / 16][8 + j]);
+          split_pair(im.x, im.y, p[i / 16][16 + j], p[i / 16][24 + j]);
+        }
       if (!__all_sync(0xffffffffu, wait(&done[r], pd, 10))) break;
       if (++r == DONE) {
         r = 0;
         pd ^= 1u;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll
-      for (int i = 0; i < 32; i += 16) {  // a k-step: 8 words of every plane
-        std::uint32_t p[32];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
-          const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
-          split_pair(re.x, re.y, p[j], p[8 + j]);
-          split_pair(im.x, im.y, p[16 + j], p[24 + j]);
-        }
-        tmem_st32(lanes + xa * TMEM_A_BLOCK + i * 2, p);
-      }
+      tmem_st32(lanes + xa * TMEM_A_BLOCK, p[0]);
+      tmem_st32(lanes + xa * TMEM_A_BLOCK + 32, p[1]);
       // Exponents live in a ring of their own: the MMAs of the block two
       // back are done, so every epilogue warp has read the exponents of the
       // block three back.
@@ -525,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_full[xa]);
+      if (lane == 0) arrive(&a_full[xa]);
       xa ^= 1;
       if (++x == EXP_RING) x = 0;
       if (++s == A_RING) {
@@ -570,7 +631,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[h]);
+      if (lane == 0) arrive(&acc_empty[h]);
       h = h == HALVES - 1 ? 0 : h + 1;
     };
     for (int t = first; t < total && ok; t += stride) {
@@ -723,13 +784,23 @@ __global__ void __launch_bounds__(THREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 1) {
-    // Release TMEM only after every MMA this CTA issued has completed; the
-    // wait is immediate unless the pipeline was abandoned.
+    // Release TMEM only after every MMA this CTA issued (or, in a pair, that
+    // read this CTA's memories) has completed; the wait is immediate unless
+    // the pipeline was abandoned.
     const unsigned long long t0 = now_ns();
-    while (!mbar_test(mma_done, 0) && now_ns() - t0 < WAIT_NS) {
+    while (!(PAIR ? mbar_test_cluster(mma_done, 0) : mbar_test(mma_done, 0)) && now_ns() - t0 < WAIT_NS) {
     }
+  }
+  if constexpr (PAIR) {
+    __syncthreads();
+    cluster_sync();
+  }
+  if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS));
+    if constexpr (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS));
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS));
   }
 }
 
@@ -940,6 +1011,11 @@ void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const floa
 // (32768, 64, 64) x 16 112 and 86 us (reading A and writing C alone 80),
 // (1048576, 16, 256) 498 and, in tiles of 32, 353 us (342).
 static int direct_columns(std::size_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : 128; }
+// Pairs where a second row tile exists and the MMAs of a tile take longer than
+// its store, which starts later in a pair. Single CTAs against pairs: (65536,
+// 256, k) x 4 with k = 32 104 and 106 us, 64 143 and 149, 256 301 and 286;
+// (8192, 128, 128) x 16 59 and 60.5; (4096, 1024, 4096) 272 and 240.
+static bool direct_pair(std::size_t m, std::size_t k) { return m > (std::size_t)BM && k > 128; }
 
 std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k) {
   return 2 * n * ((k + 15) / 16 * 16) + 2 * n;  // B's planes, exponents and largest components
@@ -970,7 +1046,8 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
   launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   const int bn = direct_columns(n);
-  const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, bn, 64);
+  const bool pair = bn == 128 && direct_pair(m, k);
+  const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, pair ? bn / 2 : bn, 64);
   CUtensorMap ma;
   std::memset(&ma, 0, sizeof(ma));
   if (gather.boxes && gather.plain) {
@@ -990,24 +1067,49 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   }
   CUtensorMap mc;
   const int tma_c = output_map(C, m, n, ac_stride, batch, &mc) ? 1 : 0;
-  const std::size_t tiles = ((m + BM - 1) / BM) * ((n + bn - 1) / bn) * (std::size_t)batch;
-  auto run = [&](auto columns) {
+  const std::size_t rows = pair ? 2 * BM : BM;
+  const std::size_t tiles = ((m + rows - 1) / rows) * ((n + bn - 1) / bn) * (std::size_t)batch;
+  auto run = [&](auto columns, auto paired) {
     constexpr int BN = decltype(columns)::value;
-    auto* kernel = cgemm_fp16x3_direct_kernel<BN>;
+    constexpr bool PAIR = decltype(paired)::value;
+    auto* kernel = cgemm_fp16x3_direct_kernel<BN, PAIR>;
+    cudaLaunchConfig_t lc = {};
+    lc.blockDim = dim3(THREADS, 1, 1);
+    lc.dynamicSmemBytes = Layout<BN, PAIR>::SMEM;
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = PAIR ? 1 : 0;
     static std::once_flag attr;
+    static int resident = 0;  // pairs (SMs pair up within a GPC)
     std::call_once(attr, [&] {
-      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BN>::SMEM),
+      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BN, PAIR>::SMEM),
             "cudaFuncSetAttribute");
+      lc.gridDim = dim3(2, 1, 1);
+      if (PAIR && (cudaOccupancyMaxActiveClusters(&resident, kernel, &lc) != cudaSuccess || resident < 1)) {
+        cudaGetLastError();
+        resident = (int)persistent_grid(1u << 20) / 2;
+      }
     });
-    kernel<<<persistent_grid(tiles), THREADS, Layout<BN>::SMEM, s>>>(ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n,
-                                                                     (int)k, batch, ac_stride, err, eb);
+    lc.gridDim = dim3(PAIR ? 2 * (unsigned)std::min<std::size_t>(tiles, (std::size_t)resident) : persistent_grid(tiles),
+                      1, 1);
+    check(cudaLaunchKernelEx(&lc, kernel, ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err,
+                             (const int*)eb),
+          "cgemm_fp16x3_direct");
   };
-  if (bn == 32)
-    run(std::integral_constant<int, 32>{});
+  using std::integral_constant;
+  if (pair)
+    run(integral_constant<int, 128>{}, std::true_type{});
+  else if (bn == 128)
+    run(integral_constant<int, 128>{}, std::false_type{});
   else if (bn == 64)
-    run(std::integral_constant<int, 64>{});
+    run(integral_constant<int, 64>{}, std::false_type{});
   else
-    run(std::integral_constant<int, 128>{});
+    run(integral_constant<int, 32>{}, std::false_type{});
   check(cudaGetLastError(), "cgemm_fp16x3_direct");
 }
 

@@ -60,3 +60,12 @@ def test_direct_product(built_lib, kind, m, n, k, batch, extra):
 def test_narrow_tiles(built_lib, kind, m, n, k, batch, extra):
     """Tiles of 32 and 64 columns, also of products that FP32 kernels ran."""
     test_direct_product(built_lib, kind, m, n, k, batch, extra)
+
+
+@pytest.mark.parametrize("kind", ["gauss", "jump", "tiny"])
+@pytest.mark.parametrize("m,n,k,batch,extra", [
+    (129, 128, 160, 1, 0), (256, 129, 256, 1, 0), (257, 640, 161, 1, 1), (640, 1100, 192, 2, 0), (383, 1500, 130, 1, 0),
+    (20000, 256, 256, 1, 0), (128, 1100, 192, 1, 0)])
+def test_pairs(built_lib, kind, m, n, k, batch, extra):
+    """Tiles of two CTAs, also with an empty second half, and of one beside them."""
+    test_direct_product(built_lib, kind, m, n, k, batch, extra)
