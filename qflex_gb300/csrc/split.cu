@@ -12,13 +12,15 @@
 // imaginary planes), 12 (BF16x3) or 16 (3xTF32; 24) B written per element.
 // Measured at 4096 x 4096, against two values per thread, a second pass over
 // every 3xFP16 row, and a permutation (42 us) before the rows of a row-major B:
-//   3xFP16 rows 100 -> 50 us, columns 142 -> 87 us (with the negated copy)
+//   3xFP16 rows 100 -> 50 us, columns 142 -> 87 us (with the negated copy), in
+//   one pass (without) 63; at 1100 x 690 8.4 -> 6.4 us and two launches fewer
 //   3xTF32 rows  79 -> 74 us, columns 134 -> 83 us (with the negated copy)
 //   BF16x3 rows  68 -> 57 us, columns 110 -> 52 us
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <mutex>
 #include <string>
 
 #include "half_split.cuh"
@@ -240,8 +242,87 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float2* __restric
   }
 }
 
-// Columns of a row-major k x n matrix become the rows of planes. The largest
-// component of every column first (bit patterns, by integer maxima): blocks
+// Columns of a row-major k x n matrix become the rows of planes. 3xFP16, whose
+// scale is a column's, in one pass: a cluster of CTAs holds 16 columns, each a
+// run of `deep` values of k, in shared memory, exchanges the largest
+// components and writes the planes. Rows of 17 elements: the two halves of a
+// k-step, 8 rows apart, lie in different banks.
+constexpr int SLAB = 16, PITCH = SLAB + 1;
+template <int NP>
+__global__ void __launch_bounds__(256, 3) split_cols_cluster_kernel(const float2* __restrict__ src,
+                                                                 void* __restrict__ main_planes, int* __restrict__ exps,
+                                                                 std::uint64_t n, std::uint64_t k, std::uint64_t kpad,
+                                                                 std::uint64_t src_stride, std::uint64_t main_stride,
+                                                                 int deep, int ranks) {
+  extern __shared__ float2 slab[];
+  __shared__ std::uint32_t part[8][SLAB], top[SLAB];
+  __shared__ int scale[SLAB];
+  const std::uint64_t b = blockIdx.y;
+  src += b * src_stride;
+  main_planes = static_cast<char*>(main_planes) + b * main_stride;
+  const std::uint32_t rank = cluster_rank();
+  const std::uint64_t n0 = std::uint64_t(blockIdx.x / ranks) * SLAB, k0 = std::uint64_t(rank) * deep;
+  {
+    const int c = threadIdx.x % SLAB, w = threadIdx.x / 32;
+    const bool in = n0 + c < n;
+    const float2* s = src + n0 + c;
+    std::uint32_t mx = 0;
+    for (int r0 = threadIdx.x / SLAB; r0 < deep; r0 += 256) {  // 16 rows in flight
+      float2 v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int r = r0 + 16 * i;
+        v[i] = in && r < deep && k0 + r < k ? __ldg(s + (k0 + r) * n) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (r0 + 16 * i < deep) slab[(r0 + 16 * i) * PITCH + c] = v[i];
+        mx = max(mx, max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
+      }
+    }
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, SLAB));
+    if (threadIdx.x % 32 < SLAB) part[w][c] = mx;
+  }
+  __syncthreads();
+  if (threadIdx.x < SLAB) {
+    std::uint32_t mx = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = max(mx, part[w][threadIdx.x]);
+    top[threadIdx.x] = mx;
+  }
+  __syncthreads();
+  cluster_sync();
+  if (threadIdx.x < SLAB) {
+    std::uint32_t mx = 0;
+    for (int q = 0; q < ranks; ++q) {
+      std::uint32_t v;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(&top[threadIdx.x], q)) : "memory");
+      mx = max(mx, v);
+    }
+    const int e = scale_exponent(mx);
+    scale[threadIdx.x] = e;
+    if (rank == 0 && n0 + threadIdx.x < n) exps[b * n + n0 + threadIdx.x] = e;
+  }
+  __syncthreads();
+  // No CTA ends while another still reads its maxima: waited for below.
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  const int c = (threadIdx.x >> 1) % SLAB;
+  if (n0 + c < n) {
+    const int e = scale[c];
+    for (int at = (threadIdx.x >> 5) * 16 + (threadIdx.x & 1) * 8; at < deep && k0 + at < kpad; at += 128) {
+      float2 v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = slab[(at + j) * PITCH + c];
+      emit<KIND_FP16, NP>(v, e, main_planes, nullptr, n, n0 + c, k0 + at);
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Columns longer than the clusters hold with three CTAs on an SM (4096
+// values; with one CTA on an SM 13000 x 1000 took 127 us, this way 62). The
+// largest component of every column first (bit patterns, by integer maxima): blocks
 // of 32 columns x `depth` rows.
 __global__ void __launch_bounds__(256) column_max_kernel(const float2* __restrict__ src, std::uint32_t* __restrict__ top,
                                                          std::uint64_t n, std::uint64_t k, std::uint64_t src_stride,
@@ -354,7 +435,38 @@ void run_split(const SplitOut& out, const float2* src, std::size_t rows, std::si
     return;
   }
   const unsigned cols = (unsigned)((rows + 31) / 32);
-  if (KIND == KIND_FP16) {
+  if constexpr (KIND == KIND_FP16) {
+    // As many CTAs as keep three on an SM (512 values of k each), then as many
+    // as give every SM two, of at least 32 values.
+    const std::size_t slabs = (rows + SLAB - 1) / SLAB * (std::size_t)batch;
+    int ranks = 1;
+    while (ranks < 8 && (st.kpad > 512u * ranks || (slabs * ranks < 304 && st.kpad >= 64u * ranks))) ranks *= 2;
+    const std::size_t deep = (st.kpad / 16 + ranks - 1) / ranks * 16, bytes = deep * PITCH * sizeof(float2);
+    if (deep <= 512) {
+      auto* kernel = split_cols_cluster_kernel<NP>;
+      static std::once_flag attr;
+      std::call_once(attr, [&] {
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   512 * PITCH * (int)sizeof(float2)),
+              "cudaFuncSetAttribute");
+      });
+      cudaLaunchConfig_t lc = {};
+      lc.gridDim = dim3((unsigned)((rows + SLAB - 1) / SLAB * ranks), (unsigned)batch, 1);
+      lc.blockDim = dim3(256, 1, 1);
+      lc.dynamicSmemBytes = bytes;
+      lc.stream = s;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)ranks;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      lc.attrs = at;
+      lc.numAttrs = 1;
+      check(cudaLaunchKernelEx(&lc, kernel, src, out.main, out.exps, (std::uint64_t)rows, (std::uint64_t)k,
+                               (std::uint64_t)st.kpad, src_stride, (std::uint64_t)st.main_bytes, (int)deep, ranks),
+            "split_cols_cluster");
+      return;
+    }
     check(cudaMemsetAsync(out.top, 0, rows * (std::size_t)batch * sizeof(std::uint32_t), s), "cudaMemsetAsync");
     // Deep enough to amortize a block, shallow enough for several on each SM.
     const std::size_t want = std::max<std::size_t>(1, 152 * 8 / ((std::size_t)cols * batch));
