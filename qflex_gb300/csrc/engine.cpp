@@ -200,14 +200,20 @@ void Engine::set_tc_variant(std::size_t m, std::size_t n, std::size_t k, int var
   ++options_version_;
 }
 
-// Whether the 3xFP16 product splits A inside the kernel, as every 128 columns
+static SplitKind split_kind(int precision) {
+  return precision == TF32X3 ? KIND_TF32 : precision == BF16X3 ? KIND_BF16 : KIND_FP16;
+}
+
+// Whether the 3xFP16 or 3xTF32 product splits A inside the kernel, as every 128 columns
 // of the product then do again, beside the MMAs, instead of in a pass over A
 // before it. Split + product against direct: (65536, 256, 256) x 4 211 + 309
 // and 286 us, (4096, 4096, 4096) 49 + 965 and 901 us, (256, 4096, 4096) 5 +
 // 130 and 121 us, (128, 4096, 4096), too few rows for a pair of CTAs, 4 + 129
-// and 150 us: there the passes are left out while n is small.
+// and 150 us: there the passes are left out while n is small. 3xTF32: (4096,
+// 4096, 4096) 72 + 1747 and 1495 us, (65536, 256, 16) x 4 17 + 104 and 97 us.
 bool Engine::direct_product(std::size_t m, std::size_t n, const TcConfig& cfg) const {
-  return precision_ == FP16X3 && cfg.variant == 0 && cfg.chunk == 2 && (m > 128 || n <= 1024);
+  return (precision_ == FP16X3 || precision_ == TF32X3) && cfg.variant == 0 && cfg.chunk == 2 &&
+         (m > 128 || n <= 1024);
 }
 
 // Products of 16 to 63 columns in the direct kernel's tiles of 32 or 64, from
@@ -217,11 +223,12 @@ bool Engine::direct_product(std::size_t m, std::size_t n, const TcConfig& cfg) c
 // 32, 256) 194 and 63, (256, 16, 256) 39 and 15, (1000, 50, 100) 26 and 14.
 // Contractions with fewer rows may run as one small program instead.
 bool Engine::narrow_product(std::size_t m, std::size_t n, std::size_t k) const {
-  return m >= 256 && n >= 16 && n < 64 && k >= 96 && tc_runs(m, n, k) && direct_product(m, n, tc_config(m, n, k));
+  return precision_ == FP16X3 && m >= 256 && n >= 16 && n < 64 && k >= 96 && tc_runs(m, n, k) &&
+         direct_product(m, n, tc_config(m, n, k));
 }
 
 std::size_t Engine::workspace_elems(std::size_t m, std::size_t n, std::size_t k) const {
-  return direct_product(m, n, tc_config(m, n, k)) ? tc_direct_workspace_elems(n, k) : tc_workspace_elems(m, n, k);
+  return direct_product(m, n, tc_config(m, n, k)) ? tc_direct_workspace_elems(split_kind(precision_), n, k) : tc_workspace_elems(m, n, k);
 }
 
 void Engine::launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
@@ -231,8 +238,8 @@ void Engine::launch_split_product(const float2* A, const float2* B, BLayout b_la
   if (direct_product(m, n, cfg)) {
     const bool aligned = (reinterpret_cast<std::uintptr_t>(A) & 15) == 0 && k % 2 == 0 &&
                          (batch == 1 || ac_stride % 2 == 0);
-    launch_cgemm_fp16x3_direct(A, make_a_rows(k, aligned), B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws,
-                               error_flag(), cfg, stream_);
+    launch_cgemm_direct(split_kind(precision_), A, make_a_rows(k, aligned), B, b_layout, C, m, n, k, ac_stride,
+                        b_stride, batch, ws, error_flag(), cfg, stream_);
   } else if (precision_ == FP16X3) {
     launch_cgemm_fp16x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
   } else if (precision_ == BF16X3) {
@@ -361,7 +368,7 @@ Engine::Plan* Engine::get_plan(const std::string& circuit, const std::string& or
   key += open_terminals_ ? "o" : "p";
   key += std::to_string(exact_gates_);
   if (!fuse_splits_) key += "n";
-  if (precision_ == FP16X3) {
+  if (precision_ == FP16X3 || precision_ == TF32X3) {
     // What decides which products run in the direct kernel.
     key += cat("f", tc_cfg_.chunk == 2 ? 1 : 0, ",", tc_cfg_.variant);
     for (const auto& [shape, variant] : tc_variant_)
@@ -574,8 +581,8 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
       const bool a_planes = p.fused[i] == (int)i;
       const TcConfig cfg = tc_config(op.m, op.n, op.k);
       if (op.a_gather)
-        launch_cgemm_fp16x3_direct(arena + op.a, p.gather[gathered++], arena + op.b, BLayout::nk, arena + op.c, op.m, op.n,
-                                   op.k, stride, stride, batch, tc_ws, error_flag(), cfg, stream_);
+        launch_cgemm_direct(split_kind(precision_), arena + op.a, p.gather[gathered++], arena + op.b, BLayout::nk,
+                            arena + op.c, op.m, op.n, op.k, stride, stride, batch, tc_ws, error_flag(), cfg, stream_);
       else if (a_planes)
         launch_cgemm_fp16x3(arena + op.a, arena + op.b, BLayout::nk, arena + op.c, op.m, op.n, op.k, stride, stride,
                             batch, tc_ws, error_flag(), cfg, stream_, true);

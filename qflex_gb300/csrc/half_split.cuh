@@ -1,10 +1,16 @@
-// Splitting FP32 values into FP16 hi + lo.
+// Splitting FP32 values into FP16 hi + lo, rounding them to TF32.
 #pragma once
 
 #include <cstdint>
 
 namespace qfx {
 namespace {
+
+__device__ __forceinline__ float tf32_rn(float x) {
+  std::uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r);
+}
 
 // hi = fp16(x), lo = fp16(x - hi), both to nearest, for two values: a packs
 // into the low halves, b into the high ones. x - hi is one mixed-precision FMA

@@ -29,12 +29,6 @@
 namespace qfx {
 namespace {
 
-__device__ __forceinline__ float tf32_rn(float x) {
-  std::uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
 // The exponent e of a 3xFP16 row whose largest component has the bit pattern
 // `mb`: max * 2^e in [2^14, 2^15). Rows of zeros, and rows with infinities or
 // NaN, keep 0.

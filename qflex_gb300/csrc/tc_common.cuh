@@ -10,9 +10,13 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "tc_gemm.h"
+
 namespace qfx {
 
 // Host helpers, defined in tc_gemm.cu next to the plane layouts.
+CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
+                      int row_floats = 32, int box_inner = 32);
 // Map over complex64 elements (`dims`, byte `strides` of the dimensions from
 // the second on) for boxes with rows of 16 elements, 128-byte swizzle.
 CUtensorMap element_map(const float2* base, int rank, const std::uint64_t* dims, const std::uint64_t* strides,
@@ -22,12 +26,6 @@ CUtensorMap plane_map_f16(const __half* base, std::uint64_t rows, std::uint64_t 
 bool output_map(float2* C, std::size_t m, std::size_t n, std::uint64_t batch_stride, int batch, CUtensorMap* map,
                 bool narrow = false);
 unsigned persistent_grid(std::size_t tiles);
-// Operand kinds of the single-CTA kernel: 3xTF32 planes (8 values of 4
-// bytes per plane and k-step) or 3xFP16 planes (16 values of 2 bytes, rows
-// scaled by powers of two).
-// BF16x3: three BF16 pieces per value (x = b0 + b1 + b2 to ~24 bits).
-enum SplitKind : int { KIND_TF32 = 0, KIND_FP16 = 1, KIND_BF16 = 2 };
-
 // Splits `batch` operands into planes (split.cu): `rows` rows of k values, or
 // with `columns` the columns of a row-major k x rows matrix. `nplanes` 4, or 6
 // with the negated imaginary planes (not BF16). `top` holds rows * batch words

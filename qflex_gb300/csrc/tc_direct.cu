@@ -1,16 +1,18 @@
-// The 3xFP16 product that splits A itself (sm_103a, tcgen05 + TMEM + TMA).
+// The 3xFP16 and 3xTF32 products that split A themselves (sm_103a, tcgen05 +
+// TMEM + TMA).
 //
-// C = A * B, A complex64 in global memory, B as FP16 planes of Bt (n x k,
-// K-major, see split_fp16_kernel). A is brought in as it lies -- row-major,
+// C = A * B, A complex64 in global memory, B as planes of Bt (n x k, K-major,
+// see split.cu). A is brought in as it lies -- row-major,
 // or through the index permutation that would have laid it out so (AGather)
-// -- and split into its four FP16 planes inside the kernel. Against a split
+// -- and split into its four planes inside the kernel. Against a split
 // kernel (or a plane-writing permutation) before the product that saves one
 // pass over A: 8 B read and 8 B written per element.
 //
 // Structure: persistent, one CTA per SM over tiles of 128 rows x BN (128, 64
 // or 32) columns, 512 threads in four warpgroups whose registers setmaxnreg divides (56, 176,
 // 176, 104 per thread: 128 on average, the launch's own share). Work goes by
-// blocks of A, 128 rows x 32 values (two k-steps of 16):
+// blocks of A, 128 rows x two k-steps (32 values; 3xTF32, whose k-steps are
+// of 8 and which scales nothing, 16: half a place in A's ring):
 //   warp 0       B producer: four 8 KB TMA boxes a block (re and im rows of
 //                64 bytes, hi and lo, of each k-step)
 //   warp 1       TMEM allocation; issues every MMA
@@ -44,6 +46,9 @@
 // pipe idle for 3300; (4096, 1024, 4096) from 319 to 240; (65536, 256, 16) x
 // 4 takes 96, of which writing C alone is 80.
 //
+// 3xTF32: (2048, 2048, 2048) 18 + 256 + 22 us with both operands split before
+// the product, 218 + 17; (65536, 256, 256) x 4 228 + 495 and 436.
+//
 // B holds no negated copy: the real part takes -Ai Bi by the descriptor's
 // negate-A bit, and a k-step loads 16 KB of B, not 24. MMAs of N = 128 run at
 // the rate of N = 256 when A lies in TMEM.
@@ -66,12 +71,16 @@ namespace qfx {
 namespace {
 
 constexpr int BM = 128;
-constexpr int A_BLOCK = 128 * 32 * 8;  // bytes
+constexpr int A_BLOCK = 128 * 32 * 8;  // bytes of A as it lies, 32 values of a row
 constexpr int A_BUFS = 2;              // blocks of planes in TMEM
 constexpr int HALVES = 3;              // sums, the real or imaginary part of a block
 constexpr int EXP_RING = 4;            // block exponents, see the converter
 constexpr int SLOT = 4096;             // output box: 32 rows x 16 complex
 constexpr int TMEM_A_BLOCK = 64;       // 2 k-steps x 4 planes x 8 words
+template <int KIND>
+__host__ __device__ constexpr int block_values() {  // values of a row in two k-steps
+  return KIND == KIND_TF32 ? 16 : 32;
+}
 constexpr int THREADS = 512;
 constexpr int LOADERS = 64, CONVERTERS = 128;
 
@@ -105,15 +114,16 @@ struct Layout {
 // TMEM (re hi, lo, im hi, lo, 8 columns each from `a`) against B's re rows
 // (`blo`, hi and lo 32 bytes apart) and im rows (B_PART further), small terms
 // first.
-template <int BN, bool PAIR, int IM>
+template <int KIND, int BN, bool PAIR, int IM>
 __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std::uint32_t blo, std::uint32_t bhi) {
   constexpr int rows = PAIR ? 2 * BM : BM;
-  constexpr std::uint32_t pos = idesc_f16(rows, BN, false), neg = idesc_f16(rows, BN, true);
+  constexpr std::uint32_t pos = KIND == KIND_TF32 ? idesc_tf32(rows, BN, false) : idesc_f16(rows, BN, false);
+  constexpr std::uint32_t neg = KIND == KIND_TF32 ? idesc_tf32(rows, BN, true) : idesc_f16(rows, BN, true);
   constexpr std::uint32_t part = Layout<BN, PAIR>::B_PART / 16;
   // Ar multiplies B's part of the same name, Ai the other one (negated for
   // the real part).
   const std::uint32_t x = IM ? blo + part : blo, y = IM ? blo : blo + part;
-#define QFX_MMA(g, a_, b_, id, p) " tcgen05.mma.cta_group::" g ".kind::f16 [%0], [" a_ "], " b_ ", " id ", " p ";\n"
+#define QFX_MMA(g, a_, b_, id, p) " tcgen05.mma.cta_group::" g " [%0], [" a_ "], " b_ ", " id ", " p ";\n"
 #define QFX_KSTEP(g, rh, rl, ih, il, p)                                                                  \
   QFX_MMA(g, rh, "xl", "%5", p)                                                                          \
   QFX_MMA(g, rl, "xh", "%5", "p1")                                                                       \
@@ -132,10 +142,14 @@ __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std:
         " add.u32 x0, %2, %7;\n add.u32 y0, %3, %7;\n add.u32 x1, x0, 2;\n add.u32 y1, y0, 2;\n" \
         QFX_BDESC QFX_KSTEP(g, "a4", "a5", "a6", "a7", "p1") "}\n" ::"r"(d), \
         "r"(a), "r"(x), "r"(y), "r"(bhi), "r"(pos), "r"(IM ? pos : neg), "n"(2 * part))
-  if constexpr (PAIR)
-    QFX_BLOCK("2");
+  if constexpr (PAIR && KIND == KIND_TF32)
+    QFX_BLOCK("2.kind::tf32");
+  else if constexpr (PAIR)
+    QFX_BLOCK("2.kind::f16");
+  else if constexpr (KIND == KIND_TF32)
+    QFX_BLOCK("1.kind::tf32");
   else
-    QFX_BLOCK("1");
+    QFX_BLOCK("1.kind::f16");
 #undef QFX_BLOCK
 #undef QFX_BDESC
 #undef QFX_KSTEP
@@ -189,9 +203,9 @@ __device__ __forceinline__ void cp_async_arrive(std::uint64_t* bar) {
 #define QFX_SETMAXNREG_DEC(n) asm volatile("setmaxnreg.dec.sync.aligned.u32 " #n ";")
 #define QFX_SETMAXNREG_INC(n) asm volatile("setmaxnreg.inc.sync.aligned.u32 " #n ";")
 
-template <int BN, bool PAIR>
+template <int KIND, int BN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
-    cgemm_fp16x3_direct_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+    cgemm_direct_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ AGather g,
                                const float2* __restrict__ A, float2* __restrict__ C, int tma_c, int m, int n, int k,
                                int batches, std::uint64_t ac_stride, int* __restrict__ err,
@@ -256,7 +270,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     else
       umma_commit(bar);
   };
-  const int blocks = (k + 31) / 32;
+  constexpr int VALUES = block_values<KIND>();
+  const int blocks = (k + VALUES - 1) / VALUES, loads = (k + 31) / 32;  // of a tile
   // Blocks of all the CTA's tiles.
   const int work = first < total ? ((total - 1 - first) / stride + 1) * blocks : 0;
 
@@ -302,6 +317,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     QFX_SETMAXNREG_DEC(56);
     if (warp == 0 && lane == 0) {
       // B producer.
+      constexpr int X_IM = KIND == KIND_TF32 ? 16 : 32;  // im rows in the map
       int q = 0, s = 0;
       for (int t = first; t < total && !*abort_flag; t += stride) {
         int mt, nt, batch;
@@ -320,15 +336,15 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (rank == 0) mbar_expect_tx(&b_full[s], 2 * B_STAGE);
             const std::uint32_t bar = peer_addr(&b_full[s], 0);
             tma_load_4d_pair(&map_b, bar, st, 0, col, 2 * b, batch);
-            tma_load_4d_pair(&map_b, bar, st + B_PART, 32, col, 2 * b, batch);
+            tma_load_4d_pair(&map_b, bar, st + B_PART, X_IM, col, 2 * b, batch);
             tma_load_4d_pair(&map_b, bar, st + 2 * B_PART, 0, col, 2 * b + 1, batch);
-            tma_load_4d_pair(&map_b, bar, st + 3 * B_PART, 32, col, 2 * b + 1, batch);
+            tma_load_4d_pair(&map_b, bar, st + 3 * B_PART, X_IM, col, 2 * b + 1, batch);
           } else {
             mbar_expect_tx(&b_full[s], B_STAGE);
             tma_load_4d(&map_b, &b_full[s], st, 0, col, 2 * b, batch);
-            tma_load_4d(&map_b, &b_full[s], st + B_PART, 32, col, 2 * b, batch);
+            tma_load_4d(&map_b, &b_full[s], st + B_PART, X_IM, col, 2 * b, batch);
             tma_load_4d(&map_b, &b_full[s], st + 2 * B_PART, 0, col, 2 * b + 1, batch);
-            tma_load_4d(&map_b, &b_full[s], st + 3 * B_PART, 32, col, 2 * b + 1, batch);
+            tma_load_4d(&map_b, &b_full[s], st + 3 * B_PART, X_IM, col, 2 * b + 1, batch);
           }
           ++q;
           if (++s == B_STAGES) s = 0;
@@ -378,7 +394,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;");
         const std::uint32_t a = tmem + TMEM_A + xa * TMEM_A_BLOCK, b = b_lo0 + sb * (B_STAGE >> 4);
         if (leader) {
-          mma_block<BN, PAIR, 0>(tmem + h * BN, a, b, b_hi);
+          mma_block<KIND, BN, PAIR, 0>(tmem + h * BN, a, b, b_hi);
           commit(&re_full[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
@@ -387,7 +403,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!__all_sync(0xffffffffu, kind != 3 || wait(bars + at, parity, 4))) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (leader) {
-          mma_block<BN, PAIR, 1>(tmem + h * BN, a, b, b_hi);
+          mma_block<KIND, BN, PAIR, 1>(tmem + h * BN, a, b, b_hi);
           commit(&done[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
@@ -417,7 +433,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           if (!g.plain)
             for (int x = 0; x < AGather::kBits && (mt >> x); ++x)
               if ((mt >> x) & 1) tile_src += g.tile_src[x];
-          for (int b = 0; b < blocks; ++b) {
+          for (int b = 0; b < loads; ++b) {
             if (q >= A_RING && !wait(&raw_empty[s], ph ^ 1u, 5)) break;
             const std::uint32_t dst = ring + s * A_BLOCK;
             mbar_expect_tx(&raw_full[s], bytes);
@@ -470,7 +486,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         else
           for (int b = 0; b < AGather::kBits && (mt >> b); ++b)
             if ((mt >> b) & 1) tile_src += g.tile_src[b];
-        for (int b = 0; b < blocks; ++b) {
+        for (int b = 0; b < loads; ++b) {
           if (q >= A_RING && !wait(&raw_empty[s], ph ^ 1u, 5)) {
             ok = false;
             break;
@@ -525,52 +541,71 @@ __global__ void __launch_bounds__(THREADS, 1)
     const std::uint32_t lanes = tmem + TMEM_A + (std::uint32_t((warp - 12) * 32) << 16);
     int s = 0, x = 0, xa = 0, r = DONE - A_BUFS;
     std::uint32_t ph = 0, pd = 1;  // block w - A_BUFS: barrier r
-    for (int w = 0; w < work; ++w) {
-      if (!__all_sync(0xffffffffu, wait(&raw_full[s], ph, 6))) break;
+    // Block w: its values lie in one place of the ring, or (3xTF32) in half of
+    // one, b counting the tile's blocks.
+    for (int w = 0, b = 0; w < work; ++w) {
+      const int half = VALUES == 16 ? b & 1 : 0;
+      b = b == blocks - 1 ? 0 : b + 1;
+      const bool first_half = half == 0, last = VALUES == 32 || half || b == 0;
+      if (first_half && !__all_sync(0xffffffffu, wait(&raw_full[s], ph, 6))) break;
       const std::uint32_t block = ring + s * A_BLOCK;
-      float2 v[32];
+      const std::uint32_t at0 = half ? row_at ^ g.value_at[16] : row_at;
+      float2 v[VALUES];
       if (g.pairs) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2)
+        for (int i = 0; i < VALUES; i += 2)
           asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                        : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i + 1].x), "=f"(v[i + 1].y)
-                       : "r"(block + (row_at ^ g.value_at[i]))
+                       : "r"(block + (at0 ^ g.value_at[i]))
                        : "memory");
       } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
+        for (int i = 0; i < VALUES; ++i)
           asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
                        : "=f"(v[i].x), "=f"(v[i].y)
-                       : "r"(block + (row_at ^ g.value_at[i]))
+                       : "r"(block + (at0 ^ g.value_at[i]))
                        : "memory");
       }
-      // Bit patterns of non-negative floats order like their values.
-      std::uint32_t mx[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        mx[i & 3] = max(mx[i & 3], max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
-      // e with max * 2^e in [2^14, 2^15), at most 126 (2^e and 2^-e stay
-      // normal floats; smaller blocks keep all their bits: below 2^-112 the
-      // lo planes reach further down than FP32 itself). A block of zeros
-      // takes 126 so that it never sets the scale of the sum; infinities
-      // and NaN keep 0.
-      const int be = int(max(max(mx[0], mx[1]), max(mx[2], mx[3])) >> 23);
-      const int e = be == 255 ? 0 : min(141 - be, 126);
-      const float sc = __uint_as_float(std::uint32_t(e + 127) << 23);
-      const float2 sc2 = make_float2(sc, sc);
-      // The block is in registers: its place in the ring is free.
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&raw_empty[s]);
       std::uint32_t p[2][32];  // of each k-step: 8 words of every plane
+      int e = 0;
+      if constexpr (KIND == KIND_FP16) {
+        // Bit patterns of non-negative floats order like their values.
+        std::uint32_t mx[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-      for (int i = 0; i < 32; i += 16)
+        for (int i = 0; i < VALUES; ++i)
+          mx[i & 3] = max(mx[i & 3], max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
+        // e with max * 2^e in [2^14, 2^15), at most 126 (2^e and 2^-e stay
+        // normal floats; smaller blocks keep all their bits: below 2^-112 the
+        // lo planes reach further down than FP32 itself). A block of zeros
+        // takes 126 so that it never sets the scale of the sum; infinities
+        // and NaN keep 0.
+        const int be = int(max(max(mx[0], mx[1]), max(mx[2], mx[3])) >> 23);
+        e = be == 255 ? 0 : min(141 - be, 126);
+        const float sc = __uint_as_float(std::uint32_t(e + 127) << 23);
+        const float2 sc2 = make_float2(sc, sc);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
-          const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
-          split_pair(re.x, re.y, p[i / 16][j], p[i / 16][8 + j]);
-          split_pair(im.x, im.y, p[i / 16][16 + j], p[i / 16][24 + j]);
+        for (int i = 0; i < VALUES; i += 16)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
+            const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
+            split_pair(re.x, re.y, p[i / 16][j], p[i / 16][8 + j]);
+            split_pair(im.x, im.y, p[i / 16][16 + j], p[i / 16][24 + j]);
+          }
+      } else {
+#pragma unroll
+        for (int i = 0; i < VALUES; ++i) {
+          std::uint32_t* o = p[i / 8] + i % 8;
+          const float rh = tf32_rn(v[i].x), ih = tf32_rn(v[i].y);
+          o[0] = __float_as_uint(rh);
+          o[8] = __float_as_uint(tf32_rn(v[i].x - rh));
+          o[16] = __float_as_uint(ih);
+          o[24] = __float_as_uint(tf32_rn(v[i].y - ih));
         }
+      }
+      // The values are in registers: their place in the ring is free.
+      __syncwarp();
+      if (last && lane == 0) mbar_arrive(&raw_empty[s]);
       if (!__all_sync(0xffffffffu, wait(&done[r], pd, 10))) break;
       if (++r == DONE) {
         r = 0;
@@ -582,14 +617,14 @@ __global__ void __launch_bounds__(THREADS, 1)
       // Exponents live in a ring of their own: the MMAs of the block two
       // back are done, so every epilogue warp has read the exponents of the
       // block three back.
-      exps[x * BM + row] = std::int8_t(e);
+      if constexpr (KIND == KIND_FP16) exps[x * BM + row] = std::int8_t(e);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) arrive(&a_full[xa]);
       xa ^= 1;
       if (++x == EXP_RING) x = 0;
-      if (++s == A_RING) {
+      if (last && ++s == A_RING) {
         s = 0;
         ph ^= 1u;
       }
@@ -606,7 +641,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const std::int8_t* exps = reinterpret_cast<const std::int8_t*>(smem + L::OFF_EXP);
     std::uint8_t* staging = smem + L::OFF_STAGING + (warp - 4) * L::SLOTS * SLOT;
     int* sc_row = reinterpret_cast<int*>(smem + L::OFF_SCALE) + (warp - 4) * COLS;
-    const float beta = debias_beta<KIND_FP16>(err, 2, (k + 15) / 16);
+    const float beta = debias_beta<KIND>(err, 2, (k + VALUES / 2 - 1) / (VALUES / 2));
     const float2 beta2 = make_float2(beta, beta);
     int h = 0, x = 0, r = 0;
     std::uint32_t pr = 0;
@@ -641,8 +676,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int ncols = n - n0;
       // Exponents of the lane's columns, fetched before the drain.
       const int* eb = exp_b + std::uint64_t(batch) * n + n0;
-      const int eb0 = lane < min(ncols, COLS) ? eb[lane] : 0;
-      const int eb1 = COLS > 32 && 32 + lane < ncols ? eb[32 + lane] : eb0;
+      const int eb0 = KIND == KIND_FP16 && lane < min(ncols, COLS) ? eb[lane] : 0;
+      const int eb1 = KIND == KIND_FP16 && COLS > 32 && 32 + lane < ncols ? eb[32 + lane] : eb0;
       float2 re[COLS / 2], im[COLS / 2];  // columns 2 j, 2 j + 1
 #pragma unroll
       for (int j = 0; j < COLS / 2; ++j) re[j] = im[j] = make_float2(0.f, 0.f);
@@ -657,11 +692,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const int e = exps[x * BM + row];
+        const int e = KIND == KIND_FP16 ? exps[x * BM + row] : 0;
         if (++x == EXP_RING) x = 0;
         if (b == 0) {
-          eref = e - 2;
-        } else if (__any_sync(0xffffffffu, e < eref)) {
+          eref = KIND == KIND_FP16 ? e - 2 : 0;
+        } else if (KIND == KIND_FP16 && __any_sync(0xffffffffu, e < eref)) {
           const int next = e < eref ? e - 2 : eref;
           const float f = pow2(next - eref);
           const float2 f2 = make_float2(f, f);
@@ -1015,16 +1050,19 @@ static int direct_columns(std::size_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : 
 // its store, which starts later in a pair. Single CTAs against pairs: (65536,
 // 256, k) x 4 with k = 32 104 and 106 us, 64 143 and 149, 256 301 and 286;
 // (8192, 128, 128) x 16 59 and 60.5; (4096, 1024, 4096) 272 and 240.
-static bool direct_pair(std::size_t m, std::size_t k) { return m > (std::size_t)BM && k > 128; }
+static bool direct_pair(SplitKind kind, std::size_t m, std::size_t k) {
+  return m > (std::size_t)BM && k > (kind == KIND_TF32 ? 64u : 128u);
+}
 
-std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k) {
+std::size_t tc_direct_workspace_elems(SplitKind kind, std::size_t n, std::size_t k) {
+  if (kind == KIND_TF32) return 4 * n * ((k + 7) / 8 * 8);
   return 2 * n * ((k + 15) / 16 * 16) + 2 * n;  // B's planes, exponents and largest components
 }
 
-void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* B, BLayout b_layout, float2* C,
-                                std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
-                                std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
-                                cudaStream_t s) {
+void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather, const float2* B, BLayout b_layout,
+                         float2* C, std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
+                         std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
+                         cudaStream_t s) {
   if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk != 2)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct product takes chunks of 2 k-steps");
@@ -1034,20 +1072,28 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
     const std::uint64_t most = ((std::uint64_t(1) << 35) - (std::uint64_t(1) << gather.nbits)) / ac_stride + 1;
     if (most < (std::uint64_t)batch) {
       for (int at = 0; at < batch; at += (int)most)
-        launch_cgemm_fp16x3_direct(A + at * ac_stride, gather, B + at * b_stride, b_layout, C + at * ac_stride, m, n, k,
-                                   ac_stride, b_stride, (int)std::min<std::uint64_t>(most, batch - at), workspace, err,
-                                   cfg, s);
+        launch_cgemm_direct(kind, A + at * ac_stride, gather, B + at * b_stride, b_layout, C + at * ac_stride, m, n, k,
+                            ac_stride, b_stride, (int)std::min<std::uint64_t>(most, batch - at), workspace, err, cfg,
+                            s);
       return;
     }
   }
-  const std::size_t kpad = (k + 15) / 16 * 16;
-  __half* pb = reinterpret_cast<__half*>(workspace);
-  int* eb = reinterpret_cast<int*>(pb + 4 * n * kpad * (std::size_t)batch);
-  std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
-  launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
-  const int bn = direct_columns(n);
-  const bool pair = bn == 128 && direct_pair(m, k);
-  const CUtensorMap mb = plane_map_f16(pb, n, kpad, batch, pair ? bn / 2 : bn, 64);
+  const int bn = kind == KIND_FP16 ? direct_columns(n) : 128;
+  const bool pair = bn == 128 && direct_pair(kind, m, k);
+  const int b_cols = pair ? bn / 2 : bn;
+  int* eb = nullptr;
+  CUtensorMap mb;
+  if (kind == KIND_FP16) {
+    const std::size_t kpad = (k + 15) / 16 * 16;
+    __half* pb = reinterpret_cast<__half*>(workspace);
+    eb = reinterpret_cast<int*>(pb + 4 * n * kpad * (std::size_t)batch);
+    std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
+    launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
+    mb = plane_map_f16(pb, n, kpad, batch, b_cols, 64);
+  } else {
+    launch_split(KIND_TF32, 4, {workspace}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
+    mb = plane_map(workspace, n, (k + 7) / 8 * 8, batch, b_cols, 32, 16);
+  }
   CUtensorMap ma;
   std::memset(&ma, 0, sizeof(ma));
   if (gather.boxes && gather.plain) {
@@ -1069,10 +1115,10 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
   const int tma_c = output_map(C, m, n, ac_stride, batch, &mc) ? 1 : 0;
   const std::size_t rows = pair ? 2 * BM : BM;
   const std::size_t tiles = ((m + rows - 1) / rows) * ((n + bn - 1) / bn) * (std::size_t)batch;
-  auto run = [&](auto columns, auto paired) {
+  auto run = [&](auto of_kind, auto columns, auto paired) {
     constexpr int BN = decltype(columns)::value;
     constexpr bool PAIR = decltype(paired)::value;
-    auto* kernel = cgemm_fp16x3_direct_kernel<BN, PAIR>;
+    auto* kernel = cgemm_direct_kernel<decltype(of_kind)::value, BN, PAIR>;
     cudaLaunchConfig_t lc = {};
     lc.blockDim = dim3(THREADS, 1, 1);
     lc.dynamicSmemBytes = Layout<BN, PAIR>::SMEM;
@@ -1099,18 +1145,21 @@ void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const fl
                       1, 1);
     check(cudaLaunchKernelEx(&lc, kernel, ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err,
                              (const int*)eb),
-          "cgemm_fp16x3_direct");
+          "cgemm_direct");
   };
   using std::integral_constant;
-  if (pair)
-    run(integral_constant<int, 128>{}, std::true_type{});
+  const integral_constant<int, KIND_FP16> fp16;
+  const integral_constant<int, KIND_TF32> tf32;
+  const integral_constant<int, 128> c128;
+  if (kind == KIND_TF32)
+    pair ? run(tf32, c128, std::true_type{}) : run(tf32, c128, std::false_type{});
   else if (bn == 128)
-    run(integral_constant<int, 128>{}, std::false_type{});
+    pair ? run(fp16, c128, std::true_type{}) : run(fp16, c128, std::false_type{});
   else if (bn == 64)
-    run(integral_constant<int, 64>{}, std::false_type{});
+    run(fp16, integral_constant<int, 64>{}, std::false_type{});
   else
-    run(integral_constant<int, 32>{}, std::false_type{});
-  check(cudaGetLastError(), "cgemm_fp16x3_direct");
+    run(fp16, integral_constant<int, 32>{}, std::false_type{});
+  check(cudaGetLastError(), "cgemm_direct");
 }
 
 }  // namespace qfx

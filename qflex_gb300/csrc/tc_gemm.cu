@@ -996,29 +996,6 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// 4-D map over split planes laid out [batch][kpad / 8][rows][row_floats] (32:
-// re hi, lo, im hi, lo; 48: also -im hi, lo). Box {32, box_rows, 1, 1}: whole
-// 128-byte rows, 128-byte swizzle; or with box_inner = 16 the hi and lo planes
-// of one part as 64-byte rows, 64-byte swizzle.
-CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
-                      int row_floats = 32, int box_inner = 32) {
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  const std::uint64_t kb = kpad / 8, rb = std::uint64_t(row_floats) * 4;
-  const cuuint64_t dims[4] = {(cuuint64_t)row_floats, rows, kb, (cuuint64_t)batch};
-  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
-  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides,
-                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
-        std::to_string((int)r);
-  return map;
-}
-
 // 4-D map over BF16 planes laid out [batch][kpad / 16][rows][inner]; box
 // {box_inner, box_rows, 1, 1}: rows of 128, 64 or 32 bytes in the swizzle of
 // that width.
@@ -1048,6 +1025,29 @@ void check(cudaError_t e, const char* what) {
 }
 
 }  // namespace
+
+// 4-D map over split planes laid out [batch][kpad / 8][rows][row_floats] (32:
+// re hi, lo, im hi, lo; 48: also -im hi, lo). Box {32, box_rows, 1, 1}: whole
+// 128-byte rows, 128-byte swizzle; or with box_inner = 16 the hi and lo planes
+// of one part as 64-byte rows, 64-byte swizzle.
+CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
+                      int row_floats, int box_inner) {
+  CUtensorMap map;
+  std::memset(&map, 0, sizeof(map));
+  const std::uint64_t kb = kpad / 8, rb = std::uint64_t(row_floats) * 4;
+  const cuuint64_t dims[4] = {(cuuint64_t)row_floats, rows, kb, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
+  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides,
+                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
+        std::to_string((int)r);
+  return map;
+}
 
 // 4-D map over FP16 planes laid out [batch][kpad / 16][rows][row_halves]
 // (64: re hi, lo, im hi, lo; 96: also -im hi, lo). Box {32, box_rows, 1, 1}:

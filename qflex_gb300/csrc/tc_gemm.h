@@ -8,6 +8,12 @@
 
 namespace qfx {
 
+// Operand kinds: 3xTF32 planes (8 values of 4
+// bytes per plane and k-step) or 3xFP16 planes (16 values of 2 bytes, rows
+// scaled by powers of two).
+// BF16x3: three BF16 pieces per value (x = b0 + b1 + b2 to ~24 bits).
+enum SplitKind : int { KIND_TF32 = 0, KIND_FP16 = 1, KIND_BF16 = 2 };
+
 // Shapes that a contraction gives to the tensor-core kernels (smaller products
 // stay on the CUDA-core kernels).
 bool tc_eligible(std::size_t m, std::size_t n, std::size_t k);
@@ -109,16 +115,16 @@ bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size
 // checks: dst is the m x k operand the product sees. Tests use it.
 void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const float2* src, float2* dst);
 
-// fp32 elements that launch_cgemm_fp16x3_direct's workspace takes per batch entry.
-std::size_t tc_direct_workspace_elems(std::size_t n, std::size_t k);
-// The same product with A split inside the kernel: A is read as complex64
-// through `gather`, every 32 values of a row scaled by their own power of
-// two, and no A planes exist in memory. Single CTA, cfg.chunk 2 (a TMEM
-// chunk is one of A's blocks); cfg.variant is ignored.
-void launch_cgemm_fp16x3_direct(const float2* A, const AGather& gather, const float2* B, BLayout b_layout, float2* C,
-                                std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
-                                std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
-                                cudaStream_t s);
+// fp32 elements that launch_cgemm_direct's workspace takes per batch entry.
+std::size_t tc_direct_workspace_elems(SplitKind kind, std::size_t n, std::size_t k);
+// The 3xFP16 or 3xTF32 product with A split inside the kernel: A is read as
+// complex64 through `gather` (3xFP16: every 32 values of a row scaled by their
+// own power of two), and no A planes exist in memory. cfg.chunk 2 (a TMEM chunk
+// is one of A's blocks); cfg.variant is ignored.
+void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather, const float2* B, BLayout b_layout,
+                         float2* C, std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
+                         std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
+                         cudaStream_t s);
 
 // The same product with BF16x3 planes: x = b0 + b1 + b2 in BF16 (no
 // scaling: BF16 has the FP32 exponent range), six products per real

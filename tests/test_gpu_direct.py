@@ -4,7 +4,7 @@ and on rows whose magnitude changes from one block of 32 values to the next."""
 import numpy as np
 import pytest
 
-from qflex_gb300 import FP16X3, Context
+from qflex_gb300 import FP16X3, TF32X3, Context
 
 pytestmark = pytest.mark.gpu
 
@@ -27,7 +27,7 @@ def _rows(kind, g, m, k):
 @pytest.mark.parametrize("m,n,k,batch,extra", [
     (64, 64, 16, 1, 0), (128, 128, 32, 1, 0), (129, 64, 64, 2, 0), (300, 128, 64, 1, 1), (192, 256, 128, 3, 1),
     (1024, 1024, 32, 1, 0), (20000, 64, 16, 1, 0)])
-def test_direct_product(built_lib, kind, m, n, k, batch, extra):
+def test_direct_product(built_lib, kind, m, n, k, batch, extra, precision=FP16X3, tol=TOL):
     import torch
     g = np.random.default_rng(m + n + k)
     stride = m * k + k * n + m * n + extra  # an odd stride leaves rows on 8-byte boundaries
@@ -39,7 +39,7 @@ def test_direct_product(built_lib, kind, m, n, k, batch, extra):
             row[m * k:m * k + k * n] = (g.standard_normal(k * n) + 1j * g.standard_normal(k * n)) * scale_b
     d = torch.from_numpy(buf).cuda()
     torch.cuda.synchronize()
-    ctx = Context(0, FP16X3)
+    ctx = Context(0, precision)
     at = d.data_ptr()
     ctx.multiply(at, at + 8 * m * k, at + 8 * (m * k + k * n), m, n, k, batch, stride)
     ctx.synchronize()
@@ -48,7 +48,7 @@ def test_direct_product(built_lib, kind, m, n, k, batch, extra):
         A, B = row[:m * k].reshape(m, k).astype(complex), row[m * k:m * k + k * n].reshape(k, n).astype(complex)
         C = got[m * k + k * n:m * k + k * n + m * n].reshape(m, n)
         assert np.isfinite(C).all()
-        assert np.max(np.abs(C - A @ B) / (np.abs(A) @ np.abs(B) + 1e-300)) < TOL
+        assert np.max(np.abs(C - A @ B) / (np.abs(A) @ np.abs(B) + 1e-300)) < tol
         assert np.array_equal(got[:m * k + k * n], row[:m * k + k * n])
         assert np.array_equal(got[m * k + k * n + m * n:], row[m * k + k * n + m * n:])
 
@@ -69,3 +69,11 @@ def test_narrow_tiles(built_lib, kind, m, n, k, batch, extra):
 def test_pairs(built_lib, kind, m, n, k, batch, extra):
     """Tiles of two CTAs, also with an empty second half, and of one beside them."""
     test_direct_product(built_lib, kind, m, n, k, batch, extra)
+
+
+# 3xTF32: chunks of 16 values, so k / 16 FP32 additions: below 6e-6 for k <= 400.
+@pytest.mark.parametrize("m,n,k,batch,extra", [
+    (64, 64, 16, 1, 0), (128, 128, 32, 1, 0), (129, 64, 64, 2, 0), (300, 130, 97, 1, 1), (257, 640, 111, 1, 1),
+    (640, 1100, 160, 2, 0), (383, 1500, 400, 1, 0), (20000, 256, 64, 1, 0), (128, 1100, 192, 1, 0)])
+def test_tf32(built_lib, m, n, k, batch, extra):
+    test_direct_product(built_lib, "gauss", m, n, k, batch, extra, TF32X3, 6e-6)
