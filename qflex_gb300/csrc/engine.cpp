@@ -204,16 +204,16 @@ static SplitKind split_kind(int precision) {
   return precision == TF32X3 ? KIND_TF32 : precision == BF16X3 ? KIND_BF16 : KIND_FP16;
 }
 
-// Whether the 3xFP16 or 3xTF32 product splits A inside the kernel, as every 128 columns
+// Whether the product splits A inside the kernel, as every 128 columns
 // of the product then do again, beside the MMAs, instead of in a pass over A
 // before it. Split + product against direct: (65536, 256, 256) x 4 211 + 309
 // and 286 us, (4096, 4096, 4096) 49 + 965 and 901 us, (256, 4096, 4096) 5 +
 // 130 and 121 us, (128, 4096, 4096), too few rows for a pair of CTAs, 4 + 129
 // and 150 us: there the passes are left out while n is small. 3xTF32: (4096,
 // 4096, 4096) 72 + 1747 and 1495 us, (65536, 256, 16) x 4 17 + 104 and 97 us.
-bool Engine::direct_product(std::size_t m, std::size_t n, const TcConfig& cfg) const {
-  return (precision_ == FP16X3 || precision_ == TF32X3) && cfg.variant == 0 && cfg.chunk == 2 &&
-         (m > 128 || n <= 1024);
+bool Engine::direct_product(std::size_t m, std::size_t n, std::size_t k, const TcConfig& cfg) const {
+  if (precision_ == FP32 || is_complex128(precision_) || cfg.variant != 0 || cfg.chunk != 2) return false;
+  return precision_ == BF16X3 ? tc_direct_pair(KIND_BF16, m, k) : m > 128 || n <= 1024;
 }
 
 // Products of 16 to 63 columns in the direct kernel's tiles of 32 or 64, from
@@ -224,18 +224,18 @@ bool Engine::direct_product(std::size_t m, std::size_t n, const TcConfig& cfg) c
 // Contractions with fewer rows may run as one small program instead.
 bool Engine::narrow_product(std::size_t m, std::size_t n, std::size_t k) const {
   return precision_ == FP16X3 && m >= 256 && n >= 16 && n < 64 && k >= 96 && tc_runs(m, n, k) &&
-         direct_product(m, n, tc_config(m, n, k));
+         direct_product(m, n, k, tc_config(m, n, k));
 }
 
 std::size_t Engine::workspace_elems(std::size_t m, std::size_t n, std::size_t k) const {
-  return direct_product(m, n, tc_config(m, n, k)) ? tc_direct_workspace_elems(split_kind(precision_), n, k) : tc_workspace_elems(m, n, k);
+  return direct_product(m, n, k, tc_config(m, n, k)) ? tc_direct_workspace_elems(split_kind(precision_), n, k) : tc_workspace_elems(m, n, k);
 }
 
 void Engine::launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
                                   std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride,
                                   int batch, float* ws) {
   const TcConfig cfg = tc_config(m, n, k);
-  if (direct_product(m, n, cfg)) {
+  if (direct_product(m, n, k, cfg)) {
     const bool aligned = (reinterpret_cast<std::uintptr_t>(A) & 15) == 0 && k % 2 == 0 &&
                          (batch == 1 || ac_stride % 2 == 0);
     launch_cgemm_direct(split_kind(precision_), A, make_a_rows(k, aligned), B, b_layout, C, m, n, k, ac_stride,
@@ -368,7 +368,7 @@ Engine::Plan* Engine::get_plan(const std::string& circuit, const std::string& or
   key += open_terminals_ ? "o" : "p";
   key += std::to_string(exact_gates_);
   if (!fuse_splits_) key += "n";
-  if (precision_ == FP16X3 || precision_ == TF32X3) {
+  if (precision_ != FP32 && !is_complex128(precision_)) {
     // What decides which products run in the direct kernel.
     key += cat("f", tc_cfg_.chunk == 2 ? 1 : 0, ",", tc_cfg_.variant);
     for (const auto& [shape, variant] : tc_variant_)
@@ -536,7 +536,7 @@ void Engine::plan_fusion(Plan& p) {
       if (g.kind == DevOp::PERMUTE) continue;
       if (!g.b_nk || g.a != ops[i].c || g.m * g.k != (std::size_t(1) << ops[i].nbits)) break;
       const TcConfig cfg = tc_config(g.m, g.n, g.k);
-      if (g.k < 32 || (g.k & (g.k - 1)) != 0 || cfg.chunk > 2 || direct_product(g.m, g.n, cfg)) break;
+      if (g.k < 32 || (g.k & (g.k - 1)) != 0 || cfg.chunk > 2 || direct_product(g.m, g.n, g.k, cfg)) break;
       if (only_read_by(ops, i, j)) {
         p.fused[i] = (int)j;
         p.fused[j] = (int)j;
@@ -589,7 +589,7 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
       else
         launch_split_product(arena + op.a, arena + op.b, BLayout::nk, arena + op.c, op.m, op.n, op.k, stride, stride,
                              batch, tc_ws);
-      launches += a_planes || direct_product(op.m, op.n, cfg) ? 2 : 3;  // plane splits and the product
+      launches += a_planes || direct_product(op.m, op.n, op.k, cfg) ? 2 : 3;  // plane splits and the product
     } else if (op.a_gather) {
       launch_cgemm_tiled(arena + op.a, &p.tile_gather[tile_gathered++], arena + op.b, arena + op.c, op.m, op.n, op.k,
                          stride, batch, stream_);
@@ -707,7 +707,7 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
       gather_a = [&](std::size_t m, std::size_t n, std::size_t k, int nbits, const std::uint8_t* perm) {
         if (b_kmajor && b_kmajor(m, n, k)) {
           AGather g;
-          if (!direct_product(m, n, tc_config(m, n, k)) || !make_a_gather(nbits, perm, m, k, &g)) return false;
+          if (!direct_product(m, n, k, tc_config(m, n, k)) || !make_a_gather(nbits, perm, m, k, &g)) return false;
           p.gather.push_back(g);
         } else {
           TileGather g;

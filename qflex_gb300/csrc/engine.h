@@ -130,7 +130,7 @@ class Engine {
   bool debias_ = true;    // tensor-core products compensate the truncation bias
   unsigned options_version_ = 0;  // part of the graph key: options change launches
   TcConfig tc_config(std::size_t m, std::size_t n, std::size_t k) const;
-  bool direct_product(std::size_t m, std::size_t n, const TcConfig& cfg) const;
+  bool direct_product(std::size_t m, std::size_t n, std::size_t k, const TcConfig& cfg) const;
   bool split_multiply(std::size_t m, std::size_t n, std::size_t k) const;
   // fp32 elements of split planes that one product of this shape needs.
   bool narrow_product(std::size_t m, std::size_t n, std::size_t k) const;

@@ -138,19 +138,11 @@ __device__ __forceinline__ void emit(const float2 (&v)[unit_values<KIND>()], int
       o[10] = make_float4(-il[0], -il[1], -il[2], -il[3]);
     }
   } else {
-    __nv_bfloat162 r0[4], r1[4], r2[4], i0[4], i1[4], i2[4];
+    std::uint32_t r0[4], r1[4], r2[4], i0[4], i1[4], i2[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float2 x = v[2 * j], y = v[2 * j + 1];
-      r0[j] = __floats2bfloat162_rn(x.x, y.x);
-      i0[j] = __floats2bfloat162_rn(x.y, y.y);
-      const float2 r0f = __bfloat1622float2(r0[j]), i0f = __bfloat1622float2(i0[j]);
-      const float2 rr = make_float2(x.x - r0f.x, y.x - r0f.y), ir = make_float2(x.y - i0f.x, y.y - i0f.y);
-      r1[j] = __floats2bfloat162_rn(rr.x, rr.y);
-      i1[j] = __floats2bfloat162_rn(ir.x, ir.y);
-      const float2 r1f = __bfloat1622float2(r1[j]), i1f = __bfloat1622float2(i1[j]);
-      r2[j] = __floats2bfloat162_rn(rr.x - r1f.x, rr.y - r1f.y);
-      i2[j] = __floats2bfloat162_rn(ir.x - i1f.x, ir.y - i1f.y);
+      split_bf16(v[2 * j].x, v[2 * j + 1].x, r0[j], r1[j], r2[j]);
+      split_bf16(v[2 * j].y, v[2 * j + 1].y, i0[j], i1[j], i2[j]);
     }
     const std::uint64_t at = (kk / 16) * rows + row;
     uint4* o = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(main_planes) + at * 64 + kk % 16);

@@ -5,6 +5,7 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <cstddef>
@@ -17,6 +18,8 @@ namespace qfx {
 // Host helpers, defined in tc_gemm.cu next to the plane layouts.
 CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad, int batch, int box_rows,
                       int row_floats = 32, int box_inner = 32);
+CUtensorMap plane_map_bf16(const __nv_bfloat16* base, std::uint64_t rows, std::uint64_t kpad, int batch,
+                           int box_rows, int inner, int box_inner);
 // Map over complex64 elements (`dims`, byte `strides` of the dimensions from
 // the second on) for boxes with rows of 16 elements, 128-byte swizzle.
 CUtensorMap element_map(const float2* base, int rank, const std::uint64_t* dims, const std::uint64_t* strides,
@@ -199,6 +202,15 @@ __device__ __forceinline__ void umma_f16(std::uint32_t d_tmem, std::uint64_t a, 
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+// kind::f16 with BF16 A and B (format 1), F32 D.
+__host__ __device__ constexpr std::uint32_t idesc_bf16(int m, int n, bool negate_a) {
+  return idesc_f16(m, n, negate_a) | (1u << 7) | (1u << 10);
+}
+template <int KIND>
+__host__ __device__ constexpr std::uint32_t idesc_kind(int m, int n, bool negate_a) {
+  return KIND == KIND_TF32 ? idesc_tf32(m, n, negate_a)
+                           : (KIND == KIND_FP16 ? idesc_f16(m, n, negate_a) : idesc_bf16(m, n, negate_a));
 }
 // True in one lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {

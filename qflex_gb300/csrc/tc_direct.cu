@@ -1,10 +1,10 @@
-// The 3xFP16 and 3xTF32 products that split A themselves (sm_103a, tcgen05 +
+// The split-precision products that split A themselves (sm_103a, tcgen05 +
 // TMEM + TMA).
 //
 // C = A * B, A complex64 in global memory, B as planes of Bt (n x k, K-major,
 // see split.cu). A is brought in as it lies -- row-major,
 // or through the index permutation that would have laid it out so (AGather)
-// -- and split into its four planes inside the kernel. Against a split
+// -- and split into its planes inside the kernel. Against a split
 // kernel (or a plane-writing permutation) before the product that saves one
 // pass over A: 8 B read and 8 B written per element.
 //
@@ -12,7 +12,7 @@
 // or 32) columns, 512 threads in four warpgroups whose registers setmaxnreg divides (56, 176,
 // 176, 104 per thread: 128 on average, the launch's own share). Work goes by
 // blocks of A, 128 rows x two k-steps (32 values; 3xTF32, whose k-steps are
-// of 8 and which scales nothing, 16: half a place in A's ring):
+// of 8 16: half a place in A's ring):
 //   warp 0       B producer: four 8 KB TMA boxes a block (re and im rows of
 //                64 bytes, hi and lo, of each k-step)
 //   warp 1       TMEM allocation; issues every MMA
@@ -46,13 +46,17 @@
 // pipe idle for 3300; (4096, 1024, 4096) from 319 to 240; (65536, 256, 16) x
 // 4 takes 96, of which writing C alone is 80.
 //
-// 3xTF32: (2048, 2048, 2048) 18 + 256 + 22 us with both operands split before
-// the product, 218 + 17; (65536, 256, 256) x 4 228 + 495 and 436.
+// The other kinds scale nothing. 3xTF32: (2048, 2048, 2048) 18 + 256 + 22 us
+// with both operands split before the product, 216 + 17; (65536, 256, 256) x 4
+// 228 + 495 and 436. BF16x3, six planes of A (192 TMEM columns and two sums),
+// 48 MMAs a block: (4096, 1024, 2048) 28 + 279 and 217 us, (65536, 256, 256) x
+// 4 193 + 485 and 427.
 //
 // B holds no negated copy: the real part takes -Ai Bi by the descriptor's
 // negate-A bit, and a k-step loads 16 KB of B, not 24. MMAs of N = 128 run at
 // the rate of N = 256 when A lies in TMEM.
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -73,10 +77,8 @@ namespace {
 constexpr int BM = 128;
 constexpr int A_BLOCK = 128 * 32 * 8;  // bytes of A as it lies, 32 values of a row
 constexpr int A_BUFS = 2;              // blocks of planes in TMEM
-constexpr int HALVES = 3;              // sums, the real or imaginary part of a block
 constexpr int EXP_RING = 4;            // block exponents, see the converter
 constexpr int SLOT = 4096;             // output box: 32 rows x 16 complex
-constexpr int TMEM_A_BLOCK = 64;       // 2 k-steps x 4 planes x 8 words
 template <int KIND>
 __host__ __device__ constexpr int block_values() {  // values of a row in two k-steps
   return KIND == KIND_TF32 ? 16 : 32;
@@ -86,15 +88,19 @@ constexpr int LOADERS = 64, CONVERTERS = 128;
 
 // Shared memory and TMEM for tiles of 128 rows and BN columns; of a PAIR, with
 // half of B's columns.
-template <int BN, bool PAIR>
+template <int KIND, int BN, bool PAIR>
 struct Layout {
+  static constexpr int PLANES = KIND == KIND_BF16 ? 6 : 4;   // of A
+  static constexpr int HALVES = KIND == KIND_BF16 ? 2 : 3;  // sums, the real or imaginary part of a block
+  static constexpr int TMEM_A_BLOCK = 2 * PLANES * 8;       // 2 k-steps x planes x 8 words
   static constexpr int A_RING = BN == 128 ? 3 : BN == 64 ? 4 : 5;  // blocks of 128 rows x 32 values
   static constexpr int B_COLS = PAIR ? BN / 2 : BN;
-  static constexpr int B_PART = B_COLS * 64;      // re or im rows of a k-step (hi, lo)
-  static constexpr int B_STAGES = PAIR ? 4 : 2;  // two k-steps each
+  static constexpr int B_PART = B_COLS * 64;               // re or im rows of a k-step (hi, lo)
+  static constexpr int B_STEP = B_COLS * PLANES * 32;      // re, im rows, BF16x3: re, im rows of the third pieces
+  static constexpr int B_STAGES = PAIR && KIND != KIND_BF16 ? 4 : 2;  // two k-steps each
   static constexpr int DONE = PAIR ? 4 : 3;      // barriers of finished blocks in turn
   static_assert(DONE >= B_STAGES && DONE > A_BUFS, "a barrier's phase is read before the next but one");
-  static constexpr int B_STAGE = 4 * B_PART;
+  static constexpr int B_STAGE = 2 * B_STEP;
   static constexpr int SLOTS = BN == 32 ? 1 : 2;  // of each epilogue warp
   static constexpr int COLS = BN / 2;             // columns of an epilogue warp
   static constexpr int OFF_B = A_RING * A_BLOCK;
@@ -119,7 +125,7 @@ __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std:
   constexpr int rows = PAIR ? 2 * BM : BM;
   constexpr std::uint32_t pos = KIND == KIND_TF32 ? idesc_tf32(rows, BN, false) : idesc_f16(rows, BN, false);
   constexpr std::uint32_t neg = KIND == KIND_TF32 ? idesc_tf32(rows, BN, true) : idesc_f16(rows, BN, true);
-  constexpr std::uint32_t part = Layout<BN, PAIR>::B_PART / 16;
+  constexpr std::uint32_t part = Layout<KIND, BN, PAIR>::B_PART / 16;
   // Ar multiplies B's part of the same name, Ai the other one (negated for
   // the real part).
   const std::uint32_t x = IM ? blo + part : blo, y = IM ? blo : blo + part;
@@ -156,6 +162,32 @@ __device__ __forceinline__ void mma_block(std::uint32_t d, std::uint32_t a, std:
 #undef QFX_MMA
 }
 
+// The same of BF16x3, one k-step: planes re 0, 1, 2, im 0, 1, 2 in TMEM; B's re
+// rows (`blo`) and im rows with pieces 0 and 1 32 bytes apart, then those of
+// piece 2, 32 bytes each. Per real product x y the terms x2 y0, x1 y1, x0 y2
+// (~2^-16), x1 y0, x0 y1 (~2^-8) and x0 y0, smallest first. Pairs only.
+template <int B_COLS, int BN, int IM>
+__device__ __forceinline__ void mma_bf16_step(std::uint32_t d, std::uint32_t a, std::uint32_t blo, std::uint32_t bhi,
+                                              std::uint32_t bhi2, std::uint32_t acc) {
+  constexpr std::uint32_t pos = idesc_bf16(2 * BM, BN, false), neg = idesc_bf16(2 * BM, BN, true);
+  constexpr std::uint32_t part = B_COLS * 64 / 16, part2 = B_COLS * 32 / 16;
+  const std::uint32_t x = IM ? blo + part : blo, y = IM ? blo : blo + part;
+  const std::uint32_t t = blo + 2 * part, x2 = IM ? t + part2 : t, y2 = IM ? t : t + part2;
+#define QFX_MMA(a_, b_, id, p) " tcgen05.mma.cta_group::2.kind::f16 [%0], [" a_ "], " b_ ", " id ", " p ";\n"
+  asm volatile(
+      "{\n .reg .pred p0, p1;\n .reg .b32 r1, r2, i0, i1, i2, x1, y1;\n .reg .b64 x0d, x1d, x2d, y0d, y1d, y2d;\n"
+      " setp.ne.b32 p0, %8, 0;\n setp.eq.b32 p1, %8, %8;\n"
+      " add.u32 r1, %1, 8;\n add.u32 r2, %1, 16;\n add.u32 i0, %1, 24;\n add.u32 i1, %1, 32;\n add.u32 i2, %1, 40;\n"
+      " add.u32 x1, %2, 2;\n add.u32 y1, %3, 2;\n mov.b64 x0d, {%2, %6};\n mov.b64 x1d, {x1, %6};\n"
+      " mov.b64 y0d, {%3, %6};\n mov.b64 y1d, {y1, %6};\n mov.b64 x2d, {%4, %7};\n mov.b64 y2d, {%5, %7};\n"  //
+      QFX_MMA("r2", "x0d", "%9", "p0") QFX_MMA("r1", "x1d", "%9", "p1") QFX_MMA("%1", "x2d", "%9", "p1")
+      QFX_MMA("i2", "y0d", "%10", "p1") QFX_MMA("i1", "y1d", "%10", "p1") QFX_MMA("i0", "y2d", "%10", "p1")
+      QFX_MMA("r1", "x0d", "%9", "p1") QFX_MMA("%1", "x1d", "%9", "p1") QFX_MMA("i1", "y0d", "%10", "p1")
+      QFX_MMA("i0", "y1d", "%10", "p1") QFX_MMA("%1", "x0d", "%9", "p1") QFX_MMA("i0", "y0d", "%10", "p1") "}\n" ::"r"(d),
+      "r"(a), "r"(x), "r"(y), "r"(x2), "r"(y2), "r"(bhi), "r"(bhi2), "r"(acc), "r"(pos), "r"(IM ? pos : neg));
+#undef QFX_MMA
+}
+
 // 32 words of the thread's TMEM lane.
 __device__ __forceinline__ void tmem_st32(std::uint32_t at, const std::uint32_t* w) {
   asm volatile(
@@ -165,6 +197,16 @@ __device__ __forceinline__ void tmem_st32(std::uint32_t at, const std::uint32_t*
       "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15]), "r"(w[16]), "r"(w[17]), "r"(w[18]),
       "r"(w[19]), "r"(w[20]), "r"(w[21]), "r"(w[22]), "r"(w[23]), "r"(w[24]), "r"(w[25]), "r"(w[26]), "r"(w[27]),
       "r"(w[28]), "r"(w[29]), "r"(w[30]), "r"(w[31])
+      : "memory");
+}
+
+// 16 words.
+__device__ __forceinline__ void tmem_st16(std::uint32_t at, const std::uint32_t* w) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15, %16};" ::"r"(at),
+      "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+      "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
       : "memory");
 }
 
@@ -206,12 +248,13 @@ __device__ __forceinline__ void cp_async_arrive(std::uint64_t* bar) {
 template <int KIND, int BN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
     cgemm_direct_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                               const __grid_constant__ CUtensorMap map_b2,
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ AGather g,
                                const float2* __restrict__ A, float2* __restrict__ C, int tma_c, int m, int n, int k,
                                int batches, std::uint64_t ac_stride, int* __restrict__ err,
                                const int* __restrict__ exp_b) {
-  using L = Layout<BN, PAIR>;
-  constexpr int B_STAGES = L::B_STAGES, DONE = L::DONE;
+  using L = Layout<KIND, BN, PAIR>;
+  constexpr int B_STAGES = L::B_STAGES, DONE = L::DONE, HALVES = L::HALVES, TMEM_A_BLOCK = L::TMEM_A_BLOCK;
   constexpr int A_RING = L::A_RING, B_PART = L::B_PART, B_STAGE = L::B_STAGE, TMEM_A = L::TMEM_A, COLS = L::COLS;
   extern __shared__ __align__(1024) std::uint8_t smem[];
   std::uint64_t* raw_full = reinterpret_cast<std::uint64_t*>(smem + L::OFF_BAR);  // a block of A has landed
@@ -331,20 +374,20 @@ __global__ void __launch_bounds__(THREADS, 1)
           // the map and arrive as zeros.
           std::uint8_t* st = smem + L::OFF_B + s * B_STAGE;
           const int col = nt * BN + int(rank) * L::B_COLS;
-          if constexpr (PAIR) {
-            // Both CTAs' halves complete on CTA 0's barrier.
-            if (rank == 0) mbar_expect_tx(&b_full[s], 2 * B_STAGE);
-            const std::uint32_t bar = peer_addr(&b_full[s], 0);
-            tma_load_4d_pair(&map_b, bar, st, 0, col, 2 * b, batch);
-            tma_load_4d_pair(&map_b, bar, st + B_PART, X_IM, col, 2 * b, batch);
-            tma_load_4d_pair(&map_b, bar, st + 2 * B_PART, 0, col, 2 * b + 1, batch);
-            tma_load_4d_pair(&map_b, bar, st + 3 * B_PART, X_IM, col, 2 * b + 1, batch);
-          } else {
-            mbar_expect_tx(&b_full[s], B_STAGE);
-            tma_load_4d(&map_b, &b_full[s], st, 0, col, 2 * b, batch);
-            tma_load_4d(&map_b, &b_full[s], st + B_PART, X_IM, col, 2 * b, batch);
-            tma_load_4d(&map_b, &b_full[s], st + 2 * B_PART, 0, col, 2 * b + 1, batch);
-            tma_load_4d(&map_b, &b_full[s], st + 3 * B_PART, X_IM, col, 2 * b + 1, batch);
+          if (rank == 0) mbar_expect_tx(&b_full[s], (PAIR ? 2 : 1) * B_STAGE);  // both CTAs' halves
+          for (int h = 0; h < 2; ++h, st += L::B_STEP) {
+            if constexpr (PAIR) {
+              const std::uint32_t bar = peer_addr(&b_full[s], 0);
+              tma_load_4d_pair(&map_b, bar, st, 0, col, 2 * b + h, batch);
+              tma_load_4d_pair(&map_b, bar, st + B_PART, X_IM, col, 2 * b + h, batch);
+              if constexpr (KIND == KIND_BF16) {
+                tma_load_4d_pair(&map_b2, bar, st + 2 * B_PART, 0, col, 2 * b + h, batch);
+                tma_load_4d_pair(&map_b2, bar, st + 2 * B_PART + B_PART / 2, 16, col, 2 * b + h, batch);
+              }
+            } else {
+              tma_load_4d(&map_b, &b_full[s], st, 0, col, 2 * b + h, batch);
+              tma_load_4d(&map_b, &b_full[s], st + B_PART, X_IM, col, 2 * b + h, batch);
+            }
           }
           ++q;
           if (++s == B_STAGES) s = 0;
@@ -382,6 +425,16 @@ __global__ void __launch_bounds__(THREADS, 1)
       const bool leader = elect_one();
       const std::uint64_t db = smem_desc_sw64(smem_u32(smem + L::OFF_B));
       const std::uint32_t b_hi = std::uint32_t(db >> 32), b_lo0 = std::uint32_t(db);
+      const std::uint32_t b_hi2 = std::uint32_t(smem_desc_sw32(0) >> 32);
+      auto issue = [&](auto im, std::uint32_t d, std::uint32_t a, std::uint32_t b) {
+        constexpr int IM = decltype(im)::value;
+        if constexpr (KIND == KIND_BF16) {
+          mma_bf16_step<L::B_COLS, BN, IM>(d, a, b, b_hi, b_hi2, 0);
+          mma_bf16_step<L::B_COLS, BN, IM>(d, a + 48, b + (L::B_STEP >> 4), b_hi, b_hi2, 1);
+        } else {
+          mma_block<KIND, BN, PAIR, IM>(d, a, b, b_hi);
+        }
+      };
       const int kind = lane & 3;
       std::uint64_t* const bars = kind == 1 ? a_full : kind == 2 ? b_full : acc_empty;
       const int ring = kind == 1 ? A_BUFS : kind == 2 ? B_STAGES : HALVES;
@@ -394,7 +447,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;");
         const std::uint32_t a = tmem + TMEM_A + xa * TMEM_A_BLOCK, b = b_lo0 + sb * (B_STAGE >> 4);
         if (leader) {
-          mma_block<KIND, BN, PAIR, 0>(tmem + h * BN, a, b, b_hi);
+          issue(std::integral_constant<int, 0>{}, tmem + h * BN, a, b);
           commit(&re_full[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
@@ -403,7 +456,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!__all_sync(0xffffffffu, kind != 3 || wait(bars + at, parity, 4))) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (leader) {
-          mma_block<KIND, BN, PAIR, 1>(tmem + h * BN, a, b, b_hi);
+          issue(std::integral_constant<int, 1>{}, tmem + h * BN, a, b);
           commit(&done[r]);
         }
         h = h == HALVES - 1 ? 0 : h + 1;
@@ -541,83 +594,119 @@ __global__ void __launch_bounds__(THREADS, 1)
     const std::uint32_t lanes = tmem + TMEM_A + (std::uint32_t((warp - 12) * 32) << 16);
     int s = 0, x = 0, xa = 0, r = DONE - A_BUFS;
     std::uint32_t ph = 0, pd = 1;  // block w - A_BUFS: barrier r
-    // Block w: its values lie in one place of the ring, or (3xTF32) in half of
-    // one, b counting the tile's blocks.
-    for (int w = 0, b = 0; w < work; ++w) {
-      const int half = VALUES == 16 ? b & 1 : 0;
-      b = b == blocks - 1 ? 0 : b + 1;
-      const bool first_half = half == 0, last = VALUES == 32 || half || b == 0;
-      if (first_half && !__all_sync(0xffffffffu, wait(&raw_full[s], ph, 6))) break;
-      const std::uint32_t block = ring + s * A_BLOCK;
-      const std::uint32_t at0 = half ? row_at ^ g.value_at[16] : row_at;
-      float2 v[VALUES];
+    // Values of the thread's row from the first (h = 0) or second 16 of place s
+    // of the ring on.
+    auto read = [&](auto& v, int s, int h) {
+      const std::uint32_t block = ring + s * A_BLOCK, at = h ? row_at ^ g.value_at[16] : row_at;
+      constexpr int N = sizeof(v) / sizeof(v[0]);
       if (g.pairs) {
 #pragma unroll
-        for (int i = 0; i < VALUES; i += 2)
+        for (int i = 0; i < N; i += 2)
           asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                        : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i + 1].x), "=f"(v[i + 1].y)
-                       : "r"(block + (at0 ^ g.value_at[i]))
+                       : "r"(block + (at ^ g.value_at[i]))
                        : "memory");
       } else {
 #pragma unroll
-        for (int i = 0; i < VALUES; ++i)
+        for (int i = 0; i < N; ++i)
           asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
                        : "=f"(v[i].x), "=f"(v[i].y)
-                       : "r"(block + (at0 ^ g.value_at[i]))
+                       : "r"(block + (at ^ g.value_at[i]))
                        : "memory");
       }
-      std::uint32_t p[2][32];  // of each k-step: 8 words of every plane
-      int e = 0;
-      if constexpr (KIND == KIND_FP16) {
-        // Bit patterns of non-negative floats order like their values.
-        std::uint32_t mx[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-        for (int i = 0; i < VALUES; ++i)
-          mx[i & 3] = max(mx[i & 3], max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
-        // e with max * 2^e in [2^14, 2^15), at most 126 (2^e and 2^-e stay
-        // normal floats; smaller blocks keep all their bits: below 2^-112 the
-        // lo planes reach further down than FP32 itself). A block of zeros
-        // takes 126 so that it never sets the scale of the sum; infinities
-        // and NaN keep 0.
-        const int be = int(max(max(mx[0], mx[1]), max(mx[2], mx[3])) >> 23);
-        e = be == 255 ? 0 : min(141 - be, 126);
-        const float sc = __uint_as_float(std::uint32_t(e + 127) << 23);
-        const float2 sc2 = make_float2(sc, sc);
-#pragma unroll
-        for (int i = 0; i < VALUES; i += 16)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
-            const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
-            split_pair(re.x, re.y, p[i / 16][j], p[i / 16][8 + j]);
-            split_pair(im.x, im.y, p[i / 16][16 + j], p[i / 16][24 + j]);
-          }
-      } else {
-#pragma unroll
-        for (int i = 0; i < VALUES; ++i) {
-          std::uint32_t* o = p[i / 8] + i % 8;
-          const float rh = tf32_rn(v[i].x), ih = tf32_rn(v[i].y);
-          o[0] = __float_as_uint(rh);
-          o[8] = __float_as_uint(tf32_rn(v[i].x - rh));
-          o[16] = __float_as_uint(ih);
-          o[24] = __float_as_uint(tf32_rn(v[i].y - ih));
-        }
-      }
-      // The values are in registers: their place in the ring is free.
+    };
+    // The values read are in registers: their place in the ring is free.
+    auto release = [&] {
       __syncwarp();
-      if (last && lane == 0) mbar_arrive(&raw_empty[s]);
-      if (!__all_sync(0xffffffffu, wait(&done[r], pd, 10))) break;
+      if (lane == 0) mbar_arrive(&raw_empty[s]);
+    };
+    // Waits for the MMAs of the block two back, whose place in TMEM comes next.
+    auto place = [&] {
+      if (!__all_sync(0xffffffffu, wait(&done[r], pd, 10))) return false;
       if (++r == DONE) {
         r = 0;
         pd ^= 1u;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-      tmem_st32(lanes + xa * TMEM_A_BLOCK, p[0]);
-      tmem_st32(lanes + xa * TMEM_A_BLOCK + 32, p[1]);
-      // Exponents live in a ring of their own: the MMAs of the block two
-      // back are done, so every epilogue warp has read the exponents of the
-      // block three back.
-      if constexpr (KIND == KIND_FP16) exps[x * BM + row] = std::int8_t(e);
+      return true;
+    };
+    // Block w: its values lie in one place of the ring, or (3xTF32) in half of
+    // one, b counting the tile's blocks.
+    for (int w = 0, b = 0; w < work; ++w) {
+      const int half = VALUES == 16 ? b & 1 : 0;
+      b = b == blocks - 1 ? 0 : b + 1;
+      const bool last = VALUES == 32 || half || b == 0;
+      if (!half && !__all_sync(0xffffffffu, wait(&raw_full[s], ph, 6))) break;
+      const std::uint32_t to = lanes + xa * TMEM_A_BLOCK;
+      if constexpr (KIND == KIND_BF16) {
+        bool ok = true;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float2 v[16];
+          read(v, s, h);
+          if (h == 1) release();
+          std::uint32_t p[48];  // 8 words of every plane
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            split_bf16(v[2 * j].x, v[2 * j + 1].x, p[j], p[8 + j], p[16 + j]);
+            split_bf16(v[2 * j].y, v[2 * j + 1].y, p[24 + j], p[32 + j], p[40 + j]);
+          }
+          if (h == 0) ok = place();
+          if (!ok) break;
+          tmem_st32(to + 48 * h, p);
+          tmem_st16(to + 48 * h + 32, p + 32);
+        }
+        if (!ok) break;
+      } else {
+        float2 v[VALUES];
+        read(v, s, half);
+        std::uint32_t p[2][32];  // of each k-step: 8 words of every plane
+        int e = 0;
+        if constexpr (KIND == KIND_FP16) {
+          // Bit patterns of non-negative floats order like their values.
+          std::uint32_t mx[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int i = 0; i < VALUES; ++i)
+            mx[i & 3] =
+                max(mx[i & 3], max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu));
+          // e with max * 2^e in [2^14, 2^15), at most 126 (2^e and 2^-e stay
+          // normal floats; smaller blocks keep all their bits: below 2^-112 the
+          // lo planes reach further down than FP32 itself). A block of zeros
+          // takes 126 so that it never sets the scale of the sum; infinities
+          // and NaN keep 0.
+          const int be = int(max(max(mx[0], mx[1]), max(mx[2], mx[3])) >> 23);
+          e = be == 255 ? 0 : min(141 - be, 126);
+          const float sc = __uint_as_float(std::uint32_t(e + 127) << 23);
+          const float2 sc2 = make_float2(sc, sc);
+#pragma unroll
+          for (int i = 0; i < VALUES; i += 16)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float2 a = v[i + 2 * j], b2 = v[i + 2 * j + 1];
+              const float2 re = mul2(make_float2(a.x, b2.x), sc2), im = mul2(make_float2(a.y, b2.y), sc2);
+              split_pair(re.x, re.y, p[i / 16][j], p[i / 16][8 + j]);
+              split_pair(im.x, im.y, p[i / 16][16 + j], p[i / 16][24 + j]);
+            }
+        } else {
+#pragma unroll
+          for (int i = 0; i < VALUES; ++i) {
+            std::uint32_t* o = p[i / 8] + i % 8;
+            const float rh = tf32_rn(v[i].x), ih = tf32_rn(v[i].y);
+            o[0] = __float_as_uint(rh);
+            o[8] = __float_as_uint(tf32_rn(v[i].x - rh));
+            o[16] = __float_as_uint(ih);
+            o[24] = __float_as_uint(tf32_rn(v[i].y - ih));
+          }
+        }
+        if (last) release();
+        if (!place()) break;
+        tmem_st32(to, p[0]);
+        tmem_st32(to + 32, p[1]);
+        // Exponents live in a ring of their own: the MMAs of the block two
+        // back are done, so every epilogue warp has read the exponents of the
+        // block three back.
+        if constexpr (KIND == KIND_FP16) exps[x * BM + row] = std::int8_t(e);
+      }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
@@ -1047,15 +1136,19 @@ void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const floa
 // (1048576, 16, 256) 498 and, in tiles of 32, 353 us (342).
 static int direct_columns(std::size_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : 128; }
 // Pairs where a second row tile exists and the MMAs of a tile take longer than
-// its store, which starts later in a pair. Single CTAs against pairs: (65536,
-// 256, k) x 4 with k = 32 104 and 106 us, 64 143 and 149, 256 301 and 286;
-// (8192, 128, 128) x 16 59 and 60.5; (4096, 1024, 4096) 272 and 240.
-static bool direct_pair(SplitKind kind, std::size_t m, std::size_t k) {
-  return m > (std::size_t)BM && k > (kind == KIND_TF32 ? 64u : 128u);
+// its store, which starts later in a pair. 3xFP16, single CTAs against pairs:
+// (65536, 256, k) x 4 with k = 32 104 and 106 us, 64 143 and 149, 256 301 and
+// 286; (8192, 128, 128) x 16 59 and 60.5; (4096, 1024, 4096) 272 and 240.
+// 3xTF32 takes twice the MMAs. BF16x3 runs in pairs alone: split and product,
+// and this, (65536, 256, k) x 4 with k = 16 122 and 98 us, 64 200 and 154;
+// (32768, 64, 64) x 16 220 and 133; (256, 256, 64) 12 and 12.
+bool tc_direct_pair(SplitKind kind, std::size_t m, std::size_t k) {
+  return m > (std::size_t)BM && k > (kind == KIND_FP16 ? 128u : kind == KIND_TF32 ? 64u : 0u);
 }
 
 std::size_t tc_direct_workspace_elems(SplitKind kind, std::size_t n, std::size_t k) {
   if (kind == KIND_TF32) return 4 * n * ((k + 7) / 8 * 8);
+  if (kind == KIND_BF16) return 3 * n * ((k + 15) / 16 * 16);
   return 2 * n * ((k + 15) / 16 * 16) + 2 * n;  // B's planes, exponents and largest components
 }
 
@@ -1079,10 +1172,13 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     }
   }
   const int bn = kind == KIND_FP16 ? direct_columns(n) : 128;
-  const bool pair = bn == 128 && direct_pair(kind, m, k);
+  const bool pair = bn == 128 && tc_direct_pair(kind, m, k);
+  if (kind == KIND_BF16 && !pair)
+    throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct BF16x3 product runs in pairs");
   const int b_cols = pair ? bn / 2 : bn;
   int* eb = nullptr;
-  CUtensorMap mb;
+  CUtensorMap mb, mb2;
+  std::memset(&mb2, 0, sizeof(mb2));
   if (kind == KIND_FP16) {
     const std::size_t kpad = (k + 15) / 16 * 16;
     __half* pb = reinterpret_cast<__half*>(workspace);
@@ -1090,6 +1186,13 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     std::uint32_t* top = reinterpret_cast<std::uint32_t*>(eb + n * (std::size_t)batch);
     launch_split(KIND_FP16, 4, {pb, nullptr, eb, top}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
     mb = plane_map_f16(pb, n, kpad, batch, b_cols, 64);
+  } else if (kind == KIND_BF16) {
+    const std::size_t kpad = (k + 15) / 16 * 16;
+    __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(workspace);
+    __nv_bfloat16* pt = pb + 4 * n * kpad * (std::size_t)batch;
+    launch_split(KIND_BF16, 4, {pb, pt}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
+    mb = plane_map_bf16(pb, n, kpad, batch, b_cols, 64, 32);
+    mb2 = plane_map_bf16(pt, n, kpad, batch, b_cols, 32, 16);
   } else {
     launch_split(KIND_TF32, 4, {workspace}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
     mb = plane_map(workspace, n, (k + 7) / 8 * 8, batch, b_cols, 32, 16);
@@ -1117,11 +1220,12 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
   const std::size_t tiles = ((m + rows - 1) / rows) * ((n + bn - 1) / bn) * (std::size_t)batch;
   auto run = [&](auto of_kind, auto columns, auto paired) {
     constexpr int BN = decltype(columns)::value;
+    constexpr int KIND = decltype(of_kind)::value;
     constexpr bool PAIR = decltype(paired)::value;
-    auto* kernel = cgemm_direct_kernel<decltype(of_kind)::value, BN, PAIR>;
+    auto* kernel = cgemm_direct_kernel<KIND, BN, PAIR>;
     cudaLaunchConfig_t lc = {};
     lc.blockDim = dim3(THREADS, 1, 1);
-    lc.dynamicSmemBytes = Layout<BN, PAIR>::SMEM;
+    lc.dynamicSmemBytes = Layout<KIND, BN, PAIR>::SMEM;
     lc.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1133,7 +1237,7 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     static std::once_flag attr;
     static int resident = 0;  // pairs (SMs pair up within a GPC)
     std::call_once(attr, [&] {
-      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BN, PAIR>::SMEM),
+      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<KIND, BN, PAIR>::SMEM),
             "cudaFuncSetAttribute");
       lc.gridDim = dim3(2, 1, 1);
       if (PAIR && (cudaOccupancyMaxActiveClusters(&resident, kernel, &lc) != cudaSuccess || resident < 1)) {
@@ -1143,7 +1247,7 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     });
     lc.gridDim = dim3(PAIR ? 2 * (unsigned)std::min<std::size_t>(tiles, (std::size_t)resident) : persistent_grid(tiles),
                       1, 1);
-    check(cudaLaunchKernelEx(&lc, kernel, ma, mb, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err,
+    check(cudaLaunchKernelEx(&lc, kernel, ma, mb, mb2, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err,
                              (const int*)eb),
           "cgemm_direct");
   };
@@ -1151,7 +1255,9 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
   const integral_constant<int, KIND_FP16> fp16;
   const integral_constant<int, KIND_TF32> tf32;
   const integral_constant<int, 128> c128;
-  if (kind == KIND_TF32)
+  if (kind == KIND_BF16)
+    run(integral_constant<int, KIND_BF16>{}, c128, std::true_type{});
+  else if (kind == KIND_TF32)
     pair ? run(tf32, c128, std::true_type{}) : run(tf32, c128, std::false_type{});
   else if (bn == 128)
     pair ? run(fp16, c128, std::true_type{}) : run(fp16, c128, std::false_type{});

@@ -129,15 +129,6 @@ __device__ __forceinline__ void umma(std::uint32_t d, std::uint64_t a, std::uint
   else
     umma_f16(d, a, b, id, acc);
 }
-// kind::f16 with BF16 A and B (format 1), F32 D.
-__host__ __device__ constexpr std::uint32_t idesc_bf16(int m, int n, bool negate_a) {
-  return idesc_f16(m, n, negate_a) | (1u << 7) | (1u << 10);
-}
-template <int KIND>
-__host__ __device__ constexpr std::uint32_t idesc_kind(int m, int n, bool negate_a) {
-  return KIND == KIND_TF32 ? idesc_tf32(m, n, negate_a)
-                           : (KIND == KIND_FP16 ? idesc_f16(m, n, negate_a) : idesc_bf16(m, n, negate_a));
-}
 
 #define TMEM_LD32(taddr, r)                                                                            \
   asm volatile(                                                                                        \
@@ -996,30 +987,6 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// 4-D map over BF16 planes laid out [batch][kpad / 16][rows][inner]; box
-// {box_inner, box_rows, 1, 1}: rows of 128, 64 or 32 bytes in the swizzle of
-// that width.
-CUtensorMap plane_map_bf16(const __nv_bfloat16* base, std::uint64_t rows, std::uint64_t kpad, int batch,
-                           int box_rows, int inner, int box_inner) {
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  const std::uint64_t kb = kpad / 16, rb = std::uint64_t(inner) * 2;
-  const cuuint64_t dims[4] = {(cuuint64_t)inner, rows, kb, (cuuint64_t)batch};
-  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
-  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(base), dims,
-                           strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           box_inner == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
-                           : box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                             : CU_TENSOR_MAP_SWIZZLE_32B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
-        std::to_string((int)r);
-  return map;
-}
-
 void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: CUDA ") + what + ") --> " + cudaGetErrorString(e);
 }
@@ -1042,6 +1009,30 @@ CUtensorMap plane_map(const float* base, std::uint64_t rows, std::uint64_t kpad,
   CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides,
                            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +
+        std::to_string((int)r);
+  return map;
+}
+
+// 4-D map over BF16 planes laid out [batch][kpad / 16][rows][inner]; box
+// {box_inner, box_rows, 1, 1}: rows of 128, 64 or 32 bytes in the swizzle of
+// that width.
+CUtensorMap plane_map_bf16(const __nv_bfloat16* base, std::uint64_t rows, std::uint64_t kpad, int batch,
+                           int box_rows, int inner, int box_inner) {
+  CUtensorMap map;
+  std::memset(&map, 0, sizeof(map));
+  const std::uint64_t kb = kpad / 16, rb = std::uint64_t(inner) * 2;
+  const cuuint64_t dims[4] = {(cuuint64_t)inner, rows, kb, (cuuint64_t)batch};
+  const cuuint64_t strides[3] = {rb, rows * rb, kb * rows * rb};
+  const cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(base), dims,
+                           strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           box_inner == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                           : box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                             : CU_TENSOR_MAP_SWIZZLE_32B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> cuTensorMapEncodeTiled failed: ") +

@@ -115,9 +115,12 @@ bool make_a_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size
 // checks: dst is the m x k operand the product sees. Tests use it.
 void a_gather_on_host(const AGather& g, std::size_t m, std::size_t k, const float2* src, float2* dst);
 
+// Whether the direct product of m rows and k terms runs on pairs of CTAs
+// (BF16x3: whether it runs).
+bool tc_direct_pair(SplitKind kind, std::size_t m, std::size_t k);
 // fp32 elements that launch_cgemm_direct's workspace takes per batch entry.
 std::size_t tc_direct_workspace_elems(SplitKind kind, std::size_t n, std::size_t k);
-// The 3xFP16 or 3xTF32 product with A split inside the kernel: A is read as
+// The split product with A split inside the kernel: A is read as
 // complex64 through `gather` (3xFP16: every 32 values of a row scaled by their
 // own power of two), and no A planes exist in memory. cfg.chunk 2 (a TMEM chunk
 // is one of A's blocks); cfg.variant is ignored.

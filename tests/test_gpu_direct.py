@@ -4,7 +4,7 @@ and on rows whose magnitude changes from one block of 32 values to the next."""
 import numpy as np
 import pytest
 
-from qflex_gb300 import FP16X3, TF32X3, Context
+from qflex_gb300 import BF16X3, FP16X3, TF32X3, Context
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +77,11 @@ def test_pairs(built_lib, kind, m, n, k, batch, extra):
     (640, 1100, 160, 2, 0), (383, 1500, 400, 1, 0), (20000, 256, 64, 1, 0), (128, 1100, 192, 1, 0)])
 def test_tf32(built_lib, m, n, k, batch, extra):
     test_direct_product(built_lib, "gauss", m, n, k, batch, extra, TF32X3, 6e-6)
+
+
+# BF16x3: 24 truncating additions per chunk of two k-steps of 16.
+@pytest.mark.parametrize("m,n,k,batch,extra", [
+    (129, 64, 65, 1, 0), (256, 128, 128, 1, 0), (300, 130, 97, 1, 1), (257, 640, 111, 1, 1), (640, 1100, 160, 2, 0),
+    (383, 1500, 400, 1, 0), (20000, 256, 80, 1, 0)])
+def test_bf16(built_lib, m, n, k, batch, extra):
+    test_direct_product(built_lib, "gauss", m, n, k, batch, extra, BF16X3, 6e-6)
