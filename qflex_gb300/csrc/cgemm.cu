@@ -31,6 +31,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.h"
@@ -63,11 +64,24 @@ __device__ __forceinline__ void copy16(float2* dst, const float2* src) {
 // so that the rows a quarter-warp reads start in different banks.
 constexpr int a_row(int BK) { return BK + 2; }
 
-template <int BM, int BN, int BK, int TM, int TN, int STAGES, bool GATHER>
+// What one variant of the kernel takes besides the matrices: a gather, or the
+// split of k (`splits` runs of `terms`, whose sums go to `partial` as
+// [entry][split][m][n]); nothing for the others, whose launches it would slow.
+struct SplitK {
+  float2* partial;
+  int splits, terms;
+};
+struct Nothing {};
+enum Variant { PLAIN, GATHERED, SPLIT };
+template <int VARIANT>
+using Extra = std::conditional_t<VARIANT == GATHERED, TileGather, std::conditional_t<VARIANT == SPLIT, SplitK, Nothing>>;
+
+template <int BM, int BN, int BK, int TM, int TN, int STAGES, int VARIANT>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     cgemm_kernel(const float2* __restrict__ A, const float2* __restrict__ B, float2* __restrict__ C, int m, int n,
                  int k, std::uint64_t batch_stride, int tiles_m, long long tiles, int pairs,
-                 const __grid_constant__ TileGather g) {
+                 const __grid_constant__ Extra<VARIANT> g) {
+  constexpr bool GATHER = VARIANT == GATHERED;
   constexpr int NT = (BM / TM) * (BN / TN);
   constexpr int TX = BN / TN, TY = BM / TM;
   constexpr int LA = BM * BK / NT, LB = (BK * BN + NT - 1) / NT;
@@ -77,22 +91,25 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   extern __shared__ __align__(16) float2 ring[];
   const int t = threadIdx.x;
   const int tx = t % TX, ty = t / TX;
-  const int ktiles = k > 0 ? (k + BK - 1) / BK : 1;  // no terms: one k-step of zeros
+  int ktiles = k > 0 ? (k + BK - 1) / BK : 1;  // no terms: one k-step of zeros
+  if constexpr (VARIANT == SPLIT) ktiles = g.terms / BK;
   const int tiles_n = (n + BN - 1) / BN;
   const long long mine = (long long)blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   const long long steps = mine * ktiles;
-  // Consecutive tiles share their rows of A.
+  // Consecutive tiles share their rows of A. A split product counts the runs
+  // of k like batch entries: `at` is the run's number.
+  const std::uint64_t entry_stride = VARIANT == SPLIT ? 1 : batch_stride;
   auto place = [&](long long tile, unsigned& mt, unsigned& nt, std::uint64_t& at) {
     if (tiles <= 0xffffffffll) {  // 32-bit divisions are much the shorter
       const unsigned r = unsigned(tile) / unsigned(tiles_n);
       nt = unsigned(tile) % unsigned(tiles_n);
       mt = r % unsigned(tiles_m);
-      at = std::uint64_t(r / unsigned(tiles_m)) * batch_stride;
+      at = std::uint64_t(r / unsigned(tiles_m)) * entry_stride;
     } else {
       const long long r = tile / tiles_n;
       nt = unsigned(tile % tiles_n);
       mt = unsigned(r % tiles_m);
-      at = std::uint64_t(r / tiles_m) * batch_stride;
+      at = std::uint64_t(r / tiles_m) * entry_stride;
     }
   };
 
@@ -115,7 +132,12 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     unsigned mt, nt;
     std::uint64_t at;
     place(lt, mt, nt, at);
-    const int k0 = lk * BK;
+    int k0 = lk * BK;
+    if constexpr (VARIANT == SPLIT) {
+      const unsigned run = unsigned(at);
+      k0 += int(run % unsigned(g.splits)) * g.terms;
+      at = std::uint64_t(run / unsigned(g.splits)) * batch_stride;
+    }
     if constexpr (GATHER) {
       const float2* src = lane_src + at;
       for (int b = 0; b < TileGather::kBits && (mt >> b); ++b)
@@ -231,6 +253,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
         const unsigned r = mt * BM + ty + i * TY;
         if (r >= unsigned(m)) continue;
         float2* c = C + at + std::uint64_t(r) * n;
+        if constexpr (VARIANT == SPLIT) c = g.partial + (at * std::uint64_t(m) + r) * n;
 #pragma unroll
         for (int j = 0; j < TN; j += 2) {
           const unsigned col = nt * BN + 2 * tx + j * TX;
@@ -248,6 +271,36 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// Adds the sums of a split product's runs: blocks of 32 elements of C, whose
+// eight warps take every eighth run (one thread for all runs of an element
+// took 15 us at 64).
+__global__ void __launch_bounds__(256) split_finish_kernel(const float2* __restrict__ partial, float2* __restrict__ C,
+                                                           std::uint64_t outputs, int splits,
+                                                           std::uint64_t batch_stride) {
+  __shared__ double2 part[8][32];
+  const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
+  const std::uint64_t at = std::uint64_t(blockIdx.x) * 32 + lane;
+  double2 sum = make_double2(0, 0);
+  if (at < outputs) {
+    const float2* p = partial + blockIdx.y * outputs * splits + at;
+#pragma unroll 8
+    for (int q = w; q < splits; q += 8) {
+      const float2 v = p[q * outputs];
+      sum.x += double(v.x);
+      sum.y += double(v.y);
+    }
+  }
+  part[w][lane] = sum;
+  __syncthreads();
+  if (w || at >= outputs) return;
+#pragma unroll
+  for (int q = 1; q < 8; ++q) {
+    sum.x += part[q][lane].x;
+    sum.y += part[q][lane].y;
+  }
+  C[blockIdx.y * batch_stride + at] = make_float2(float(sum.x), float(sum.y));
+}
+
 struct Tile {
   int bm, bn, bk, threads;
 };
@@ -257,10 +310,10 @@ struct Shape {
   static constexpr Tile tile{BM, BN, BK, nt};
   static constexpr int smem = STAGES * (BM * a_row(BK) + BK * BN) * (int)sizeof(float2);
 
-  template <bool GATHER>
+  template <int VARIANT>
   static void run(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
-                  std::uint64_t stride, int batch, const TileGather& g, cudaStream_t s) {
-    auto* kernel = cgemm_kernel<BM, BN, BK, TM, TN, STAGES, GATHER>;
+                  std::uint64_t stride, int batch, const Extra<VARIANT>& g, cudaStream_t s) {
+    auto* kernel = cgemm_kernel<BM, BN, BK, TM, TN, STAGES, VARIANT>;
     // Blocks that are resident at once on the current device.
     static std::once_flag once;
     static int resident = 152;
@@ -273,13 +326,15 @@ struct Shape {
       resident = sms * std::max(per, 1);
     });
     const long long tiles_m = (long long)((m + BM - 1) / BM);
-    const long long tiles = tiles_m * (long long)((n + BN - 1) / BN) * batch;
+    long long tiles = tiles_m * (long long)((n + BN - 1) / BN) * batch;
+    if constexpr (VARIANT == SPLIT) tiles *= g.splits;
     // Which of C's, A's and B's rows start on 16 bytes (bits 0, 1, 2).
     const bool even = batch == 1 || stride % 2 == 0;
     auto rows16 = [&](const float2* p, std::size_t row) {
       return even && row % 2 == 0 && (reinterpret_cast<std::uintptr_t>(p) & 15) == 0;
     };
-    const int pairs = (rows16(C, n) ? 1 : 0) | (rows16(A, k) ? 2 : 0) | (rows16(B, n) ? 4 : 0);
+    const bool c16 = VARIANT == SPLIT ? n % 2 == 0 : rows16(C, n);
+    const int pairs = (c16 ? 1 : 0) | (rows16(A, k) ? 2 : 0) | (rows16(B, n) ? 4 : 0);
     kernel<<<(unsigned)std::min<long long>(tiles, resident), nt, smem, s>>>(A, B, C, (int)m, (int)n, (int)k, stride,
                                                                             (int)tiles_m, tiles, pairs, g);
     const cudaError_t e = cudaGetLastError();
@@ -288,9 +343,9 @@ struct Shape {
   static void launch(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
                      std::uint64_t stride, int batch, const TileGather* g, cudaStream_t s) {
     if (g)
-      run<true>(A, B, C, m, n, k, stride, batch, *g, s);
+      run<GATHERED>(A, B, C, m, n, k, stride, batch, *g, s);
     else
-      run<false>(A, B, C, m, n, k, stride, batch, TileGather{}, s);
+      run<PLAIN>(A, B, C, m, n, k, stride, batch, Nothing{}, s);
   }
 };
 
@@ -384,9 +439,40 @@ void tile_gather_on_host(const TileGather& g, std::size_t m, std::size_t n, std:
 }
 
 void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
-                        std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, cudaStream_t s) {
+                        std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, float2* scratch,
+                        cudaStream_t s) {
   if (m > 0x7fffffffull || n > 0x7fffffffull || k > 0x7fffffffull)
     throw std::string("ERROR (qflex_gb300: cgemm) --> dimension exceeds 2^31");
+  // Few tiles: a product is then as long as one tile's chain of k-steps. Small
+  // tiles and six steps in flight shorten the chain, and where they are fewer
+  // than the SMs hold (two each), so does splitting k into runs of 64 or more.
+  // The shapes above against these: (16, 16, 32) 10 and 4 us, (256, 16, 64) 19
+  // and 5.5, (512, 512, 512) 104 and 42; with runs (256, 16, 512) 80 and 9,
+  // (16, 16, 4096) 500 and 12. A gather is made for the shapes above.
+  const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
+  const std::size_t tiles = ((m + tile.bm - 1) / tile.bm) * ((n + tile.bn - 1) / tile.bn) * (std::size_t)batch;
+  if (!gather && tiles && tiles <= 38) {
+    auto small = [&](auto shape) {
+      using S = decltype(shape);
+      constexpr Tile t = S::tile;
+      const std::size_t own = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn) * (std::size_t)batch;
+      std::size_t splits = scratch ? std::min<std::size_t>(304 / own, k / 64) : 1;
+      splits = std::min<std::size_t>(splits, kSkinnyScratchElems / (m * n * (std::size_t)batch));
+      if (splits < 3) {
+        S::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, Nothing{}, s);
+        return;
+      }
+      const std::size_t terms = ((k + splits - 1) / splits + t.bk - 1) / t.bk * t.bk;
+      splits = (k + terms - 1) / terms;
+      S::template run<SPLIT>(A, B, C, m, n, k, batch_stride, batch, SplitK{scratch, (int)splits, (int)terms}, s);
+      dim3 grid((unsigned)((m * n + 31) / 32), (unsigned)batch);
+      split_finish_kernel<<<grid, 256, 0, s>>>(scratch, C, m * n, (int)splits, batch_stride);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch split_finish) --> ") + cudaGetErrorString(e);
+    };
+    n <= 8 ? small(Shape<64, 8, 16, 2, 2, 6>{}) : small(Shape<32, 32, 16, 2, 2, 6>{});
+    return;
+  }
   with_shape(m, n, k, [&](auto shape) {
     decltype(shape)::launch(A, B, C, m, n, k, batch_stride, batch, gather, s);
     return 0;

@@ -592,7 +592,7 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
       launches += a_planes || direct_product(op.m, op.n, op.k, cfg) ? 2 : 3;  // plane splits and the product
     } else if (op.a_gather) {
       launch_cgemm_tiled(arena + op.a, &p.tile_gather[tile_gathered++], arena + op.b, arena + op.c, op.m, op.n, op.k,
-                         stride, batch, stream_);
+                         stride, batch, nullptr, stream_);
       launches += 1;
     } else {
       launch_cgemm_fp32(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, batch,

@@ -545,7 +545,7 @@ void launch_cgemm_fp32(const float2* A, const float2* B, float2* C, std::size_t 
     check_launch("gemv_cols");
     return;
   }
-  launch_cgemm_tiled(A, nullptr, B, C, m, n, k, stride, batch, s);
+  launch_cgemm_tiled(A, nullptr, B, C, m, n, k, stride, batch, scratch, s);
 }
 
 void launch_reduce_amplitudes(const float2* results, std::uint64_t stride, const std::uint32_t* ptr,

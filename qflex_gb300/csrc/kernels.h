@@ -160,8 +160,10 @@ bool make_tile_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::s
 void tile_gather_on_host(const TileGather& g, std::size_t m, std::size_t n, std::size_t k, const float2* src,
                          float2* dst);
 // The tiled product, A row-major or (gather not null) through a permutation.
+// Products of few tiles split k when they have `scratch` (kSkinnyScratchElems).
 void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
-                        std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, cudaStream_t s);
+                        std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, float2* scratch,
+                        cudaStream_t s);
 
 // One skinny product (m * n outputs) with k split over `splits` blocks per
 // output; `partial` holds m * n * splits float2, every one of which is

@@ -2,17 +2,17 @@
 // TMEM + TMA).
 //
 // C = A * B, A complex64 in global memory, B as planes of Bt (n x k, K-major,
-// see split.cu). A is brought in as it lies -- row-major,
-// or through the index permutation that would have laid it out so (AGather)
-// -- and split into its planes inside the kernel. Against a split
-// kernel (or a plane-writing permutation) before the product that saves one
-// pass over A: 8 B read and 8 B written per element.
+// see split.cu). A is brought in as it lies -- row-major, or through the index
+// permutation that would have laid it out so (AGather) -- and split into its
+// planes inside the kernel. Against a split kernel (or a plane-writing
+// permutation) before the product that saves one pass over A: 8 B read and 8
+// (3xFP16), 12 (BF16x3) or 16 (3xTF32) written per element.
 //
 // Structure: persistent, one CTA per SM over tiles of 128 rows x BN (128, 64
-// or 32) columns, 512 threads in four warpgroups whose registers setmaxnreg divides (56, 176,
-// 176, 104 per thread: 128 on average, the launch's own share). Work goes by
-// blocks of A, 128 rows x two k-steps (32 values; 3xTF32, whose k-steps are
-// of 8 16: half a place in A's ring):
+// or 32) columns, 512 threads in four warpgroups whose registers setmaxnreg
+// divides (56, 176, 176, 104 per thread: 128 on average, the launch's own
+// share). Work goes by blocks of A, 128 rows x two k-steps: 32 values, or in
+// 3xTF32, whose k-steps are of 8, 16, half a place of A's ring.
 //   warp 0       B producer: four 8 KB TMA boxes a block (re and im rows of
 //                64 bytes, hi and lo, of each k-step)
 //   warp 1       TMEM allocation; issues every MMA
@@ -24,9 +24,9 @@
 //                into [2^14, 2^15), splits into hi + lo and writes the planes
 //                to its TMEM lane, where the MMAs read A
 // TMEM holds two blocks of planes (128 columns) and three sums of BN columns:
-// a block's real part is summed from zero into one, its imaginary
-// part into the next, and the epilogue, which applies the block's exponent as
-// it adds a sum to the tile, drains one while the others fill.
+// a block's real part is summed from zero into one, its imaginary part into
+// the next, and the epilogue, which applies the block's exponent as it adds a
+// sum to the tile, drains one while the others fill.
 //
 // PAIR (clusters of two CTAs, cta_group::2): CTA r has rows 128 r .. + 127 of a
 // tile of 256, their planes in its own tensor memory, and half of B's columns

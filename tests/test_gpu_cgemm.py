@@ -45,3 +45,12 @@ def test_product_without_terms_is_zero(built_lib):
     ctx.multiply(C.data_ptr() + 8, C.data_ptr() + 16, C.data_ptr(), 300, 20, 0)
     ctx.synchronize()
     assert not C.any()
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (16, 16, 32), (33, 31, 17), (64, 8, 191), (65, 7, 192), (16, 16, 192), (31, 33, 257), (130, 9, 1000), (64, 64, 4096),
+    (2, 3, 700), (1000, 24, 300), (512, 130, 511)])
+@pytest.mark.parametrize("batch,extra", [(1, 0), (3, 1)])
+def test_few_tiles(built_lib, m, n, k, batch, extra):
+    """Small tiles, and k in runs (from 192 terms on) summed afterwards."""
+    test_tiled_product(built_lib, m, n, k, batch, extra)
