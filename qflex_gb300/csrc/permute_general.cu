@@ -33,8 +33,18 @@ FastDiv fast_div(std::uint32_t d) {
   return f;
 }
 
+// What the kernel takes of the schedule, for up to CAP indices: a small tensor's
+// call is as long as its launch, to which 1.4 KB of arguments added 0.4 us.
+template <int CAP>
+struct RunPlan {
+  std::uint32_t runs, last_run, run, n_div;
+  FastDiv div[CAP];
+  std::uint32_t div_in[CAP], div_out[CAP], run_out[16];
+};
+
 // Input and output offset of thread r's run; its length.
-__host__ __device__ inline std::uint32_t run_of(const GeneralPerm& g, std::uint32_t r, std::uint32_t* in,
+template <typename Plan>
+__host__ __device__ inline std::uint32_t run_of(const Plan& g, std::uint32_t r, std::uint32_t* in,
                                                 std::uint32_t* out) {
   std::uint32_t i = 0, o = 0, digit = 0;
   for (std::uint32_t j = 0; j < g.n_div; ++j) {
@@ -50,8 +60,8 @@ __host__ __device__ inline std::uint32_t run_of(const GeneralPerm& g, std::uint3
   return digit + 1 == g.div[g.n_div - 1].d ? g.last_run : g.run;
 }
 
-template <int RUN>
-__global__ void __launch_bounds__(256) permute_runs_kernel(const __grid_constant__ GeneralPerm g,
+template <int RUN, int CAP>
+__global__ void __launch_bounds__(256) permute_runs_kernel(const __grid_constant__ RunPlan<CAP> g,
                                                            const float2* __restrict__ src, float2* __restrict__ dst,
                                                            std::uint64_t batch_stride) {
   src += std::uint64_t(blockIdx.y) * batch_stride;
@@ -99,6 +109,7 @@ void plan_runs(GeneralPerm* g) {
   // The permuted indices in output order, neighbours that stay neighbours as
   // one, then fastest output index first.
   std::vector<Dim> dims;
+  dims.reserve(kGeneralPermMaxRank + 1);
   std::uint64_t out = g->size;
   for (std::uint32_t i = 0; i < g->rank; ++i) {
     const std::uint32_t d = (std::uint32_t)g->out_dims[i], in = (std::uint32_t)g->in_stride[i];
@@ -205,18 +216,37 @@ void permute_general_on_host(const GeneralPerm& g, const float2* src, float2* ds
   }
 }
 
+template <int CAP>
+static void launch_runs(const GeneralPerm& g, const float2* src, float2* dst, std::uint64_t batch_stride, dim3 grid,
+                        cudaStream_t s) {
+  RunPlan<CAP> p;
+  p.runs = g.runs;
+  p.last_run = g.last_run;
+  p.run = g.run;
+  p.n_div = g.n_div;
+  std::copy_n(g.div, g.n_div, p.div);
+  std::copy_n(g.div_in, g.n_div, p.div_in);
+  std::copy_n(g.div_out, g.n_div, p.div_out);
+  std::copy_n(g.run_out, 16, p.run_out);
+  auto* kernel = g.run == 1   ? permute_runs_kernel<1, CAP>
+                 : g.run <= 4 ? permute_runs_kernel<4, CAP>
+                 : g.run <= 8 ? permute_runs_kernel<8, CAP>
+                              : permute_runs_kernel<16, CAP>;
+  kernel<<<grid, 256, 0, s>>>(p, src, dst, batch_stride);
+}
+
 void launch_permute_general(const GeneralPerm& g, const float2* src, float2* dst, std::uint64_t batch_stride,
                             int batch, cudaStream_t s) {
   if (g.size == 0 || batch == 0) return;
   const std::uint64_t threads = g.runs ? g.runs : g.size;
   const std::uint64_t blocks = std::min<std::uint64_t>((threads + 255) / 256, 152ull * 64ull);
   dim3 grid((unsigned)blocks, (unsigned)batch, 1);
-  auto* kernel = !g.runs         ? permute_general_kernel
-                 : g.run == 1    ? permute_runs_kernel<1>
-                 : g.run <= 4    ? permute_runs_kernel<4>
-                 : g.run <= 8    ? permute_runs_kernel<8>
-                                 : permute_runs_kernel<16>;
-  kernel<<<grid, 256, 0, s>>>(g, src, dst, batch_stride);
+  if (!g.runs)
+    permute_general_kernel<<<grid, 256, 0, s>>>(g, src, dst, batch_stride);
+  else if (g.n_div <= 8)
+    launch_runs<8>(g, src, dst, batch_stride, grid, s);
+  else
+    launch_runs<kGeneralPermMaxRank + 1>(g, src, dst, batch_stride, grid, s);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     throw std::string("ERROR (qflex_gb300: launch permute_general) --> ") + cudaGetErrorString(e);
