@@ -39,9 +39,9 @@ WORKLOAD = "c3"
 FP32_PEAK_NOMINAL = 152 * 128 * 2 * 2.07e9 / 1e12  # TFLOP/s, FP32 CUDA-core FMA
 # DRAM bytes (read + write) per product of the dominant shape, from the ncu
 # captures summarised in profiles/ (dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch divided by its products): 3xTF32 at 1
-# product per launch, 3xFP16 at 4 (the step's pass size), 5.728 GB / 4.
-TRAFFIC = {("tf32x3", 4096, 4096, 4096): 2.322e9, ("fp16x3", 4096, 4096, 4096): 1.432e9}
+# dram__bytes_write.sum of a launch of one product; 3xTF32: the kernel that
+# loads both operands' planes).
+TRAFFIC = {("tf32x3", 4096, 4096, 4096): 2.322e9, ("fp16x3", 4096, 4096, 4096): 0.997e9}
 
 
 def parse():
@@ -528,7 +528,7 @@ def main():
                          "unit": "TFLOP/s algorithmic"},
                 "traffic": (TRAFFIC[(args.precision, m, n, k)] * pbatch
                             if (args.precision, m, n, k) in TRAFFIC else None),
-                "traffic_source": "ncu dram__bytes_read+write per product of this shape (profiles/tc_*_4096.md), "
+                "traffic_source": "ncu dram__bytes_read+write per product of this shape (profiles/tc_direct.md, tc_gemm_4096.md), "
                                   "times the products per launch",
                 "algorithmic_bytes": 8.0 * (m * k + k * n + m * n) * pbatch,
                 "timing": f"CUDA events around each of the {launches} launches of this shape (batch {pbatch}) "
