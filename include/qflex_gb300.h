@@ -138,10 +138,10 @@ size_t qflex_gb300_last_ops(const qflex_gb300_context* ctx, double* out, size_t 
  *                replay it (default 1, or QFLEX_GB300_GRAPHS)
  *   "max_batch"  most output strings per device pass of evaluate_many
  *                (0: as many as fit in device memory; default 0)
- *   "fuse_splits" 1: CUDA-core products, and 3xFP16 products of up to 1024
- *                columns (kernel choice 0), read A through the permutation
- *                that would lay it out, and no permutation runs; for the
- *                other 3xFP16 products a permutation whose
+ *   "fuse_splits" 1: CUDA-core products, and split products that split A
+ *                inside the kernel (kernel choice 0, chunks of two k-steps),
+ *                read A through the permutation that would lay it out, and no
+ *                permutation runs; for other 3xFP16 products a permutation whose
  *                output is the next product's A operand and read by nothing
  *                else writes the FP16 planes (scaled per 32 values of a row)
  *                directly instead of complex64, and the product skips

@@ -59,6 +59,12 @@ __device__ __forceinline__ void copy16(float2* dst, const float2* src) {
                "l"(src)
                : "memory");
 }
+__device__ __forceinline__ void copy16(float2* dst, const float2* src, bool real) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   static_cast<std::uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(real ? 16u : 0u)
+               : "memory");
+}
 
 // Row stride of a staged A tile in elements: 16 bytes more than its values,
 // so that the rows a quarter-warp reads start in different banks.
@@ -156,6 +162,28 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       for (int i = 0; i < LP; ++i) {
         if (BM * P % NT == 0 || r + i * ROWS < BM) copy16(As + (r + i * ROWS) * AR + c, src);
         src += std::uint64_t(ROWS) * k;
+      }
+    } else if ((pairs & 2) && k0 + BK <= k) {
+      // Rows on 16 bytes, some of them past the last.
+      constexpr int P = BK / 2, LP = (BM * P + NT - 1) / NT, ROWS = NT / P;
+      const int r = t / P, c = 2 * (t % P), rows = m - int(mt * BM) - r;
+      const float2* src = A + at + std::uint64_t(mt * BM + r) * k + k0 + c;
+#pragma unroll
+      for (int i = 0; i < LP; ++i) {
+        if (BM * P % NT == 0 || r + i * ROWS < BM)
+          copy16(As + (r + i * ROWS) * AR + c, i * ROWS < rows ? src : A, i * ROWS < rows);
+        src += std::uint64_t(ROWS) * k;
+      }
+    } else if (k0 + BK <= k) {
+      // Rows on 8 bytes.
+      static_assert(NT % BK == 0, "values of a row of A / threads");
+      const int r = t / BK, c = t % BK, rows = m - int(mt * BM) - r;
+      const float2* src = A + at + std::uint64_t(mt * BM + r) * k + k0 + c;
+#pragma unroll
+      for (int i = 0; i < LA; ++i) {
+        const bool real = i * (NT / BK) < rows;
+        copy8(As + (r + i * (NT / BK)) * AR + c, real ? src : A, real);
+        src += std::uint64_t(NT / BK) * k;
       }
     } else {
 #pragma unroll
@@ -359,6 +387,7 @@ auto with_shape(std::size_t m, std::size_t n, std::size_t k, F&& f) {
   if (n <= 16) return f(Shape<256, 16, 8, 8, 4, 2>{});
   if (n <= 32) return f(Shape<128, 32, 8, 8, 4, 3>{});
   if (m <= 32) return f(Shape<16, 256, 8, 4, 8, 3>{});
+  if (m <= 64 && n >= 128 && k > 8) return f(Shape<64, 128, 16, 8, 4, 3>{});  // (50, 1642, 1993) x 7 804 -> 438 us
   if (k <= 8) return f(Shape<128, 64, 8, 8, 4, 3>{});
   return f(Shape<128, 64, 16, 8, 4, 3>{});
 }
@@ -448,11 +477,14 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
   // than the SMs hold (two each), so does splitting k into runs of 64 or more.
   // The shapes above against these: (16, 16, 32) 10 and 4 us, (256, 16, 64) 19
   // and 5.5, (512, 512, 512) 104 and 42; with runs (256, 16, 512) 80 and 9,
-  // (16, 16, 4096) 500 and 12. A gather is made for the shapes above.
+  // (16, 16, 4096) 500 and 12. Up to 101 tiles with 512 terms take runs too, in
+  // the shapes above: (1586, 161, 3221) 686 and 342, (1000, 512, 1000) 202 and
+  // 140. A gather is made for the shapes above.
   const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
   const std::size_t tiles = ((m + tile.bm - 1) / tile.bm) * ((n + tile.bn - 1) / tile.bn) * (std::size_t)batch;
-  if (!gather && tiles && tiles <= 38) {
-    auto small = [&](auto shape) {
+  const bool runs = scratch && tiles <= 101 && k >= 512 && 3 * m * n * (std::size_t)batch <= kSkinnyScratchElems;
+  if (!gather && tiles && (tiles <= 38 || runs)) {
+    auto few = [&](auto shape) {
       using S = decltype(shape);
       constexpr Tile t = S::tile;
       const std::size_t own = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn) * (std::size_t)batch;
@@ -460,7 +492,7 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
       splits = std::min<std::size_t>(splits, kSkinnyScratchElems / (m * n * (std::size_t)batch));
       if (splits < 3) {
         S::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, Nothing{}, s);
-        return;
+        return 0;
       }
       const std::size_t terms = ((k + splits - 1) / splits + t.bk - 1) / t.bk * t.bk;
       splits = (k + terms - 1) / terms;
@@ -469,9 +501,26 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
       split_finish_kernel<<<grid, 256, 0, s>>>(scratch, C, m * n, (int)splits, batch_stride);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch split_finish) --> ") + cudaGetErrorString(e);
+      return 0;
     };
-    n <= 8 ? small(Shape<64, 8, 16, 2, 2, 6>{}) : small(Shape<32, 32, 16, 2, 2, 6>{});
+    if (tiles > 38)
+      with_shape(m, n, k, few);
+    else
+      n <= 8 ? few(Shape<64, 8, 16, 2, 2, 6>{}) : few(Shape<32, 32, 16, 2, 2, 6>{});
     return;
+  }
+  // Where one or two blocks on an SM hold all tiles: up to 32 columns in tiles
+  // of 64 rows, more of them with fewer outputs a thread ((16384, 16, 256) 40
+  // and 20 us, (25646, 10, 112) x 2 34 and 23, (30000, 32, 64) 16.8 and 15.6);
+  // more columns in k-steps of 32, half the barriers ((2000, 512, 256) 54.7 and
+  // 51.2, (92, 717, 148) x 7 37.2 and 34.7).
+  if (!gather && n > 8 && tiles <= (n <= 32 ? 304u : 152u)) {
+    auto plain = [&](auto shape) {
+      decltype(shape)::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, Nothing{}, s);
+    };
+    if (n <= 16) return plain(Shape<64, 16, 16, 4, 2, 4>{});
+    if (n <= 32) return plain(Shape<64, 32, 16, 4, 4, 3>{});
+    if (m > 64 && k >= 128) return plain(Shape<128, 64, 32, 8, 4, 2>{});
   }
   with_shape(m, n, k, [&](auto shape) {
     decltype(shape)::launch(A, B, C, m, n, k, batch_stride, batch, gather, s);

@@ -219,9 +219,9 @@ bool Engine::direct_product(std::size_t m, std::size_t n, std::size_t k, const T
 // Products of 16 to 63 columns in the direct kernel's tiles of 32 or 64, from
 // the number of terms on where its error is below that of FP32 sums (see
 // split_multiply): A is then nearly all there is to read. FP32 products
-// against these, with B's split: (1048576, 16, 256) 746 and 361 us, (131072,
-// 32, 256) 194 and 63, (256, 16, 256) 39 and 15, (1000, 50, 100) 26 and 14.
-// Contractions with fewer rows may run as one small program instead.
+// against these, with B's split: (1048576, 16, 256) 746 and 350 us, (131072,
+// 32, 256) 194 and 59, (65536, 16, 256) 69 and 36. Contractions with fewer rows
+// may run as one small program instead.
 bool Engine::narrow_product(std::size_t m, std::size_t n, std::size_t k) const {
   return precision_ == FP16X3 && m >= 256 && n >= 16 && n < 64 && k >= 96 && tc_runs(m, n, k) &&
          direct_product(m, n, k, tc_config(m, n, k));
@@ -292,18 +292,22 @@ void Engine::check_error_flag() {
 // sums or more so. Relative RMS errors against complex128 products of
 // Gaussian operands, (1000, 256, k), FP32 / 3xFP16 / 3xTF32 / BF16x3:
 // k = 64 2.0 / 1.6 / 1.5 / 2.3e-7, 128 2.9 / 1.7 / 1.6 / 2.3e-7,
-// 1024 8.1 / 1.9 / 2.1 / 2.5e-7. (3001, 690, 1100) in 3xFP16: 424 -> 65 us.
-bool Engine::split_multiply(std::size_t m, std::size_t n, std::size_t k) const {
-  if (m >= 64 && n >= 64 && k >= 96 && tc_runs(m, n, k)) return true;
-  if (narrow_product(m, n, k)) return true;
-  return tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
+// 1024 8.1 / 1.9 / 2.1 / 2.5e-7. (3001, 690, 1100) in 3xFP16: 424 -> 45 us.
+// Below 2^25 terms in all the FP32 kernel's few small tiles are ahead, FP32
+// against 3xFP16 with B's split, us a call: (128, 64, 96) 8 and 15, (1024, 128,
+// 128) 10 and 19, (256, 256, 256) 19 and 23; kernels (2048, 16, 256) 12 and 13,
+// (4096, 32, 128) 9 and 11, (8192, 32, 128) 19 and 11, (16384, 16, 256) 40 and 14.
+bool Engine::split_multiply(std::size_t m, std::size_t n, std::size_t k, int batch) const {
+  if (tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0) return true;
+  if (k < 96 || double(m) * n * k * batch < double(1 << 25)) return false;
+  return narrow_product(m, n, k) || (m >= 64 && n >= 64 && tc_runs(m, n, k));
 }
 
 void Engine::multiply(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n,
                       std::size_t k, std::uint64_t stride, int batch) {
   if (is_complex128(precision_))
     throw QFX_ERR("The complex64 tensor operations need a complex64 precision mode (this context is complex128).");
-  if (precision_ != FP32 && split_multiply(m, n, k)) {
+  if (precision_ != FP32 && split_multiply(m, n, k, batch)) {
     const std::size_t bytes = workspace_elems(m, n, k) * (std::size_t)batch * sizeof(float);
     // A product that FP32 can run as well needs no more memory than that.
     const bool contraction = tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
@@ -711,6 +715,10 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
           p.gather.push_back(g);
         } else {
           TileGather g;
+          // Few outputs of many terms run faster from a row-major A, in the
+          // small tiles and runs of k that gathers have no tables for: (16, 16,
+          // 256) 54 us gathered, 12 with its permutation.
+          if (k >= 64 && m * n <= 4096) return false;
           if (m < 2 || n < 2 || m * n <= 64 || !make_tile_gather(nbits, perm, m, n, k, &g)) return false;
           p.tile_gather.push_back(g);
         }

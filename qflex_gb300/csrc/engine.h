@@ -131,7 +131,7 @@ class Engine {
   unsigned options_version_ = 0;  // part of the graph key: options change launches
   TcConfig tc_config(std::size_t m, std::size_t n, std::size_t k) const;
   bool direct_product(std::size_t m, std::size_t n, std::size_t k, const TcConfig& cfg) const;
-  bool split_multiply(std::size_t m, std::size_t n, std::size_t k) const;
+  bool split_multiply(std::size_t m, std::size_t n, std::size_t k, int batch) const;
   // fp32 elements of split planes that one product of this shape needs.
   bool narrow_product(std::size_t m, std::size_t n, std::size_t k) const;
   std::size_t workspace_elems(std::size_t m, std::size_t n, std::size_t k) const;

@@ -54,3 +54,12 @@ def test_product_without_terms_is_zero(built_lib):
 def test_few_tiles(built_lib, m, n, k, batch, extra):
     """Small tiles, and k in runs (from 192 terms on) summed afterwards."""
     test_tiled_product(built_lib, m, n, k, batch, extra)
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (10000, 16, 33), (9999, 9, 16), (16001, 12, 100), (5000, 32, 40), (6001, 17, 15), (3000, 200, 128), (2999, 193, 131),
+    (64, 3000, 20), (33, 2999, 131), (1586, 161, 513), (1001, 300, 700)])
+@pytest.mark.parametrize("batch,extra", [(1, 0), (2, 1)])
+def test_one_wave(built_lib, m, n, k, batch, extra):
+    """Tiles for products that the SMs hold at once, and of 64 rows."""
+    test_tiled_product(built_lib, m, n, k, batch, extra)
