@@ -15,14 +15,15 @@
 //   (32768, 64, 64) x 16      462 ->  342 us (50 TFLOP/s)
 //   (32768, 64, 8) x 16       221 ->   71 us
 //   (32768, 8, 64) x 16       113 ->   72 us
-//   (2^20, 16, 16)             75 ->   65 us (4.1 TB/s)
+//   (2^20, 16, 16)             75 ->   63 us (4.2 TB/s)
 //   (2^20, 16, 256)           847 ->  747 us
 // Copies of 16 bytes are worth 10 to 25 % of that against copies of 8; k-steps
 // of 8 keep four blocks of the narrow tiles on an SM. Two-lane FMAs
 // (fma.rn.f32x2) have the same rate from registers and lose more to packing
 // their operands: 2049 us at 2048^3.
 //
-// Sums run over k in ascending order with four FMAs per complex term.
+// Sums run over k in ascending order with four FMAs per complex term; products
+// of few tiles may sum runs of k so and then add the runs in 64 bits.
 //
 // A is read as it lies or, for the tensors of a contraction, through the digit
 // permutation that would have laid it out row-major (TileGather): then lanes
