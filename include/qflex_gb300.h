@@ -125,12 +125,13 @@ size_t qflex_gb300_last_ops(const qflex_gb300_context* ctx, double* out, size_t 
  * no device kernels to tune). Names and values:
  *   "tc_chunk"   k-steps per TMEM accumulation chunk of the split
  *                tensor-core product, 1..64 (default 2, or QFLEX_TC_CHUNK;
- *                longer chunks are faster and less accurate: the tensor
- *                core's FP32 accumulation truncates, which shrinks every
- *                product by an amount that grows with the chunk)
+ *                longer chunks are less accurate: the tensor core's FP32
+ *                accumulation truncates, which shrinks every product by an
+ *                amount that grows with the chunk; lengths other than 2 run
+ *                the kernels that load both operands' planes)
  *   "tc_pair"    1: 3xTF32 products with m >= 256 use the CTA-pair
  *                (cta_group::2, 256 x 128 tile) kernel; 0: every product uses
- *                the single-CTA 128 x 128 tile (default 0, or QFLEX_TC_PAIR)
+ *                kernel choice 0 (default 0, or QFLEX_TC_PAIR)
  *   "tc_variant" tensor-core kernel of every product without a per-shape
  *                choice (qflex_gb300_set_tc_variant): 0..4 as listed there
  *                (default 0; "tc_pair" sets 0 or the pair-for-m >= 256 rule)
@@ -172,11 +173,13 @@ size_t qflex_gb300_last_ops(const qflex_gb300_context* ctx, double* out, size_t 
 int qflex_gb300_set_option(qflex_gb300_context* ctx, const char* name, double value);
 int qflex_gb300_get_option(const qflex_gb300_context* ctx, const char* name, double* value);
 /* Tensor-core kernel for products of shape (m, n, k), e.g. chosen by an
- * autotuner: 0 single CTA, 1 CTA pair (needs m >= 64), 2 single CTA with a
- * deeper operand pipeline (3xFP16), 3 single CTA with 16 epilogue warps
- * (3xFP16; outputs that cannot take bulk tensor stores use 0), 4 single CTA
- * with 64-column tiles and four TMEM chunk buffers (3xFP16); the other
- * precisions take 0. -1 removes the override. Overrides "tc_pair" for that
+ * autotuner: 0 the kernel that splits A itself (pairs of CTAs from 129 rows
+ * on) where it runs, else the single CTA that loads both operands' planes;
+ * from planes, 1 CTA pair (needs m >= 64), 2 single CTA with a deeper operand
+ * pipeline (3xFP16), 3 single CTA with 16 epilogue warps (3xFP16; outputs that
+ * cannot take bulk tensor stores use the plain one), 4 single CTA with
+ * 64-column tiles and four TMEM chunk buffers (3xFP16); the other precisions
+ * take the plain one. -1 removes the override. Overrides "tc_pair" for that
  * shape. */
 int qflex_gb300_set_tc_variant(qflex_gb300_context* ctx, size_t m, size_t n, size_t k, int variant);
 

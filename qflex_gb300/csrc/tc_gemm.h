@@ -27,7 +27,8 @@ std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k);
 // Kernel choice of one product.
 struct TcConfig {
   int chunk = 2;     // k-steps per TMEM accumulation chunk, 1..64 (QFLEX_TC_CHUNK)
-  int variant = 0;   // 0: single CTA; 1: CTA pair; -1: CTA pair when m >= 256, else single;
+  int variant = 0;   // 0: the product that splits A itself (tc_direct.cu) where it runs, else single
+                     // CTA; 1: CTA pair from planes; -1: CTA pair when m >= 256, else single;
                      // 2: 3xFP16 single CTA with five stages; 3: 3xFP16 single CTA with 16
                      // epilogue warps; 4: 3xFP16 single CTA with 64-column tiles and four
                      // TMEM chunk buffers (others: single CTA)
