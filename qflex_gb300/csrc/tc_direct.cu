@@ -108,7 +108,8 @@ struct Layout {
   static constexpr int OFF_SCALE = OFF_STAGING + 8 * SLOTS * SLOT;
   static constexpr int OFF_EXP = OFF_SCALE + 8 * COLS * 4;  // after each epilogue warp's column exponents
   static constexpr int OFF_BAR = OFF_EXP + EXP_RING * BM;
-  static constexpr int N_BARS = 2 * A_RING + A_BUFS + B_STAGES + 2 * DONE + HALVES + 1;
+  static constexpr int EXP_BARS = KIND == KIND_FP16 ? EXP_RING : 0;
+  static constexpr int N_BARS = 2 * A_RING + A_BUFS + B_STAGES + 2 * DONE + HALVES + 1 + 2 * EXP_BARS;
   static constexpr int SMEM = OFF_BAR + N_BARS * 8 + 8;
   static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
   static constexpr int TMEM_A = HALVES * BN;  // the planes, after the sums
@@ -265,7 +266,9 @@ __global__ void __launch_bounds__(THREADS, 1)
   std::uint64_t* done = re_full + DONE;         // all MMAs of a block are done
   std::uint64_t* acc_empty = done + DONE;       // an accumulator was drained
   std::uint64_t* mma_done = acc_empty + HALVES;
-  std::uint32_t* tmem_slot = reinterpret_cast<std::uint32_t*>(mma_done + 1);
+  std::uint64_t* exp_full = mma_done + 1;             // a block's exponents are written
+  std::uint64_t* exp_empty = exp_full + L::EXP_BARS;  // and read by the epilogue
+  std::uint32_t* tmem_slot = reinterpret_cast<std::uint32_t*>(exp_empty + L::EXP_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   if (smem_u32(smem) & 1023) {  // the swizzles need it; the layout leaves no room to round up
     if (threadIdx.x == 0) atomicExch(err, 9);
@@ -295,7 +298,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   };
   // Waits and arrivals keep CTA scope in a pair as well: what the barriers
   // between its CTAs order are tensor-memory accesses (with the tcgen05
-  // fences) and TMA writes. At cluster scope a block took 3200 cycles.
+  // fences) and TMA writes. At cluster scope a block took 3200 cycles. The
+  // blocks' exponents, ordinary shared memory, have barriers of their own
+  // inside the CTA (exp_full, exp_empty): neither an arrival at the other
+  // CTA nor a commit orders them.
   auto wait = [&](std::uint64_t* bar, std::uint32_t parity, int code) {
     return mbar_wait(bar, parity, abort_flag, err, code);
   };
@@ -331,6 +337,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     for (int s = 0; s < HALVES; ++s) mbar_init(&acc_empty[s], PAIR ? 16 : 8);
     mbar_init(mma_done, 1);
+    for (int s = 0; s < L::EXP_BARS; ++s) {
+      mbar_init(&exp_full[s], CONVERTERS / 32);
+      mbar_init(&exp_empty[s], 8);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -444,6 +454,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       int xa = 0, sb = 0, h = 0, r = 0;
       for (int w = 0; w < work; ++w) {
         if (!__all_sync(0xffffffffu, kind == 3 || wait(bars + at, parity, 2))) break;
+        __syncwarp();  // what one lane's wait orders, it orders for the leader
         asm volatile("tcgen05.fence::after_thread_sync;");
         const std::uint32_t a = tmem + TMEM_A + xa * TMEM_A_BLOCK, b = b_lo0 + sb * (B_STAGE >> 4);
         if (leader) {
@@ -454,6 +465,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // The epilogue's TMEM reads of a buffer precede the MMAs that
         // overwrite it.
         if (!__all_sync(0xffffffffu, kind != 3 || wait(bars + at, parity, 4))) break;
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (leader) {
           issue(std::integral_constant<int, 1>{}, tmem + h * BN, a, b);
@@ -593,7 +605,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const std::uint32_t ring = smem_u32(smem);
     const std::uint32_t lanes = tmem + TMEM_A + (std::uint32_t((warp - 12) * 32) << 16);
     int s = 0, x = 0, xa = 0, r = DONE - A_BUFS;
-    std::uint32_t ph = 0, pd = 1;  // block w - A_BUFS: barrier r
+    std::uint32_t ph = 0, pd = 1, pe = 1;  // block w - A_BUFS: barrier r
+    const bool odd = KIND == KIND_FP16 && (lane & 1);
     // Values of the thread's row from the first (h = 0) or second 16 of place s
     // of the ring on.
     auto read = [&](auto& v, int s, int h) {
@@ -620,9 +633,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&raw_empty[s]);
     };
-    // Waits for the MMAs of the block two back, whose place in TMEM comes next.
+    // Waits for the MMAs of the block two back, whose place in TMEM comes
+    // next, and (the odd lanes meanwhile) for the epilogue's reads of the
+    // exponents EXP_RING blocks back.
     auto place = [&] {
-      if (!__all_sync(0xffffffffu, wait(&done[r], pd, 10))) return false;
+      if (!__all_sync(0xffffffffu, wait(odd ? &exp_empty[x] : &done[r], odd ? pe : pd, 10))) return false;
+      __syncwarp();
       if (++r == DONE) {
         r = 0;
         pd ^= 1u;
@@ -702,17 +718,20 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (!place()) break;
         tmem_st32(to, p[0]);
         tmem_st32(to + 32, p[1]);
-        // Exponents live in a ring of their own: the MMAs of the block two
-        // back are done, so every epilogue warp has read the exponents of the
-        // block three back.
         if constexpr (KIND == KIND_FP16) exps[x * BM + row] = std::int8_t(e);
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
-      if (lane == 0) arrive(&a_full[xa]);
+      if (lane == 0) {
+        if constexpr (KIND == KIND_FP16) mbar_arrive(&exp_full[x]);
+        arrive(&a_full[xa]);
+      }
       xa ^= 1;
-      if (++x == EXP_RING) x = 0;
+      if (++x == EXP_RING) {
+        x = 0;
+        pe ^= 1u;
+      }
       if (last && ++s == A_RING) {
         s = 0;
         ph ^= 1u;
@@ -733,7 +752,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     const float beta = debias_beta<KIND>(err, 2, (k + VALUES / 2 - 1) / (VALUES / 2));
     const float2 beta2 = make_float2(beta, beta);
     int h = 0, x = 0, r = 0;
-    std::uint32_t pr = 0;
+    std::uint32_t pr = 0, px = 0;
+    const bool odd = KIND == KIND_FP16 && (lane & 1);
     bool ok = true;
     const std::uint32_t base0 = tmem + (std::uint32_t(q * 32) << 16) + part * COLS;
     // Adds the next TMEM buffer, times `f`, to `sum`.
@@ -776,13 +796,23 @@ __global__ void __launch_bounds__(THREADS, 1)
       // only when a later block is more than four times larger.
       int eref = 0;
       for (int b = 0; b < blocks; ++b) {
-        if (!__all_sync(0xffffffffu, wait(&re_full[r], pr, 3))) {
+        // The odd lanes wait for the block's exponents.
+        if (!__all_sync(0xffffffffu, wait(odd ? &exp_full[x] : &re_full[r], odd ? px : pr, 3))) {
           ok = false;
           break;
         }
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const int e = KIND == KIND_FP16 ? exps[x * BM + row] : 0;
-        if (++x == EXP_RING) x = 0;
+        int e = 0;
+        if constexpr (KIND == KIND_FP16) {
+          e = exps[x * BM + row];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&exp_empty[x]);
+          if (++x == EXP_RING) {
+            x = 0;
+            px ^= 1u;
+          }
+        }
         if (b == 0) {
           eref = KIND == KIND_FP16 ? e - 2 : 0;
         } else if (KIND == KIND_FP16 && __any_sync(0xffffffffu, e < eref)) {
