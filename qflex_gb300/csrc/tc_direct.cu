@@ -110,7 +110,7 @@ struct Layout {
   static constexpr int OFF_BAR = OFF_EXP + EXP_RING * BM;
   static constexpr int EXP_BARS = KIND == KIND_FP16 ? EXP_RING : 0;
   static constexpr int N_BARS = 2 * A_RING + A_BUFS + B_STAGES + 2 * DONE + HALVES + 1 + 2 * EXP_BARS;
-  static constexpr int SMEM = OFF_BAR + N_BARS * 8 + 8;
+  static constexpr int SMEM = OFF_BAR + N_BARS * 8 + 24;  // and tmem_slot .. peer_abort
   static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
   static constexpr int TMEM_A = HALVES * BN;  // the planes, after the sums
   static constexpr int TMEM_COLS = BN == 32 ? 256 : 512;
@@ -270,6 +270,12 @@ __global__ void __launch_bounds__(THREADS, 1)
   std::uint64_t* exp_empty = exp_full + L::EXP_BARS;  // and read by the epilogue
   std::uint32_t* tmem_slot = reinterpret_cast<std::uint32_t*>(exp_empty + L::EXP_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  // What lands if the pipeline is abandoned: blocks of A by boxes and stages of
+  // B asked for, in a pair those of B by CTA 1; whether the other CTA gave up.
+  volatile int* issued_a = abort_flag + 1;
+  volatile int* issued_b = issued_a + 1;
+  volatile int* peer_b = issued_b + 1;
+  volatile int* peer_abort = peer_b + 1;
   if (smem_u32(smem) & 1023) {  // the swizzles need it; the layout leaves no room to round up
     if (threadIdx.x == 0) atomicExch(err, 9);
     return;
@@ -342,6 +348,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_init(&exp_empty[s], 8);
     }
     *abort_flag = 0;
+    *issued_a = *issued_b = *peer_b = *peer_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // The second half of a block that a k of 16 does not have.
@@ -403,19 +410,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           if (++s == B_STAGES) s = 0;
         }
       }
-      if (*abort_flag) {
-        // The copies already issued land before the CTA's shared memory is
-        // released (bounded as well). Those of a pair's CTA 1 complete on CTA
-        // 0, which may have expected fewer: time for them to land.
-        const unsigned long long t1 = now_ns();
-        while (rank == 1 && now_ns() - t1 < 1000000) {
-        }
-        for (int w = q > B_STAGES ? q - B_STAGES : 0; w < q && rank == 0; ++w) {
-          const unsigned long long t0 = now_ns();
-          while (!mbar_test(&b_full[w % B_STAGES], (w / B_STAGES) & 1) && now_ns() - t0 < WAIT_NS) {
-          }
-        }
-      }
+      *issued_b = q;
     } else if (warp == 1 && rank == 0) {
       // MMA issuer (of a pair: CTA 0). The whole warp runs the loop in step and one elected lane
       // issues: the descriptors then live in uniform registers. Run by one
@@ -518,13 +513,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
           }
         }
-        if (*abort_flag) {
-          for (int w = q > A_RING ? q - A_RING : 0; w < q; ++w) {
-            const unsigned long long t0 = now_ns();
-            while (!mbar_test(&raw_full[w % A_RING], (w / A_RING) & 1) && now_ns() - t0 < WAIT_NS) {
-            }
-          }
-        }
+        *issued_a = q;
       }
     } else if (warp >= 2) {
       // A loader. A block is 2048 copies of 16 bytes (a pair of elements
@@ -946,8 +935,43 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   }
   if constexpr (PAIR) {
+    if (threadIdx.x == 0) {
+      auto tell = [&](volatile int* word, int v) {
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_addr(const_cast<int*>(word), rank ^ 1)), "r"(v)
+                     : "memory");
+      };
+      tell(peer_abort, *abort_flag);
+      if (rank == 1) tell(peer_b, *issued_b);
+    }
     __syncthreads();
     cluster_sync();
+  }
+  if (*abort_flag || *peer_abort) {
+    // Every copy asked for lands before shared memory is released (waits are
+    // bounded here as well). A pair's stages of B complete on CTA 0's barriers:
+    // where one CTA alone asked for its half of a stage, CTA 0 makes the
+    // barrier expect that half only.
+    if (threadIdx.x == 0) {
+      auto land = [&](std::uint64_t* bar, std::uint32_t parity) {
+        const unsigned long long t0 = now_ns();
+        while (!mbar_test(bar, parity) && now_ns() - t0 < WAIT_NS) {
+        }
+      };
+      const int qa = *issued_a, qb = *issued_b, qp = PAIR ? *peer_b : qb;
+      for (int w = max(qa - A_RING, 0); w < qa; ++w) land(&raw_full[w % A_RING], (w / A_RING) & 1);
+      const int last = max(qb, qp);
+      for (int w = max(last - B_STAGES, 0); w < last && rank == 0; ++w) {
+        std::uint64_t* bar = &b_full[w % B_STAGES];
+        if (w >= qb)
+          mbar_expect_tx(bar, B_STAGE);
+        else if (w >= qp)
+          asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(B_STAGE)
+                       : "memory");
+        land(bar, (w / B_STAGES) & 1);
+      }
+    }
+    __syncthreads();
+    if constexpr (PAIR) cluster_sync();
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;");

@@ -61,3 +61,33 @@ def test_block_exponents(built_lib, m, n, k, batch):
     scale = torch.randint(-30, 31, (batch, m, (k + 31) // 32), device="cuda", generator=gen)
     A = randn((batch, m, k), k) * torch.exp2(scale.repeat_interleave(32, -1)[..., :k])
     check(FP16X3, A, randn((batch, k, n), n), 0, 6e-6)
+
+
+@pytest.mark.parametrize("precision,m,n,k", [
+    (FP16X3, 300, 640, 200), (FP16X3, 20000, 256, 256), (FP16X3, 100, 1000, 400), (FP16X3, 60000, 32, 128),
+    (TF32X3, 300, 640, 200), (TF32X3, 20000, 256, 256), (TF32X3, 100, 1000, 400), (BF16X3, 300, 640, 200),
+    (BF16X3, 20000, 256, 256)])
+def test_abandoned_products(built_lib, precision, m, n, k):
+    """Products whose pipeline waits run out at once (limit 1 ns), in pairs and
+    alone, end with the error and with every copy landed: the products after
+    them, in the same context and at the default limit, are right."""
+    import torch
+
+    from qflex_gb300 import QflexGb300Error
+    A, B = randn((1, m, k), k)[0], randn((1, k, n), n)[0]
+    C = torch.zeros((m, n), dtype=torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    ctx = Context(0, precision)
+    want = A.to(torch.complex128) @ B.to(torch.complex128)
+    bound = A.abs().double() @ B.abs().double()
+    for _ in range(3):
+        ctx.set_option("tc_wait_ns", 1)
+        for _ in range(4):
+            ctx.multiply(A.data_ptr(), B.data_ptr(), C.data_ptr(), m, n, k)
+            with pytest.raises(QflexGb300Error, match="pipeline wait expired"):
+                ctx.synchronize()
+        ctx.set_option("tc_wait_ns", 0)
+        ctx.multiply(A.data_ptr(), B.data_ptr(), C.data_ptr(), m, n, k)
+        ctx.synchronize()
+        # Bound as for test_block_exponents, k <= 400 (3xTF32: chunks of 16 terms).
+        assert float(((C - want).abs() / bound).max()) < 8e-6
