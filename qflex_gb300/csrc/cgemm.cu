@@ -30,12 +30,12 @@
 // follow the source's order and each copy goes to its place in the tile.
 #include <algorithm>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <type_traits>
 #include <vector>
 
 #include "kernels.h"
+#include "per_device.h"
 
 namespace qfx {
 
@@ -344,15 +344,14 @@ struct Shape {
                   std::uint64_t stride, int batch, const Extra<VARIANT>& g, cudaStream_t s) {
     auto* kernel = cgemm_kernel<BM, BN, BK, TM, TN, STAGES, VARIANT>;
     // Blocks that are resident at once on the current device.
-    static std::once_flag once;
-    static int resident = 152;
-    std::call_once(once, [&] {
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static PerDevice blocks;
+    const int resident = blocks([&] {
+      raise_smem_limit(kernel, smem);
       int dev = 0, sms = 152, per = 1;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, nt, smem);
-      resident = sms * std::max(per, 1);
+      return sms * std::max(per, 1);
     });
     const long long tiles_m = (long long)((m + BM - 1) / BM);
     long long tiles = tiles_m * (long long)((n + BN - 1) / BN) * batch;

@@ -13,11 +13,11 @@
 //
 // The arithmetic is that of the separate kernels: the same gate chains, sums
 // over k in ascending order with four FMAs per complex term.
-#include <mutex>
 #include <string>
 
 #include "flatten.cuh"
 #include "kernels.h"
+#include "per_device.h"
 
 namespace qfx {
 namespace {
@@ -208,10 +208,11 @@ std::size_t small_program_smem(const SmallProgram& p) {
 void launch_small_program(const SmallProgram& p, const std::uint8_t* init_bits, const std::uint8_t* final_bits,
                           double2* amps, int batch, cudaStream_t s) {
   const std::size_t smem = small_program_smem(p);
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice raised;
+  raised([] {
     for (auto* kernel : {small_program_kernel<false>, small_program_kernel<true>})
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SmallProgram::kMaxSmem);
+      raise_smem_limit(kernel, (int)SmallProgram::kMaxSmem);
+    return 1;
   });
   auto run = [&](auto* kernel) {
     kernel<<<(unsigned)batch, NT, smem, s>>>(p, init_bits, final_bits, amps);

@@ -20,10 +20,10 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <mutex>
 #include <string>
 
 #include "half_split.cuh"
+#include "per_device.h"
 #include "tc_common.cuh"
 
 namespace qfx {
@@ -430,11 +430,10 @@ void run_split(const SplitOut& out, const float2* src, std::size_t rows, std::si
     const std::size_t deep = (st.kpad / 16 + ranks - 1) / ranks * 16, bytes = deep * PITCH * sizeof(float2);
     if (deep <= 512) {
       auto* kernel = split_cols_cluster_kernel<NP>;
-      static std::once_flag attr;
-      std::call_once(attr, [&] {
-        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   512 * PITCH * (int)sizeof(float2)),
-              "cudaFuncSetAttribute");
+      static PerDevice raised;
+      raised([&] {
+        raise_smem_limit(kernel, 512 * PITCH * (int)sizeof(float2));
+        return 1;
       });
       cudaLaunchConfig_t lc = {};
       lc.gridDim = dim3((unsigned)((rows + SLAB - 1) / SLAB * ranks), (unsigned)batch, 1);

@@ -62,12 +62,12 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <type_traits>
 #include <vector>
 
 #include "half_split.cuh"
+#include "per_device.h"
 #include "tc_common.cuh"
 #include "tc_gemm.h"
 
@@ -1288,16 +1288,16 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     at[0].val.clusterDim.z = 1;
     lc.attrs = at;
     lc.numAttrs = PAIR ? 1 : 0;
-    static std::once_flag attr;
-    static int resident = 0;  // pairs (SMs pair up within a GPC)
-    std::call_once(attr, [&] {
-      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<KIND, BN, PAIR>::SMEM),
-            "cudaFuncSetAttribute");
+    static PerDevice pairs;  // resident at once (SMs pair up within a GPC)
+    const int resident = pairs([&] {
+      raise_smem_limit(kernel, Layout<KIND, BN, PAIR>::SMEM);
+      int v = 1;
       lc.gridDim = dim3(2, 1, 1);
-      if (PAIR && (cudaOccupancyMaxActiveClusters(&resident, kernel, &lc) != cudaSuccess || resident < 1)) {
+      if (PAIR && (cudaOccupancyMaxActiveClusters(&v, kernel, &lc) != cudaSuccess || v < 1)) {
         cudaGetLastError();
-        resident = (int)persistent_grid(1u << 20) / 2;
+        v = (int)persistent_grid(1u << 20) / 2;
       }
+      return v;
     });
     lc.gridDim = dim3(PAIR ? 2 * (unsigned)std::min<std::size_t>(tiles, (std::size_t)resident) : persistent_grid(tiles),
                       1, 1);

@@ -49,6 +49,7 @@
 #include <string>
 
 #include "kernels.h"
+#include "per_device.h"
 #include "tc_common.cuh"
 #include "tc_gemm.h"
 
@@ -1169,13 +1170,11 @@ void launch_cgemm_tf32x3(const float2* A, const float2* B, BLayout b_layout, flo
   if (cfg.chunk < 1 || cfg.chunk > 64)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> chunk length must be 1..64");
   const int chunk = cfg.chunk;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    check(cudaFuncSetAttribute(cgemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-          "cudaFuncSetAttribute");
-    check(cudaFuncSetAttribute(cgemm_tf32x3_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               P_SMEM_BYTES),
-          "cudaFuncSetAttribute");
+  static PerDevice raised;
+  raised([] {
+    raise_smem_limit(cgemm_tf32x3_kernel, SMEM_BYTES);
+    raise_smem_limit(cgemm_tf32x3_pair_kernel, P_SMEM_BYTES);
+    return 1;
   });
   const bool use_pair = cfg.variant == 1 || (cfg.variant < 0 && m >= 2 * PBM);
   float* pa = workspace;
@@ -1226,19 +1225,14 @@ void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, flo
     throw std::string("ERROR (qflex_gb300: tensor cores) --> chunk length must be 1..64");
   if (a_in_planes && (k < 32 || (k & (k - 1)) != 0 || cfg.chunk > 2))
     throw std::string("ERROR (qflex_gb300: tensor cores) --> A in planes needs k = 2^j >= 32 and chunk <= 2");
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    check(cudaFuncSetAttribute(cgemm_fp16x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-          "cudaFuncSetAttribute");
-    check(cudaFuncSetAttribute(cgemm_fp16x3_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-          "cudaFuncSetAttribute");
-    check(cudaFuncSetAttribute(cgemm_fp16x3_deep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               DEEP_SMEM_BYTES),
-          "cudaFuncSetAttribute");
-    check(cudaFuncSetAttribute(cgemm_fp16x3_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-          "cudaFuncSetAttribute");
-    check(cudaFuncSetAttribute(cgemm_fp16x3_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-          "cudaFuncSetAttribute");
+  static PerDevice raised;
+  raised([] {
+    raise_smem_limit(cgemm_fp16x3_kernel, SMEM_BYTES);
+    raise_smem_limit(cgemm_fp16x3_pair_kernel, SMEM_BYTES);
+    raise_smem_limit(cgemm_fp16x3_deep_kernel, DEEP_SMEM_BYTES);
+    raise_smem_limit(cgemm_fp16x3_wide_kernel, SMEM_BYTES);
+    raise_smem_limit(cgemm_fp16x3_narrow_kernel, SMEM_BYTES);
+    return 1;
   });
   const bool use_pair = cfg.variant == 1 || (cfg.variant < 0 && m >= 2 * BM);
   const std::size_t kpad = (k + 15) / 16 * 16;
@@ -1262,7 +1256,8 @@ void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, flo
     const std::size_t tiles = ((m + 2 * BM - 1) / (2 * BM)) * ((n + BN - 1) / BN) * (std::size_t)batch;
     // As many clusters as can be resident at once (SMs pair up within a
     // GPC), at most one per tile.
-    static const int resident = [] {
+    static PerDevice pairs;
+    const int resident = pairs([] {
       cudaLaunchConfig_t lc = {};
       lc.gridDim = dim3(2, 1, 1);
       lc.blockDim = dim3(THREADS, 1, 1);
@@ -1280,7 +1275,7 @@ void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, flo
         v = (int)persistent_grid(1u << 20) / 2;
       }
       return std::max(1, v);
-    }();
+    });
     const unsigned clusters = (unsigned)std::min<std::size_t>(tiles, (std::size_t)resident);
     cgemm_fp16x3_pair_kernel<<<2 * clusters, THREADS, SMEM_BYTES, s>>>(
         ma, mb, mc, tma_c, C, (int)m, (int)n, (int)k, batch, batch_stride, err, cfg.chunk, ea, eb, a_blocks);
@@ -1323,10 +1318,10 @@ void launch_cgemm_bf16x3(const float2* A, const float2* B, BLayout b_layout, flo
   if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk < 1 || cfg.chunk > 64)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> chunk length must be 1..64");
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    check(cudaFuncSetAttribute(cgemm_bf16x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-          "cudaFuncSetAttribute");
+  static PerDevice raised;
+  raised([] {
+    raise_smem_limit(cgemm_bf16x3_kernel, SMEM_BYTES);
+    return 1;
   });
   const std::size_t kpad = (k + 15) / 16 * 16;
   const std::size_t nb = (std::size_t)batch;

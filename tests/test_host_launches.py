@@ -1,0 +1,32 @@
+"""What the library's host code launches, on a CUDA runtime without a GPU."""
+from tests.fake_cuda import fake_lib, run_fake  # noqa: F401  (fixtures)
+
+
+def test_every_kernel_runs_on_every_device(run_fake):  # noqa: F811
+    """One process, contexts on two devices: whatever runs on the first runs on
+    the second. Limits of dynamic shared memory belong to a device."""
+    run_fake('''
+fake.fake_devices(2)
+products = [(70000, 8, 16), (70000, 16, 16), (70000, 32, 16), (32, 70000, 16), (64, 70000, 16), (70000, 64, 16),
+            (70000, 64, 8), (64, 8, 600), (64, 64, 600), (5000, 12, 100), (3000, 200, 128)]
+splits = [(128, 128, 32), (4096, 64, 256), (4096, 256, 16), (4096, 256, 256), (65536, 32, 128), (512, 9000, 4096),
+          (100, 2048, 64)]
+circuit, grid, ordering = rqc.random_circuit(3, 3, 8, seed=1), rqc.grid_text(3, 3), rqc.row_sweep_ordering(3, 3)
+seen = []
+for device in (0, 1):
+    for precision in (FP32, TF32X3, FP16X3, BF16X3):
+        ctx = Context(device, precision)
+        for m, n, k in products if precision == FP32 else splits:
+            ctx.multiply(A, B, C, m, n, k)
+            ctx.multiply(A, B, C, m, n, k, 3, 1 << 30)
+        ctx.evaluate(circuit, ordering, grid, "0" * 9, "1" * 9, 1 << 40)
+        if precision not in (FP32, TF32X3):
+            ctx.set_option("exact_gates", 0)
+            ctx.evaluate(circuit, ordering, grid, "0" * 9, "1" * 9, 1 << 40)
+        if precision != FP32:
+            for variant in range(1, 5):
+                ctx.set_option("tc_variant", variant)
+                ctx.multiply(A, B, C, 4096, 256, 256)
+    seen.append(kernels())
+assert seen[0] == seen[1] and len(set(seen[0])) > 20, (len(seen[0]), len(seen[1]))
+''')
