@@ -228,7 +228,16 @@ int qflex_gb300_reorder(qflex_gb300_context* ctx, void* data, void* scratch, siz
 /* C[m,n] = A[m,k] * B[k,n], row-major complex64, alpha = 1, beta = 0: the
  * products multiply() hands to cblas_cgemm / cgemv / cdotu_sub
  * (src/tensor.cpp:960-1042). `batch` products at a distance of
- * `batch_stride` elements. */
+ * `batch_stride` elements.
+ *
+ * In a split precision these run on the tensor cores: m, n >= 64 and k >= 16
+ * with n and k powers of two (the sizes of contractions); and, with k >= 96
+ * and m * n * k * batch >= 2^25, any sizes with m, n >= 64 and in 3xFP16 also
+ * those with m >= 256 and 16 <= n < 64. All others run in FP32. The tensor
+ * cores need memory for the planes of B. Where that of all entries cannot be
+ * had, fewer entries run at a time, with the same results; where that of one
+ * entry cannot, the sizes of contractions fail and the others run in FP32,
+ * whose results differ in rounding. */
 int qflex_gb300_multiply(qflex_gb300_context* ctx, const void* A, const void* B, void* C, size_t m,
                          size_t n, size_t k, size_t batch, size_t batch_stride);
 

@@ -286,6 +286,11 @@ void Engine::check_error_flag() {
   }
 }
 
+// Sizes that a contraction gives to the tensor cores.
+static bool contraction_sizes(std::size_t m, std::size_t n, std::size_t k) {
+  return tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
+}
+
 // Whether multiply runs a product on the tensor cores in a split precision:
 // the sizes that contractions have (n and k powers of two), and any others
 // with at least 96 terms, where every split precision is as accurate as FP32
@@ -298,7 +303,7 @@ void Engine::check_error_flag() {
 // 128) 10 and 19, (256, 256, 256) 19 and 23; kernels (2048, 16, 256) 12 and 13,
 // (4096, 32, 128) 9 and 11, (8192, 32, 128) 19 and 11, (16384, 16, 256) 40 and 14.
 bool Engine::split_multiply(std::size_t m, std::size_t n, std::size_t k, int batch) const {
-  if (tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0) return true;
+  if (contraction_sizes(m, n, k)) return true;
   if (k < 96 || double(m) * n * k * batch < double(1 << 25)) return false;
   return narrow_product(m, n, k) || (m >= 64 && n >= 64 && tc_runs(m, n, k));
 }
@@ -308,12 +313,18 @@ void Engine::multiply(const float2* A, const float2* B, float2* C, std::size_t m
   if (is_complex128(precision_))
     throw QFX_ERR("The complex64 tensor operations need a complex64 precision mode (this context is complex128).");
   if (precision_ != FP32 && split_multiply(m, n, k, batch)) {
-    const std::size_t bytes = workspace_elems(m, n, k) * (std::size_t)batch * sizeof(float);
-    // A product that FP32 can run as well needs no more memory than that.
-    const bool contraction = tc_eligible(m, n, k) && (n & (n - 1)) == 0 && (k & (k - 1)) == 0;
-    if (contraction || fits(bytes, 4)) {
-      float* ws = tc_workspace(bytes / sizeof(float));
-      launch_split_product(A, B, BLayout::kn, C, m, n, k, stride, stride, batch, ws);
+    // Where the planes of all entries find no room, fewer entries at a time
+    // (the results are the same); where those of one entry do not, the sizes
+    // that only a multiply has run in FP32, which needs no planes.
+    const std::size_t entry = workspace_elems(m, n, k) * sizeof(float);
+    int piece = batch;
+    void* ws = nullptr;
+    while (piece > 0 && !(ws = try_reserve(entry * (std::size_t)piece, 4))) piece /= 2;
+    if (!ws && contraction_sizes(m, n, k)) ws = tc_workspace(entry / sizeof(float));  // throws
+    if (ws) {
+      for (int b = 0; b < batch; b += piece)
+        launch_split_product(A + b * stride, B + b * stride, BLayout::kn, C + b * stride, m, n, k, stride, stride,
+                             std::min(piece, batch - b), (float*)ws);
       return;
     }
   }
@@ -329,7 +340,7 @@ void Engine::set_stream(cudaStream_t s) {
   stream_ = s;
 }
 
-void* Engine::reserve(std::size_t bytes, int slot) {
+void* Engine::try_reserve(std::size_t bytes, int slot) {
   if ((int)bufs_.size() <= slot) bufs_.resize(slot + 1);
   DevBuf& b = bufs_[slot];
   if (b.bytes < bytes) {
@@ -337,18 +348,22 @@ void* Engine::reserve(std::size_t bytes, int slot) {
     if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
     b.bytes = 0;
-    QFX_CUDA(cudaMalloc(&b.ptr, bytes));
+    const cudaError_t e = cudaMalloc(&b.ptr, bytes);
+    if (e != cudaSuccess) b.ptr = nullptr;
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // the next launch is not to report it
+      return nullptr;
+    }
+    QFX_CUDA(e);
     b.bytes = bytes;
   }
   return b.ptr;
 }
 
-bool Engine::fits(std::size_t bytes, int slot) const {
-  const std::size_t have = (int)bufs_.size() > slot ? bufs_[slot].bytes : 0;
-  if (have >= bytes) return true;
-  std::size_t free_b = 0, total_b = 0;
-  QFX_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  return bytes < free_b + have;
+void* Engine::reserve(std::size_t bytes, int slot) {
+  void* p = try_reserve(bytes, slot);
+  if (!p) throw cuda_error_string(cudaErrorMemoryAllocation, "cudaMalloc(&b.ptr, bytes)");
+  return p;
 }
 
 const std::vector<GemmShape>& Engine::last_shapes() const {

@@ -132,11 +132,11 @@ class Engine {
   TcConfig tc_config(std::size_t m, std::size_t n, std::size_t k) const;
   bool direct_product(std::size_t m, std::size_t n, std::size_t k, const TcConfig& cfg) const;
   bool split_multiply(std::size_t m, std::size_t n, std::size_t k, int batch) const;
-  // fp32 elements of split planes that one product of this shape needs.
   bool narrow_product(std::size_t m, std::size_t n, std::size_t k) const;
+  // fp32 elements of split planes that one product of this shape needs.
   std::size_t workspace_elems(std::size_t m, std::size_t n, std::size_t k) const;
-  // Whether device buffer `slot` holds `bytes` or can be made to.
-  bool fits(std::size_t bytes, int slot) const;
+  // Device buffer `slot` of at least `bytes`; null when the device has no room.
+  void* try_reserve(std::size_t bytes, int slot);
   // C = A * B on the tensor cores in the context's split precision.
   void launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
                             std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride, int batch,

@@ -17,7 +17,7 @@
 namespace {
 
 int g_devices = 1, g_current = 0;
-size_t g_free = size_t(64) << 30;
+size_t g_free = size_t(64) << 30, g_largest = ~size_t(0);
 cudaError_t g_last = cudaSuccess;
 std::string g_log;
 std::map<const void*, std::string> g_names;
@@ -62,6 +62,7 @@ extern "C" {
 // ---- what tests set and read ----
 void fake_devices(int n) { g_devices = n; }
 void fake_memory(size_t bytes) { g_free = bytes; }
+void fake_largest_block(size_t bytes) { g_largest = bytes; }
 void fake_capturing(void* stream, int on) {
   if (on)
     g_capturing.insert(stream);
@@ -153,7 +154,7 @@ cudaError_t cudaGetSymbolAddress(void** p, const void*) {
 
 // ---- memory ----
 cudaError_t cudaMalloc(void** p, size_t bytes) {
-  if (bytes > g_free) {
+  if (bytes > g_free || bytes > g_largest) {
     line("malloc %zu failed", bytes);
     return set(cudaErrorMemoryAllocation);
   }

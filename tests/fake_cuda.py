@@ -19,7 +19,7 @@ from qflex_gb300 import *
 from qflex_gb300 import rqc
 fake = _lib.load_library()
 fake.fake_log.restype = ctypes.c_char_p
-fake.fake_memory.argtypes = [ctypes.c_size_t]
+fake.fake_memory.argtypes = fake.fake_largest_block.argtypes = [ctypes.c_size_t]
 fake.fake_capturing.argtypes = [ctypes.c_void_p, ctypes.c_int]
 def log():
     "The runtime's calls since the last time, without stream and event creation."

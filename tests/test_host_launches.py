@@ -30,3 +30,40 @@ for device in (0, 1):
     seen.append(kernels())
 assert seen[0] == seen[1] and len(set(seen[0])) > 20, (len(seen[0]), len(seen[1]))
 ''')
+
+
+def test_multiply_without_room_for_planes(run_fake):  # noqa: F811
+    """A multiply of sizes that no contraction has takes its planes' memory
+    when it can be had; otherwise fewer entries at a time, and FP32 when those
+    of one entry find no room. Free memory that comes in no large enough piece
+    is no error, and neither is what follows."""
+    run_fake('''
+m, n, k, batch = 1000, 700, 1100, 6
+entry = 4 * (2 * n * 1104 + 2 * n)  # planes, scales and largest components of B
+for limit in (fake.fake_largest_block, fake.fake_memory):
+    for room, piece in ((1 << 40, 6), (6 * entry, 6), (3 * entry, 3), (entry, 1), (entry - (1 << 16), 0), (1 << 20, 0)):
+        ctx = Context(0, FP16X3)
+        ctx.multiply(A, B, C, 4, 4, 4)  # the context's FP32 scratch and control block exist
+        ctx.multiply(A, B, C, 64, 64, 16)
+        log()
+        limit(room)
+        ctx.multiply(A, B, C, m, n, k, batch, 1 << 30)
+        names = kernels()
+        direct = [x for x in names if x.startswith("cgemm_direct_kernel")]
+        fp32 = [x for x in names if x.startswith("cgemm_kernel")]
+        assert (len(direct), len(fp32)) == ((-(-batch // piece), 0) if piece else (0, 1)), (room, names)
+        ctx.multiply(A, B, C, 70000, 64, 5)
+        ctx.synchronize()
+        limit(1 << 40)
+        # Sizes of contractions have no other way.
+        limit(1 << 16)
+        try:
+            ctx.multiply(A, B, C, 4096, 4096, 4096)
+            raise SystemExit("no error")
+        except QflexGb300Error as e:
+            assert e.code == 2 and "out of memory" in str(e), str(e)
+        limit(1 << 40)
+        ctx.multiply(A, B, C, 4096, 4096, 4096)
+        assert kernels()[-1].startswith("cgemm_direct_kernel")
+        ctx.close()
+''')
