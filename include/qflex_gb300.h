@@ -237,7 +237,14 @@ int qflex_gb300_reorder(qflex_gb300_context* ctx, void* data, void* scratch, siz
  * cores need memory for the planes of B. Where that of all entries cannot be
  * had, fewer entries run at a time, with the same results; where that of one
  * entry cannot, the sizes of contractions fail and the others run in FP32,
- * whose results differ in rounding. */
+ * whose results differ in rounding.
+ *
+ * Operands keep 22 bits in 3xFP16 and 3xTF32 and 24 in BF16x3; 3xFP16 counts
+ * its bits from the largest component of 32 values of a row of A (or of the
+ * whole row) and of a column of B, so that components 2^17 below it lose bits
+ * and those 2^39 below it vanish. An infinity makes its products NaN at the
+ * sizes of contractions; a product of the other sizes that meets infinities,
+ * NaN or overflow runs again in FP32. */
 int qflex_gb300_multiply(qflex_gb300_context* ctx, const void* A, const void* B, void* C, size_t m,
                          size_t n, size_t k, size_t batch, size_t batch_stride);
 

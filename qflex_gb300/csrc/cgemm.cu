@@ -71,17 +71,17 @@ __device__ __forceinline__ void copy16(float2* dst, const float2* src, bool real
 // so that the rows a quarter-warp reads start in different banks.
 constexpr int a_row(int BK) { return BK + 2; }
 
-// What one variant of the kernel takes besides the matrices: a gather, or the
-// split of k (`splits` runs of `terms`, whose sums go to `partial` as
-// [entry][split][m][n]); nothing for the others, whose launches it would slow.
+// What one variant of the kernel takes besides the matrices, no more, since a
+// larger argument slows the launch: a gather, the split of k (`splits` runs of
+// `terms`, whose sums go to `partial` as [entry][split][m][n]), or the
+// condition under which it does anything.
 struct SplitK {
   float2* partial;
   int splits, terms;
 };
-struct Nothing {};
 enum Variant { PLAIN, GATHERED, SPLIT };
 template <int VARIANT>
-using Extra = std::conditional_t<VARIANT == GATHERED, TileGather, std::conditional_t<VARIANT == SPLIT, SplitK, Nothing>>;
+using Extra = std::conditional_t<VARIANT == GATHERED, TileGather, std::conditional_t<VARIANT == SPLIT, SplitK, OnlyIf>>;
 
 template <int BM, int BN, int BK, int TM, int TN, int STAGES, int VARIANT>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
@@ -96,6 +96,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   constexpr int A_ELEMS = BM * AR, STAGE = A_ELEMS + BK * BN;
   static_assert(LA * NT == BM * BK && BK % 2 == 0 && TN % 2 == 0, "tile / threads mismatch");
   extern __shared__ __align__(16) float2 ring[];
+  if constexpr (VARIANT == PLAIN)
+    if (g.flag && *g.flag != g.value) return;
   const int t = threadIdx.x;
   const int tx = t % TX, ty = t / TX;
   int ktiles = k > 0 ? (k + BK - 1) / BK : 1;  // no terms: one k-step of zeros
@@ -330,6 +332,19 @@ __global__ void __launch_bounds__(256) split_finish_kernel(const float2* __restr
   C[blockIdx.y * batch_stride + at] = make_float2(float(sum.x), float(sum.y));
 }
 
+// Sets *flag to `value` when an element of a product is no finite number.
+__global__ void __launch_bounds__(256) flag_not_finite_kernel(const float2* __restrict__ C, std::uint64_t outputs,
+                                                              std::uint64_t batch_stride, int* flag, int value) {
+  C += blockIdx.y * batch_stride;
+  float zero = 0.f;  // NaN once an infinity or NaN was met
+  for (std::uint64_t i = std::uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < outputs;
+       i += std::uint64_t(gridDim.x) * blockDim.x) {
+    const float2 v = C[i];
+    zero = fmaf(v.x, 0.f, fmaf(v.y, 0.f, zero));
+  }
+  if (zero != 0.f) atomicExch(flag, value);
+}
+
 struct Tile {
   int bm, bn, bk, threads;
 };
@@ -369,11 +384,11 @@ struct Shape {
     if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch cgemm) --> ") + cudaGetErrorString(e);
   }
   static void launch(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
-                     std::uint64_t stride, int batch, const TileGather* g, cudaStream_t s) {
+                     std::uint64_t stride, int batch, const TileGather* g, OnlyIf only_if, cudaStream_t s) {
     if (g)
       run<GATHERED>(A, B, C, m, n, k, stride, batch, *g, s);
     else
-      run<PLAIN>(A, B, C, m, n, k, stride, batch, Nothing{}, s);
+      run<PLAIN>(A, B, C, m, n, k, stride, batch, only_if, s);
   }
 };
 
@@ -393,6 +408,14 @@ auto with_shape(std::size_t m, std::size_t n, std::size_t k, F&& f) {
 }
 
 }  // namespace
+
+void launch_flag_not_finite(const float2* C, std::size_t outputs, std::uint64_t batch_stride, int batch, int* flag,
+                            int value, cudaStream_t s) {
+  dim3 grid((unsigned)std::min<std::size_t>((outputs + 1023) / 1024, 152 * 8), (unsigned)batch);
+  flag_not_finite_kernel<<<grid, 256, 0, s>>>(C, outputs, batch_stride, flag, value);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch flag_not_finite) --> ") + cudaGetErrorString(e);
+}
 
 bool make_tile_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::size_t n, std::size_t k, TileGather* g) {
   const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
@@ -469,7 +492,7 @@ void tile_gather_on_host(const TileGather& g, std::size_t m, std::size_t n, std:
 
 void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
                         std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, float2* scratch,
-                        cudaStream_t s) {
+                        cudaStream_t s, OnlyIf only_if) {
   if (m > 0x7fffffffull || n > 0x7fffffffull || k > 0x7fffffffull)
     throw std::string("ERROR (qflex_gb300: cgemm) --> dimension exceeds 2^31");
   // Few tiles: a product is then as long as one tile's chain of k-steps. Small
@@ -491,7 +514,7 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
       std::size_t splits = scratch ? std::min<std::size_t>(304 / own, k / 64) : 1;
       splits = std::min<std::size_t>(splits, kSkinnyScratchElems / (m * n * (std::size_t)batch));
       if (splits < 3) {
-        S::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, Nothing{}, s);
+        S::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, only_if, s);
         return 0;
       }
       const std::size_t terms = ((k + splits - 1) / splits + t.bk - 1) / t.bk * t.bk;
@@ -516,14 +539,14 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
   // 51.2, (92, 717, 148) x 7 37.2 and 34.7).
   if (!gather && n > 8 && tiles <= (n <= 32 ? 304u : 152u)) {
     auto plain = [&](auto shape) {
-      decltype(shape)::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, Nothing{}, s);
+      decltype(shape)::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, only_if, s);
     };
     if (n <= 16) return plain(Shape<64, 16, 16, 4, 2, 4>{});
     if (n <= 32) return plain(Shape<64, 32, 16, 4, 4, 3>{});
     if (m > 64 && k >= 128) return plain(Shape<128, 64, 32, 8, 4, 2>{});
   }
   with_shape(m, n, k, [&](auto shape) {
-    decltype(shape)::launch(A, B, C, m, n, k, batch_stride, batch, gather, s);
+    decltype(shape)::launch(A, B, C, m, n, k, batch_stride, batch, gather, only_if, s);
     return 0;
   });
 }

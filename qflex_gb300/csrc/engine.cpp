@@ -233,20 +233,23 @@ std::size_t Engine::workspace_elems(std::size_t m, std::size_t n, std::size_t k)
 
 void Engine::launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
                                   std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride,
-                                  int batch, float* ws) {
+                                  int batch, float* ws, int watch) {
   const TcConfig cfg = tc_config(m, n, k);
   if (direct_product(m, n, k, cfg)) {
     const bool aligned = (reinterpret_cast<std::uintptr_t>(A) & 15) == 0 && k % 2 == 0 &&
                          (batch == 1 || ac_stride % 2 == 0);
     launch_cgemm_direct(split_kind(precision_), A, make_a_rows(k, aligned), B, b_layout, C, m, n, k, ac_stride,
-                        b_stride, batch, ws, error_flag(), cfg, stream_);
-  } else if (precision_ == FP16X3) {
+                        b_stride, batch, ws, error_flag(), cfg, stream_, watch);
+    return;
+  }
+  if (precision_ == FP16X3) {
     launch_cgemm_fp16x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
   } else if (precision_ == BF16X3) {
     launch_cgemm_bf16x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
   } else {
     launch_cgemm_tf32x3(A, B, b_layout, C, m, n, k, ac_stride, b_stride, batch, ws, error_flag(), cfg, stream_);
   }
+  if (watch) launch_flag_not_finite(C, m * n, ac_stride, batch, error_flag() + 4, watch, stream_);
 }
 
 TcConfig Engine::tc_config(std::size_t m, std::size_t n, std::size_t k) const {
@@ -257,13 +260,14 @@ TcConfig Engine::tc_config(std::size_t m, std::size_t n, std::size_t k) const {
 }
 
 int* Engine::error_flag() {
-  // The context's control block for the tensor-core kernels, int[4]: the
+  // The context's control block for the tensor-core kernels, int[8]: the
   // error code they set, the truncation-bias compensation switch, then
-  // (bytes 8..15) the limit of their pipeline waits in ns (0: 2 s).
-  const bool fresh = (int)bufs_.size() <= 5 || bufs_[5].bytes < 4 * sizeof(int);
-  int* p = (int*)reserve(sizeof(int) * 4, 5);
+  // (bytes 8..15) the limit of their pipeline waits in ns (0: 2 s), and the
+  // number of the last watched product with a sum that is no finite number.
+  const bool fresh = (int)bufs_.size() <= 5 || bufs_[5].bytes < 8 * sizeof(int);
+  int* p = (int*)reserve(sizeof(int) * 8, 5);
   if (fresh) {
-    int init[4] = {0, debias_ ? 1 : 0, 0, 0};
+    int init[8] = {0, debias_ ? 1 : 0};
     std::memcpy(init + 2, &wait_ns_, sizeof(wait_ns_));
     QFX_CUDA(cudaMemcpyAsync(p, init, sizeof(init), cudaMemcpyHostToDevice, stream_));
     QFX_CUDA(cudaStreamSynchronize(stream_));
@@ -322,9 +326,16 @@ void Engine::multiply(const float2* A, const float2* B, float2* C, std::size_t m
     while (piece > 0 && !(ws = try_reserve(entry * (std::size_t)piece, 4))) piece /= 2;
     if (!ws && contraction_sizes(m, n, k)) ws = tc_workspace(entry / sizeof(float));  // throws
     if (ws) {
+      // An infinity has no rest to split off, so that its products become NaN;
+      // a value next to the largest ones rounds to infinity. Where the sizes
+      // allow FP32, a product with such a sum runs again there.
+      int watch = 0;
+      if (!contraction_sizes(m, n, k)) watch = watched_ = watched_ % 0x7fffffff + 1;
       for (int b = 0; b < batch; b += piece)
         launch_split_product(A + b * stride, B + b * stride, BLayout::kn, C + b * stride, m, n, k, stride, stride,
-                             std::min(piece, batch - b), (float*)ws);
+                             std::min(piece, batch - b), (float*)ws, watch);
+      if (watch)
+        launch_cgemm_tiled(A, nullptr, B, C, m, n, k, stride, batch, nullptr, stream_, {error_flag() + 4, watch});
       return;
     }
   }

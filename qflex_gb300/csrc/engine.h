@@ -137,10 +137,13 @@ class Engine {
   std::size_t workspace_elems(std::size_t m, std::size_t n, std::size_t k) const;
   // Device buffer `slot` of at least `bytes`; null when the device has no room.
   void* try_reserve(std::size_t bytes, int slot);
-  // C = A * B on the tensor cores in the context's split precision.
+  // C = A * B on the tensor cores in the context's split precision. With
+  // `watch` != 0 the control block takes that number when a sum is no finite
+  // number.
   void launch_split_product(const float2* A, const float2* B, BLayout b_layout, float2* C, std::size_t m,
                             std::size_t n, std::size_t k, std::uint64_t ac_stride, std::uint64_t b_stride, int batch,
-                            float* ws);
+                            float* ws, int watch = 0);
+  int watched_ = 0;  // number of the last watched product
   std::vector<cudaEvent_t> prof_events_;
   std::vector<double> op_ms_;
   std::unique_ptr<Plan> plan_;

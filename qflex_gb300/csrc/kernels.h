@@ -159,11 +159,22 @@ bool make_tile_gather(int nbits, const std::uint8_t* perm, std::size_t m, std::s
 // operand that the product sees. Tests use it.
 void tile_gather_on_host(const TileGather& g, std::size_t m, std::size_t n, std::size_t k, const float2* src,
                          float2* dst);
+// A condition on the device: *flag == value when the kernel starts (always
+// true without a flag).
+struct OnlyIf {
+  const int* flag = nullptr;
+  int value = 0;
+};
 // The tiled product, A row-major or (gather not null) through a permutation.
-// Products of few tiles split k when they have `scratch` (kSkinnyScratchElems).
+// Products of few tiles split k when they have `scratch` (kSkinnyScratchElems);
+// a product under a condition has neither a gather nor scratch.
 void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
                         std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, float2* scratch,
-                        cudaStream_t s);
+                        cudaStream_t s, OnlyIf only_if = {});
+// Sets *flag to `value` when one of `outputs` elements per entry of C is an
+// infinity or NaN.
+void launch_flag_not_finite(const float2* C, std::size_t outputs, std::uint64_t batch_stride, int batch, int* flag,
+                            int value, cudaStream_t s);
 
 // One skinny product (m * n outputs) with k split over `splits` blocks per
 // output; `partial` holds m * n * splits float2, every one of which is

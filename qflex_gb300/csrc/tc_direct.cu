@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ AGather g,
                                const float2* __restrict__ A, float2* __restrict__ C, int tma_c, int m, int n, int k,
                                int batches, std::uint64_t ac_stride, int* __restrict__ err,
-                               const int* __restrict__ exp_b) {
+                               const int* __restrict__ exp_b, int watch) {
   using L = Layout<KIND, BN, PAIR>;
   constexpr int B_STAGES = L::B_STAGES, DONE = L::DONE, HALVES = L::HALVES, TMEM_A_BLOCK = L::TMEM_A_BLOCK;
   constexpr int A_RING = L::A_RING, B_PART = L::B_PART, B_STAGE = L::B_STAGE, TMEM_A = L::TMEM_A, COLS = L::COLS;
@@ -868,6 +868,16 @@ __global__ void __launch_bounds__(THREADS, 1)
         re[j] = fma2(re[j], beta2, re[j]);
         im[j] = fma2(im[j], beta2, im[j]);
       }
+      if (watch) {
+        float2 z[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // NaN once a sum is no number
+#pragma unroll
+        for (int j = 0; j < COLS / 2; ++j) {
+          z[0] = fma2(re[j], make_float2(0.f, 0.f), z[0]);
+          z[1] = fma2(im[j], make_float2(0.f, 0.f), z[1]);
+        }
+        const float zero = (z[0].x + z[0].y) + (z[1].x + z[1].y);
+        if (__any_sync(0xffffffffu, zero != 0.f) && lane == 0) atomicExch(err + 4, watch);
+      }
       float2* cb = C + std::uint64_t(batch) * ac_stride;
       // Boxes of 32 rows x 16 complex, the warp's slots in turn. (Boxes of 8
       // columns: twice the fences and barriers, a tile's store took 7200
@@ -1209,7 +1219,7 @@ std::size_t tc_direct_workspace_elems(SplitKind kind, std::size_t n, std::size_t
 void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather, const float2* B, BLayout b_layout,
                          float2* C, std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
                          std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
-                         cudaStream_t s) {
+                         cudaStream_t s, int watch) {
   if (!tc_runs(m, n, k)) throw std::string("ERROR (qflex_gb300: tensor cores) --> shape not eligible");
   if (cfg.chunk != 2)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct product takes chunks of 2 k-steps");
@@ -1221,7 +1231,7 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
       for (int at = 0; at < batch; at += (int)most)
         launch_cgemm_direct(kind, A + at * ac_stride, gather, B + at * b_stride, b_layout, C + at * ac_stride, m, n, k,
                             ac_stride, b_stride, (int)std::min<std::uint64_t>(most, batch - at), workspace, err, cfg,
-                            s);
+                            s, watch);
       return;
     }
   }
@@ -1302,7 +1312,7 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     lc.gridDim = dim3(PAIR ? 2 * (unsigned)std::min<std::size_t>(tiles, (std::size_t)resident) : persistent_grid(tiles),
                       1, 1);
     check(cudaLaunchKernelEx(&lc, kernel, ma, mb, mb2, mc, gather, A, C, tma_c, (int)m, (int)n, (int)k, batch, ac_stride, err,
-                             (const int*)eb),
+                             (const int*)eb, watch),
           "cgemm_direct");
   };
   using std::integral_constant;

@@ -124,11 +124,12 @@ std::size_t tc_direct_workspace_elems(SplitKind kind, std::size_t n, std::size_t
 // The split product with A split inside the kernel: A is read as
 // complex64 through `gather` (3xFP16: every 32 values of a row scaled by their
 // own power of two), and no A planes exist in memory. cfg.chunk 2 (a TMEM chunk
-// is one of A's blocks); cfg.variant is ignored.
+// is one of A's blocks); cfg.variant is ignored. With `watch` != 0 err[4] takes
+// that value when a sum is an infinity or NaN.
 void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather, const float2* B, BLayout b_layout,
                          float2* C, std::size_t m, std::size_t n, std::size_t k, std::uint64_t ac_stride,
                          std::uint64_t b_stride, int batch, float* workspace, int* err, const TcConfig& cfg,
-                         cudaStream_t s);
+                         cudaStream_t s, int watch = 0);
 
 // The same product with BF16x3 planes: x = b0 + b1 + b2 in BF16 (no
 // scaling: BF16 has the FP32 exponent range), six products per real

@@ -91,3 +91,58 @@ def test_abandoned_products(built_lib, precision, m, n, k):
         ctx.synchronize()
         # Bound as for test_block_exponents, k <= 400 (3xTF32: chunks of 16 terms).
         assert float(((C - want).abs() / bound).max()) < 8e-6
+
+
+def _parts(A, B):
+    """Real and imaginary part of A B by products of real matrices in 64 bits:
+    where they have infinities and NaN."""
+    a, b = A.cdouble(), B.cdouble()
+    return a.real @ b.real - a.imag @ b.imag, a.real @ b.imag + a.imag @ b.real
+
+
+@pytest.mark.parametrize("precision,m,n,k,batch,options", [
+    (FP32, 300, 70, 161, 3, {}), (FP32, 40, 30, 700, 2, {}), (FP32, 70000, 16, 19, 1, {}), (FP32, 20, 600, 9, 1, {}),
+    (FP16X3, 640, 500, 161, 1, {}), (FP16X3, 3001, 70, 200, 2, {}), (FP16X3, 40000, 17, 100, 1, {}),
+    (FP16X3, 100, 2051, 255, 2, {}), (FP16X3, 640, 500, 161, 1, {"tc_chunk": 1}),
+    (TF32X3, 640, 500, 161, 1, {}), (TF32X3, 100, 2051, 255, 2, {}), (BF16X3, 640, 500, 161, 1, {}),
+    (BF16X3, 100, 2051, 255, 2, {})])
+@pytest.mark.parametrize("case", ["inf_a", "inf_b", "nan_a", "nan_b", "largest", "none"])
+def test_infinities_and_nan(built_lib, precision, m, n, k, batch, options, case):
+    """Sizes that only a multiply has: infinities stay infinities and reach no
+    other element, also next to values that round to infinity in fewer bits."""
+    import torch
+    A, B = randn((batch, m, k), k), randn((batch, k, n), n)
+    if case == "inf_a":
+        A[-1, m - 1, k - 1] = complex(float("inf"), 1)
+    elif case == "inf_b":
+        B[0, 3, n - 2] = complex(2, -float("inf"))
+        B[0, 5, n - 2] = complex(-1, -float("inf"))
+    elif case == "nan_a":
+        A[0, 5, 7] = complex(0, float("nan"))
+    elif case == "nan_b":
+        B[-1, k - 1, 0] = complex(float("nan"), 0)
+    elif case == "largest":
+        A[0, 2, 1] = 3.4028234e38
+        B *= 2.0 ** -40
+    buf = torch.zeros((batch, m * k + k * n + m * n), dtype=torch.complex64, device="cuda")
+    buf[:, :m * k] = A.reshape(batch, -1)
+    buf[:, m * k:m * k + k * n] = B.reshape(batch, -1)
+    torch.cuda.synchronize()
+    ctx = Context(0, precision)
+    for name, value in options.items():
+        ctx.set_option(name, value)
+    at = buf.data_ptr()
+    for again in range(2):  # a product without them afterwards is not run twice
+        ctx.multiply(at, at + 8 * m * k, at + 8 * (m * k + k * n), m, n, k, batch, buf.shape[1])
+        ctx.synchronize()
+    for a, b, row in zip(A, B, buf):
+        c = row[m * k + k * n:].view(m, n)
+        for got, want in zip((c.real, c.imag), _parts(a, b)):
+            assert torch.equal(got.isnan(), want.isnan())
+            assert torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+        good = c.isfinite()
+        # 2 k additions of each part at 2^-24, and as for test_block_exponents.
+        tol = 2 * k * 2.0 ** -24 * 2 ** 0.5 + 6e-6
+        want, bound = (x.nan_to_num(0, 0, 0) for x in (a.to(torch.complex128) @ b.to(torch.complex128),
+                                                      a.abs().double() @ b.abs().double()))
+        assert float((torch.where(good, c.to(torch.complex128) - want, 0).abs() / (bound + 1e-300))[good].max()) < tol
