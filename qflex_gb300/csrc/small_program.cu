@@ -12,7 +12,8 @@
 // 152, 548 -> 343 us for 1024.
 //
 // The arithmetic is that of the separate kernels: the same gate chains, sums
-// over k in ascending order with four FMAs per complex term.
+// over k in ascending order with four FMAs per complex term, and in products
+// of vectors the same partial sums added in the same order.
 #include <string>
 
 #include "flatten.cuh"
@@ -74,6 +75,47 @@ __device__ __forceinline__ void tile_product(const float2* A, const float2* B, f
       for (int j = 0; j < TN; ++j)
         if (c0 + j < n) C[r * n + c0 + j] = acc[i][j];
     }
+  }
+}
+
+__device__ __forceinline__ float2 warp_sum(float2 v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
+
+// Products with one column (m x k times a vector of more than 32) or one row
+// (of up to 255 columns): a warp per output, as the separate kernels for
+// vectors sum them (gemv_rows_warp, gemv_cols_block). One thread per output
+// would add up to 1024 terms one after the other.
+__device__ __forceinline__ void column_product(const float2* A, const float2* B, float2* C, int m, int k) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int i = threadIdx.x >> 5; i < m; i += NT / 32) {
+    float2 acc = make_float2(0.f, 0.f);
+    for (int kk = lane; kk < k; kk += 32) acc = cfma(A[i * k + kk], B[kk], acc);
+    acc = warp_sum(acc);
+    if (lane == 0) C[i] = acc;
+  }
+}
+__device__ __forceinline__ void row_product(const float2* A, const float2* B, float2* C, int n, int k) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int j = threadIdx.x >> 5; j < n; j += NT / 32) {
+    // The sums of eight warps of which each takes 32 terms in turn.
+    float2 part = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int w = 0; w < 8 && 32 * w < k; ++w) {
+      float2 acc = make_float2(0.f, 0.f);
+      for (int kk = 32 * w + lane; kk < k; kk += 256) acc = cfma(A[kk], B[kk * n + j], acc);
+      acc = warp_sum(acc);
+      if (lane == w) part = acc;
+    }
+    part = warp_sum(part);
+    if (lane == 0) C[j] = part;
   }
 }
 
@@ -173,7 +215,11 @@ __global__ void __launch_bounds__(NT, 1)
       // two rows per thread 7300.)
       const int cols4 = (n + 3) / 4, rows4 = (m + 3) / 4;
       const bool even = ((op.b | op.c | n) & 1) == 0;
-      if (m * n >= 2048) {
+      if (n == 1 && k > 32) {
+        column_product(A, B, C, m, k);
+      } else if (m == 1 && n > 1 && n < 256) {
+        row_product(A, B, C, n, k);
+      } else if (m * n >= 2048) {
         for (int i = t; i < rows4 * cols4; i += NT)
           tile_product<4, 4>(A, B, C, m, n, k, i / cols4, rows4, i % cols4 * 4, even, col, row);
       } else if (m * n >= 512) {
