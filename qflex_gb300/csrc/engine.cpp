@@ -38,6 +38,17 @@ struct GraphKey {
   }
 };
 
+// What a string of a small program takes.
+struct SmallCost {
+  double ops = 0;            // operations
+  double multiply_adds = 0;  // complex ones of all products
+  double moved = 0;          // elements of all permutations
+  double gates = 0;          // applied, over all elements of the grid tensors
+  double gate_lanes = 0;     // the same with every column in pieces of 128 elements
+  double longest = 0;        // gates of the longest column
+  bool compensated = false;  // gate chains in float-float
+};
+
 struct Engine::Plan {
   std::string key;
   Circuit circuit;
@@ -71,6 +82,7 @@ struct Engine::Plan {
   std::uint32_t* d_leaves = nullptr;
   // The program as one kernel, when it is small (small.n_ops != 0).
   SmallProgram small = {};
+  SmallCost small_cost;
   SmallOp* d_small_ops = nullptr;
   // Captured device pass and the buffers it was captured with.
   cudaGraphExec_t graph = nullptr;
@@ -492,15 +504,10 @@ T* upload(const std::vector<T>& v) {
 namespace {
 
 // The ops of a program as the one-kernel form takes them; empty when it does
-// not. A block runs its string's operations one after the other, at about 9
-// complex multiply-adds a cycle (256 x 16 x 16: 7000 cycles, 3.7 us) plus
-// 0.4 us per operation, against 3.3 us for the launch of an operation of its
-// own: the line lies where the average operation takes as long either way.
+// not.
 std::vector<SmallOp> small_ops(const Program& prog) {
-  constexpr double kFlopPerOp = 400e3;
   std::vector<SmallOp> out;
-  if (prog.arena_elems * sizeof(float2) > SmallProgram::kMaxSmem || prog.gemm_flop > kFlopPerOp * prog.ops.size())
-    return out;
+  if (prog.arena_elems * sizeof(float2) > SmallProgram::kMaxSmem) return out;
   for (const DevOp& op : prog.ops) {
     SmallOp s{};
     s.a = (std::uint32_t)op.a;
@@ -523,6 +530,29 @@ std::vector<SmallOp> small_ops(const Program& prog) {
     out.push_back(s);
   }
   return out;
+}
+
+// Whether `batch` strings of a program run faster as one kernel, by estimates
+// of both forms' device time in us. A block runs a string's gate chains and
+// operations one after the other and has an SM to itself, so a chip full of
+// strings takes as long as one; the separate kernels share their launches among
+// all strings, and the host takes 15 us longer to replay them. Fitted to 70
+// row-sweep programs of 2 x 2 to 5 x 6 sites with 1 to 4096 strings, with plain
+// and with compensated gate chains: the estimates miss by 6 % (standard
+// deviation), and choosing by them costs 0.4 % of the device time against
+// always the faster form, where one kernel for all costs 1 (plain) and 14 %.
+// Gate chains weigh most: 2 x 3 sites of depth 32, one string in 3xFP16, take
+// 293 us as one kernel and 53 separate.
+bool one_kernel_faster(const SmallCost& c, int batch) {
+  const double waves = (batch + 151) / 152;
+  const double work = 0.39 * c.ops + 4.65e-5 * c.multiply_adds + 9.7e-4 * c.moved;
+  const double one = 6.3 + waves * (c.compensated ? 6.2 + work + 1.17e-3 * c.gate_lanes : 3.2 + work + 1.22e-4 * c.gate_lanes);
+  const double separate =
+      c.compensated ? 2.5 + 2.2 * c.ops + 0.85 * c.longest + 5.2e-5 * c.multiply_adds +
+                          batch * (4.36e-3 * c.ops + 1.0e-7 * c.multiply_adds + 9.68e-6 * c.gates)
+                    : 3.7 + 2.2 * c.ops + 0.43 * c.longest + 3.8e-5 * c.multiply_adds +
+                          batch * (3.7e-3 * c.ops + 1.5e-7 * c.multiply_adds + 2.19e-6 * c.gates);
+  return one < 0.9 * separate + 15;
 }
 
 bool overlaps(std::size_t a0, std::size_t a1, std::size_t b0, std::size_t b1) { return a0 < b1 && b0 < a1; }
@@ -800,6 +830,17 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
         p.small.arena_elems = (std::uint32_t)p.prog.arena_elems;
         p.small.results = (std::uint32_t)p.prog.results_offset;
         if (small_program_smem(p.small) > SmallProgram::kMaxSmem) p.small.n_ops = 0;
+        SmallCost& cost = p.small_cost;
+        cost.ops = double(small.size());
+        cost.multiply_adds = p.prog.gemm_flop / 8;
+        cost.moved = p.prog.permute_bytes / 16;
+        cost.compensated = p.d_mats_lo != nullptr;
+        for (const ColumnDesc& c : cols) {
+          const double gates = c.step_end - c.step_begin;
+          cost.gates += std::ldexp(gates, (int)c.size_log2);
+          cost.gate_lanes += std::ldexp(gates, std::max((int)c.size_log2, 7));
+          cost.longest = std::max(cost.longest, gates);
+        }
       }
     }
     p.built = true;
@@ -851,8 +892,9 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
 
   // How many final states fit on the device at once. A program that runs as
   // one kernel keeps its tensors in shared memory.
-  const bool small = p.small.n_ops != 0 && !profile_;
   int chunk = std::min(total, 65535);
+  const bool small = p.small.n_ops != 0 && !profile_ &&
+                     one_kernel_faster(p.small_cost, max_batch_ > 0 ? std::min(chunk, max_batch_) : chunk);
   float2* arena = nullptr;
   float* tc_ws = nullptr;
   if (!small) {

@@ -68,3 +68,31 @@ for limit in (fake.fake_largest_block, fake.fake_memory):
         assert kernels()[-1].startswith("cgemm_direct_kernel")
         ctx.close()
 ''')
+
+
+def test_one_kernel_or_separate_kernels(run_fake):  # noqa: F811
+    """Which form a small program takes depends on the strings of a call and on
+    its gate chains: separate kernels where one SM would be the slower (each of
+    these was measured in both forms)."""
+    run_fake('''
+from qflex_gb300 import FP16X3, FP32
+for (rows, cols, depth), precision, strings, one in [
+        ((4, 5, 16), FP32, 1, True), ((4, 5, 16), FP16X3, 1, True), ((4, 5, 16), FP32, 152, True),
+        ((4, 5, 16), FP32, 4096, False), ((4, 5, 16), FP16X3, 1024, False), ((2, 3, 32), FP32, 1, False),
+        ((2, 3, 32), FP16X3, 1, False), ((2, 3, 32), FP16X3, 32, False), ((2, 3, 32), FP16X3, 152, True),
+        ((2, 3, 32), FP32, 4096, True), ((3, 3, 21), FP16X3, 1, False), ((3, 3, 21), FP16X3, 304, True),
+        ((3, 3, 12), FP16X3, 152, True), ((3, 3, 12), FP16X3, 4096, False), ((5, 5, 8), FP32, 4096, True)]:
+    net = (rqc.random_circuit(rows, cols, depth, seed=depth), rqc.row_sweep_ordering(rows, cols), rqc.grid_text(rows, cols))
+    ctx = Context(0, precision)
+    log()
+    ctx.evaluate_many(*net, "0" * (rows * cols), ["0" * (rows * cols)] * strings, 1 << 40)
+    assert (ctx.stats()["launches"] == 1) == one, (rows, cols, depth, precision, strings)
+    # Passes of one string at a time are calls of one string.
+    if strings > 1:
+        ctx.set_option("max_batch", 1)
+        ctx.evaluate_many(*net, "0" * (rows * cols), ["0" * (rows * cols)] * 3, 1 << 40)
+        single = ctx.stats()["launches"] == 3
+        ctx.set_option("max_batch", 0)
+        ctx.evaluate_many(*net, "0" * (rows * cols), ["0" * (rows * cols)], 1 << 40)
+        assert (ctx.stats()["launches"] == 1) == single
+''')
