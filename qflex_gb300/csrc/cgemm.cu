@@ -407,7 +407,53 @@ auto with_shape(std::size_t m, std::size_t n, std::size_t k, F&& f) {
   return f(Shape<128, 64, 16, 8, 4, 3>{});
 }
 
+// Few tiles: a product is then as long as one tile's chain of k-steps. Small
+// tiles and six steps in flight shorten the chain, and where they are fewer
+// than the SMs hold (two each), so does splitting k into runs of 64 or more.
+// The shapes above against these: (16, 16, 32) 10 and 4 us, (256, 16, 64) 19
+// and 5.5, (512, 512, 512) 104 and 42; with runs (256, 16, 512) 80 and 9,
+// (16, 16, 4096) 500 and 12. Up to 101 tiles with 512 terms take runs too, in
+// the shapes above: (1586, 161, 3221) 686 and 342, (1000, 512, 1000) 202 and
+// 140. Calls f with the shape of such a product; false for other products.
+template <typename F>
+bool with_few_tiles(std::size_t m, std::size_t n, std::size_t k, int batch, bool scratch, F&& f) {
+  const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
+  const std::size_t tiles = ((m + tile.bm - 1) / tile.bm) * ((n + tile.bn - 1) / tile.bn) * (std::size_t)batch;
+  const bool runs = scratch && tiles <= 101 && k >= 512 && 3 * m * n * (std::size_t)batch <= kSkinnyScratchElems;
+  if (!tiles || (tiles > 38 && !runs)) return false;
+  if (tiles > 38)
+    with_shape(m, n, k, [&](auto shape) {
+      f(shape);
+      return 0;
+    });
+  else
+    n <= 8 ? f(Shape<64, 8, 16, 2, 2, 6>{}) : f(Shape<32, 32, 16, 2, 2, 6>{});
+  return true;
+}
+
+// The runs of k (and their terms) in which the tiles of shape S sum a product
+// that has scratch: 0 for none.
+template <typename S>
+int runs_of(std::size_t m, std::size_t n, std::size_t k, int batch, std::size_t* terms) {
+  constexpr Tile t = S::tile;
+  const std::size_t own = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn) * (std::size_t)batch;
+  std::size_t splits = std::min<std::size_t>(304 / own, k / 64);
+  splits = std::min<std::size_t>(splits, kSkinnyScratchElems / (m * n * (std::size_t)batch));
+  if (splits < 3) return 0;
+  *terms = ((k + splits - 1) / splits + t.bk - 1) / t.bk * t.bk;
+  return (int)((k + *terms - 1) / *terms);
+}
+
 }  // namespace
+
+int tiled_splits(std::size_t m, std::size_t n, std::size_t k, int batch) {
+  int splits = 0;
+  with_few_tiles(m, n, k, batch, true, [&](auto shape) {
+    std::size_t terms = 0;
+    splits = runs_of<decltype(shape)>(m, n, k, batch, &terms);
+  });
+  return splits;
+}
 
 void launch_flag_not_finite(const float2* C, std::size_t outputs, std::uint64_t batch_stride, int batch, int* flag,
                             int value, cudaStream_t s) {
@@ -495,43 +541,24 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
                         cudaStream_t s, OnlyIf only_if) {
   if (m > 0x7fffffffull || n > 0x7fffffffull || k > 0x7fffffffull)
     throw std::string("ERROR (qflex_gb300: cgemm) --> dimension exceeds 2^31");
-  // Few tiles: a product is then as long as one tile's chain of k-steps. Small
-  // tiles and six steps in flight shorten the chain, and where they are fewer
-  // than the SMs hold (two each), so does splitting k into runs of 64 or more.
-  // The shapes above against these: (16, 16, 32) 10 and 4 us, (256, 16, 64) 19
-  // and 5.5, (512, 512, 512) 104 and 42; with runs (256, 16, 512) 80 and 9,
-  // (16, 16, 4096) 500 and 12. Up to 101 tiles with 512 terms take runs too, in
-  // the shapes above: (1586, 161, 3221) 686 and 342, (1000, 512, 1000) 202 and
-  // 140. A gather is made for the shapes above.
+  // A gather is made for the usual shapes.
+  if (!gather && with_few_tiles(m, n, k, batch, scratch != nullptr, [&](auto shape) {
+        using S = decltype(shape);
+        std::size_t terms = 0;
+        const int splits = scratch ? runs_of<S>(m, n, k, batch, &terms) : 0;
+        if (!splits) {
+          S::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, only_if, s);
+          return;
+        }
+        S::template run<SPLIT>(A, B, C, m, n, k, batch_stride, batch, SplitK{scratch, splits, (int)terms}, s);
+        dim3 grid((unsigned)((m * n + 31) / 32), (unsigned)batch);
+        split_finish_kernel<<<grid, 256, 0, s>>>(scratch, C, m * n, splits, batch_stride);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch split_finish) --> ") + cudaGetErrorString(e);
+      }))
+    return;
   const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
   const std::size_t tiles = ((m + tile.bm - 1) / tile.bm) * ((n + tile.bn - 1) / tile.bn) * (std::size_t)batch;
-  const bool runs = scratch && tiles <= 101 && k >= 512 && 3 * m * n * (std::size_t)batch <= kSkinnyScratchElems;
-  if (!gather && tiles && (tiles <= 38 || runs)) {
-    auto few = [&](auto shape) {
-      using S = decltype(shape);
-      constexpr Tile t = S::tile;
-      const std::size_t own = ((m + t.bm - 1) / t.bm) * ((n + t.bn - 1) / t.bn) * (std::size_t)batch;
-      std::size_t splits = scratch ? std::min<std::size_t>(304 / own, k / 64) : 1;
-      splits = std::min<std::size_t>(splits, kSkinnyScratchElems / (m * n * (std::size_t)batch));
-      if (splits < 3) {
-        S::template run<PLAIN>(A, B, C, m, n, k, batch_stride, batch, only_if, s);
-        return 0;
-      }
-      const std::size_t terms = ((k + splits - 1) / splits + t.bk - 1) / t.bk * t.bk;
-      splits = (k + terms - 1) / terms;
-      S::template run<SPLIT>(A, B, C, m, n, k, batch_stride, batch, SplitK{scratch, (int)splits, (int)terms}, s);
-      dim3 grid((unsigned)((m * n + 31) / 32), (unsigned)batch);
-      split_finish_kernel<<<grid, 256, 0, s>>>(scratch, C, m * n, (int)splits, batch_stride);
-      const cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch split_finish) --> ") + cudaGetErrorString(e);
-      return 0;
-    };
-    if (tiles > 38)
-      with_shape(m, n, k, few);
-    else
-      n <= 8 ? few(Shape<64, 8, 16, 2, 2, 6>{}) : few(Shape<32, 32, 16, 2, 2, 6>{});
-    return;
-  }
   // Where one or two blocks on an SM hold all tiles: up to 32 columns in tiles
   // of 64 rows, more of them with fewer outputs a thread ((16384, 16, 256) 40
   // and 20 us, (25646, 10, 112) x 2 34 and 23, (30000, 32, 64) 16.8 and 15.6);

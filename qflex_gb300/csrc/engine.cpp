@@ -657,7 +657,7 @@ std::size_t Engine::run_program(Plan& p, int batch, float2* arena, float* tc_ws)
     } else {
       launch_cgemm_fp32(arena + op.a, arena + op.b, arena + op.c, op.m, op.n, op.k, stride, batch,
                         stream_, scratch);
-      launches += (vm_splits(op.m, op.n, op.k, batch) || skinny_splits(op.m, op.n, op.k, batch)) ? 2 : 1;
+      launches += cgemm_fp32_launches(op.m, op.n, op.k, batch);
     }
   }
   if (profile_) QFX_CUDA(cudaEventRecord(prof_events_[prog.ops.size()], stream_));

@@ -501,6 +501,10 @@ void launch_skinny_split(const float2* A, const float2* B, float2* C, std::size_
   check_launch("skinny_finish");
 }
 
+int cgemm_fp32_launches(std::size_t m, std::size_t n, std::size_t k, int batch) {
+  return vm_splits(m, n, k, batch) || skinny_splits(m, n, k, batch) || (m > 1 && n > 1 && tiled_splits(m, n, k, batch)) ? 2 : 1;
+}
+
 void launch_cgemm_fp32(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n,
                        std::size_t k, std::uint64_t stride, int batch, cudaStream_t s,
                        float2* scratch) {

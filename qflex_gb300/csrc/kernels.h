@@ -133,6 +133,8 @@ int skinny_splits(std::size_t m, std::size_t n, std::size_t k, int batch);
 // blocks that each read whole rows of B; 0 when the shape does not qualify.
 // Takes precedence over skinny_splits.
 int vm_splits(std::size_t m, std::size_t n, std::size_t k, int batch);
+// Kernels that launch_cgemm_fp32 launches with scratch: two when the scratch is used.
+int cgemm_fp32_launches(std::size_t m, std::size_t n, std::size_t k, int batch);
 void launch_cgemm_fp32(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n,
                        std::size_t k, std::uint64_t batch_stride, int batch, cudaStream_t s,
                        float2* scratch);
@@ -171,6 +173,9 @@ struct OnlyIf {
 void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2* B, float2* C, std::size_t m,
                         std::size_t n, std::size_t k, std::uint64_t batch_stride, int batch, float2* scratch,
                         cudaStream_t s, OnlyIf only_if = {});
+// Runs of k in which launch_cgemm_tiled sums a row-major product that has
+// scratch, as a second launch adds them up; 0: none.
+int tiled_splits(std::size_t m, std::size_t n, std::size_t k, int batch);
 // Sets *flag to `value` when one of `outputs` elements per entry of C is an
 // infinity or NaN.
 void launch_flag_not_finite(const float2* C, std::size_t outputs, std::uint64_t batch_stride, int batch, int* flag,

@@ -96,3 +96,32 @@ for (rows, cols, depth), precision, strings, one in [
         ctx.evaluate_many(*net, "0" * (rows * cols), ["0" * (rows * cols)], 1 << 40)
         assert (ctx.stats()["launches"] == 1) == single
 ''')
+
+
+def test_launch_count(run_fake):  # noqa: F811
+    """stats()["launches"] is the number of kernels an evaluation launches, also
+    where FP32 products sum k in runs, added up by a second kernel."""
+    run_fake('''
+runs = 0
+nets = [(4, 4, 16), (4, 5, 16), (4, 4, 24), (5, 5, 16)]
+nets = [(rqc.random_circuit(r, c, d, seed=3), rqc.row_sweep_ordering(r, c), rqc.grid_text(r, c), r * c) for r, c, d in nets]
+nets.append((rqc.random_circuit(6, 6, 24, seed=0), rqc.ordering_6x6(cut_values=(1,)), rqc.grid_text(6, 6), 36))
+nets.append((rqc.random_circuit(7, 7, 32, seed=0), rqc.ordering_7x7((0,), (1,)), rqc.grid_text(7, 7), 49))
+# Patches that share four bonds of dimension 4 and keep others: (4, 64, 256).
+merge = [f"expand a {q}" for q in range(5)] + [f"expand b {q}" for q in (5, 6, 7)] + ["merge a b"]
+nets.append((rqc.random_circuit(4, 4, 16, seed=3), "\\n".join(merge + [f"expand b {q}" for q in range(8, 16)]) + "\\n",
+             rqc.grid_text(4, 4), 16))
+fake.fake_memory(1 << 45)
+for circuit, ordering, grid, qubits in nets:
+    for precision in (FP32, TF32X3, FP16X3, BF16X3, FP64):
+        for strings in (1, 2):
+            ctx = Context(0, precision)
+            ctx.set_profiling(True)  # operation by operation
+            log()
+            ctx.evaluate_many(circuit, ordering, grid, "0" * qubits, ["0" * qubits] * strings, float(1 << 50))
+            names = kernels()
+            runs += sum(x.startswith("split_finish_kernel") for x in names)
+            assert len(names) == ctx.stats()["launches"], (qubits, precision, strings, len(names), ctx.stats())
+            ctx.close()
+assert runs > 4, runs
+''')
