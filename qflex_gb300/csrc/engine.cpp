@@ -116,6 +116,7 @@ Engine::Engine(int device, int precision) : device_(device), precision_(precisio
   if (const char* f = std::getenv("QFLEX_GB300_FUSE")) fuse_splits_ = std::atoi(f) != 0;
   QFX_CUDA(cudaEventCreate(&ev0_));
   QFX_CUDA(cudaEventCreate(&ev1_));
+  QFX_CUDA(cudaEventCreateWithFlags(&buffers_free_, cudaEventDisableTiming));
   set_precision(precision);
 }
 
@@ -127,6 +128,7 @@ Engine::~Engine() {
   for (auto& b : bufs_) cudaFree(b.ptr);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
+  if (buffers_free_) cudaEventDestroy(buffers_free_);
   for (auto e : prof_events_) cudaEventDestroy(e);
   if (own_stream_ && stream_) cudaStreamDestroy(stream_);
 }
@@ -338,6 +340,7 @@ void Engine::multiply(const float2* A, const float2* B, float2* C, std::size_t m
     while (piece > 0 && !(ws = try_reserve(entry * (std::size_t)piece, 4))) piece /= 2;
     if (!ws && contraction_sizes(m, n, k)) ws = tc_workspace(entry / sizeof(float));  // throws
     if (ws) {
+      buffers_wait();
       // An infinity has no rest to split off, so that its products become NaN;
       // a value next to the largest ones rounds to infinity. Where the sizes
       // allow FP32, a product with such a sum runs again there.
@@ -348,10 +351,31 @@ void Engine::multiply(const float2* A, const float2* B, float2* C, std::size_t m
                              std::min(piece, batch - b), (float*)ws, watch);
       if (watch)
         launch_cgemm_tiled(A, nullptr, B, C, m, n, k, stride, batch, nullptr, stream_, {error_flag() + 4, watch});
+      buffers_used();
       return;
     }
   }
-  launch_cgemm_fp32(A, B, C, m, n, k, stride, batch, stream_, skinny_scratch());
+  float2* scratch = skinny_scratch();
+  const bool used = cgemm_fp32_launches(m, n, k, batch) > 1;
+  if (used) buffers_wait();
+  launch_cgemm_fp32(A, B, C, m, n, k, stride, batch, stream_, scratch);
+  if (used) buffers_used();
+}
+
+void Engine::buffers_wait() {
+  if (!buffers_stream_ || buffers_stream_ == stream_) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  QFX_CUDA(cudaStreamIsCapturing(stream_, &capture));
+  if (capture == cudaStreamCaptureStatusNone) QFX_CUDA(cudaStreamWaitEvent(stream_, buffers_free_, 0));
+}
+
+void Engine::buffers_used() {
+  if (own_stream_) return;  // set_stream waits for it
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  QFX_CUDA(cudaStreamIsCapturing(stream_, &capture));
+  if (capture != cudaStreamCaptureStatusNone) return;
+  QFX_CUDA(cudaEventRecord(buffers_free_, stream_));
+  buffers_stream_ = stream_;
 }
 
 void Engine::set_stream(cudaStream_t s) {
@@ -908,6 +932,7 @@ std::vector<EvalResult> Engine::evaluate(const std::string& circuit, const std::
     chunk = (int)std::max<std::size_t>(1, std::min<std::size_t>((std::size_t)chunk, usable / std::max<std::size_t>(per_entry, 1)));
   }
   if (max_batch_ > 0) chunk = std::min(chunk, max_batch_);
+  buffers_wait();
   if (!small) {
     arena = (float2*)reserve(arena_bytes * (std::size_t)chunk, 0);
     tc_ws = p.tc_ws_elems ? tc_workspace(p.tc_ws_elems * (std::size_t)chunk) : nullptr;

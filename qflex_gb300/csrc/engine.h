@@ -135,6 +135,14 @@ class Engine {
   bool narrow_product(std::size_t m, std::size_t n, std::size_t k) const;
   // fp32 elements of split planes that one product of this shape needs.
   std::size_t workspace_elems(std::size_t m, std::size_t n, std::size_t k) const;
+  // The context's device buffers serve one product after the other. A caller
+  // may give it another stream while the last one's work is still queued:
+  // products that use the buffers start after those before them, on whatever
+  // stream (not inside a capture, whose order is the caller's).
+  void buffers_wait();
+  void buffers_used();
+  cudaEvent_t buffers_free_ = nullptr;
+  cudaStream_t buffers_stream_ = nullptr;  // where buffers_free_ was recorded
   // Device buffer `slot` of at least `bytes`; null when the device has no room.
   void* try_reserve(std::size_t bytes, int slot);
   // C = A * B on the tensor cores in the context's split precision. With

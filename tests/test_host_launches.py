@@ -125,3 +125,39 @@ for circuit, ordering, grid, qubits in nets:
             ctx.close()
 assert runs > 4, runs
 ''')
+
+
+def test_buffers_across_streams(run_fake):  # noqa: F811
+    """A product that uses the context's buffers (planes, runs of k) on another
+    stream than the one before it waits for that one; products that use none run
+    side by side, and a captured product waits for nothing outside its graph."""
+    run_fake('''
+def steps():
+    return [(w[0], x.split("stream=")[1].split()[0]) for x in log() for w in [x.split()]
+            if w[0] in ("launch", "wait", "record")]
+for precision, size in ((FP32, (64, 64, 600)), (FP32, (1, 4, 9000)), (FP16X3, (4096, 256, 256)), (BF16X3, (640, 700, 200))):
+    ctx = Context(0, precision)
+    ctx.multiply(A, B, C, *size)
+    assert not [s for s in steps() if s[0] != "launch"]  # the context's own stream
+    ctx.set_stream(0x10)
+    last = None
+    for stream in ("0x10", "0x20", "0x20", "0x10"):
+        ctx.set_stream(int(stream, 16))
+        ctx.multiply(A, B, C, *size)
+        got = steps()
+        assert {s for _, s in got} == {stream} and got[-1][0] == "record", got
+        assert [w for w, _ in got].count("wait") == (last not in (None, stream)), (precision, size, got)
+        assert last in (None, stream) or got[0][0] == "wait", got
+        last = stream
+    ctx.set_stream(0x30)
+    plain = Context(0, FP32)
+    for stream in (0x10, 0x20):
+        plain.set_stream(stream)
+        plain.multiply(A, B, C, 70000, 64, 16)
+        assert [w for w, _ in steps()] == ["launch"]
+    # 0x30 is being captured.
+    fake.fake_capturing(0x30, 1)
+    ctx.multiply(A, B, C, *size)
+    assert all(w == "launch" for w, _ in steps())
+    fake.fake_capturing(0x30, 0)
+''')
