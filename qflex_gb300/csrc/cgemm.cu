@@ -22,6 +22,10 @@
 // (fma.rn.f32x2) have the same rate from registers and lose more to packing
 // their operands: 2049 us at 2048^3.
 //
+// Where the persistent blocks' rounds of tiles leave half of the chip idle, or
+// rows do not start on 16 bytes, one tile per block is faster: those products
+// run as they did before (cgemm_staged_kernel, staged_is_faster).
+//
 // Sums run over k in ascending order with four FMAs per complex term; products
 // of few tiles may sum runs of k so and then add the runs in 64 bits.
 //
@@ -302,6 +306,90 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// One tile per block, operands staged through registers: the next k-step's
+// are loaded while one is multiplied. A block of 128 x 64 has an SM to itself
+// (164 registers), where it is as fast as two persistent ones, so its rounds
+// of tiles are half as long; and rows that do not start on 16 bytes cost it
+// nothing, where the persistent blocks' copies of 8 bytes cost them 3 to 10 %.
+// The rule is staged_is_faster. The sums are the same.
+template <int BM, int BN, int BK, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+    cgemm_staged_kernel(const float2* __restrict__ A, const float2* __restrict__ B, float2* __restrict__ C, int m,
+                        int n, int k, std::uint64_t batch_stride) {
+  constexpr int NT = (BM / TM) * (BN / TN);
+  constexpr int TX = BN / TN;
+  constexpr int LA = BM * BK / NT, LB = BK * BN / NT;
+  static_assert(LA * NT == BM * BK && LB * NT == BK * BN, "tile / threads mismatch");
+  __shared__ __align__(16) float2 As[BK][BM + 2];
+  __shared__ __align__(16) float2 Bs[BK][BN + 2];
+  const std::uint64_t at = std::uint64_t(blockIdx.z) * batch_stride;
+  A += at;
+  B += at;
+  C += at;
+  const int tiles_m = (m + BM - 1) / BM;
+  const int m0 = int(blockIdx.x % tiles_m) * BM, n0 = int(blockIdx.x / tiles_m) * BN;
+  const int t = threadIdx.x, tx = t % TX, ty = t / TX;
+  float2 acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  float2 ra[LA], rb[LB];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+      const int r = m0 + (t + i * NT) / BK, c = k0 + (t + i * NT) % BK;
+      ra[i] = r < m && c < k ? A[std::size_t(r) * k + c] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < LB; ++i) {
+      const int r = k0 + (t + i * NT) / BN, c = n0 + (t + i * NT) % BN;
+      rb[i] = r < k && c < n ? B[std::size_t(r) * n + c] : make_float2(0.f, 0.f);
+    }
+  };
+  auto store = [&] {
+#pragma unroll
+    for (int i = 0; i < LA; ++i) As[(t + i * NT) % BK][(t + i * NT) / BK] = ra[i];
+#pragma unroll
+    for (int i = 0; i < LB; ++i) Bs[(t + i * NT) / BN][(t + i * NT) % BN] = rb[i];
+  };
+  const int ktiles = (k + BK - 1) / BK;
+  load(0);
+  store();
+  __syncthreads();
+  for (int kt = 0; kt < ktiles; ++kt) {
+    const bool more = kt + 1 < ktiles;
+    if (more) load((kt + 1) * BK);
+#pragma unroll
+    for (int kk = 0; kk < BK; ++kk) {
+      float2 a[TM], b[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx * TN + j];
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) cfma(acc[i][j], a[i], b[j]);
+    }
+    __syncthreads();
+    if (more) {
+      store();
+      __syncthreads();
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int r = m0 + ty * TM + i;
+    if (r >= m) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int c = n0 + tx * TN + j;
+      if (c < n) C[std::size_t(r) * n + c] = acc[i][j];
+    }
+  }
+}
+
 // Adds the sums of a split product's runs: blocks of 32 elements of C, whose
 // eight warps take every eighth run (one thread for all runs of an element
 // took 15 us at 64).
@@ -444,6 +532,49 @@ int runs_of(std::size_t m, std::size_t n, std::size_t k, int batch, std::size_t*
   return (int)((k + *terms - 1) / *terms);
 }
 
+// Whether one tile per block is faster, for products of `tiles` tiles of the
+// usual shape (and no gather).
+// Tiles of 128 x 64, by estimates in us from the rounds of tiles, one on an SM
+// (rounds) or two (pairs; a last round of up to 112 tiles finds an SM for each,
+// from there on some SMs get two), and the padded terms, fitted to 1172 products
+// of 39 to 3000 tiles (2 to 4 % standard deviation). 161 of those take over 2 %
+// more in persistent blocks than in one tile per block, and 15 as chosen here;
+// most is lost between 417 and 456 tiles: (5573, 290, 1392) x 2 838 us in one
+// tile per block, 1049 in persistent ones.
+// Tiles of 256 x 16 with rows on 8 bytes: up to 304 of them by how many 64-row
+// tiles an SM gets, (74497, 11, 1713) 455 and 664, (10143, 11, 585) x 4 160 and
+// 136; more where steps of 16 terms pad no more than those of 8, (157583, 13,
+// 27) x 4 83 and 87, (157583, 13, 9) x 7 91 and 81, or terms are many.
+bool staged_is_faster(const Tile& tile, std::size_t tiles, std::size_t m, std::size_t n, std::size_t k, int batch) {
+  if (tile.bm == 256 && tile.bn == 16) {
+    if (k % 2 == 0 || k < 25) return false;
+    const std::size_t per_sm = ((m + 63) / 64 * (std::size_t)batch + 151) / 152;
+    return tiles <= 152 ? per_sm >= 4 : tiles <= 304 ? per_sm >= 6 : k % 16 > 8 || k >= 150;
+  }
+  if (tile.bm != 128 || tile.bn != 64 || tile.bk != 16) return false;
+  const double rounds = double((tiles + 151) / 152), terms = double((k + 15) / 16 * 16);
+  const double staged = 6.9 + rounds * (4.1 + 0.1884 * terms);
+  if (tiles <= 152) {
+    const double q = m > 64 && k >= 128 ? double((k + 31) / 32 * 32) : terms;  // steps of 32, see below
+    return staged < (k % 2 ? 7.9 + 0.2104 * q : n % 2 ? 9.4 + 0.1937 * q : 8.2 + 0.1884 * q);
+  }
+  const std::size_t last = tiles % 304;
+  const bool spread = tiles > 304 && last > 0 && last <= 112;
+  const double pairs = double(tiles / 304) + (last > 0 && !spread), alone = spread;
+  return staged < (k % 2   ? 6.7 + pairs * (3.0 + 0.3847 * terms) + alone * (1.4 + 0.194 * terms)
+                   : n % 2 ? 6.7 + pairs * (3.2 + 0.38 * terms) + alone * (1.6 + 0.195 * terms)
+                           : 6.4 + pairs * (1.8 + 0.3702 * terms) + alone * (1.4 + 0.1951 * terms));
+}
+
+template <int BM, int BN, int BK, int TM, int TN>
+void run_staged(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
+                std::uint64_t stride, int batch, cudaStream_t s) {
+  dim3 grid((unsigned)(((m + BM - 1) / BM) * ((n + BN - 1) / BN)), 1, (unsigned)batch);
+  cgemm_staged_kernel<BM, BN, BK, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, s>>>(A, B, C, (int)m, (int)n, (int)k, stride);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch cgemm_staged) --> ") + cudaGetErrorString(e);
+}
+
 }  // namespace
 
 int tiled_splits(std::size_t m, std::size_t n, std::size_t k, int batch) {
@@ -559,6 +690,13 @@ void launch_cgemm_tiled(const float2* A, const TileGather* gather, const float2*
     return;
   const Tile tile = with_shape(m, n, k, [](auto shape) { return decltype(shape)::tile; });
   const std::size_t tiles = ((m + tile.bm - 1) / tile.bm) * ((n + tile.bn - 1) / tile.bn) * (std::size_t)batch;
+  if (!gather && !only_if.flag && staged_is_faster(tile, tiles, m, n, k, batch)) {
+    if (tile.bm == 256)
+      run_staged<256, 16, 16, 8, 2>(A, B, C, m, n, k, batch_stride, batch, s);
+    else
+      run_staged<128, 64, 16, 8, 4>(A, B, C, m, n, k, batch_stride, batch, s);
+    return;
+  }
   // Where one or two blocks on an SM hold all tiles: up to 32 columns in tiles
   // of 64 rows, more of them with fewer outputs a thread ((16384, 16, 256) 40
   // and 20 us, (25646, 10, 112) x 2 34 and 23, (30000, 32, 64) 16.8 and 15.6);

@@ -161,3 +161,19 @@ for precision, size in ((FP32, (64, 64, 600)), (FP32, (1, 4, 9000)), (FP16X3, (4
     assert all(w == "launch" for w, _ in steps())
     fake.fake_capturing(0x30, 0)
 ''')
+
+
+def test_fp32_tiles_per_block(run_fake):  # noqa: F811
+    """Which FP32 products run one tile per block: those measured slower in
+    persistent blocks (rounds of tiles that fill half the chip, rows on 8
+    bytes), and none of the sizes that contractions have beside them."""
+    from tests.test_gpu_staged import STAGED
+    run_fake(f"staged = {STAGED!r}" + '''
+persistent = [(2048, 2048, 2048, 1), (32768, 64, 64, 16), (1024, 1024, 1024, 4), (157583, 13, 9, 7), (40000, 40, 10, 1),
+              (65536, 16, 512, 1), (10143, 11, 585, 4), (5000, 200, 300, 1), (1048576, 16, 16, 1), (300, 30, 700, 1)]
+ctx = Context(0, FP32)
+for product in staged + persistent:
+    ctx.multiply(A, B, C, *product[:4], 1 << 30)
+    name = kernels()[0]
+    assert name.startswith("cgemm_staged_kernel" if product in staged else "cgemm_kernel"), (product, name)
+''')
