@@ -103,6 +103,10 @@ __global__ void __launch_bounds__(256) permute_general_kernel(const __grid_const
 }
 
 void plan_runs(GeneralPerm* g) {
+  // Small tensors need the threads more than whole sectors: of 10000 to 100000
+  // elements, one launch behind the other, runs of 13 to 16 took 6.2 us, runs of
+  // up to 4 take 4.2.
+  const std::uint32_t most = g->size <= (1u << 17) ? 4 : 16;
   struct Dim {
     std::uint32_t d, in, out;
   };
@@ -124,8 +128,8 @@ void plan_runs(GeneralPerm* g) {
   std::reverse(dims.begin(), dims.end());
   g->run = g->last_run = 1;
   std::uint32_t chunks = 1, chunk_in = 0, chunk_out = 0;
-  // The input's fastest index: in runs of up to 16 when long, else with the
-  // next faster ones up to 16 elements; never with the output's fastest
+  // The input's fastest index: in runs of up to `most` when long, else with the
+  // next faster ones up to that many elements; never with the output's fastest
   // index, which the lanes follow.
   auto fastest = [&](std::uint32_t in) {
     for (std::size_t i = 1; i < dims.size(); ++i)
@@ -134,8 +138,8 @@ void plan_runs(GeneralPerm* g) {
   };
   if (std::size_t i = fastest(1)) {
     const Dim f = dims[i];
-    if (f.d > 16) {
-      chunks = (f.d + 15) / 16;
+    if (f.d > most) {
+      chunks = (f.d + most - 1) / most;
       g->run = (f.d + chunks - 1) / chunks;
       chunks = (f.d + g->run - 1) / g->run;
       g->last_run = f.d - g->run * (chunks - 1);
@@ -146,7 +150,7 @@ void plan_runs(GeneralPerm* g) {
     } else {
       while (i) {
         const Dim e = dims[i];
-        if (g->run * e.d > 16) break;
+        if (g->run * e.d > most) break;
         for (std::uint32_t u = g->run; u < g->run * e.d; ++u)
           g->run_out[u] = g->run_out[u % g->run] + u / g->run * e.out;
         g->run *= e.d;

@@ -177,3 +177,22 @@ for product in staged + persistent:
     name = kernels()[0]
     assert name.startswith("cgemm_staged_kernel" if product in staged else "cgemm_kernel"), (product, name)
 ''')
+
+
+def test_small_permutations_move_short_runs(run_fake):  # noqa: F811
+    """Runs of at most four elements up to 2^17, where longer ones leave too few
+    threads; the schedules on either side of the line are right."""
+    run_fake('''
+import numpy as np
+ctx = Context(0, FP32)
+for dims, order in [((25, 5, 24, 4), (0, 2, 3, 1)), ((16, 24, 26), (1, 2, 0)), ((3, 3, 2, 5, 2, 5, 4, 4), (7, 5, 2, 0, 4, 1, 6, 3)),
+                    ((8, 16, 1023), (2, 1, 0)), ((131071,), (0,)), ((1025, 128), (1, 0)), ((7, 18725), (1, 0)),
+                    ((13, 9, 16, 71), (3, 1, 0, 2)), ((71, 13, 9, 16), (1, 3, 0, 2))]:
+    ctx.permute(A, B, dims, order)
+    name = kernels()[0]
+    run = int(name.split("<")[1].split(",")[0])
+    size = int(np.prod(dims))
+    assert name.startswith("permute_runs_kernel") and (run <= 4 if size <= 1 << 17 else run in (1, 8, 16)), (dims, name)
+    x = np.arange(size).astype(np.complex64)
+    assert np.array_equal(_lib.check_permute(x, dims, order), x.reshape(dims).transpose(order).reshape(-1)), dims
+''')
