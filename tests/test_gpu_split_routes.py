@@ -146,3 +146,55 @@ def test_infinities_and_nan(built_lib, precision, m, n, k, batch, options, case)
         want, bound = (x.nan_to_num(0, 0, 0) for x in (a.to(torch.complex128) @ b.to(torch.complex128),
                                                       a.abs().double() @ b.abs().double()))
         assert float((torch.where(good, c.to(torch.complex128) - want, 0).abs() / (bound + 1e-300))[good].max()) < tol
+
+
+EDGES = [(300, 1000, 113, 1, 1), (129, 4097, 97, 1, 0), (40000, 130, 97, 1, 1), (4097, 257, 111, 2, 1),
+         (128, 1024, 300, 1, 1), (64, 5467, 96, 1, 0), (383, 1500, 130, 1, 0), (640, 1100, 192, 2, 0),
+         (257, 640, 257, 1, 1), (8193, 129, 161, 1, 0), (3001, 690, 319, 1, 0)]
+# Few columns: 3xFP16, tiles of 32 and 64, with rows on 16 and on 8 bytes.
+NARROW = [(65537, 17, 100, 1, 0), (40001, 31, 129, 2, 1), (262144, 16, 96, 1, 0), (20000, 32, 256, 1, 1),
+          (70001, 50, 97, 1, 1), (20001, 63, 112, 1, 0), (30000, 64, 97, 2, 1), (16385, 33, 128, 1, 0),
+          (100000, 48, 96, 1, 0)]
+
+
+@pytest.mark.parametrize("precision,m,n,k,batch,extra",
+                         [(p, *e) for p in (FP16X3, TF32X3, BF16X3) for e in EDGES] + [(FP16X3, *e) for e in NARROW])
+def test_edges(built_lib, precision, m, n, k, batch, extra):
+    """Partial tiles, k-steps and blocks, one row into a pair's second half, odd
+    sizes and strides, and columns of B of very different size."""
+    import torch
+    B = randn((batch, k, n), n) * torch.exp2(torch.arange(n, device="cuda") % 41 - 20.0)
+    check(precision, randn((batch, m, k), k), B, extra, 8e-6)  # as for test_block_exponents; 3xTF32 chunks of 16
+
+
+@pytest.mark.parametrize("precision,m,n,k", [
+    (p, m, n, k) for p in (FP16X3, TF32X3, BF16X3) for m, n, k in [(1000, 500, 200), (129, 4096, 256)]] + [
+    (FP16X3, 60000, 31, 128), (FP16X3, 20000, 60, 97), (FP16X3, 100, 2000, 255)])
+def test_wide_ranges(built_lib, precision, m, n, k):
+    """Components from 1 down to 2^-60 side by side in a row of A and in a column
+    of B. 3xTF32 and BF16x3 keep the bits of each; 3xFP16 counts them from the
+    largest of 32 values of A's row (of the row, where A's planes are made
+    before the product: m <= 128 with n > 1024) and of B's column."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    A, B = (randn((1, *s), s[0]) * torch.exp2(-torch.randint(0, 61, s, device="cuda", generator=gen))
+            for s in ((m, k), (k, n)))
+    if precision != FP16X3:
+        check(precision, A, B, 0, 8e-6)
+        return
+    buf = torch.cat([A.reshape(1, -1), B.reshape(1, -1), torch.zeros((1, m * n), dtype=torch.complex64, device="cuda")], 1)
+    C = _multiply(precision, buf, m, n, k)[0, m * k + k * n:].view(m, n).cdouble()
+    assert not torch.equal(C, _multiply(FP32, buf, m, n, k)[0, m * k + k * n:].view(m, n).cdouble())
+    a, b = A[0].cdouble(), B[0].cdouble()
+
+    def largest(x, dim):
+        return torch.maximum(x.real.abs(), x.imag.abs()).amax(dim, keepdim=True)
+    if m <= 128 and n > 1024:
+        top_a = largest(a, 1).expand(m, k)
+    else:
+        pad = torch.nn.functional.pad(torch.view_as_real(a), (0, 0, 0, -k % 32)).abs().amax(-1)
+        top_a = pad.view(m, -1, 32).amax(-1).repeat_interleave(32, -1)[:, :k]
+    top_b = largest(b, 0).expand(k, n)
+    # A value within 2^-22 of the largest component, each part of a complex one.
+    bound = 2.0 ** -22 * 2 ** 0.5 * (top_a @ b.abs() + a.abs() @ top_b) + 8e-6 * (a.abs() @ b.abs())
+    assert float(((C - a @ b).abs() / bound).max()) < 1

@@ -196,3 +196,58 @@ for dims, order in [((25, 5, 24, 4), (0, 2, 3, 1)), ((16, 24, 26), (1, 2, 0)), (
     x = np.arange(size).astype(np.complex64)
     assert np.array_equal(_lib.check_permute(x, dims, order), x.reshape(dims).transpose(order).reshape(-1)), dims
 ''')
+
+
+def test_products_of_a_split_precision(run_fake):  # noqa: F811
+    """Which products of a split-precision context run on the tensor cores, and
+    in which tiles."""
+    from tests.test_gpu_split_routes import EDGES, NARROW
+    run_fake(f"edges, narrow = {EDGES!r}, {NARROW!r}" + '''
+kinds = {FP16X3: 1, TF32X3: 0, BF16X3: 2}
+for precision, kind in kinds.items():
+    ctx = Context(0, precision)
+    def direct(m, n, k, batch=1, extra=0):
+        ctx.multiply(A, B, C, m, n, k, batch, 1 << 30)
+        return [x for x in kernels() if x.startswith(("cgemm_direct", "cgemm_tf32", "cgemm_fp16", "cgemm_bf16"))]
+    for e in edges:
+        m, n = e[:2]
+        name, = direct(*e)
+        if precision == BF16X3 and m <= 128 or m <= 128 and n > 1024:
+            assert not name.startswith("cgemm_direct"), (e, name)
+        else:
+            columns = 128 if n > 64 or kind != 1 else 64 if n > 32 else 32
+            assert name.startswith(f"cgemm_direct_kernel<{kind}, {columns},"), (e, name)
+            assert name.endswith("true>") == (m > 128 and e[2] > {1: 128, 0: 64, 2: 0}[kind] and columns == 128), (e, name)
+    for e in narrow:
+        names = direct(*e)
+        if precision == FP16X3:
+            assert len(names) == 1 and names[0].startswith(f"cgemm_direct_kernel<1, {32 if e[1] <= 32 else 64}, false>"), (e, names)
+        else:
+            assert bool(names) == (e[1] == 64), (e, names)
+    # Below 2^25 terms in all, or 96 a sum, FP32 kernels.
+    for m, n, k in [(64, 5461, 96), (40000, 130, 95), (257, 640, 161), (300, 130, 97), (262144, 15, 96), (255, 50, 4000)]:
+        assert not direct(m, n, k), (precision, m, n, k)
+    assert direct(64, 64, 16) and direct(128, 128, 32)  # sizes of contractions
+''')
+
+
+def test_kernels_of_an_evaluation(run_fake):  # noqa: F811
+    """The 3xFP16 products of one 7x7 slice: at the default choices they split A
+    themselves and no permutation writes planes; in chunks of one k-step, or at
+    another kernel choice, permutations write planes and the product loads them."""
+    run_fake('''
+net = (rqc.random_circuit(7, 7, 32, seed=0), rqc.ordering_7x7((0,), (1,)), rqc.grid_text(7, 7), "0" * 49, ["0" * 49])
+for option, kernel in ((None, "cgemm_direct_kernel<1,"), (("tc_chunk", 1), "cgemm_fp16x3_kernel"),
+                       (("tc_variant", 1), "cgemm_fp16x3_pair_kernel"), (("tc_variant", 2), "cgemm_fp16x3_deep_kernel"),
+                       (("tc_variant", 3), "cgemm_fp16x3_wide_kernel"), (("tc_variant", 4), "cgemm_fp16x3_narrow_kernel")):
+    ctx = Context(0, FP16X3)
+    if option:
+        ctx.set_option(*option)
+    log()
+    ctx.evaluate_many(*net, float(1 << 50))
+    names = kernels()
+    writing = [x for x in names if x.startswith("permute_kernel<float2, true>")]
+    assert [x for x in names if x.startswith(kernel)], (option, set(names))
+    assert bool(writing) == (option is not None), (option, len(writing))
+    assert option is None or not [x for x in names if x.startswith("cgemm_direct")], option
+''')
