@@ -17,14 +17,25 @@ def _cases():
            rqc.random_bitstrings(49, 2, 5))
 
 
+@pytest.fixture(scope="module")
+def cases(built_lib):
+    """The networks and their amplitudes by the complex128 oracle."""
+    from oracle import qflex_oracle as qo
+    out = []
+    for circuit, ordering, grid, initial, finals in _cases():
+        inp = [qo.Input(qo.Circuit.loads(circuit), qo.load_ordering(ordering), qo.Grid.loads(grid), initial, f) for f in finals]
+        out.append((circuit, ordering, grid, initial, finals,
+                    [qo.evaluate_circuit(i, np.complex128, float(1 << 40))[0][1] for i in inp]))
+    return out
+
+
 @pytest.mark.parametrize("option", [("tc_chunk", 1), ("tc_variant", 1), ("tc_variant", 2), ("tc_variant", 3),
                                     ("tc_variant", 4)], ids=lambda o: f"{o[0]}_{o[1]}")
-def test_permutations_write_planes(built_lib, option):
+def test_permutations_write_planes(cases, option):
     """Planes written by permutations (scaled per 32 values of a row) against
     planes split from permuted operands (scaled per row), and both against the
     complex128 oracle; fewer kernels are launched where permutations write them."""
-    from oracle import qflex_oracle as qo
-    for circuit, ordering, grid, initial, finals in _cases():
+    for circuit, ordering, grid, initial, finals, want in cases:
         got = []
         for fuse in (1, 0):
             ctx = Context(0, FP16X3)
@@ -35,6 +46,4 @@ def test_permutations_write_planes(built_lib, option):
             got.append(ctx.stats()["launches"])
         written, few, split, many = got
         assert few < many
-        inp = [qo.Input(qo.Circuit.loads(circuit), qo.load_ordering(ordering), qo.Grid.loads(grid), initial, f) for f in finals]
-        want = [qo.evaluate_circuit(i, np.complex128, float(1 << 40))[0][1] for i in inp]
         assert rel_err(written, want) < 1e-5 and rel_err(split, want) < 1e-5
