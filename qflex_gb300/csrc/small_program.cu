@@ -91,7 +91,7 @@ __device__ __forceinline__ float2 warp_sum(float2 v) {
 // (of up to 255 columns): a warp per output, as the separate kernels for
 // vectors sum them (gemv_rows_warp, gemv_cols_block). One thread per output
 // would add up to 1024 terms one after the other.
-__device__ __forceinline__ void column_product(const float2* A, const float2* B, float2* C, int m, int k) {
+__device__ __noinline__ void column_product(const float2* A, const float2* B, float2* C, int m, int k) {
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int i = threadIdx.x >> 5; i < m; i += NT / 32) {
@@ -101,7 +101,7 @@ __device__ __forceinline__ void column_product(const float2* A, const float2* B,
     if (lane == 0) C[i] = acc;
   }
 }
-__device__ __forceinline__ void row_product(const float2* A, const float2* B, float2* C, int n, int k) {
+__device__ __noinline__ void row_product(const float2* A, const float2* B, float2* C, int n, int k) {
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int j = threadIdx.x >> 5; j < n; j += NT / 32) {
