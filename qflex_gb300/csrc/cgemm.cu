@@ -101,7 +101,10 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   static_assert(LA * NT == BM * BK && BK % 2 == 0 && TN % 2 == 0, "tile / threads mismatch");
   extern __shared__ __align__(16) float2 ring[];
   if constexpr (VARIANT == PLAIN)
-    if (g.flag && *g.flag != g.value) return;
+    if (g.flag) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (*reinterpret_cast<const volatile int*>(g.flag) != g.value) return;
+    }
   const int t = threadIdx.x;
   const int tx = t % TX, ty = t / TX;
   int ktiles = k > 0 ? (k + BK - 1) / BK : 1;  // no terms: one k-step of zeros
@@ -433,6 +436,12 @@ __global__ void __launch_bounds__(256) flag_not_finite_kernel(const float2* __re
   if (zero != 0.f) atomicExch(flag, value);
 }
 
+bool is_conditional(const OnlyIf& c) { return c.flag != nullptr; }
+template <typename T>
+bool is_conditional(const T&) {
+  return false;
+}
+
 struct Tile {
   int bm, bn, bk, threads;
 };
@@ -466,9 +475,25 @@ struct Shape {
     };
     const bool c16 = VARIANT == SPLIT ? n % 2 == 0 : rows16(C, n);
     const int pairs = (c16 ? 1 : 0) | (rows16(A, k) ? 2 : 0) | (rows16(B, n) ? 4 : 0);
-    kernel<<<(unsigned)std::min<long long>(tiles, resident), nt, smem, s>>>(A, B, C, (int)m, (int)n, (int)k, stride,
-                                                                            (int)tiles_m, tiles, pairs, g);
-    const cudaError_t e = cudaGetLastError();
+    const unsigned grid = (unsigned)std::min<long long>(tiles, resident);
+    cudaError_t e;
+    if (VARIANT == PLAIN && is_conditional(g)) {
+      // Launched while the kernel before it ends, for which it waits.
+      cudaLaunchConfig_t lc = {};
+      lc.gridDim = dim3(grid, 1, 1);
+      lc.blockDim = dim3(nt, 1, 1);
+      lc.dynamicSmemBytes = smem;
+      lc.stream = s;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      lc.attrs = at;
+      lc.numAttrs = 1;
+      e = cudaLaunchKernelEx(&lc, kernel, A, B, C, (int)m, (int)n, (int)k, stride, (int)tiles_m, tiles, pairs, g);
+    } else {
+      kernel<<<grid, nt, smem, s>>>(A, B, C, (int)m, (int)n, (int)k, stride, (int)tiles_m, tiles, pairs, g);
+      e = cudaGetLastError();
+    }
     if (e != cudaSuccess) throw std::string("ERROR (qflex_gb300: launch cgemm) --> ") + cudaGetErrorString(e);
   }
   static void launch(const float2* A, const float2* B, float2* C, std::size_t m, std::size_t n, std::size_t k,
