@@ -198,3 +198,43 @@ def test_wide_ranges(built_lib, precision, m, n, k):
     # A value within 2^-22 of the largest component, each part of a complex one.
     bound = 2.0 ** -22 * 2 ** 0.5 * (top_a @ b.abs() + a.abs() @ top_b) + 8e-6 * (a.abs() @ b.abs())
     assert float(((C - a @ b).abs() / bound).max()) < 1
+
+
+@pytest.mark.parametrize("precision,m,n,k", [(FP16X3, 640, 500, 161), (BF16X3, 100, 2051, 255), (FP16X3, 65537, 17, 100),
+                                             (FP32, 64, 64, 600)])
+@pytest.mark.parametrize("how", ["legacy stream", "graph"])
+def test_streams(built_lib, precision, m, n, k, how):
+    """The legacy stream, and a caller's graph replayed on new operands, with an
+    infinity in some of them."""
+    import torch
+    buf = torch.zeros((1, m * k + k * n + m * n), dtype=torch.complex64, device="cuda")
+    at = buf.data_ptr()
+    args = (at, at + 8 * m * k, at + 8 * (m * k + k * n), m, n, k, 1, buf.shape[1])
+    ctx = Context(0, precision)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    if how == "graph":
+        ctx.set_stream(side.cuda_stream)
+        with torch.cuda.stream(side):
+            ctx.multiply(*args)  # takes the context's buffers
+            ctx.synchronize()
+            graph.capture_begin()
+            ctx.multiply(*args)
+            graph.capture_end()
+    else:
+        ctx.set_stream(0)
+    for seed in range(4):
+        x = randn((1, m * k + k * n), seed)
+        if seed in (1, 2):
+            x[0, 3 * k + 5] = complex(float("inf"), 1)
+        buf[:, :m * k + k * n] = x
+        torch.cuda.synchronize()
+        graph.replay() if how == "graph" else ctx.multiply(*args)
+        torch.cuda.synchronize()
+        ctx.synchronize()
+        a, b = x[0, :m * k].view(m, k), x[0, m * k:].view(k, n)
+        c = buf[0, m * k + k * n:].view(m, n)
+        rows = torch.arange(m, device="cuda") != (3 if seed in (1, 2) else -1)
+        want, bound = a[rows].cdouble() @ b.cdouble(), a[rows].abs().double() @ b.abs().double()
+        assert float(((c[rows] - want).abs() / bound).max()) < 2 * k * 2.0 ** -24 * 2 ** 0.5 + 6e-6
+        for got, part in zip((c.real, c.imag), _parts(a, b)):
+            assert torch.equal(got.isnan(), part.isnan()) and torch.equal(got.isposinf(), part.isposinf())
