@@ -2,9 +2,9 @@
 
 Chosen by measurement on the current GPU:
   * for every tensor-core product shape of the plan, the kernel variant --
-    the single-CTA 128 x 128 tile or the CTA-pair (cta_group::2) 256 x 128
-    tile -- timing both on random operands of that shape through the C
-    ABI's multiply (qflex_gb300_multiply);
+    the product that splits A itself, or one of those that load both
+    operands' planes -- timing each on random operands of that shape through
+    the C ABI's multiply (qflex_gb300_multiply);
   * the number of output strings per device pass (the "max_batch" option),
     timing evaluate_many on the workload's own strings.
 The TMEM chunk length is not tuned: it trades accuracy for speed, and 2
@@ -20,8 +20,8 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 from ._lib import FP16X3, TF32X3, Context
 
-VARIANTS = (0, 1)  # single CTA, CTA pair
-FP16_VARIANTS = (0, 1, 2, 3, 4)  # + five stages, 16 epilogue warps, 64-column tiles (3xFP16)
+VARIANTS = (0, 1)  # A split inside the kernel, CTA pair from planes
+FP16_VARIANTS = (0, 1, 2, 3, 4)  # + from planes: five stages, 16 epilogue warps, 64-column tiles (3xFP16)
 
 
 def variants(ctx: Context) -> Tuple[int, ...]:

@@ -95,7 +95,8 @@ void launch_permute_fp16_planes(const PermPlan& plan, const float2* src, std::ui
 // sum_i digit_i(o) * in_stride[i], where in_stride[i] is the input stride of
 // the index that goes to position i.
 constexpr int kGeneralPermMaxRank = 32;
-// Division by a constant: n / d = (hi32(n * mul) + n) >> shift for n < 2^31.
+// Division by a constant (Granlund and Montgomery 1994): n / d =
+// (hi32(n * mul) + n) >> shift for n < 2^31.
 struct FastDiv {
   std::uint32_t d, mul, shift;
 };

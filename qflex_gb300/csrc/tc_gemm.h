@@ -74,7 +74,7 @@ void launch_cgemm_fp16x3(const float2* A, const float2* B, BLayout b_layout, flo
                          float* workspace, int* err, const TcConfig& cfg, cudaStream_t s,
                          bool a_in_planes = false);
 
-// Where the direct 3xFP16 product finds A: TMA boxes or, where no box fits,
+// Where the direct products find A: TMA boxes or, where no box fits,
 // cp.async copies (16 bytes: two elements adjacent in the source; 8 bytes for
 // plain rows on odd addresses) fill a block of 128 rows x 32 values, copy
 // u = lt + 64 i by loader thread lt. Offsets of sources are in elements and

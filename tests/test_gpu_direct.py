@@ -1,6 +1,7 @@
-"""The 3xFP16 product that splits A inside the kernel (products of up to 1024
-columns at the default kernel choice), at the edges of its tiles and blocks
-and on rows whose magnitude changes from one block of 32 values to the next."""
+"""Split-precision products at the edges of tiles and blocks of the kernel that
+splits A itself, and on rows whose magnitude changes from one block of 32 values
+to the next. Sizes that no contraction has run in FP32 here below 2^25 terms in
+all or 96 a sum; test_gpu_split_routes.py has such edges above that line."""
 import numpy as np
 import pytest
 

@@ -1,7 +1,7 @@
-"""Split-precision products whose sizes fill no tile, k-step or vector: any n
-and any k from 96 on run on the tensor cores. B is split from the columns of
-the row-major matrix, A from its rows (3xFP16: inside the product up to 1024
-columns)."""
+"""Split-precision products whose sizes fill no tile, k-step or vector: from 2^25
+terms in all on, any n and any k from 96 on run on the tensor cores, smaller ones
+in FP32 (test_gpu_split_routes.py checks the route as well). B is split from the
+columns of the row-major matrix, A from its rows, mostly inside the product."""
 import numpy as np
 import pytest
 
