@@ -1203,7 +1203,11 @@ static int direct_columns(std::size_t n) { return n <= 32 ? 32 : n <= 64 ? 64 : 
 // its store, which starts later in a pair. 3xFP16, single CTAs against pairs:
 // (65536, 256, k) x 4 with k = 32 104 and 106 us, 64 143 and 149, 256 301 and
 // 286; (8192, 128, 128) x 16 59 and 60.5; (4096, 1024, 4096) 272 and 240.
-// 3xTF32 takes twice the MMAs. BF16x3 runs in pairs alone: split and product,
+// 3xTF32 takes twice the MMAs; with k = 32 and 64 pairs cost a short launch 2 us
+// and win from some 1000 tiles on: (16384, 256, 32) x 4 46 and 44, (16384, 8192,
+// 32) 253 and 242, (65536, 256, 64) x 4 187 and 173, but (512, 512, 64) 19 and
+// 21, and with half a tile of columns (65536, 64, 64) x 4 85 and 88. BF16x3 runs
+// in pairs alone: split and product,
 // and this, (65536, 256, k) x 4 with k = 16 122 and 98 us, 64 200 and 154;
 // (32768, 64, 64) x 16 220 and 133; (256, 256, 64) 12 and 12.
 bool tc_direct_pair(SplitKind kind, std::size_t m, std::size_t k) {
@@ -1236,7 +1240,9 @@ void launch_cgemm_direct(SplitKind kind, const float2* A, const AGather& gather,
     }
   }
   const int bn = kind == KIND_FP16 ? direct_columns(n) : 128;
-  const bool pair = bn == 128 && tc_direct_pair(kind, m, k);
+  const std::size_t singles = ((m + BM - 1) / BM) * ((n + 127) / 128) * (std::size_t)batch;
+  const bool pair = bn == 128 && (tc_direct_pair(kind, m, k) ||
+                                  (kind == KIND_TF32 && m > (std::size_t)BM && n > 64 && k > 16 && singles >= 1000));
   if (kind == KIND_BF16 && !pair)
     throw std::string("ERROR (qflex_gb300: tensor cores) --> the direct BF16x3 product runs in pairs");
   const int b_cols = pair ? bn / 2 : bn;

@@ -194,7 +194,11 @@ __device__ __forceinline__ void umma_f16_pair(std::uint32_t d_tmem, std::uint64_
 // MMAs are N = 128, a stage is 28 KB (five of them), and TMEM holds four
 // chunk buffers instead of two, so the MMAs can run three chunks ahead of an
 // epilogue that is storing a tile (products with a short k).
-template <int KIND, bool PAIR = false, bool DEEP = false, int EPI = EPI_WARPS, int TBN = BN>
+//
+// SEPARATE (3xTF32): B as the same four planes as A, in 128-byte rows, and the
+// real and imaginary parts in MMAs of N = 128, -Ai Bi by the negate-A bit: a
+// k-step loads 32 KB instead of 40, for which its MMAs read more shared memory.
+template <int KIND, bool PAIR = false, bool DEEP = false, int EPI = EPI_WARPS, int TBN = BN, bool SEPARATE = false>
 __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const CUtensorMap* map_b,
                                                  const CUtensorMap* map_a2, const CUtensorMap* map_b2,
                                                  const CUtensorMap* map_c, bool tma_c,
@@ -205,9 +209,10 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
   constexpr int KSTEP = KIND == KIND_TF32 ? 8 : 16;  // k values per plane row of 32 bytes
   constexpr int TAIL = BM * 64;                       // BF16 third-piece tile of one operand
   constexpr bool NARROW = TBN != BN;
-  constexpr int NST = KIND == KIND_BF16 ? 3 : (PAIR || DEEP || NARROW ? 5 : 4);
+  constexpr int NST = KIND == KIND_BF16 ? 3 : (PAIR || DEEP || NARROW || SEPARATE ? 5 : 4);
   constexpr int F16_BBLOCK = TBN * 64;  // one B block: TBN rows of 64 bytes
   constexpr int SBYTES = KIND == KIND_BF16 ? 2 * (TILE_A + TAIL)
+                         : SEPARATE        ? STAGE_BYTES
                                            : (PAIR ? 4 * F16_BLOCK : 2 * F16_BLOCK + 3 * F16_BBLOCK);
   // x coordinate of B's re, im and -im blocks (hi and lo: 64 bytes each).
   constexpr int BX = KIND == KIND_TF32 ? 16 : 32;
@@ -219,6 +224,7 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
   constexpr int STAGE_REGION = DEEP ? DEEP_STAGES * F16_STAGE_BYTES : STAGES * STAGE_BYTES;
   constexpr int STG_BYTES = DEEP ? DEEP_STAGING_BYTES : STAGING_BYTES;
   static_assert(NST * SBYTES <= STAGE_REGION, "stages fit the shared memory of the launch");
+  static_assert(!SEPARATE || (KIND == KIND_TF32 && !PAIR && !DEEP && !NARROW), "a 3xTF32 kernel");
   static_assert(!PAIR || KIND == KIND_FP16, "the CTA pair is a 3xFP16 kernel");
   static_assert(!DEEP || (KIND == KIND_FP16 && !PAIR), "the deep variant is a single-CTA 3xFP16 kernel");
   static_assert(EPI == EPI_WARPS || (EPI == WIDE_EPI_WARPS && KIND == KIND_FP16 && !PAIR && !DEEP),
@@ -324,7 +330,10 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
           tma_load_4d_pair(map_b, bar, st + 3 * F16_BLOCK, rank ? 0 : 64, n0, kb, batch);
         } else {
           mbar_expect_tx(&full[s], SBYTES);
-          if constexpr (KIND != KIND_BF16) {
+          if constexpr (SEPARATE) {
+            tma_load_4d(map_a, &full[s], st, 0, m0, kb, batch);
+            tma_load_4d(map_b, &full[s], st + TILE_A, 0, n0, kb, batch);
+          } else if constexpr (KIND != KIND_BF16) {
             // A: one box of whole 128-byte rows (16 KB); B: -im, re and im,
             // hi and lo each.
             tma_load_4d(map_a, &full[s], st, 0, m0, kb, batch);
@@ -425,6 +434,24 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
             umma_f16_pair(d_re, arh, b1h, idw, 1);
             umma_f16_pair(d_re, aih, b2h, idw, 1);
             (void)d_im;
+          } else if constexpr (SEPARATE) {
+            const std::uint32_t b0 = a0 + TILE_A;
+            const std::uint64_t arh = smem_desc_sw128(a0), arl = smem_desc_sw128(a0 + 32),
+                                aih = smem_desc_sw128(a0 + 64), ail = smem_desc_sw128(a0 + 96);
+            const std::uint64_t brh = smem_desc_sw128(b0), brl = smem_desc_sw128(b0 + 32),
+                                bih = smem_desc_sw128(b0 + 64), bil = smem_desc_sw128(b0 + 96);
+            umma<KIND>(d_re, arh, brl, idp, acc);
+            umma<KIND>(d_re, arl, brh, idp, 1);
+            umma<KIND>(d_re, aih, bil, idn, 1);
+            umma<KIND>(d_re, ail, bih, idn, 1);
+            umma<KIND>(d_re, arh, brh, idp, 1);
+            umma<KIND>(d_re, aih, bih, idn, 1);
+            umma<KIND>(d_im, arh, bil, idp, acc);
+            umma<KIND>(d_im, arl, bih, idp, 1);
+            umma<KIND>(d_im, aih, brl, idp, 1);
+            umma<KIND>(d_im, ail, brh, idp, 1);
+            umma<KIND>(d_im, arh, bih, idp, 1);
+            umma<KIND>(d_im, aih, brh, idp, 1);
           } else if constexpr (KIND != KIND_BF16) {
             // One M = 128, N = 256 product gives C_re (columns 0..127) and
             // C_im (128..255) together: Ar against the B rows (Br; Bi) and Ai
@@ -706,6 +733,16 @@ __global__ void __launch_bounds__(THREADS, 1)
                         int k, int batches, std::uint64_t c_batch_stride, int* __restrict__ err, int CHUNK) {
   cgemm_split_body<KIND_TF32>(&map_a, &map_b, nullptr, nullptr, &map_c, tma_c != 0, C, m, n, k, batches, c_batch_stride, err, CHUNK,
                               nullptr, nullptr, 0);
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+    cgemm_tf32x3_separate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                 const __grid_constant__ CUtensorMap map_c, int tma_c, float2* __restrict__ C, int m,
+                                 int n, int k, int batches, std::uint64_t c_batch_stride, int* __restrict__ err,
+                                 int CHUNK) {
+  cgemm_split_body<KIND_TF32, false, false, EPI_WARPS, BN, true>(&map_a, &map_b, nullptr, nullptr, &map_c, tma_c != 0,
+                                                                 C, m, n, k, batches, c_batch_stride, err, CHUNK,
+                                                                 nullptr, nullptr, 0);
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -1117,6 +1154,10 @@ bool tc_eligible(std::size_t m, std::size_t n, std::size_t k) {
   return m >= 64 && n >= 64 && k >= 16 && k % 4 == 0 && m < (1u << 31) && n < (1u << 31) && k < (1u << 31);
 }
 
+bool tf32_separate(std::size_t m, std::size_t n, std::size_t k) {
+  return k > 16 && k <= 32 && n >= 1024 && m * n >= (std::size_t(1) << 25);
+}
+
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k) {
   // The largest of the 3xTF32 planes (4 fp32 per element of A, 6 of Bt), the
   // 3xFP16 planes (4 fp16 per element of A, 6 of Bt) plus their exponents and the BF16x3
@@ -1173,6 +1214,7 @@ void launch_cgemm_tf32x3(const float2* A, const float2* B, BLayout b_layout, flo
   static PerDevice raised;
   raised([] {
     raise_smem_limit(cgemm_tf32x3_kernel, SMEM_BYTES);
+    raise_smem_limit(cgemm_tf32x3_separate_kernel, SMEM_BYTES);
     raise_smem_limit(cgemm_tf32x3_pair_kernel, P_SMEM_BYTES);
     return 1;
   });
@@ -1181,7 +1223,8 @@ void launch_cgemm_tf32x3(const float2* A, const float2* B, BLayout b_layout, flo
   const std::size_t kpad = (k + BK - 1) / BK * BK;
   float* pb = workspace + 4 * m * kpad * (std::size_t)batch;
   launch_split(KIND_TF32, 4, {pa}, A, m, k, batch_stride, batch, false, s);
-  launch_split(KIND_TF32, use_pair ? 4 : 6, {pb}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
+  const bool separate = !use_pair && tf32_separate(m, n, k);
+  launch_split(KIND_TF32, use_pair || separate ? 4 : 6, {pb}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   if (use_pair) {
     const CUtensorMap ma = plane_map(pa, m, kpad, batch, PBM);
     const CUtensorMap mb = plane_map(pb, n, kpad, batch, PBN_CTA);
@@ -1193,13 +1236,13 @@ void launch_cgemm_tf32x3(const float2* A, const float2* B, BLayout b_layout, flo
     return;
   }
   const CUtensorMap ma = plane_map(pa, m, kpad, batch, BM);
-  const CUtensorMap mb = plane_map(pb, n, kpad, batch, BN, 48, 16);
+  const CUtensorMap mb = separate ? plane_map(pb, n, kpad, batch, BN) : plane_map(pb, n, kpad, batch, BN, 48, 16);
   const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
   dim3 grid(persistent_grid(tiles * (std::size_t)batch), 1, 1);
   CUtensorMap mc;
   const int tma_c = output_map(C, m, n, batch_stride, batch, &mc) ? 1 : 0;
-  cgemm_tf32x3_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, mc, tma_c, C, (int)m, (int)n, (int)k, batch,
-                                                        batch_stride, err, chunk);
+  auto* kernel = separate ? cgemm_tf32x3_separate_kernel : cgemm_tf32x3_kernel;
+  kernel<<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, mc, tma_c, C, (int)m, (int)n, (int)k, batch, batch_stride, err, chunk);
   check(cudaGetLastError(), "cgemm_tf32x3");
 }
 

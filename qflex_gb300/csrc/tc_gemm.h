@@ -21,6 +21,10 @@ bool tc_eligible(std::size_t m, std::size_t n, std::size_t k);
 bool tc_runs(std::size_t m, std::size_t n, std::size_t k);
 // How B lies in memory: n rows of k values, or k rows of n.
 enum class BLayout { nk, kn };
+// 3xTF32 products of 17 to 32 terms with many columns and outputs: loading both
+// operands' planes, with the real and imaginary parts in MMAs of their own, is
+// then ahead of splitting A inside the kernel, as a tile's store bounds both.
+bool tf32_separate(std::size_t m, std::size_t n, std::size_t k);
 // fp32 elements of split planes one batch entry needs (A and B of any split kind).
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k);
 

@@ -238,3 +238,11 @@ def test_streams(built_lib, precision, m, n, k, how):
         assert float(((c[rows] - want).abs() / bound).max()) < 2 * k * 2.0 ** -24 * 2 ** 0.5 + 6e-6
         for got, part in zip((c.real, c.imag), _parts(a, b)):
             assert torch.equal(got.isnan(), part.isnan()) and torch.equal(got.isposinf(), part.isposinf())
+
+
+@pytest.mark.parametrize("m,n,k,batch,extra", [(32769, 1024, 32, 1, 1), (4100, 8192, 32, 1, 0), (2100, 16384, 32, 2, 1),
+                                               (16385, 256, 32, 4, 1), (3000, 4096, 64, 2, 0)])
+def test_tf32_short_sums(built_lib, m, n, k, batch, extra):
+    """3xTF32 products of 32 and 64 terms: real and imaginary parts in MMAs of
+    their own where a tile's store bounds it, and pairs for many tiles."""
+    check(TF32X3, randn((batch, m, k), m), randn((batch, k, n), n), extra, 8e-6)

@@ -251,3 +251,20 @@ for option, kernel in ((None, "cgemm_direct_kernel<1,"), (("tc_chunk", 1), "cgem
     assert bool(writing) == (option is not None), (option, len(writing))
     assert option is None or not [x for x in names if x.startswith("cgemm_direct")], option
 ''')
+
+
+def test_tf32_products_of_few_terms(run_fake):  # noqa: F811
+    """Which kernel 3xTF32 products of 16 to 64 terms take (each line measured
+    on both sides)."""
+    run_fake('''
+ctx = Context(0, TF32X3)
+for (m, n, k, batch), want in [
+        ((16384, 4096, 32, 1), "cgemm_tf32x3_separate_kernel"), ((32769, 1024, 32, 1), "cgemm_tf32x3_separate_kernel"),
+        ((65536, 512, 32, 1), "cgemm_direct_kernel<0, 128, true>"), ((16384, 256, 32, 4), "cgemm_direct_kernel<0, 128, true>"),
+        ((16384, 8192, 64, 1), "cgemm_direct_kernel<0, 128, true>"), ((16384, 8192, 16, 1), "cgemm_direct_kernel<0, 128, false>"),
+        ((512, 512, 64, 1), "cgemm_direct_kernel<0, 128, false>"), ((65536, 64, 64, 4), "cgemm_direct_kernel<0, 128, false>"),
+        ((512, 512, 128, 1), "cgemm_direct_kernel<0, 128, true>")]:
+    ctx.multiply(A, B, C, m, n, k, batch, 1 << 31)
+    names = kernels()
+    assert names[-1].startswith(want), (m, n, k, batch, names)
+''')
