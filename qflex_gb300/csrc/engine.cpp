@@ -228,6 +228,7 @@ static SplitKind split_kind(int precision) {
 bool Engine::direct_product(std::size_t m, std::size_t n, std::size_t k, const TcConfig& cfg) const {
   if (precision_ == FP32 || is_complex128(precision_) || cfg.variant != 0 || cfg.chunk != 2) return false;
   if (precision_ == TF32X3 && tf32_separate(m, n, k)) return false;
+  if (precision_ == BF16X3 && bf16_separate(m, n, k)) return false;
   return precision_ == BF16X3 ? tc_direct_pair(KIND_BF16, m, k) : m > 128 || n <= 1024;
 }
 

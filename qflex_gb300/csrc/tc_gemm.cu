@@ -195,9 +195,10 @@ __device__ __forceinline__ void umma_f16_pair(std::uint32_t d_tmem, std::uint64_
 // chunk buffers instead of two, so the MMAs can run three chunks ahead of an
 // epilogue that is storing a tile (products with a short k).
 //
-// SEPARATE (3xTF32): B as the same four planes as A, in 128-byte rows, and the
-// real and imaginary parts in MMAs of N = 128, -Ai Bi by the negate-A bit: a
-// k-step loads 32 KB instead of 40, for which its MMAs read more shared memory.
+// SEPARATE (3xTF32, BF16x3): B lies in a stage as A does, rows of whole planes,
+// and the real and imaginary parts are MMAs of N = 128, -Ai Bi by the negate-A
+// bit. A k-step takes fewer boxes (3xTF32: 32 KB instead of 40), for which its
+// MMAs read more shared memory.
 template <int KIND, bool PAIR = false, bool DEEP = false, int EPI = EPI_WARPS, int TBN = BN, bool SEPARATE = false>
 __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const CUtensorMap* map_b,
                                                  const CUtensorMap* map_a2, const CUtensorMap* map_b2,
@@ -224,7 +225,7 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
   constexpr int STAGE_REGION = DEEP ? DEEP_STAGES * F16_STAGE_BYTES : STAGES * STAGE_BYTES;
   constexpr int STG_BYTES = DEEP ? DEEP_STAGING_BYTES : STAGING_BYTES;
   static_assert(NST * SBYTES <= STAGE_REGION, "stages fit the shared memory of the launch");
-  static_assert(!SEPARATE || (KIND == KIND_TF32 && !PAIR && !DEEP && !NARROW), "a 3xTF32 kernel");
+  static_assert(!SEPARATE || (KIND != KIND_FP16 && !PAIR && !DEEP && !NARROW), "a 3xTF32 or BF16x3 kernel");
   static_assert(!PAIR || KIND == KIND_FP16, "the CTA pair is a 3xFP16 kernel");
   static_assert(!DEEP || (KIND == KIND_FP16 && !PAIR), "the deep variant is a single-CTA 3xFP16 kernel");
   static_assert(EPI == EPI_WARPS || (EPI == WIDE_EPI_WARPS && KIND == KIND_FP16 && !PAIR && !DEEP),
@@ -333,6 +334,10 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
           if constexpr (SEPARATE) {
             tma_load_4d(map_a, &full[s], st, 0, m0, kb, batch);
             tma_load_4d(map_b, &full[s], st + TILE_A, 0, n0, kb, batch);
+            if constexpr (KIND == KIND_BF16) {
+              tma_load_4d(map_a2, &full[s], st + 2 * TILE_A, 0, m0, kb, batch);
+              tma_load_4d(map_b2, &full[s], st + 2 * TILE_A + TAIL, 0, n0, kb, batch);
+            }
           } else if constexpr (KIND != KIND_BF16) {
             // A: one box of whole 128-byte rows (16 KB); B: -im, re and im,
             // hi and lo each.
@@ -440,18 +445,38 @@ __device__ __forceinline__ void cgemm_split_body(const CUtensorMap* map_a, const
                                 aih = smem_desc_sw128(a0 + 64), ail = smem_desc_sw128(a0 + 96);
             const std::uint64_t brh = smem_desc_sw128(b0), brl = smem_desc_sw128(b0 + 32),
                                 bih = smem_desc_sw128(b0 + 64), bil = smem_desc_sw128(b0 + 96);
-            umma<KIND>(d_re, arh, brl, idp, acc);
-            umma<KIND>(d_re, arl, brh, idp, 1);
-            umma<KIND>(d_re, aih, bil, idn, 1);
-            umma<KIND>(d_re, ail, bih, idn, 1);
-            umma<KIND>(d_re, arh, brh, idp, 1);
-            umma<KIND>(d_re, aih, bih, idn, 1);
-            umma<KIND>(d_im, arh, bil, idp, acc);
-            umma<KIND>(d_im, arl, bih, idp, 1);
-            umma<KIND>(d_im, aih, brl, idp, 1);
-            umma<KIND>(d_im, ail, brh, idp, 1);
-            umma<KIND>(d_im, arh, bih, idp, 1);
-            umma<KIND>(d_im, aih, brh, idp, 1);
+            // C_re = Ar Br - Ai Bi, C_im = Ar Bi + Ai Br, small terms first. A
+            // BF16x3 row has pieces 0 and 1 (named h and l), its tail piece 2.
+            const std::uint32_t at = a0 + 2 * TILE_A, bt = at + TAIL;
+            auto part = [&](std::uint32_t d, std::uint64_t xh, std::uint64_t xl, std::uint64_t yh, std::uint64_t yl,
+                            std::uint32_t x2, std::uint32_t y2, std::uint32_t id2) {
+              if constexpr (KIND == KIND_BF16) {
+                const std::uint64_t ar2 = smem_desc_sw64(at), ai2 = smem_desc_sw64(at + 32);
+                const std::uint64_t x2d = smem_desc_sw64(bt + x2), y2d = smem_desc_sw64(bt + y2);
+                umma<KIND>(d, ar2, xh, idp, acc);
+                umma<KIND>(d, arl, xl, idp, 1);
+                umma<KIND>(d, arh, x2d, idp, 1);
+                umma<KIND>(d, ai2, yh, id2, 1);
+                umma<KIND>(d, ail, yl, id2, 1);
+                umma<KIND>(d, aih, y2d, id2, 1);
+                umma<KIND>(d, arl, xh, idp, 1);
+                umma<KIND>(d, arh, xl, idp, 1);
+              } else {
+                umma<KIND>(d, arh, xl, idp, acc);
+                umma<KIND>(d, arl, xh, idp, 1);
+              }
+              if constexpr (KIND == KIND_BF16) {
+                umma<KIND>(d, ail, yh, id2, 1);
+                umma<KIND>(d, aih, yl, id2, 1);
+              } else {
+                umma<KIND>(d, aih, yl, id2, 1);
+                umma<KIND>(d, ail, yh, id2, 1);
+              }
+              umma<KIND>(d, arh, xh, idp, 1);
+              umma<KIND>(d, aih, yh, id2, 1);
+            };
+            part(d_re, brh, brl, bih, bil, 0, 32, idn);
+            part(d_im, bih, bil, brh, brl, 32, 0, idp);
           } else if constexpr (KIND != KIND_BF16) {
             // One M = 128, N = 256 product gives C_re (columns 0..127) and
             // C_im (128..255) together: Ar against the B rows (Br; Bi) and Ai
@@ -741,6 +766,17 @@ __global__ void __launch_bounds__(THREADS, 1)
                                  int n, int k, int batches, std::uint64_t c_batch_stride, int* __restrict__ err,
                                  int CHUNK) {
   cgemm_split_body<KIND_TF32, false, false, EPI_WARPS, BN, true>(&map_a, &map_b, nullptr, nullptr, &map_c, tma_c != 0,
+                                                                 C, m, n, k, batches, c_batch_stride, err, CHUNK,
+                                                                 nullptr, nullptr, 0);
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+    cgemm_bf16x3_separate_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                 const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_b2,
+                                 const __grid_constant__ CUtensorMap map_c, int tma_c, float2* __restrict__ C, int m,
+                                 int n, int k, int batches, std::uint64_t c_batch_stride, int* __restrict__ err,
+                                 int CHUNK) {
+  cgemm_split_body<KIND_BF16, false, false, EPI_WARPS, BN, true>(&map_a, &map_b, &map_a2, &map_b2, &map_c, tma_c != 0,
                                                                  C, m, n, k, batches, c_batch_stride, err, CHUNK,
                                                                  nullptr, nullptr, 0);
 }
@@ -1158,6 +1194,10 @@ bool tf32_separate(std::size_t m, std::size_t n, std::size_t k) {
   return k > 16 && k <= 32 && n >= 1024 && m * n >= (std::size_t(1) << 25);
 }
 
+bool bf16_separate(std::size_t m, std::size_t n, std::size_t k) {
+  return k > 32 && k <= 64 && n >= 1024 && m * n >= (std::size_t(1) << 25);
+}
+
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k) {
   // The largest of the 3xTF32 planes (4 fp32 per element of A, 6 of Bt), the
   // 3xFP16 planes (4 fp16 per element of A, 6 of Bt) plus their exponents and the BF16x3
@@ -1364,6 +1404,7 @@ void launch_cgemm_bf16x3(const float2* A, const float2* B, BLayout b_layout, flo
   static PerDevice raised;
   raised([] {
     raise_smem_limit(cgemm_bf16x3_kernel, SMEM_BYTES);
+    raise_smem_limit(cgemm_bf16x3_separate_kernel, SMEM_BYTES);
     return 1;
   });
   const std::size_t kpad = (k + 15) / 16 * 16;
@@ -1375,14 +1416,16 @@ void launch_cgemm_bf16x3(const float2* A, const float2* B, BLayout b_layout, flo
   launch_split(KIND_BF16, 4, {am, at}, A, m, k, batch_stride, batch, false, s);
   launch_split(KIND_BF16, 4, {bm, bt}, B, n, k, b_stride, batch, b_layout == BLayout::kn, s);
   const CUtensorMap ma = plane_map_bf16(am, m, kpad, batch, BM, 64, 64);
-  const CUtensorMap mb = plane_map_bf16(bm, n, kpad, batch, BN, 64, 32);
+  const bool separate = bf16_separate(m, n, k);
+  const CUtensorMap mb = plane_map_bf16(bm, n, kpad, batch, BN, 64, separate ? 64 : 32);
   const CUtensorMap ma2 = plane_map_bf16(at, m, kpad, batch, BM, 32, 32);
-  const CUtensorMap mb2 = plane_map_bf16(bt, n, kpad, batch, BN, 32, 16);
+  const CUtensorMap mb2 = plane_map_bf16(bt, n, kpad, batch, BN, 32, separate ? 32 : 16);
   const std::size_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
   dim3 grid(persistent_grid(tiles * (std::size_t)batch), 1, 1);
   CUtensorMap mc;
   const int tma_c = output_map(C, m, n, batch_stride, batch, &mc) ? 1 : 0;
-  cgemm_bf16x3_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, ma2, mb2, mc, tma_c, C, (int)m, (int)n, (int)k, batch,
+  auto* kernel = separate ? cgemm_bf16x3_separate_kernel : cgemm_bf16x3_kernel;
+  kernel<<<grid, THREADS, SMEM_BYTES, s>>>(ma, mb, ma2, mb2, mc, tma_c, C, (int)m, (int)n, (int)k, batch,
                                                         batch_stride, err, cfg.chunk);
   check(cudaGetLastError(), "cgemm_bf16x3");
 }

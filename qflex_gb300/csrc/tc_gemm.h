@@ -25,6 +25,8 @@ enum class BLayout { nk, kn };
 // operands' planes, with the real and imaginary parts in MMAs of their own, is
 // then ahead of splitting A inside the kernel, as a tile's store bounds both.
 bool tf32_separate(std::size_t m, std::size_t n, std::size_t k);
+// The same of BF16x3 with 33 to 64 terms.
+bool bf16_separate(std::size_t m, std::size_t n, std::size_t k);
 // fp32 elements of split planes one batch entry needs (A and B of any split kind).
 std::size_t tc_workspace_elems(std::size_t m, std::size_t n, std::size_t k);
 

@@ -240,9 +240,11 @@ def test_streams(built_lib, precision, m, n, k, how):
             assert torch.equal(got.isnan(), part.isnan()) and torch.equal(got.isposinf(), part.isposinf())
 
 
-@pytest.mark.parametrize("m,n,k,batch,extra", [(32769, 1024, 32, 1, 1), (4100, 8192, 32, 1, 0), (2100, 16384, 32, 2, 1),
-                                               (16385, 256, 32, 4, 1), (3000, 4096, 64, 2, 0)])
-def test_tf32_short_sums(built_lib, m, n, k, batch, extra):
-    """3xTF32 products of 32 and 64 terms: real and imaginary parts in MMAs of
-    their own where a tile's store bounds it, and pairs for many tiles."""
-    check(TF32X3, randn((batch, m, k), m), randn((batch, k, n), n), extra, 8e-6)
+@pytest.mark.parametrize("precision,m,n,k,batch,extra", [
+    (TF32X3, 32769, 1024, 32, 1, 1), (TF32X3, 4100, 8192, 32, 1, 0), (TF32X3, 2100, 16384, 32, 2, 1),
+    (TF32X3, 16385, 256, 32, 4, 1), (TF32X3, 3000, 4096, 64, 2, 0), (BF16X3, 32769, 1024, 64, 1, 1),
+    (BF16X3, 4100, 8192, 64, 1, 0), (BF16X3, 2100, 16384, 64, 2, 1)])
+def test_short_sums(built_lib, precision, m, n, k, batch, extra):
+    """Products of 32 and 64 terms: real and imaginary parts in MMAs of their own
+    where a tile's store bounds it, and pairs for many tiles."""
+    check(precision, randn((batch, m, k), m), randn((batch, k, n), n), extra, 8e-6)

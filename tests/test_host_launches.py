@@ -253,18 +253,21 @@ for option, kernel in ((None, "cgemm_direct_kernel<1,"), (("tc_chunk", 1), "cgem
 ''')
 
 
-def test_tf32_products_of_few_terms(run_fake):  # noqa: F811
-    """Which kernel 3xTF32 products of 16 to 64 terms take (each line measured
-    on both sides)."""
+def test_products_of_few_terms(run_fake):  # noqa: F811
+    """Which kernel 3xTF32 and BF16x3 products of 16 to 64 terms take (each line
+    measured on both sides)."""
     run_fake('''
-ctx = Context(0, TF32X3)
-for (m, n, k, batch), want in [
-        ((16384, 4096, 32, 1), "cgemm_tf32x3_separate_kernel"), ((32769, 1024, 32, 1), "cgemm_tf32x3_separate_kernel"),
-        ((65536, 512, 32, 1), "cgemm_direct_kernel<0, 128, true>"), ((16384, 256, 32, 4), "cgemm_direct_kernel<0, 128, true>"),
-        ((16384, 8192, 64, 1), "cgemm_direct_kernel<0, 128, true>"), ((16384, 8192, 16, 1), "cgemm_direct_kernel<0, 128, false>"),
-        ((512, 512, 64, 1), "cgemm_direct_kernel<0, 128, false>"), ((65536, 64, 64, 4), "cgemm_direct_kernel<0, 128, false>"),
-        ((512, 512, 128, 1), "cgemm_direct_kernel<0, 128, true>")]:
+for precision, (m, n, k, batch), want in [
+        (TF32X3, (16384, 4096, 32, 1), "cgemm_tf32x3_separate_kernel"), (TF32X3, (32769, 1024, 32, 1), "cgemm_tf32x3_separate_kernel"),
+        (TF32X3, (65536, 512, 32, 1), "cgemm_direct_kernel<0, 128, true>"), (TF32X3, (16384, 256, 32, 4), "cgemm_direct_kernel<0, 128, true>"),
+        (TF32X3, (16384, 8192, 64, 1), "cgemm_direct_kernel<0, 128, true>"), (TF32X3, (16384, 8192, 16, 1), "cgemm_direct_kernel<0, 128, false>"),
+        (TF32X3, (512, 512, 64, 1), "cgemm_direct_kernel<0, 128, false>"), (TF32X3, (65536, 64, 64, 4), "cgemm_direct_kernel<0, 128, false>"),
+        (TF32X3, (512, 512, 128, 1), "cgemm_direct_kernel<0, 128, true>"), (BF16X3, (16384, 4096, 64, 1), "cgemm_bf16x3_separate_kernel"),
+        (BF16X3, (65536, 512, 64, 1), "cgemm_direct_kernel<2, 128, true>"), (BF16X3, (16384, 4096, 32, 1), "cgemm_direct_kernel<2, 128, true>"),
+        (BF16X3, (16384, 4096, 128, 1), "cgemm_direct_kernel<2, 128, true>"), (BF16X3, (2048, 2048, 64, 1), "cgemm_direct_kernel<2, 128, true>")]:
+    ctx = Context(0, precision)
     ctx.multiply(A, B, C, m, n, k, batch, 1 << 31)
     names = kernels()
-    assert names[-1].startswith(want), (m, n, k, batch, names)
+    assert names[-1].startswith(want), (precision, m, n, k, batch, names)
+    ctx.close()
 ''')
